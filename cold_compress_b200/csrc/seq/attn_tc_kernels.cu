@@ -1,0 +1,471 @@
+// attn_tc_kernels.cu -- attention of a prompt portion over position-addressed bf16 rows on the tensor cores
+// (cc_seq_attention for bf16 caches; the fp32 FMA kernel of seq_kernels.cu serves fp32 caches and odd row widths).
+//
+// Scores and softmax weights stay 32-bit: a bf16 x bf16 product is exact in fp32, so an fp32 operand is cut into
+// three bf16 parts that add up to it EXACTLY (truncation takes 8 of the 24 significant bits at a time) and multiplied
+// part by part: S = (q1 + q2 + q3) K^T and (p1 + p2 + p3) V, smallest part first.  The tensor core truncates where an FMA
+// rounds, so an accumulator lives for one tile of 128 keys only; the sum over the tiles is an fp32 FMA in registers
+// that also applies the softmax's rescaling.
+//
+// Bound: tensor pipe, 2 x 24 MMAs of 128 x 128 x 16 per 128 x 128 scores at head size 128 (3072 cycles at the nominal
+// rate) beside ~14 instructions per score on the other pipes (about 1700 cycles when all four schedulers issue).  Layout
+// that follows: the query parts stay in shared memory (96 KB) and the weight parts go to tensor memory, over the scores
+// they came from, as the A operand -- through shared memory they would cost more bandwidth than the MMAs have.
+//
+// Measured on a B200: 4096 tokens, 32 / 8 heads of 128, learned sinks, 6.17 ms on the FMA kernel -> 0.67 ms (204 TFLOP/s of
+// the attention, 3 times that on the tensor pipe); 1001 tokens behind 3333 in a window of 1024, 16 / 4 heads, 0.435 ms ->
+// 0.081 ms.  Error of fp32 outputs against 64 bits over shapes, masks and score ranges: 0.15-0.8e-6 relative, on the FMA
+// kernel 0.1-2.5e-6, never larger than it there.
+#include <cuda_bf16.h>
+#include <cuda_runtime.h>
+#include <math.h>
+#include <stdint.h>
+
+#include "../../../include/cc_b200_seq.h"
+
+namespace ccs {
+
+int fail(int code, const char* msg);
+int cuda_check(const char* where);
+
+namespace {
+
+typedef __nv_bfloat16 bf16;
+
+constexpr int BM = 128, BN = 128;             // score tile: rows = (query, query head of the group) pairs, keys
+constexpr int TILE_BYTES = 128 * 128;         // 128 rows x 64 bf16, 128-byte swizzled
+constexpr int SOFT_THREADS = 256;             // two threads per row (64 keys and half of the value columns each)
+constexpr int THREADS = SOFT_THREADS + 128;   // + MMA warp, K warp, V warp, one warp without work
+constexpr int RING = 8;                       // tiles in flight, for the marks of their live keys
+constexpr int TM_O = 256, TM_P3 = 384, TM_COLS = 512;   // tensor memory: scores 2 x 128 | tile result 128 | third part 2 x 64
+constexpr float LOG2E = 1.4426950408889634f;
+constexpr uint32_t WAIT_LIMIT = 1u << 22;
+
+__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
+}
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
+    uint32_t done;
+    asm volatile(
+        "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
+        : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+    return done != 0;
+}
+// Bounded: a wait that runs out raises `failed`; every later wait of the CTA then gives up at once, the kernel runs to its
+// end and stores NaN.
+__device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity, volatile int* failed) {
+    if (mbar_try(bar, parity)) return;
+    for (uint32_t n = 0; !mbar_try(bar, parity); ++n)
+        if (n >= WAIT_LIMIT || *failed) { *failed = 1; return; }
+}
+__device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void fence_async() { asm volatile("fence.proxy.async;" ::: "memory"); }
+// shared-memory matrix descriptor, 128-byte swizzle, descriptor version 1 (sm_100)
+__device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
+    return (uint64_t)((addr >> 4) & 0x3FFFu) | ((uint64_t)((lbo >> 4) & 0x3FFFu) << 16) | ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) |
+           (1ull << 46) | (2ull << 61);
+}
+// bf16 x bf16 -> fp32, M = 128, A K-major, B K-major or MN-major
+__device__ __forceinline__ uint32_t idesc(int N, bool b_mn) {
+    return (1u << 4) | (1u << 7) | (1u << 10) | ((b_mn ? 1u : 0u) << 16) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+}
+__device__ __forceinline__ void mma_ss(uint32_t d, uint64_t a, uint64_t b, uint32_t id, uint32_t acc) {
+    asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
+                 ::"r"(d), "l"(a), "l"(b), "r"(id), "r"(acc) : "memory");
+}
+__device__ __forceinline__ void mma_ts(uint32_t d, uint32_t a, uint64_t b, uint32_t id, uint32_t acc) {
+    asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
+                 ::"r"(d), "r"(a), "l"(b), "r"(id), "r"(acc) : "memory");
+}
+__device__ __forceinline__ void mma_commit(uint32_t bar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+// 32 lanes x 32 consecutive columns -> registers; the caller waits with tmem_wait_ld
+__device__ __forceinline__ void tmem_ld32(uint32_t t, float* v) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];\n"
+        : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]), "=f"(v[8]), "=f"(v[9]),
+          "=f"(v[10]), "=f"(v[11]), "=f"(v[12]), "=f"(v[13]), "=f"(v[14]), "=f"(v[15]), "=f"(v[16]), "=f"(v[17]), "=f"(v[18]),
+          "=f"(v[19]), "=f"(v[20]), "=f"(v[21]), "=f"(v[22]), "=f"(v[23]), "=f"(v[24]), "=f"(v[25]), "=f"(v[26]), "=f"(v[27]),
+          "=f"(v[28]), "=f"(v[29]), "=f"(v[30]), "=f"(v[31])
+        : "r"(t) : "memory");
+}
+__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void tmem_st16(uint32_t t, const uint32_t* v) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};\n"
+        ::"r"(t), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]),
+          "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]) : "memory");
+}
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool have) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(have ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ float ex2(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+// the high halves of two fp32 words as a bf16 pair (a in the low half)
+__device__ __forceinline__ uint32_t high_pair(float a, float b) { return __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632); }
+__device__ __forceinline__ float high_part(float x) { return __uint_as_float(__float_as_uint(x) & 0xffff0000u); }
+// two fp32 values as three bf16 pairs whose sums are the values
+__device__ __forceinline__ void split3(float a, float b, uint32_t& p1, uint32_t& p2, uint32_t& p3) {
+    p1 = high_pair(a, b);
+    a -= high_part(a);
+    b -= high_part(b);
+    p2 = high_pair(a, b);
+    a -= high_part(a);
+    b -= high_part(b);
+    p3 = high_pair(a, b);
+}
+__device__ __forceinline__ void st_out(float* p, size_t i, float v) { p[i] = v; }
+__device__ __forceinline__ void st_out(bf16* p, size_t i, float v) { p[i] = __float2bfloat16_rn(v); }
+
+struct Keys {   // the keys of one CTA in order: the kept first positions below the window, then j_lo, j_lo + 1, ...
+    int p0, kx, j_lo, n;
+    __device__ __forceinline__ int at(int u) const { return u < kx ? u : j_lo + (u - kx); }
+};
+
+// Global row of key `u` (element offset of its first column), or nullptr when no slot holds it.
+__device__ __forceinline__ const bf16* key_row(const CcSeqAttn& a, const Keys& ks, int u, int g, int width, const void* cache, const void* fresh) {
+    if (u >= ks.n) return nullptr;
+    const int j = ks.at(u);
+    if (j >= ks.p0) return (const bf16*)fresh + ((size_t)(j - ks.p0) * a.G + g) * width;
+    const int slot = j < a.keep_first ? j : a.keep_first + (j - a.keep_first) % (a.L - a.keep_first);
+    return a.pos[slot] == j ? (const bf16*)cache + ((size_t)g * a.L + slot) * width : nullptr;
+}
+
+// One warp copies the 128 rows of a tile into the swizzled layout; lane l knows rows l, l + 32, ...
+__device__ __forceinline__ void copy_tile(uint32_t dst, const bf16* const (&src)[4], const void* any, int chunks, int chunks_padded, int lane) {
+    const int c = lane & 15;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const unsigned long long mine = (unsigned long long)src[q];
+#pragma unroll 4
+        for (int it = 0; it < 16; ++it) {
+            const int r = 2 * it + (lane >> 4), row = 32 * q + r;
+            const unsigned long long from = __shfl_sync(0xffffffffu, mine, r);
+            if (c < chunks_padded) {
+                const bool have = from != 0 && c < chunks;
+                cp_async16(dst + (c >> 3) * TILE_BYTES + row * 128 + (((c & 7) ^ (row & 7)) << 4), have ? (const void*)(from + 16 * c) : any, have);
+            }
+        }
+    }
+}
+
+struct Small {
+    uint64_t bars[11];          // k full[2], v full[2], scores[2], weights[2], product[2], result read
+    uint32_t tmem;
+    int failed;
+    float max[2][2][BM], sum[BM];
+    uint32_t live[RING][BN / 32];   // bit of key u % 32 of the tile: a slot holds it
+};
+
+// NO: value columns per thread (half of the padded value width).  SHAPED: soft cap and distance penalty.
+template <typename YT, int NO, bool SHAPED>
+__global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const CcSeqAttn a) {
+    extern __shared__ __align__(1024) uint8_t smem_raw[];   // operand tiles, then Small
+
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int R = a.H / a.G, Dk = a.Dk, Dv = a.Dv;
+    const int n_rows = a.T * R, n_tiles = (n_rows + BM - 1) / BM;
+    const int g = blockIdx.x % a.G, tile = n_tiles - 1 - (int)blockIdx.x / a.G;   // longest rows first
+    const int f0 = tile * BM, f1 = min(f0 + BM, n_rows) - 1;
+    const int dh = (Dk + 63) / 64, ksteps = (Dk + 15) / 16;
+    const uint32_t q_part = dh * TILE_BYTES, sQ = smem_u32(smem_raw), sK = sQ + 3 * q_part, sV = sK + 2 * q_part;
+    const uint32_t v_tile = ((Dv + 63) / 64) * TILE_BYTES;
+    Small& sm = *reinterpret_cast<Small*>(smem_raw + 5 * q_part + 2 * v_tile);
+    volatile int* const failed = &sm.failed;
+    const uint32_t bar = smem_u32(sm.bars);
+    const uint32_t K_FULL = bar, V_FULL = bar + 16, S_DONE = bar + 32, P_DONE = bar + 48, PV_DONE = bar + 64, O_READ = bar + 80;
+
+    if (tid == 0) {
+        *failed = 0;
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(K_FULL + 8 * b, 32);
+            mbar_init(V_FULL + 8 * b, 32);
+            mbar_init(S_DONE + 8 * b, 1);
+            mbar_init(P_DONE + 8 * b, SOFT_THREADS / 32);
+            mbar_init(PV_DONE + 8 * b, 1);
+        }
+        mbar_init(O_READ, SOFT_THREADS / 32);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sm.tmem)), "r"(TM_COLS) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    // the query rows in three parts; columns up to the padded width and rows past the end are zero
+    const int q_chunks = 2 * ksteps;
+    for (int idx = tid; idx < BM * q_chunks; idx += THREADS) {
+        const int row = idx / q_chunks, c = idx - row * q_chunks, flat = f0 + row;
+        float v[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[e] = 0.f;
+        if (flat < n_rows && 8 * c < Dk) {
+            const int t = flat / R;
+            const float4* src = reinterpret_cast<const float4*>(a.q + ((size_t)t * a.H + g * R + (flat - t * R)) * Dk + 8 * c);
+            *reinterpret_cast<float4*>(v) = __ldg(src);
+            *reinterpret_cast<float4*>(v + 4) = __ldg(src + 1);
+        }
+        uint32_t w[3][4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) split3(v[2 * e], v[2 * e + 1], w[0][e], w[1][e], w[2][e]);
+        uint8_t* dst = smem_raw + (c >> 3) * TILE_BYTES + row * 128 + (((c & 7) ^ (row & 7)) << 4);
+#pragma unroll
+        for (int s = 0; s < 3; ++s) *reinterpret_cast<uint4*>(dst + s * q_part) = make_uint4(w[s][0], w[s][1], w[s][2], w[s][3]);
+    }
+    fence_async();
+    fence_before();
+    __syncthreads();
+    fence_after();
+    const uint32_t tmem = sm.tmem;
+
+    Keys ks;
+    ks.p0 = a.input_pos[0];
+    const int i_first = ks.p0 + f0 / R, i_last = ks.p0 + f1 / R;
+    ks.j_lo = a.block > 0 ? (i_first / a.block) * a.block : (a.window > 0 ? max(0, i_first - a.window + 1) : 0);
+    ks.kx = a.window > 0 ? min(a.keep_first, ks.j_lo) : 0;
+    ks.n = ks.kx + (i_last - ks.j_lo + 1);
+    const int N = (ks.n + BN - 1) / BN;
+
+    if (warp >= SOFT_THREADS / 32) {
+        // 384 threads x 168 registers at launch = 256 x 224 + 128 x 56
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
+        if (warp == 8) {
+            if (lane == 0) {
+                const uint32_t id_s = idesc(BN, false), id_v = idesc((Dv + 15) & ~15, true);
+                auto scores = [&](int n) {
+                    const int b = n & 1;
+                    mbar_wait(K_FULL + 8 * b, (n >> 1) & 1, failed);
+                    fence_after();
+                    uint32_t acc = 0;
+                    for (int s = 2; s >= 0; --s)
+                        for (int k = 0; k < ksteps; ++k, acc = 1) {
+                            const uint32_t off = (k >> 2) * TILE_BYTES + (k & 3) * 32;
+                            mma_ss(tmem + b * BN, smem_desc(sQ + s * q_part + off, 16, 1024), smem_desc(sK + b * q_part + off, 16, 1024), id_s, acc);
+                        }
+                    mma_commit(S_DONE + 8 * b);
+                };
+                scores(0);
+                for (int n = 0; n < N; ++n) {
+                    const int b = n & 1;
+                    if (n + 1 < N) scores(n + 1);   // its columns held the weights of tile n - 1, whose product is ahead of it in the pipe
+                    mbar_wait(P_DONE + 8 * b, (n >> 1) & 1, failed);
+                    mbar_wait(V_FULL + 8 * b, (n >> 1) & 1, failed);
+                    if (n > 0) mbar_wait(O_READ, (n - 1) & 1, failed);
+                    fence_after();
+                    uint32_t acc = 0;
+                    for (int s = 2; s >= 0; --s)
+#pragma unroll
+                        for (int k = 0; k < BN / 16; ++k, acc = 1) {
+                            const uint32_t half = k >> 2, kk = (k & 3) * 8;
+                            const uint32_t at = s < 2 ? tmem + b * BN + half * 64 + s * 32 + kk : tmem + TM_P3 + b * 64 + half * 32 + kk;
+                            mma_ts(tmem + TM_O, at, smem_desc(sV + b * v_tile + k * 2048, TILE_BYTES, 1024), id_v, acc);
+                        }
+                    mma_commit(PV_DONE + 8 * b);
+                }
+            }
+            __syncwarp();
+        } else if (warp == 9) {
+            for (int n = 0; n < N; ++n) {
+                const int b = n & 1;
+                const bf16* src[4];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) src[q] = key_row(a, ks, n * BN + 32 * q + lane, g, Dk, a.k_cache, a.k_new);
+                // buffer b is free when the scores of tile n - 2 are done; by then every thread has passed tile n - 4
+                if (n >= 2) mbar_wait(S_DONE + 8 * b, ((n - 2) >> 1) & 1, failed);
+                copy_tile(sK + b * q_part, src, a.k_new, Dk / 8, q_chunks, lane);
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const uint32_t live = __ballot_sync(0xffffffffu, src[q] != nullptr);
+                    if (lane == 0) sm.live[n & (RING - 1)][q] = live;
+                }
+                asm volatile("cp.async.wait_all;" ::: "memory");
+                fence_async();
+                mbar_arrive(K_FULL + 8 * b);
+            }
+        } else if (warp == 10) {
+            for (int n = 0; n < N; ++n) {
+                const int b = n & 1;
+                const bf16* src[4];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) src[q] = key_row(a, ks, n * BN + 32 * q + lane, g, Dv, a.v_cache, a.v_new);
+                if (n >= 2) mbar_wait(PV_DONE + 8 * b, ((n - 2) >> 1) & 1, failed);
+                copy_tile(sV + b * v_tile, src, a.v_new, Dv / 8, 2 * ((Dv + 15) / 16), lane);
+                asm volatile("cp.async.wait_all;" ::: "memory");
+                fence_async();
+                mbar_arrive(V_FULL + 8 * b);
+            }
+        }
+    } else {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 224;");
+        const int half = warp >> 2, quarter = warp & 3, row = quarter * 32 + lane, flat = min(f0 + row, n_rows - 1);
+        const int t = flat / R, h = g * R + (flat - t * R), i = ks.p0 + t;
+        const uint32_t lanes = (uint32_t)(quarter * 32) << 16;
+        const float c2 = a.scale * LOG2E;
+        const float dist_a = SHAPED && a.dist_a != nullptr ? a.dist_a[h] : 0.f, dist_b = SHAPED && a.dist_a != nullptr ? a.dist_b[h] : 0.f;
+        float m = -INFINITY, l = 0.f, corr_before = 0.f;
+        if (a.sink_mode == CC_SINK_LEARNED) { m = a.sink[h] * LOG2E; l = half == 0 ? 1.f : 0.f; }
+        else if (a.sink_mode == CC_SINK_ZERO) { m = 0.f; l = half == 0 ? 1.f : 0.f; }
+        float O[NO];
+#pragma unroll
+        for (int c = 0; c < NO; ++c) O[c] = 0.f;
+        auto add_result = [&](int n, float corr) {   // O = O corr + the product of tile n
+            mbar_wait(PV_DONE + 8 * (n & 1), (n >> 1) & 1, failed);
+            fence_after();
+#pragma unroll
+            for (int c0 = 0; c0 < NO; c0 += 32) {
+                float v[32];
+                tmem_ld32(tmem + lanes + TM_O + half * NO + c0, v);
+                tmem_wait_ld();
+#pragma unroll
+                for (int c = 0; c < 32; ++c) O[c0 + c] = fmaf(O[c0 + c], corr, v[c]);
+            }
+            fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(O_READ);
+        };
+        for (int n = 0; n < N; ++n) {
+            const int b = n & 1;
+            const int u0 = n * BN, u1 = u0 + BN - 1;
+            // whether every row of the tile sees every key of it (only where the whole tile comes from beside the kept rows)
+            const int j0 = ks.at(u0), j1 = ks.at(min(u1, ks.n - 1));
+            const bool plain = u1 < ks.n && u0 >= ks.kx && j1 <= i_first && (a.window == 0 || i_last - j0 < a.window) &&
+                               (a.block == 0 || j0 >= (i_last / a.block) * a.block);
+            mbar_wait(S_DONE + 8 * b, (n >> 1) & 1, failed);
+            fence_after();
+            float s[64];
+            tmem_ld32(tmem + lanes + b * BN + half * 64, s);
+            tmem_ld32(tmem + lanes + b * BN + half * 64 + 32, s + 32);
+            tmem_wait_ld();
+            const uint32_t live0 = sm.live[n & (RING - 1)][2 * half], live1 = sm.live[n & (RING - 1)][2 * half + 1];
+            if constexpr (SHAPED) {
+#pragma unroll
+                for (int c = 0; c < 64; ++c) {
+                    float x = s[c] * a.scale;
+                    if (a.softcap > 0.f) x = a.softcap * tanhf(x / a.softcap);
+                    if (a.dist_a != nullptr) x -= dist_a * log1pf(dist_b * (float)max(0, i - ks.at(u0 + half * 64 + c)));
+                    s[c] = x * LOG2E;
+                }
+            } else {
+#pragma unroll
+                for (int c = 0; c < 64; ++c) s[c] *= c2;
+            }
+            float m_new = m;
+            if (!(plain && (live0 & live1) == 0xffffffffu)) {
+                const int i_block = a.block > 0 ? (i / a.block) * a.block : 0, u = u0 + half * 64;
+#pragma unroll
+                for (int c = 0; c < 64; ++c) {
+                    const int j = ks.at(u + c);
+                    const bool ok = ((c < 32 ? live0 : live1) >> (c & 31) & 1u) && j <= i && (a.window == 0 || i - j < a.window || j < a.keep_first) &&
+                                    j >= i_block;
+                    if (!ok) s[c] = -INFINITY;
+                }
+            }
+            float mx[4] = {m_new, m_new, m_new, m_new};
+#pragma unroll
+            for (int c = 0; c < 64; ++c) mx[c & 3] = fmaxf(mx[c & 3], s[c]);
+            m_new = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+            sm.max[b][half][row] = m_new;
+            asm volatile("bar.sync %0, 64;" ::"r"(quarter + 1) : "memory");   // the two warps of these rows
+            m_new = fmaxf(m_new, sm.max[b][half ^ 1][row]);
+            const float ms = m_new == -INFINITY ? 0.f : m_new;
+            const float corr = m == -INFINITY ? 0.f : ex2(m - ms);
+            m = m_new;
+            float sum[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+            for (int c0 = 0; c0 < 64; c0 += 32) {
+                uint32_t p1[16], p2[16], p3[16];
+#pragma unroll
+                for (int c = 0; c < 32; c += 2) {
+                    const float x = ex2(s[c0 + c] - ms), y = ex2(s[c0 + c + 1] - ms);
+                    sum[c & 2] += x;
+                    sum[(c & 2) + 1] += y;
+                    split3(x, y, p1[c >> 1], p2[c >> 1], p3[c >> 1]);
+                }
+                const uint32_t at = tmem + lanes + b * BN + half * 64 + c0 / 2;   // 32 keys = 16 columns, over scores that are in registers
+                tmem_st16(at, p1);
+                tmem_st16(at + 32, p2);
+                tmem_st16(tmem + lanes + TM_P3 + b * 64 + half * 32 + c0 / 2, p3);
+            }
+            l = fmaf(l, corr, (sum[0] + sum[1]) + (sum[2] + sum[3]));
+            tmem_wait_st();
+            fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(P_DONE + 8 * b);
+            if (n > 0) add_result(n - 1, corr_before);
+            corr_before = corr;
+        }
+        add_result(N - 1, corr_before);
+        if (half == 1) sm.sum[row] = l;
+        asm volatile("bar.sync %0, 64;" ::"r"(quarter + 1) : "memory");
+        if (half == 0) { l += sm.sum[row]; sm.max[0][0][row] = l; }
+        asm volatile("bar.sync %0, 64;" ::"r"(quarter + 1) : "memory");
+        l = sm.max[0][0][row];
+        if (f0 + row < n_rows) {
+            float inv = l > 0.f ? 1.0f / l : 0.f;
+            if (*failed) inv = NAN;
+            YT* y = (YT*)a.y + ((size_t)t * a.H + h) * Dv + half * NO;
+            const int have = min(NO, Dv - half * NO);
+            // rows are multiples of 8 elements wide: 16-byte stores
+#pragma unroll
+            for (int c = 0; c < NO; c += 8) {
+                if (c < have) {
+                    __align__(16) YT w[8];
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) st_out(w, e, O[c + e] * inv);
+#pragma unroll
+                    for (int v = 0; v < (int)sizeof(YT) / 2; ++v) reinterpret_cast<uint4*>(y + c)[v] = reinterpret_cast<const uint4*>(w)[v];
+                }
+            }
+        }
+    }
+    fence_before();
+    __syncthreads();
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TM_COLS) : "memory");
+}
+
+template <typename YT, int NO, bool SHAPED>
+int launch_tc(const CcSeqAttn* a, cudaStream_t st) {
+    const size_t smem = sizeof(Small) + (size_t)TILE_BYTES * (5 * ((a->Dk + 63) / 64) + 2 * ((a->Dv + 63) / 64));
+    auto kern = attn_tc_kernel<YT, NO, SHAPED>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return fail(CC_SEQ_ERR_CUDA, cudaGetErrorString(e));
+    const long long tiles = ((long long)a->T * (a->H / a->G) + BM - 1) / BM;
+    kern<<<(unsigned)(tiles * a->G), THREADS, smem, st>>>(*a);
+    return cuda_check("attn_tc_kernel");
+}
+
+template <typename YT>
+int dispatch_tc(const CcSeqAttn* a, cudaStream_t st) {
+    const bool shaped = a->softcap > 0.f || a->dist_a != nullptr;
+    if (a->Dv <= 64) return shaped ? launch_tc<YT, 32, true>(a, st) : launch_tc<YT, 32, false>(a, st);
+    return shaped ? launch_tc<YT, 64, true>(a, st) : launch_tc<YT, 64, false>(a, st);
+}
+
+}  // namespace
+
+// bf16 rows of whole 16-byte vectors, up to 128 wide (the three query parts, two key and two value tiles fill the shared
+// memory), every pointer on a 16-byte boundary
+bool attn_tc_serves(const CcSeqAttn* a) {
+    const uintptr_t all = (uintptr_t)a->q | (uintptr_t)a->k_new | (uintptr_t)a->v_new | (uintptr_t)a->k_cache | (uintptr_t)a->v_cache | (uintptr_t)a->y;
+    return a->cache_dtype == CC_DT_BF16 && a->Dk % 8 == 0 && a->Dv % 8 == 0 && a->Dk <= 128 && a->Dv <= 128 && (all & 15) == 0 &&
+           (long long)a->T * (a->H / a->G) < (1ll << 30);
+}
+
+int attn_tc(const CcSeqAttn* a, cudaStream_t st) {
+    if (a->y_dtype == CC_DT_F32) return dispatch_tc<float>(a, st);
+    if (a->y_dtype == CC_DT_BF16) return dispatch_tc<bf16>(a, st);
+    return fail(CC_SEQ_ERR_INVALID_ARG, "unknown element type");
+}
+
+}  // namespace ccs

@@ -872,6 +872,9 @@ static int launch_gemv(const CcSeqGemv* g, cudaStream_t st) {
 }
 
 // ------------------------------------------------------------------------------------------------ host side
+bool attn_tc_serves(const CcSeqAttn* a);              // attn_tc_kernels.cu: bf16 rows on the tensor cores
+int attn_tc(const CcSeqAttn* a, cudaStream_t st);
+
 static int check_attn(const CcSeqAttn* a) {
     if (!a || !a->q || !a->k_new || !a->v_new || !a->k_cache || !a->v_cache || !a->pos || !a->input_pos || !a->y)
         return fail(CC_SEQ_ERR_INVALID_ARG, "attention: NULL pointer");
@@ -996,6 +999,7 @@ int cc_seq_attention(const CcSeqAttn* a, void* stream) {
     int rc = check_attn(a);
     if (rc) return rc;
     cudaStream_t st = (cudaStream_t)stream;
+    if (attn_tc_serves(a)) return attn_tc(a, st);
 #define CALL(CT, YT) dispatch_chunk<CT, YT>(a, st)
     CCS_DISPATCH2(a->cache_dtype, a->y_dtype, CALL);
 #undef CALL
