@@ -12,16 +12,17 @@
 // that follows: the query parts stay in shared memory (96 KB) and the weight parts go to tensor memory, over the scores
 // they came from, as the A operand -- through shared memory they would cost more bandwidth than the MMAs have.
 //
-// Measured on a B200: 4096 tokens, 32 / 8 heads of 128, learned sinks, 6.17 ms on the FMA kernel -> 0.67 ms (204 TFLOP/s of
+// Measured on a B200: 4096 tokens, 32 / 8 heads of 128, learned sinks, 6.17 ms on the FMA kernel -> 0.464 ms (296 TFLOP/s of
 // the attention, 3 times that on the tensor pipe); 1001 tokens behind 3333 in a window of 1024, 16 / 4 heads, 0.435 ms ->
-// 0.081 ms.  Error of fp32 outputs against 64 bits over shapes, masks and score ranges: 0.15-0.8e-6 relative, on the FMA
-// kernel 0.1-2.5e-6, never larger than it there.
+// 0.079 ms.  What is left is latency between the steps of a tile (eight warps of softmax per SM).  Error of fp32 outputs against
+// 64 bits over shapes, masks and score ranges: 0.15-0.8e-6 relative, on the FMA kernel 0.1-2.5e-6, never larger than there.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
 
 #include "../../../include/cc_b200_seq.h"
+#include "launch.cuh"
 
 namespace ccs {
 
@@ -113,17 +114,34 @@ __device__ __forceinline__ float ex2(float x) {
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
+// pairs of fp32 values: one instruction for two additions or multiply-adds, each rounded as the scalar one
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pair(float a, float b) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void unpair(f32x2 r, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(r)); }
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
 // the high halves of two fp32 words as a bf16 pair (a in the low half)
 __device__ __forceinline__ uint32_t high_pair(float a, float b) { return __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632); }
-__device__ __forceinline__ float high_part(float x) { return __uint_as_float(__float_as_uint(x) & 0xffff0000u); }
+// minus the part of x that a bf16 holds
+__device__ __forceinline__ float minus_high(float x) { return __uint_as_float((__float_as_uint(x) & 0xffff0000u) ^ 0x80000000u); }
 // two fp32 values as three bf16 pairs whose sums are the values
 __device__ __forceinline__ void split3(float a, float b, uint32_t& p1, uint32_t& p2, uint32_t& p3) {
     p1 = high_pair(a, b);
-    a -= high_part(a);
-    b -= high_part(b);
+    unpair(add2(pair(a, b), pair(minus_high(a), minus_high(b))), a, b);
     p2 = high_pair(a, b);
-    a -= high_part(a);
-    b -= high_part(b);
+    unpair(add2(pair(a, b), pair(minus_high(a), minus_high(b))), a, b);
     p3 = high_pair(a, b);
 }
 __device__ __forceinline__ void st_out(float* p, size_t i, float v) { p[i] = v; }
@@ -134,42 +152,111 @@ struct Keys {   // the keys of one CTA in order: the kept first positions below 
     __device__ __forceinline__ int at(int u) const { return u < kx ? u : j_lo + (u - kx); }
 };
 
-// Global row of key `u` (element offset of its first column), or nullptr when no slot holds it.
-__device__ __forceinline__ const bf16* key_row(const CcSeqAttn& a, const Keys& ks, int u, int g, int width, const void* cache, const void* fresh) {
-    if (u >= ks.n) return nullptr;
-    const int j = ks.at(u);
-    if (j >= ks.p0) return (const bf16*)fresh + ((size_t)(j - ks.p0) * a.G + g) * width;
-    const int slot = j < a.keep_first ? j : a.keep_first + (j - a.keep_first) % (a.L - a.keep_first);
-    return a.pos[slot] == j ? (const bf16*)cache + ((size_t)g * a.L + slot) * width : nullptr;
+// Where the 128 keys of one tile come from.  Positions below p0 sit in cache slots (the kept first ones in slots of their
+// own, the others in a ring), the others are rows of the portion; both are runs of equally spaced rows.
+struct TileRows {
+    int j0;          // position of key 0, when the tile lies beside the kept first positions
+    int ring, r0;    // ring length, and place of j0 in it
+    uint32_t live[4];
+    bool run;        // all live keys are the tile's first ones and lie in one run of rows
+    size_t first;    // ... that starts here (row), in the portion or in the cache
+    bool fresh;
+};
+
+__device__ __forceinline__ int slot_in(const CcSeqAttn& a, const Keys& ks, const TileRows& t, int u0, int row) {
+    const int u = u0 + row;
+    if (u < ks.kx) return u;
+    if (u0 < ks.kx) {
+        const int j = ks.at(u);
+        return j < a.keep_first ? j : a.keep_first + (j - a.keep_first) % t.ring;
+    }
+    if (t.j0 + row < a.keep_first) return t.j0 + row;
+    int r = t.r0 + row;
+    if (t.r0 < 0) r = (t.j0 + row - a.keep_first) % t.ring;        // a short ring, or the tile straddles the kept positions
+    else if (r >= t.ring) r -= t.ring;
+    return a.keep_first + r;
 }
 
-// One warp copies the 128 rows of a tile into the swizzled layout; lane l knows rows l, l + 32, ...
-__device__ __forceinline__ void copy_tile(uint32_t dst, const bf16* const (&src)[4], const void* any, int chunks, int chunks_padded, int lane) {
-    const int c = lane & 15;
+// The 32 lanes look the tile's 128 keys up: a key is live when it is within the portion, or its slot holds its position.
+__device__ __forceinline__ TileRows look_up(const CcSeqAttn& a, const Keys& ks, int n, int lane) {
+    TileRows t;
+    const int u0 = n * BN;
+    t.ring = a.L - a.keep_first;
+    t.j0 = ks.at(u0);
+    t.r0 = t.ring >= BN && t.j0 >= a.keep_first ? (t.j0 - a.keep_first) % t.ring : -1;
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-        const unsigned long long mine = (unsigned long long)src[q];
+        const int row = 32 * q + lane, u = u0 + row, j = ks.at(u);
+        bool live = u < ks.n;
+        if (live && j < ks.p0) live = a.pos[slot_in(a, ks, t, u0, row)] == j;
+        t.live[q] = __ballot_sync(0xffffffffu, live);
+    }
+    const int rows = min(BN, ks.n - u0), j1 = t.j0 + rows - 1;
+    uint32_t want[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) want[q] = rows >= 32 * q + 32 ? 0xffffffffu : rows <= 32 * q ? 0u : (1u << (rows - 32 * q)) - 1u;
+    const bool all = t.live[0] == want[0] && t.live[1] == want[1] && t.live[2] == want[2] && t.live[3] == want[3];
+    t.fresh = t.j0 >= ks.p0;
+    t.run = all && u0 >= ks.kx && (t.fresh || (j1 < ks.p0 && t.r0 >= 0 && t.r0 + rows <= t.ring));
+    t.first = t.fresh ? (size_t)(t.j0 - ks.p0) * a.G : (size_t)(a.keep_first + t.r0);
+    return t;
+}
+
+// One warp copies the rows of a tile into the swizzled layout: lane = 16-byte column lane % 16 of rows lane / 16, + 2, + 4, ...
+// Dead rows and columns up to the padded width become zero.  A tile that is one run of rows costs three instructions per
+// copy (a row lookup per copy made this warp the slowest part of the kernel: 0.67 against 0.49 ms for 4096 tokens).
+__device__ __forceinline__ void copy_tile(uint32_t dst, const CcSeqAttn& a, const Keys& ks, const TileRows& t, int n, int g, int width,
+                                          const void* cache, const void* fresh, int chunks, int chunks_padded, int lane) {
+    const int c = lane & 15, hi = lane >> 4;
+    if (c >= chunks_padded) return;
+    const bool col = c < chunks;
+    const bf16* const cb = (const bf16*)cache + (size_t)g * a.L * width + 8 * c;
+    const bf16* const fb = (const bf16*)fresh + (size_t)g * width + 8 * c;
+    const uint32_t at = dst + (c >> 3) * TILE_BYTES + hi * 128;
+    uint32_t sw[4];   // row 2 i + hi: the swizzle repeats every four i
+#pragma unroll
+    for (int i = 0; i < 4; ++i) sw[i] = at + ((((c & 7) ^ (2 * i + hi)) & 7) << 4);
+    if (t.run) {
+        const int step = t.fresh ? a.G * width : width;
+        const bf16* src = (t.fresh ? fb : cb) + t.first * width + (size_t)hi * step;
+        const int rows = min(BN, ks.n - n * BN);
+        if (rows == BN && col) {
+#pragma unroll 16
+            for (int i = 0; i < 64; ++i, src += 2 * step) cp_async16(sw[i & 3] + 256 * i, src, true);
+        } else {
 #pragma unroll 4
-        for (int it = 0; it < 16; ++it) {
-            const int r = 2 * it + (lane >> 4), row = 32 * q + r;
-            const unsigned long long from = __shfl_sync(0xffffffffu, mine, r);
-            if (c < chunks_padded) {
-                const bool have = from != 0 && c < chunks;
-                cp_async16(dst + (c >> 3) * TILE_BYTES + row * 128 + (((c & 7) ^ (row & 7)) << 4), have ? (const void*)(from + 16 * c) : any, have);
+            for (int i = 0; i < 64; ++i, src += 2 * step) {
+                const bool have = col && 2 * i + hi < rows;
+                cp_async16(sw[i & 3] + 256 * i, have ? (const void*)src : fresh, have);
             }
+        }
+        return;
+    }
+    const int u0 = n * BN;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const uint32_t live = t.live[q] >> hi;
+#pragma unroll 4
+        for (int i = 0; i < 16; ++i) {
+            const int row = 32 * q + 2 * i + hi, j = ks.at(u0 + row);
+            const bool have = col && (live >> (2 * i) & 1u);
+            const bf16* src = (const bf16*)fresh;
+            if (have) src = j >= ks.p0 ? fb + (size_t)(j - ks.p0) * a.G * width : cb + (size_t)slot_in(a, ks, t, u0, row) * width;
+            cp_async16(sw[i & 3] + 256 * (16 * q + i), src, have);
         }
     }
 }
 
 struct Small {
-    uint64_t bars[11];          // k full[2], v full[2], scores[2], weights[2], product[2], result read
+    uint64_t bars[12];          // k full[2], v full[2], scores[2], weights[2], product[2], result read, queries
     uint32_t tmem;
     int failed;
     float max[2][2][BM], sum[BM];
     uint32_t live[RING][BN / 32];   // bit of key u % 32 of the tile: a slot holds it
 };
 
-// NO: value columns per thread (half of the padded value width).  SHAPED: soft cap and distance penalty.
+// NO: value columns per thread (half of the padded value width).  SHAPED: soft cap, distance penalty, or a scale that is not
+// positive.
 template <typename YT, int NO, bool SHAPED>
 __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const CcSeqAttn a) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];   // operand tiles, then Small
@@ -185,7 +272,7 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const CcSeqAttn a) 
     Small& sm = *reinterpret_cast<Small*>(smem_raw + 5 * q_part + 2 * v_tile);
     volatile int* const failed = &sm.failed;
     const uint32_t bar = smem_u32(sm.bars);
-    const uint32_t K_FULL = bar, V_FULL = bar + 16, S_DONE = bar + 32, P_DONE = bar + 48, PV_DONE = bar + 64, O_READ = bar + 80;
+    const uint32_t K_FULL = bar, V_FULL = bar + 16, S_DONE = bar + 32, P_DONE = bar + 48, PV_DONE = bar + 64, O_READ = bar + 80, Q_FULL = bar + 88;
 
     if (tid == 0) {
         *failed = 0;
@@ -197,37 +284,19 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const CcSeqAttn a) 
             mbar_init(PV_DONE + 8 * b, 1);
         }
         mbar_init(O_READ, SOFT_THREADS / 32);
+        mbar_init(Q_FULL, SOFT_THREADS);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sm.tmem)), "r"(TM_COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    // the query rows in three parts; columns up to the padded width and rows past the end are zero
-    const int q_chunks = 2 * ksteps;
-    for (int idx = tid; idx < BM * q_chunks; idx += THREADS) {
-        const int row = idx / q_chunks, c = idx - row * q_chunks, flat = f0 + row;
-        float v[8];
-#pragma unroll
-        for (int e = 0; e < 8; ++e) v[e] = 0.f;
-        if (flat < n_rows && 8 * c < Dk) {
-            const int t = flat / R;
-            const float4* src = reinterpret_cast<const float4*>(a.q + ((size_t)t * a.H + g * R + (flat - t * R)) * Dk + 8 * c);
-            *reinterpret_cast<float4*>(v) = __ldg(src);
-            *reinterpret_cast<float4*>(v + 4) = __ldg(src + 1);
-        }
-        uint32_t w[3][4];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) split3(v[2 * e], v[2 * e + 1], w[0][e], w[1][e], w[2][e]);
-        uint8_t* dst = smem_raw + (c >> 3) * TILE_BYTES + row * 128 + (((c & 7) ^ (row & 7)) << 4);
-#pragma unroll
-        for (int s = 0; s < 3; ++s) *reinterpret_cast<uint4*>(dst + s * q_part) = make_uint4(w[s][0], w[s][1], w[s][2], w[s][3]);
-    }
-    fence_async();
     fence_before();
     __syncthreads();
     fence_after();
     const uint32_t tmem = sm.tmem;
+    const int q_chunks = 2 * ksteps;
+    pdl_wait_release();
 
     Keys ks;
     ks.p0 = a.input_pos[0];
@@ -255,6 +324,7 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const CcSeqAttn a) 
                         }
                     mma_commit(S_DONE + 8 * b);
                 };
+                mbar_wait(Q_FULL, 0, failed);
                 scores(0);
                 for (int n = 0; n < N; ++n) {
                     const int b = n & 1;
@@ -278,17 +348,11 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const CcSeqAttn a) 
         } else if (warp == 9) {
             for (int n = 0; n < N; ++n) {
                 const int b = n & 1;
-                const bf16* src[4];
-#pragma unroll
-                for (int q = 0; q < 4; ++q) src[q] = key_row(a, ks, n * BN + 32 * q + lane, g, Dk, a.k_cache, a.k_new);
+                const TileRows t = look_up(a, ks, n, lane);
                 // buffer b is free when the scores of tile n - 2 are done; by then every thread has passed tile n - 4
                 if (n >= 2) mbar_wait(S_DONE + 8 * b, ((n - 2) >> 1) & 1, failed);
-                copy_tile(sK + b * q_part, src, a.k_new, Dk / 8, q_chunks, lane);
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const uint32_t live = __ballot_sync(0xffffffffu, src[q] != nullptr);
-                    if (lane == 0) sm.live[n & (RING - 1)][q] = live;
-                }
+                copy_tile(sK + b * q_part, a, ks, t, n, g, Dk, a.k_cache, a.k_new, Dk / 8, q_chunks, lane);
+                if (lane < 4) sm.live[n & (RING - 1)][lane] = lane == 0 ? t.live[0] : lane == 1 ? t.live[1] : lane == 2 ? t.live[2] : t.live[3];
                 asm volatile("cp.async.wait_all;" ::: "memory");
                 fence_async();
                 mbar_arrive(K_FULL + 8 * b);
@@ -296,11 +360,9 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const CcSeqAttn a) 
         } else if (warp == 10) {
             for (int n = 0; n < N; ++n) {
                 const int b = n & 1;
-                const bf16* src[4];
-#pragma unroll
-                for (int q = 0; q < 4; ++q) src[q] = key_row(a, ks, n * BN + 32 * q + lane, g, Dv, a.v_cache, a.v_new);
+                const TileRows t = look_up(a, ks, n, lane);
                 if (n >= 2) mbar_wait(PV_DONE + 8 * b, ((n - 2) >> 1) & 1, failed);
-                copy_tile(sV + b * v_tile, src, a.v_new, Dv / 8, 2 * ((Dv + 15) / 16), lane);
+                copy_tile(sV + b * v_tile, a, ks, t, n, g, Dv, a.v_cache, a.v_new, Dv / 8, 2 * ((Dv + 15) / 16), lane);
                 asm volatile("cp.async.wait_all;" ::: "memory");
                 fence_async();
                 mbar_arrive(V_FULL + 8 * b);
@@ -308,17 +370,38 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const CcSeqAttn a) 
         }
     } else {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 224;");
+        // the query rows in three parts; columns up to the padded width and rows past the end are zero
+        for (int idx = tid; idx < BM * q_chunks; idx += SOFT_THREADS) {
+            const int row = idx / q_chunks, c = idx - row * q_chunks, flat = f0 + row;
+            float v[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) v[e] = 0.f;
+            if (flat < n_rows && 8 * c < Dk) {
+                const int t = flat / R;
+                const float4* src = reinterpret_cast<const float4*>(a.q + ((size_t)t * a.H + g * R + (flat - t * R)) * Dk + 8 * c);
+                *reinterpret_cast<float4*>(v) = src[0];
+                *reinterpret_cast<float4*>(v + 4) = src[1];
+            }
+            uint32_t w[3][4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) split3(v[2 * e], v[2 * e + 1], w[0][e], w[1][e], w[2][e]);
+            uint8_t* dst = smem_raw + (c >> 3) * TILE_BYTES + row * 128 + (((c & 7) ^ (row & 7)) << 4);
+#pragma unroll
+            for (int s = 0; s < 3; ++s) *reinterpret_cast<uint4*>(dst + s * q_part) = make_uint4(w[s][0], w[s][1], w[s][2], w[s][3]);
+        }
+        fence_async();
+        mbar_arrive(Q_FULL);
         const int half = warp >> 2, quarter = warp & 3, row = quarter * 32 + lane, flat = min(f0 + row, n_rows - 1);
         const int t = flat / R, h = g * R + (flat - t * R), i = ks.p0 + t;
         const uint32_t lanes = (uint32_t)(quarter * 32) << 16;
-        const float c2 = a.scale * LOG2E;
+        const float c2 = SHAPED ? 1.f : a.scale * LOG2E;
         const float dist_a = SHAPED && a.dist_a != nullptr ? a.dist_a[h] : 0.f, dist_b = SHAPED && a.dist_a != nullptr ? a.dist_b[h] : 0.f;
         float m = -INFINITY, l = 0.f, corr_before = 0.f;
         if (a.sink_mode == CC_SINK_LEARNED) { m = a.sink[h] * LOG2E; l = half == 0 ? 1.f : 0.f; }
         else if (a.sink_mode == CC_SINK_ZERO) { m = 0.f; l = half == 0 ? 1.f : 0.f; }
-        float O[NO];
+        f32x2 O[NO / 2];
 #pragma unroll
-        for (int c = 0; c < NO; ++c) O[c] = 0.f;
+        for (int c = 0; c < NO / 2; ++c) O[c] = 0ull;
         auto add_result = [&](int n, float corr) {   // O = O corr + the product of tile n
             mbar_wait(PV_DONE + 8 * (n & 1), (n >> 1) & 1, failed);
             fence_after();
@@ -328,7 +411,7 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const CcSeqAttn a) 
                 tmem_ld32(tmem + lanes + TM_O + half * NO + c0, v);
                 tmem_wait_ld();
 #pragma unroll
-                for (int c = 0; c < 32; ++c) O[c0 + c] = fmaf(O[c0 + c], corr, v[c]);
+                for (int c = 0; c < 32; c += 2) O[(c0 + c) / 2] = fma2(O[(c0 + c) / 2], pair(corr, corr), pair(v[c], v[c + 1]));
             }
             fence_before();
             __syncwarp();
@@ -356,11 +439,7 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const CcSeqAttn a) 
                     if (a.dist_a != nullptr) x -= dist_a * log1pf(dist_b * (float)max(0, i - ks.at(u0 + half * 64 + c)));
                     s[c] = x * LOG2E;
                 }
-            } else {
-#pragma unroll
-                for (int c = 0; c < 64; ++c) s[c] *= c2;
             }
-            float m_new = m;
             if (!(plain && (live0 & live1) == 0xffffffffu)) {
                 const int i_block = a.block > 0 ? (i / a.block) * a.block : 0, u = u0 + half * 64;
 #pragma unroll
@@ -371,25 +450,28 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const CcSeqAttn a) 
                     if (!ok) s[c] = -INFINITY;
                 }
             }
-            float mx[4] = {m_new, m_new, m_new, m_new};
+            float mx[4] = {s[0], s[1], s[2], s[3]};
 #pragma unroll
-            for (int c = 0; c < 64; ++c) mx[c & 3] = fmaxf(mx[c & 3], s[c]);
-            m_new = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+            for (int c = 4; c < 64; ++c) mx[c & 3] = fmaxf(mx[c & 3], s[c]);
+            float m_new = fmaxf(m, fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * c2);
             sm.max[b][half][row] = m_new;
             asm volatile("bar.sync %0, 64;" ::"r"(quarter + 1) : "memory");   // the two warps of these rows
             m_new = fmaxf(m_new, sm.max[b][half ^ 1][row]);
             const float ms = m_new == -INFINITY ? 0.f : m_new;
             const float corr = m == -INFINITY ? 0.f : ex2(m - ms);
             m = m_new;
-            float sum[4] = {0.f, 0.f, 0.f, 0.f};
+            const f32x2 cc = pair(c2, c2), mm = pair(-ms, -ms);
+            f32x2 sum[2] = {0ull, 0ull};
 #pragma unroll
             for (int c0 = 0; c0 < 64; c0 += 32) {
                 uint32_t p1[16], p2[16], p3[16];
 #pragma unroll
                 for (int c = 0; c < 32; c += 2) {
-                    const float x = ex2(s[c0 + c] - ms), y = ex2(s[c0 + c + 1] - ms);
-                    sum[c & 2] += x;
-                    sum[(c & 2) + 1] += y;
+                    float x, y;
+                    unpair(fma2(pair(s[c0 + c], s[c0 + c + 1]), cc, mm), x, y);
+                    x = ex2(x);
+                    y = ex2(y);
+                    sum[(c >> 1) & 1] = add2(sum[(c >> 1) & 1], pair(x, y));
                     split3(x, y, p1[c >> 1], p2[c >> 1], p3[c >> 1]);
                 }
                 const uint32_t at = tmem + lanes + b * BN + half * 64 + c0 / 2;   // 32 keys = 16 columns, over scores that are in registers
@@ -397,7 +479,9 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const CcSeqAttn a) 
                 tmem_st16(at + 32, p2);
                 tmem_st16(tmem + lanes + TM_P3 + b * 64 + half * 32 + c0 / 2, p3);
             }
-            l = fmaf(l, corr, (sum[0] + sum[1]) + (sum[2] + sum[3]));
+            float sum_x, sum_y;
+            unpair(add2(sum[0], sum[1]), sum_x, sum_y);
+            l = fmaf(l, corr, sum_x + sum_y);
             tmem_wait_st();
             fence_before();
             __syncwarp();
@@ -422,7 +506,12 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const CcSeqAttn a) 
                 if (c < have) {
                     __align__(16) YT w[8];
 #pragma unroll
-                    for (int e = 0; e < 8; ++e) st_out(w, e, O[c + e] * inv);
+                    for (int e = 0; e < 8; e += 2) {
+                        float x, x1;
+                        unpair(O[(c + e) / 2], x, x1);
+                        st_out(w, e, x * inv);
+                        st_out(w, e + 1, x1 * inv);
+                    }
 #pragma unroll
                     for (int v = 0; v < (int)sizeof(YT) / 2; ++v) reinterpret_cast<uint4*>(y + c)[v] = reinterpret_cast<const uint4*>(w)[v];
                 }
@@ -441,13 +530,13 @@ int launch_tc(const CcSeqAttn* a, cudaStream_t st) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return fail(CC_SEQ_ERR_CUDA, cudaGetErrorString(e));
     const long long tiles = ((long long)a->T * (a->H / a->G) + BM - 1) / BM;
-    kern<<<(unsigned)(tiles * a->G), THREADS, smem, st>>>(*a);
+    launch_under(kern, dim3((unsigned)(tiles * a->G)), dim3(THREADS), smem, st, *a);
     return cuda_check("attn_tc_kernel");
 }
 
 template <typename YT>
 int dispatch_tc(const CcSeqAttn* a, cudaStream_t st) {
-    const bool shaped = a->softcap > 0.f || a->dist_a != nullptr;
+    const bool shaped = a->softcap > 0.f || a->dist_a != nullptr || !(a->scale > 0.f);
     if (a->Dv <= 64) return shaped ? launch_tc<YT, 32, true>(a, st) : launch_tc<YT, 32, false>(a, st);
     return shaped ? launch_tc<YT, 64, true>(a, st) : launch_tc<YT, 64, false>(a, st);
 }
