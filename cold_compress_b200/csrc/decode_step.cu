@@ -174,6 +174,11 @@ cc_decode_kernel(const __grid_constant__ DecodeParams p) {
     // B0: this CTA has started and its exchange barriers exist; peers wait for this before they send
     cluster_arrive_release();
     bool b0_waited = false;
+    // Without the promise that the predecessor leaves this cache alone nothing of it is read before the predecessor has
+    // ended; the launch, the barriers and the cluster's start above run under it all the same.  Dependents are released
+    // only after this wait, so a kernel that does read ahead never meets one older than its own predecessor.
+    // (32 steps back to back in a graph: 64-slot sliding caches 8.8 -> 8.2 us a step, 1024 heavy-hitter slots 11.4 -> 10.9.)
+    if (!(p.a.flags & CC_FLAG_OVERLAP_PREDECESSOR)) pdl_wait();
 
     // ---- hybrid: per-head decision from scalars (every CTA of the cluster computes the same)
     int hyb_mode = kHybAppend, hyb_bits = 0, hyb_cts = 0, hyb_rw = 0;
@@ -1037,7 +1042,7 @@ int decode_step_impl(const CcCacheState* st, const CcDecodeArgs* a, cudaStream_t
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = (pdl_enabled() && (a->flags & CC_FLAG_OVERLAP_PREDECESSOR)) ? 2 : 1;
+    cfg.numAttrs = pdl_enabled() ? 2 : 1;
     cudaError_t e = cudaLaunchKernelEx(&cfg, plan.fn, p);
     if (e != cudaSuccess) return set_cuda_error(e, "cc_decode_step launch");
     return CC_OK;
