@@ -13,6 +13,7 @@
 #include <stdio.h>
 
 #include "../../../include/cc_b200_seq.h"
+#include "launch.cuh"
 
 namespace ccs {
 int fail(int code, const char* msg);
@@ -867,7 +868,7 @@ static int dispatch_latent_decode(const CcSeqLatentDecode* a, cudaStream_t st) {
 // Several independent matrix-vector products in one launch: job j is out_j = W_j xin_j with xin_j either the given
 // vector or, read from an fp32 row, act(src[off_gate + k]) * src[off_up + k] (the input side of a gated unit, or an
 // activation alone when off_up < 0).  The input is staged in shared memory rounded to the weights' type, as the
-// prompt path rounds what it hands to a product.  8 rows per CTA, a warp per row, 16-byte weight loads.
+// prompt path rounds what it hands to a product.
 __device__ __forceinline__ float round_to(float v, const float*) { return v; }
 __device__ __forceinline__ float round_to(float v, const bf16*) { return __bfloat162float(__float2bfloat16_rn(v)); }
 
@@ -936,27 +937,47 @@ __device__ __forceinline__ void bounded_row(const CcSeqBoundedSum& p, int n, flo
     else stf((float*)p.h, n, v);
 }
 
-template <typename WT, int PRE>
-__global__ void __launch_bounds__(256) gemv_multi_kernel(const CcSeqGemvMulti g) {
+// A weight vector that is read once: past L1
+__device__ __forceinline__ uint4 ld_weights(const uint4* p) {
+    uint4 u;
+    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(u.x), "=r"(u.y), "=r"(u.z), "=r"(u.w) : "l"(p));
+    return u;
+}
+
+constexpr int GEMV_AHEAD = 8;      // 16-byte weight vectors in flight per lane
+constexpr int GEMV_CTAS = 4;       // CTAs per SM (64 registers per thread)
+
+// KS warps share a row (KS == 1: a warp walks rows_per_cta / 8 rows, 8 apart).  A lane keeps GEMV_AHEAD vectors in flight
+// across the ends of rows: a slot is requested again as soon as it is used.  The first ones are on their way before the
+// kernel waits for the one before it.  (A 28-launch decode step of width 2048: 370 -> 340 us against one row per warp, four
+// loads in flight and no launch under the predecessor.)
+template <typename WT, int PRE, int KS>
+__global__ void __launch_bounds__(256, GEMV_CTAS) gemv_multi_kernel(const CcSeqGemvMulti g, int rows_per_cta) {
     extern __shared__ float4 smg4[];
     float* xs = reinterpret_cast<float*>(smg4);
     __shared__ float red[32];
+    constexpr int RW = 8 / KS;     // rows at a time
     int j = 0, first = 0;
-    while (j + 1 < g.n_jobs && (int)blockIdx.x >= first + (g.job[j].N + 7) / 8) { first += (g.job[j].N + 7) / 8; ++j; }
-    const CcSeqGemvJob& jb = g.job[j];
-    const int K = jb.K, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const WT* W = (const WT*)jb.W;
-    const int n = ((int)blockIdx.x - first) * 8 + warp;
-    const WT* w = W + (size_t)min(n, jb.N - 1) * K;
-    constexpr int VEC = 16 / (int)sizeof(WT), AHEAD = 4;
-    const bool vec = K % VEC == 0;
-    // with a shared row to form, the row's first weights are requested before it
-    uint4 ahead[PRE != CC_GEMV_PRE_NONE ? AHEAD : 1];
-    if constexpr (PRE != CC_GEMV_PRE_NONE) {
-        const uint4* w16 = reinterpret_cast<const uint4*>(w);
-#pragma unroll
-        for (int a = 0; a < AHEAD; ++a) ahead[a] = vec && lane + 32 * a < K / VEC ? __ldg(w16 + lane + 32 * a) : make_uint4(0u, 0u, 0u, 0u);
+    while (j + 1 < g.n_jobs) {
+        const int blocks = (g.job[j].N + rows_per_cta - 1) / rows_per_cta;
+        if ((int)blockIdx.x < first + blocks) break;
+        first += blocks;
+        ++j;
     }
+    const CcSeqGemvJob& jb = g.job[j];
+    const int K = jb.K, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, ks = warp % KS;
+    const WT* W = (const WT*)jb.W;
+    const int n0 = ((int)blockIdx.x - first) * rows_per_cta + warp / KS, n_end = min(((int)blockIdx.x - first + 1) * rows_per_cta, jb.N);
+    constexpr int VEC = 16 / (int)sizeof(WT);
+    const bool vec = K % VEC == 0;
+    const int nv = K / VEC, v0 = lane + 32 * ks;    // this lane's vectors of a row: v0, v0 + 32 KS, ...
+    uint4 buf[GEMV_AHEAD];
+    {
+        const uint4* w16 = reinterpret_cast<const uint4*>(W + (size_t)min(n0, jb.N - 1) * K);
+#pragma unroll
+        for (int u = 0; u < GEMV_AHEAD; ++u) buf[u] = vec && v0 + 32 * KS * u < nv ? ld_weights(w16 + v0 + 32 * KS * u) : make_uint4(0u, 0u, 0u, 0u);
+    }
+    ccs::pdl_wait_release();
     bool shared_row = false;
     if constexpr (PRE != CC_GEMV_PRE_NONE) shared_row = jb.x == nullptr;
     if (shared_row) {
@@ -969,61 +990,98 @@ __global__ void __launch_bounds__(256) gemv_multi_kernel(const CcSeqGemvMulti g)
         }
     } else if (jb.kind != CC_ACT_NONE || jb.off_up >= 0) {
         const float* src = (const float*)jb.x;
+#pragma unroll 4
         for (int k = tid; k < K; k += 256) {
             float v = unit_act(src[jb.off_gate + k], jb.kind);
             if (jb.off_up >= 0) v *= src[jb.off_up + k];
             xs[k] = round_to(v, W);
         }
     } else if (jb.x_dtype == CC_DT_F32) {
+#pragma unroll 4
         for (int k = tid; k < K; k += 256) xs[k] = round_to(((const float*)jb.x)[k], W);
     } else {
+#pragma unroll 4
         for (int k = tid; k < K; k += 256) xs[k] = __bfloat162float(((const bf16*)jb.x)[k]);
     }
     __syncthreads();
-    if (n >= jb.N) return;
-    float acc = 0.f;
-    auto dot16 = [&](const uint4& u, int i) {
-        const WT* e = reinterpret_cast<const WT*>(&u);
-        const float4* x4 = reinterpret_cast<const float4*>(xs + i * VEC);
+    if (KS == 1 && n0 >= n_end) return;
+    for (int n = n0; n < n_end || KS > 1; n += RW) {
+        float acc = 0.f, acc1 = 0.f;
+        if (vec) {
+            const uint4* w16 = reinterpret_cast<const uint4*>(W + (size_t)min(n, jb.N - 1) * K);
+            const bool more = n + RW < n_end && KS == 1;
+            for (int c0 = 32 * ks; c0 < nv; c0 += 32 * KS * GEMV_AHEAD) {      // the same for all lanes
+                const int c = c0 + lane;
+                const bool last = c0 + 32 * KS * GEMV_AHEAD >= nv;
+                const uint4* next = last ? w16 + (size_t)RW * nv + v0 : w16 + c + 32 * KS * GEMV_AHEAD;
+                const int left = last ? (more ? nv - v0 : 0) : nv - c - 32 * KS * GEMV_AHEAD;
 #pragma unroll
-        for (int q = 0; q < VEC / 4; ++q) {
-            const float4 xv = x4[q];
-            acc = fmaf(ldf(e, 4 * q + 0), xv.x, acc);
-            acc = fmaf(ldf(e, 4 * q + 1), xv.y, acc);
-            acc = fmaf(ldf(e, 4 * q + 2), xv.z, acc);
-            acc = fmaf(ldf(e, 4 * q + 3), xv.w, acc);
-        }
-    };
-    if (vec) {
-        const uint4* w16 = reinterpret_cast<const uint4*>(w);
-        const int nv = K / VEC;
-        int i = lane;
-        if constexpr (PRE != CC_GEMV_PRE_NONE) {
+                for (int u = 0; u < GEMV_AHEAD; ++u) {
+                    if (c + 32 * KS * u < nv) {
+                        const WT* e = reinterpret_cast<const WT*>(&buf[u]);
+                        const float4* x4 = reinterpret_cast<const float4*>(xs + (c + 32 * KS * u) * VEC);
+                        float& a = u & 1 ? acc1 : acc;
 #pragma unroll
-            for (int a = 0; a < AHEAD; ++a, i += 32)
-                if (i < nv) dot16(ahead[a], i);
+                        for (int q = 0; q < VEC / 4; ++q) {
+                            const float4 xv = x4[q];
+                            a = fmaf(ldf(e, 4 * q + 0), xv.x, a);
+                            a = fmaf(ldf(e, 4 * q + 1), xv.y, a);
+                            a = fmaf(ldf(e, 4 * q + 2), xv.z, a);
+                            a = fmaf(ldf(e, 4 * q + 3), xv.w, a);
+                        }
+                    }
+                    if (32 * KS * u < left) buf[u] = ld_weights(next + 32 * KS * u);
+                }
+            }
+        } else if (KS == 1 || n < n_end) {
+            const WT* w = W + (size_t)n * K;
+            for (int k = lane + 32 * ks; k < K; k += 32 * KS) acc = fmaf(ldf(w, k), xs[k], acc);
         }
-#pragma unroll 4
-        for (; i < nv; i += 32) dot16(__ldg(w16 + i), i);
-    } else {
-        for (int k = lane; k < K; k += 32) acc = fmaf(ldf(w, k), xs[k], acc);
-    }
-    acc = warp_sum(acc);
-    if (lane != 0) return;
-    if (n < jb.conv_rows) {      // this row is a channel: its past inputs, then the tail moves on
-        const int C = jb.conv_rows, taps = jb.taps;
-        const float* cw = jb.conv_w + (size_t)n * taps;
-        float c = 0.f;
-        for (int t = 0; t < taps - 1; ++t) {
-            const float u = jb.tail[(size_t)t * C + n];
-            c = fmaf(cw[t], u, c);
-            if (t > 0) jb.tail[(size_t)(t - 1) * C + n] = u;
+        acc = warp_sum(acc + acc1);
+        if constexpr (KS > 1) {      // the row's parts meet in part order
+            if (lane == 0) red[warp] = acc;
+            __syncthreads();
+            if (ks != 0 || n >= n_end) return;
+#pragma unroll
+            for (int q = 1; q < KS; ++q) acc += red[warp + q];
         }
-        if (taps > 1) jb.tail[(size_t)(taps - 2) * C + n] = acc;
-        acc = unit_act(fmaf(cw[taps - 1], acc, c), jb.conv_act);
+        if (lane == 0) {
+            if (n < jb.conv_rows) {      // this row is a channel: its past inputs, then the tail moves on
+                const int C = jb.conv_rows, taps = jb.taps;
+                const float* cw = jb.conv_w + (size_t)n * taps;
+                float c = 0.f;
+                for (int t = 0; t < taps - 1; ++t) {
+                    const float u = jb.tail[(size_t)t * C + n];
+                    c = fmaf(cw[t], u, c);
+                    if (t > 0) jb.tail[(size_t)(t - 1) * C + n] = u;
+                }
+                if (taps > 1) jb.tail[(size_t)(taps - 2) * C + n] = acc;
+                acc = unit_act(fmaf(cw[taps - 1], acc, c), jb.conv_act);
+            }
+            if (j == 0 && g.post.x != nullptr) bounded_row(g.post, n, acc);
+            if (jb.out != nullptr) ((float*)jb.out)[n] = acc;
+        }
+        if constexpr (KS > 1) return;
     }
-    if (j == 0 && g.post.x != nullptr) bounded_row(g.post, n, acc);
-    if (jb.out != nullptr) ((float*)jb.out)[n] = acc;
+}
+
+// How a launch is split: the rows of all jobs over the warps that fit the GPU at once (148 SMs x GEMV_CTAS CTAs).  Few rows:
+// two, four or eight warps share one, as long as each keeps four vectors per lane; many rows: a CTA walks several row
+// groups of 8, so that its input is staged once.
+struct GemvSplit { int ks, rows_per_cta; };
+static GemvSplit gemv_split(const CcSeqGemvMulti* g, size_t smem, int elem) {
+    int rows = 0, kmin = 1 << 30;
+    for (int j = 0; j < g->n_jobs; ++j) {
+        rows += g->job[j].N;
+        kmin = g->job[j].K < kmin ? g->job[j].K : kmin;
+    }
+    const int fit = (int)(220 * 1024 / (smem + 2048));
+    const int slots = 148 * 8 * (fit < 1 ? 1 : fit < GEMV_CTAS ? fit : GEMV_CTAS);
+    GemvSplit s = {1, 8};
+    while (s.ks < 8 && rows * s.ks * 2 <= slots && kmin * elem / 16 / (32 * s.ks * 2) >= 4) s.ks *= 2;
+    if (s.ks > 1) s.rows_per_cta = 8 / s.ks;
+    else s.rows_per_cta = 8 * ((rows + slots - 1) / slots);
+    return s;
 }
 
 template <int TB, int CH>
@@ -1285,7 +1343,7 @@ int cc_seq_latent_decode(const CcSeqLatentDecode* a, void* stream) {
 int cc_seq_gemv_multi(const CcSeqGemvMulti* g, void* stream) {
     if (!g || g->n_jobs < 1 || g->n_jobs > CC_GEMV_MAX_JOBS) return fail(CC_SEQ_ERR_INVALID_ARG, "gemv_multi: bad job count");
     const CcSeqGemvPre& p = g->pre;
-    int blocks = 0, kmax = 0;
+    int kmax = 0;
     for (int j = 0; j < g->n_jobs; ++j) {
         const CcSeqGemvJob& b = g->job[j];
         if (!b.W || (!b.out && !(j == 0 && g->post.x)) || b.N < 1 || b.K < 1 || b.kind < CC_ACT_NONE || b.kind > CC_ACT_LAST ||
@@ -1303,7 +1361,6 @@ int cc_seq_gemv_multi(const CcSeqGemvMulti* g, void* stream) {
             if (!ok || b.kind != CC_ACT_NONE || b.off_up >= 0 || g->job[0].x || b.K != g->job[0].K)
                 return fail(CC_SEQ_ERR_INVALID_ARG, "gemv_multi: bad shared input row");
         }
-        blocks += (b.N + 7) / 8;
         kmax = b.K > kmax ? b.K : kmax;
     }
     const CcSeqBoundedSum& q = g->post;
@@ -1314,16 +1371,26 @@ int cc_seq_gemv_multi(const CcSeqGemvMulti* g, void* stream) {
     const size_t smem = sizeof(float) * (size_t)((kmax + 3) & ~3);
     if (smem > 200 * 1024) return fail(CC_SEQ_ERR_UNSUPPORTED_SHAPE, "gemv_multi: input longer than 51200");
     cudaStream_t st = (cudaStream_t)stream;
-#define CALL1(ST, PRE)                                                                                             \
+    const GemvSplit split = gemv_split(g, smem, g->w_dtype == CC_DT_BF16 ? 2 : 4);
+    int blocks = 0;
+    for (int j = 0; j < g->n_jobs; ++j) blocks += (g->job[j].N + split.rows_per_cta - 1) / split.rows_per_cta;
+#define CALL2(ST, PRE, KS)                                                                                         \
     {                                                                                                              \
-        auto kern = gemv_multi_kernel<ST, PRE>;                                                                    \
+        auto kern = gemv_multi_kernel<ST, PRE, KS>;                                                                \
         static size_t configured = 48 * 1024;                                                                      \
         if (smem > configured) {                                                                                   \
             configured = smem;                                                                                     \
             if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) \
                 return cuda_check("gemv_multi: shared memory");                                                    \
         }                                                                                                          \
-        kern<<<blocks, 256, smem, st>>>(*g);                                                                       \
+        ccs::launch_under(kern, dim3(blocks), dim3(256), smem, st, *g, split.rows_per_cta);                        \
+    }
+#define CALL1(ST, PRE)                                  \
+    {                                                   \
+        if (split.ks == 8) CALL2(ST, PRE, 8)            \
+        else if (split.ks == 4) CALL2(ST, PRE, 4)       \
+        else if (split.ks == 2) CALL2(ST, PRE, 2)       \
+        else CALL2(ST, PRE, 1)                          \
     }
 #define CALL(ST)                                                                        \
     {                                                                                   \
@@ -1334,6 +1401,7 @@ int cc_seq_gemv_multi(const CcSeqGemvMulti* g, void* stream) {
     CCM_ST(g->w_dtype, CALL);
 #undef CALL
 #undef CALL1
+#undef CALL2
     return cuda_check("gemv_multi_kernel");
 }
 
