@@ -134,7 +134,7 @@ def check(rc: int, what: str = "") -> int:
 
 # --------------------------------------------------------------------------- libcc_b200_seq.so (include/cc_b200_seq.h)
 SEQ_SO_PATH = Path(os.environ.get("CC_B200_SEQ_LIB", PKG / "libcc_b200_seq.so"))
-SEQ_ABI_VERSION = 6
+SEQ_ABI_VERSION = 7
 DT_F32, DT_BF16 = 0, 1
 SINK_NONE, SINK_LEARNED, SINK_ZERO = 0, 1, 2
 
@@ -237,6 +237,10 @@ class CcSeqWkv(C.Structure):
     _fields_ = [(n, _vp) for n in ("r", "k", "v", "wraw", "w0", "u", "state", "o")] + [(n, _i32) for n in ("T", "H", "D")]
 
 
+class CcSeqMoeGrouped(C.Structure):
+    _fields_ = [(n, _vp) for n in ("wgu", "wd", "h", "perm", "counts", "xs", "act", "y")] + [(n, _i32) for n in ("n", "F", "E", "M", "kind", "gated")]
+
+
 class CcSeqMoeCombine(C.Structure):
     _fields_ = [(n, _vp) for n in ("ids", "wts", "slot", "y", "h", "shared", "sg")] + [("ld_sg", _i64), ("out", _vp)] + [
         (n, _i32) for n in ("T", "E", "top", "n_real")]
@@ -261,6 +265,7 @@ SEQ_EXPORTS.update({
     "cc_seq_moe_group": (C.c_int, [_vp, _i32, _i32, _i32, _vp, _vp, _vp, _vp]),
     "cc_seq_gather_rows": (C.c_int, [_vp, _vp, _vp, _i32, _i32, _i32, _vp]),
     "cc_seq_moe_expert_tokens": (C.c_int, [_vp, _vp, _vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _i32, _i32, _i32, _i32, _vp]),
+    "cc_seq_moe_grouped": (C.c_int, [C.POINTER(CcSeqMoeGrouped), _vp]),
     "cc_seq_moe_combine": (C.c_int, [C.POINTER(CcSeqMoeCombine), _vp]),
 })
 

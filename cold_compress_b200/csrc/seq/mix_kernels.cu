@@ -176,13 +176,21 @@ __global__ void token_shift_kernel(const float* __restrict__ h, float* state, co
 template <typename ST>
 __global__ void gated_unit_kernel(const float* __restrict__ in, int64_t ld, int off_gate, int off_up, ST* __restrict__ out,
                                   int T, int F, int kind) {
-    const int f = blockIdx.x * blockDim.x + threadIdx.x;      // column; rows stride over gridDim.y (no division per element)
-    if (f >= F) return;
+    const int f0 = blockIdx.x * (4 * blockDim.x) + threadIdx.x;      // columns f0, + blockDim.x, ...; rows stride over gridDim.y
     for (int t = blockIdx.y; t < T; t += gridDim.y) {
         const float* row = in + (size_t)t * ld;
-        float v = unit_act(row[off_gate + f], kind);
-        if (off_up >= 0) v *= row[off_up + f];
-        stf(out, (size_t)t * F + f, v);
+        float g[4], u[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {       // all loads of a thread before its arithmetic
+            const int f = f0 + i * blockDim.x;
+            g[i] = f < F ? row[off_gate + f] : 0.f;
+            u[i] = f < F && off_up >= 0 ? row[off_up + f] : 1.f;
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int f = f0 + i * blockDim.x;
+            if (f < F) stf(out, (size_t)t * F + f, off_up >= 0 ? unit_act(g[i], kind) * u[i] : unit_act(g[i], kind));
+        }
     }
 }
 
@@ -643,6 +651,49 @@ __global__ void moe_combine_kernel(const CcSeqMoeCombine a) {
             acc += g * a.shared[(size_t)t * E + e];
         }
         a.out[(size_t)t * E + e] = acc;
+    }
+}
+
+
+// The same arithmetic with 16-byte accesses, the rows of four choices in flight per thread.
+__global__ void __launch_bounds__(256) moe_combine4_kernel(const CcSeqMoeCombine a) {
+    const int t = blockIdx.x, E4 = a.E / 4;
+    const float4* const y4 = reinterpret_cast<const float4*>(a.y);
+    const float4* const h4 = reinterpret_cast<const float4*>(a.h);
+    const float g = a.shared != nullptr && a.sg ? sigmoidf_(a.sg[(size_t)t * a.ld_sg]) : 1.f;
+    for (int e = threadIdx.x; e < E4; e += blockDim.x) {
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int k0 = 0; k0 < a.top; k0 += 4) {
+            float4 v[4];
+            float w[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+                w[i] = 0.f;
+                if (k0 + i >= a.top) continue;
+                const size_t m = (size_t)t * a.top + k0 + i;
+                if (a.ids[m] < a.n_real) v[i] = y4[(size_t)(a.slot ? a.slot[m] : (int)m) * E4 + e];
+                else if (h4 != nullptr) v[i] = h4[(size_t)t * E4 + e];
+                else continue;
+                w[i] = a.wts[m];
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (k0 + i < a.top) {
+                    acc.x += w[i] * v[i].x;
+                    acc.y += w[i] * v[i].y;
+                    acc.z += w[i] * v[i].z;
+                    acc.w += w[i] * v[i].w;
+                }
+        }
+        if (a.shared != nullptr) {
+            const float4 s = reinterpret_cast<const float4*>(a.shared)[(size_t)t * E4 + e];
+            acc.x += g * s.x;
+            acc.y += g * s.y;
+            acc.z += g * s.z;
+            acc.w += g * s.w;
+        }
+        reinterpret_cast<float4*>(a.out)[(size_t)t * E4 + e] = acc;
     }
 }
 
@@ -1182,8 +1233,9 @@ int cc_seq_gated_unit(const float* in, int64_t ld, int32_t off_gate, int32_t off
 #undef CALL
         return cuda_check("gated_unit4_kernel");
     }
-    const dim3 nb((F + 255) / 256, T < 4096 ? T : 4096);
-#define CALL(ST) gated_unit_kernel<ST><<<nb, 256, 0, st>>>(in, ld, off_gate, off_up, (ST*)out, T, F, kind)
+    const int threads = F >= 1024 ? 256 : ((F + 3) / 4 + 31) / 32 * 32;
+    const dim3 nb((F + 4 * threads - 1) / (4 * threads), T < 4096 ? T : 4096);
+#define CALL(ST) gated_unit_kernel<ST><<<nb, threads, 0, st>>>(in, ld, off_gate, off_up, (ST*)out, T, F, kind)
     CCM_ST(out_dtype, CALL);
 #undef CALL
     return cuda_check("gated_unit_kernel");
@@ -1408,7 +1460,9 @@ int cc_seq_gemv_multi(const CcSeqGemvMulti* g, void* stream) {
 int cc_seq_moe_combine(const CcSeqMoeCombine* a, void* stream) {
     if (!a || !a->ids || !a->wts || !a->y || !a->out || a->T < 1 || a->E < 1 || a->top < 1)
         return fail(CC_SEQ_ERR_INVALID_ARG, "moe_combine: bad argument");   // h may be NULL when no id reaches n_real
-    moe_combine_kernel<<<a->T, 256, 0, (cudaStream_t)stream>>>(*a);
+    const uintptr_t all = (uintptr_t)a->y | (uintptr_t)a->h | (uintptr_t)a->shared | (uintptr_t)a->out;
+    if (a->E % 4 == 0 && (all & 15) == 0) moe_combine4_kernel<<<a->T, 256, 0, (cudaStream_t)stream>>>(*a);
+    else moe_combine_kernel<<<a->T, 256, 0, (cudaStream_t)stream>>>(*a);
     return cuda_check("moe_combine_kernel");
 }
 

@@ -350,8 +350,9 @@ class RoutedExperts(nn.Module):
     `weight_scale` multiplies the weights; `shared_gate=False` adds the shared expert without a gate.
 
     Steps of up to `small_t` tokens run the chosen experts through a kernel that reads the ids on the device (no host
-    round trip: a decode step stays capturable); longer portions group the (token, choice) pairs by expert, read the
-    group sizes once and run one product pair per expert."""
+    round trip: a decode step stays capturable); longer portions group the (token, choice) pairs by expert and run two
+    grouped products that read the group sizes on the device (bf16 weights), or read the sizes on the host once and run one
+    product pair per expert (fp32 weights, rows that are not whole 16-byte vectors)."""
 
     small_t = 4
 
@@ -437,6 +438,11 @@ class RoutedExperts(nn.Module):
         slot = torch.empty(M, dtype=torch.int32, device=dev)
         perm = torch.empty(M, dtype=torch.int32, device=dev)
         seq_ops.moe_group(ids, self.n_real, counts, slot, perm)
+        if seq_ops.moe_grouped_serves(self.w_gu, self.w_d, h_act):
+            xs, act = torch.empty(M, E, dtype=dt, device=dev), torch.empty(M, F, dtype=dt, device=dev)
+            y = torch.empty(M, E, dtype=torch.float32, device=dev)
+            seq_ops.moe_grouped(self.w_gu, self.w_d, h_act, perm, counts, xs, act, y, self.act)
+            return slot, y
         sizes = counts.tolist()
         rows = sum(sizes)
         y = torch.empty(max(rows, 1), E, dtype=torch.float32, device=dev)

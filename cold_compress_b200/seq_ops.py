@@ -365,6 +365,27 @@ def moe_expert_tokens(wgu, wd, h, ids, act, y, kind):
                                                             F, E, int(kind), int(rows == 2 * F), _stream()), "cc_seq_moe_expert_tokens")
 
 
+def moe_grouped_serves(wgu, wd, h) -> bool:
+    """Whether the grouped tensor-core products take these experts: bf16, rows of whole 16-byte vectors."""
+    return (h.dtype == wgu.dtype == wd.dtype == torch.bfloat16 and wgu.shape[-1] % 8 == 0 and wd.shape[-1] % 8 == 0
+            and all(t.is_contiguous() and t.data_ptr() % 16 == 0 for t in (wgu, wd, h)))
+
+
+def moe_grouped(wgu, wd, h, perm, counts, xs, act, y, kind):
+    """Experts over rows grouped by expert (moe_group), sizes read on the device: wgu [n, 2F, E] or [n, F, E], wd [n, E, F],
+    h [T, E], xs [M, E] and act [M, F] scratch -> y fp32 [M, E], rows in grouped order."""
+    _need(("wgu", wgu, torch.bfloat16), ("wd", wd, torch.bfloat16), ("h", h, torch.bfloat16), ("perm", perm, torch.int32),
+          ("counts", counts, torch.int32), ("xs", xs, torch.bfloat16), ("act", act, torch.bfloat16), ("y", y, torch.float32))
+    n, rows, E = wgu.shape
+    F = wd.shape[-1]
+    assert rows in (F, 2 * F) and wd.shape == (n, E, F) and h.shape[1] == E and counts.numel() == n
+    assert act.shape[1] == F and y.shape == xs.shape == (act.shape[0], E) and perm.numel() == act.shape[0]
+    a = _lib.CcSeqMoeGrouped()
+    a.wgu, a.wd, a.h, a.perm, a.counts, a.xs, a.act, a.y = _p(wgu), _p(wd), _p(h), _p(perm), _p(counts), _p(xs), _p(act), _p(y)
+    a.n, a.F, a.E, a.M, a.kind, a.gated = n, F, E, act.shape[0], int(kind), int(rows == 2 * F)
+    _lib.check_seq(_lib.load_seq().cc_seq_moe_grouped(C.byref(a), _stream()), "cc_seq_moe_grouped")
+
+
 def moe_combine(ids, wts, slot, y, h, shared, sg, out, n_real):
     _need(("ids", ids, torch.int32), ("wts", wts, torch.float32), ("slot", slot, torch.int32), ("y", y, torch.float32),
           ("h", h, torch.float32), ("shared", shared, torch.float32), ("out", out, torch.float32))

@@ -21,7 +21,7 @@
 extern "C" {
 #endif
 
-#define CC_SEQ_ABI_VERSION 6
+#define CC_SEQ_ABI_VERSION 7
 
 #define CC_SEQ_OK                     0
 #define CC_SEQ_ERR_INVALID_ARG       -1
@@ -368,6 +368,17 @@ int cc_seq_gather_rows(const void* src, const int32_t* perm, void* dst, int32_t 
 int cc_seq_moe_expert_tokens(const void* Wgu, const void* Wd, const void* h, const int32_t* ids, void* act, float* y,
                              int32_t dtype, int32_t T, int32_t top, int32_t n_real, int32_t F, int32_t E, int32_t kind,
                              int32_t gated, void* stream);
+
+/* Experts of a longer portion, rows grouped by expert as cc_seq_moe_group leaves them (perm, counts read on the device):
+ * xs[r] = h[perm[r]], act[r] = unit(W_gu[e] xs[r]) as above, y[r] = W_d[e] act[r].  All of wgu, wd, h, xs, act bf16, y fp32
+ * [M, E]; M = rows that xs, act and y hold (at least the sum of the counts); rows past that sum are not written.  F and E multiples of 8, pointers on
+ * 16-byte boundaries (CC_SEQ_ERR_UNSUPPORTED_SHAPE otherwise). */
+typedef struct CcSeqMoeGrouped {
+    const void* wgu;  const void* wd;  const void* h;  const int32_t* perm;  const int32_t* counts;
+    void* xs;  void* act;  float* y;
+    int32_t n, F, E, M, kind, gated;
+} CcSeqMoeGrouped;
+int cc_seq_moe_grouped(const CcSeqMoeGrouped* a, void* stream);
 
 /* out[t] = sum_k wts[t, k] * (ids[t, k] < n_real ? y[slot[t, k]] : h[t]) + sigmoid(sg[t * ld_sg]) * shared[t];
  * slot == NULL means row t * top + k; shared may be NULL; sg == NULL means no gate on it; h may be NULL when there are
