@@ -11,6 +11,7 @@
 #include <stdint.h>
 
 #include "../../../include/cc_b200_seq.h"
+#include "launch.cuh"
 
 namespace ccs {
 int fail(int code, const char* msg);
@@ -112,11 +113,12 @@ __global__ void __launch_bounds__(128) bounded_sum_kernel(const CcSeqBoundedSum 
 }
 
 template <typename ST, typename AT, int VEC>
-__global__ void __launch_bounds__(128) embed_bounded_kernel(const int32_t* __restrict__ tokens, const ST* __restrict__ embed, const CcSeqBounded emb_p,
+__global__ void __launch_bounds__(128) embed_bounded_kernel(const int32_t* tokens, const ST* __restrict__ embed, const CcSeqBounded emb_p,
                                                             float* __restrict__ x, const CcSeqBounded next_p, AT* __restrict__ h, int T, int E) {
     const int c = (blockIdx.x * blockDim.x + threadIdx.x) * VEC;
     if (c >= E) return;
     const Bounded<VEC> emb(emb_p, c), next(next_p, c);
+    ccs::pdl_wait_release();
     for (int t = blockIdx.y; t < T; t += gridDim.y) {
         Pack<VEC> s = load<VEC>(embed + (size_t)tokens[t] * E + c);
 #pragma unroll
@@ -155,6 +157,7 @@ __global__ void __launch_bounds__(544) mlstm_scan_kernel(const CcSeqMlstm a) {
     extern __shared__ float4 ml4[];
     __shared__ float s_i[SCAN_TB], s_f[SCAN_TB], s_m[SCAN_TB + 1], s_keep[SCAN_TB], s_floor[SCAN_TB], s_den[SCAN_TB];
     __shared__ int s_last;
+    ccs::pdl_wait_release();
     const int D = a.D, P = (D + CH - 1) / CH, Dp = P * CH, TB = min(a.T, SCAN_TB);
     float* qs = reinterpret_cast<float*>(ml4);      // [TB][Dp]
     float* ks = qs + TB * Dp;                       // [TB][Dp]
@@ -599,7 +602,7 @@ static int launch_scan(const CcSeqMlstm* a, cudaStream_t st) {
         if (cudaFuncSetAttribute(mlstm_scan_kernel<CH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
             return cuda_check("mlstm: shared memory");
     }
-    mlstm_scan_kernel<CH><<<dim3(a->H, (a->V + SCAN_J - 1) / SCAN_J), (P + 1) * 32, smem, st>>>(*a);
+    ccs::launch_under(mlstm_scan_kernel<CH>, dim3(a->H, (a->V + SCAN_J - 1) / SCAN_J), dim3((P + 1) * 32), smem, st, *a);
     return cuda_check("mlstm_scan_kernel");
 }
 
@@ -652,8 +655,8 @@ int cc_seq_embed_bounded(const int32_t* tokens, const void* embed, int32_t table
     const dim3 grid = row_grid(T, E, vec ? 4 : 1);
 #define EB(ST, AT)                                                                                                        \
     {                                                                                                                     \
-        if (vec) embed_bounded_kernel<ST, AT, 4><<<grid, 128, 0, st>>>(tokens, (const ST*)embed, *emb, x, nx, (AT*)h, T, E); \
-        else embed_bounded_kernel<ST, AT, 1><<<grid, 128, 0, st>>>(tokens, (const ST*)embed, *emb, x, nx, (AT*)h, T, E);     \
+        if (vec) ccs::launch_under(embed_bounded_kernel<ST, AT, 4>, grid, dim3(128), 0, st, tokens, (const ST*)embed, *emb, x, nx, (AT*)h, T, E); \
+        else ccs::launch_under(embed_bounded_kernel<ST, AT, 1>, grid, dim3(128), 0, st, tokens, (const ST*)embed, *emb, x, nx, (AT*)h, T, E);     \
     }
     if (table_dtype == CC_DT_BF16 && act_dtype == CC_DT_BF16) EB(bf16, bf16)
     else if (table_dtype == CC_DT_BF16 && act_dtype == CC_DT_F32) EB(bf16, float)

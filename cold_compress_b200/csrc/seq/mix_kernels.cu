@@ -218,6 +218,7 @@ __global__ void gated_unit4_kernel(const float* __restrict__ in, int64_t ld, int
 template <typename ST>
 __global__ void __launch_bounds__(256) latent_prepare_kernel(const CcSeqLatentPrep a) {
     __shared__ float red[32];
+    ccs::pdl_wait_release();
     const int t = blockIdx.x, tid = threadIdx.x;
     const float* in = a.in + (size_t)t * a.ld;
     const int Dk = a.kv_rank + a.rot_dim;
@@ -253,9 +254,10 @@ __global__ void __launch_bounds__(256) latent_prepare_kernel(const CcSeqLatentPr
 
 // Rotation of one segment of every head of a fused query row, in place; optionally the rotated segment is also
 // copied to `tail` (the absorbed query layout [H, tail_ld] at column tail_off).
-__global__ void rope_heads_kernel(float* __restrict__ q, int64_t ld, const int32_t* __restrict__ input_pos,
+__global__ void rope_heads_kernel(float* q, int64_t ld, const int32_t* input_pos,
                                   const float* __restrict__ inv_freq, int H, int head_w, int off, int seg, int dims,
-                                  float* __restrict__ tail, int64_t tail_ld, int tail_off, int T, int interleaved) {
+                                  float* tail, int64_t tail_ld, int tail_off, int T, int interleaved) {
+    ccs::pdl_wait_release();
     const int t = blockIdx.x, half = dims / 2;
     const float p = (float)(input_pos[0] + t);
     float* row = q + (size_t)t * ld;
@@ -312,16 +314,44 @@ __global__ void head_gate_kernel(ST* __restrict__ y, const float* __restrict__ g
     }
 }
 
-// out[h, n] = W[h, n, :] . x[h, :]  (* sigmoid(gate[h])): a block-diagonal one-token product, a warp per row.
+__device__ __forceinline__ void read8(const float* p, float* o) {     // as load8, for what a launch before has written
+    const float4 a = reinterpret_cast<const float4*>(p)[0], b = reinterpret_cast<const float4*>(p)[1];
+    o[0] = a.x; o[1] = a.y; o[2] = a.z; o[3] = a.w; o[4] = b.x; o[5] = b.y; o[6] = b.z; o[7] = b.w;
+}
+__device__ __forceinline__ void read8(const bf16* p, float* o) {
+    const uint4 u = *reinterpret_cast<const uint4*>(p);
+    const bf16* e = reinterpret_cast<const bf16*>(&u);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) o[i] = __bfloat162float(e[i]);
+}
+
+// out[h, n] = W[h, n, :] . x[h, :]  (* sigmoid(gate[h])): a block-diagonal one-token product, a warp per row whose first
+// 256 weights are requested before the launch waits.
 template <typename WT, typename XT, typename OT>
-__global__ void __launch_bounds__(256) head_gemv_kernel(const WT* __restrict__ W, const XT* __restrict__ x, int64_t sx,
-                                                        OT* __restrict__ out, int64_t so, const float* __restrict__ gate,
-                                                        int H, int N, int K) {
+__global__ void __launch_bounds__(256) head_gemv_kernel(const WT* W, const XT* x, int64_t sx, OT* out, int64_t so, const float* gate, int H, int N, int K) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int row = blockIdx.x * 8 + warp;
-    if (row >= H * N) return;
+    const int row = min((int)blockIdx.x * 8 + warp, H * N - 1);
     const int h = row / N, n = row - h * N;
-    float acc = warp_dot<WT, XT>(W + ((size_t)h * N + n) * K, x + (size_t)h * sx, K, lane);
+    const WT* w = W + ((size_t)h * N + n) * K;
+    const XT* xh = x + (size_t)h * sx;
+    const bool vec = K % 8 == 0 && (((uintptr_t)w | (uintptr_t)xh) & 15) == 0;
+    float a[8];
+    if (vec && lane * 8 < K) load8(w + lane * 8, a);
+    ccs::pdl_wait_release();
+    if ((int)blockIdx.x * 8 + warp >= H * N) return;
+    float acc = 0.f;
+    if (vec) {
+        for (int k = lane * 8; k < K; k += 256) {
+            float b[8];
+            if (k >= 256) load8(w + k, a);
+            read8(xh + k, b);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) acc = fmaf(a[i], b[i], acc);
+        }
+    } else {
+        for (int k = lane; k < K; k += 32) acc = fmaf(ldf(w, k), ldf(xh, k), acc);
+    }
+    acc = warp_sum(acc);
     if (lane == 0) {
         if (gate != nullptr) acc *= sigmoidf_(gate[h]);
         stf(out, (size_t)h * so + n, acc);
@@ -720,6 +750,7 @@ __global__ void __launch_bounds__(LD_THREADS) latent_decode_kernel(const CcSeqLa
     extern __shared__ float4 sml4[];
     float* sm = reinterpret_cast<float*>(sml4);
     const int Dk = a.Dk, C = a.C, Dkp = ld_stride(Dk), Dk4 = (Dk + 3) / 4;
+    ccs::pdl_wait_release();
     float* Qs = sm;                         // [LD_HG][Dkp]
     float* Ks = Qs + LD_HG * Dkp;           // [LD_TK][Dkp]
     float* Ps = Ks + LD_TK * Dkp;           // [LD_HG][LD_TK]
@@ -767,7 +798,7 @@ __global__ void __launch_bounds__(LD_THREADS) latent_decode_kernel(const CcSeqLa
                     for (int e = 0; e < VEC; ++e) d[e] = 0.f;
                 } else {
                     const CT* row = sl == -2 ? kn : kc + (size_t)sl * Dk;
-                    const uint4 u = __ldg(reinterpret_cast<const uint4*>(row + c));
+                    const uint4 u = *reinterpret_cast<const uint4*>(row + c);     // the new row comes from the launch before
                     const CT* e8 = reinterpret_cast<const CT*>(&u);
 #pragma unroll
                     for (int e = 0; e < VEC; ++e) d[e] = ldf(e8, e);
@@ -831,6 +862,7 @@ template <typename CT, typename YT, int NC>
 __global__ void __launch_bounds__(LC_WARPS * 32) latent_combine_kernel(const CcSeqLatentDecode a) {
     extern __shared__ float smc[];          // [LC_WARPS][C + 1]
     __shared__ float red[LC_WARPS];
+    ccs::pdl_wait_release();
     const int h = blockIdx.x, C = a.C, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int p = a.input_pos[0], kpr = ld_keys_per_run(a.L);
     const int runs = min((p - ld_first_key(a, p)) / kpr + 1, (a.L + kpr - 1) / kpr);   // never more runs than the tile kernel has
@@ -899,8 +931,8 @@ static int launch_latent_decode(const CcSeqLatentDecode* a, cudaStream_t st) {
     }
     const int kpr = ld_keys_per_run(a->L);
     dim3 grid((a->L + kpr - 1) / kpr, (a->H + LD_HG - 1) / LD_HG);
-    kern<<<grid, LD_THREADS, smem, st>>>(*a);
-    latent_combine_kernel<CT, YT, NC><<<a->H, LC_WARPS * 32, sizeof(float) * LC_WARPS * (a->C + 1), st>>>(*a);
+    ccs::launch_under(kern, grid, dim3(LD_THREADS), smem, st, *a);
+    ccs::launch_under(latent_combine_kernel<CT, YT, NC>, dim3(a->H), dim3(LC_WARPS * 32), sizeof(float) * LC_WARPS * (a->C + 1), st, *a);
     return cuda_check("latent_decode kernels");
 }
 
@@ -995,19 +1027,24 @@ __device__ __forceinline__ uint4 ld_weights(const uint4* p) {
     return u;
 }
 
-constexpr int GEMV_AHEAD = 8;      // 16-byte weight vectors in flight per lane
+constexpr int GEMV_ROWS = 2;       // rows of a warp at a time: the input, read from shared memory, serves both
+constexpr int GEMV_AHEAD = 4;      // 16-byte weight vectors in flight per lane and row
 constexpr int GEMV_CTAS = 4;       // CTAs per SM (64 registers per thread)
 
-// KS warps share a row (KS == 1: a warp walks rows_per_cta / 8 rows, 8 apart).  A lane keeps GEMV_AHEAD vectors in flight
-// across the ends of rows: a slot is requested again as soon as it is used.  The first ones are on their way before the
-// kernel waits for the one before it.  (A 28-launch decode step of width 2048: 370 -> 340 us against one row per warp, four
-// loads in flight and no launch under the predecessor.)
+// A warp takes two neighbouring rows, KS warps share them (KS == 1: a warp walks rows_per_cta / 16 pairs, 16 rows apart).  A
+// lane keeps eight weight vectors in flight across the ends of rows: a slot is requested again as soon as it is used.  The
+// first ones are on their way before the kernel waits for the one before it.
+// Bound: HBM for many rows; the input's 32 bytes from shared memory per 16 bytes of weights held one row per warp below it
+// (16384 x 2048, alone in a graph: 14.4 us, without those reads 11.4, floor 10.2).  Decode step of a 4-layer model of width
+// 2048 at 4096 positions: 370 us with one row per warp, four loads in flight and every launch behind the one before it, 338
+// with eight loads across rows and launches under their predecessor, 312 with pairs and the small launches alike.
 template <typename WT, int PRE, int KS>
 __global__ void __launch_bounds__(256, GEMV_CTAS) gemv_multi_kernel(const CcSeqGemvMulti g, int rows_per_cta) {
     extern __shared__ float4 smg4[];
     float* xs = reinterpret_cast<float*>(smg4);
     __shared__ float red[32];
-    constexpr int RW = 8 / KS;     // rows at a time
+    constexpr int RW = 8 / KS * GEMV_ROWS;     // rows of a CTA at a time
+    constexpr int STEP = 32 * KS;              // vectors between two of a lane
     int j = 0, first = 0;
     while (j + 1 < g.n_jobs) {
         const int blocks = (g.job[j].N + rows_per_cta - 1) / rows_per_cta;
@@ -1018,16 +1055,17 @@ __global__ void __launch_bounds__(256, GEMV_CTAS) gemv_multi_kernel(const CcSeqG
     const CcSeqGemvJob& jb = g.job[j];
     const int K = jb.K, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, ks = warp % KS;
     const WT* W = (const WT*)jb.W;
-    const int n0 = ((int)blockIdx.x - first) * rows_per_cta + warp / KS, n_end = min(((int)blockIdx.x - first + 1) * rows_per_cta, jb.N);
+    const int n0 = ((int)blockIdx.x - first) * rows_per_cta + warp / KS * GEMV_ROWS, n_end = min(((int)blockIdx.x - first + 1) * rows_per_cta, jb.N);
     constexpr int VEC = 16 / (int)sizeof(WT);
     const bool vec = K % VEC == 0;
-    const int nv = K / VEC, v0 = lane + 32 * ks;    // this lane's vectors of a row: v0, v0 + 32 KS, ...
-    uint4 buf[GEMV_AHEAD];
-    {
-        const uint4* w16 = reinterpret_cast<const uint4*>(W + (size_t)min(n0, jb.N - 1) * K);
+    const int nv = K / VEC, v0 = lane + 32 * ks;    // this lane's vectors of a row: v0, v0 + STEP, ...
+    auto row = [&](int n) { return reinterpret_cast<const uint4*>(W + (size_t)min(n, jb.N - 1) * K); };   // rows past the end: the last one
+    uint4 buf[GEMV_ROWS][GEMV_AHEAD];
 #pragma unroll
-        for (int u = 0; u < GEMV_AHEAD; ++u) buf[u] = vec && v0 + 32 * KS * u < nv ? ld_weights(w16 + v0 + 32 * KS * u) : make_uint4(0u, 0u, 0u, 0u);
-    }
+    for (int u = 0; u < GEMV_AHEAD; ++u)
+#pragma unroll
+        for (int r = 0; r < GEMV_ROWS; ++r)
+            buf[r][u] = vec && v0 + STEP * u < nv ? ld_weights(row(n0 + r) + v0 + STEP * u) : make_uint4(0u, 0u, 0u, 0u);
     ccs::pdl_wait_release();
     bool shared_row = false;
     if constexpr (PRE != CC_GEMV_PRE_NONE) shared_row = jb.x == nullptr;
@@ -1057,81 +1095,98 @@ __global__ void __launch_bounds__(256, GEMV_CTAS) gemv_multi_kernel(const CcSeqG
     __syncthreads();
     if (KS == 1 && n0 >= n_end) return;
     for (int n = n0; n < n_end || KS > 1; n += RW) {
-        float acc = 0.f, acc1 = 0.f;
+        float acc[GEMV_ROWS];
+#pragma unroll
+        for (int r = 0; r < GEMV_ROWS; ++r) acc[r] = 0.f;
         if (vec) {
-            const uint4* w16 = reinterpret_cast<const uint4*>(W + (size_t)min(n, jb.N - 1) * K);
-            const bool more = n + RW < n_end && KS == 1;
-            for (int c0 = 32 * ks; c0 < nv; c0 += 32 * KS * GEMV_AHEAD) {      // the same for all lanes
+            const bool more = KS == 1 && n + RW < n_end;
+            for (int c0 = 32 * ks; c0 < nv; c0 += STEP * GEMV_AHEAD) {      // the same for all lanes
                 const int c = c0 + lane;
-                const bool last = c0 + 32 * KS * GEMV_AHEAD >= nv;
-                const uint4* next = last ? w16 + (size_t)RW * nv + v0 : w16 + c + 32 * KS * GEMV_AHEAD;
-                const int left = last ? (more ? nv - v0 : 0) : nv - c - 32 * KS * GEMV_AHEAD;
+                const bool last = c0 + STEP * GEMV_AHEAD >= nv;
+                const int from = last ? v0 : c + STEP * GEMV_AHEAD;
+                const int left = last && !more ? 0 : nv - from;
+                const uint4* next[GEMV_ROWS];
+#pragma unroll
+                for (int r = 0; r < GEMV_ROWS; ++r) next[r] = row(last ? n + RW + r : n + r) + from;
 #pragma unroll
                 for (int u = 0; u < GEMV_AHEAD; ++u) {
-                    if (c + 32 * KS * u < nv) {
-                        const WT* e = reinterpret_cast<const WT*>(&buf[u]);
-                        const float4* x4 = reinterpret_cast<const float4*>(xs + (c + 32 * KS * u) * VEC);
-                        float& a = u & 1 ? acc1 : acc;
+                    if (c + STEP * u < nv) {
+                        const float4* x4 = reinterpret_cast<const float4*>(xs + (c + STEP * u) * VEC);
 #pragma unroll
                         for (int q = 0; q < VEC / 4; ++q) {
                             const float4 xv = x4[q];
-                            a = fmaf(ldf(e, 4 * q + 0), xv.x, a);
-                            a = fmaf(ldf(e, 4 * q + 1), xv.y, a);
-                            a = fmaf(ldf(e, 4 * q + 2), xv.z, a);
-                            a = fmaf(ldf(e, 4 * q + 3), xv.w, a);
+#pragma unroll
+                            for (int r = 0; r < GEMV_ROWS; ++r) {
+                                const WT* e = reinterpret_cast<const WT*>(&buf[r][u]);
+                                acc[r] = fmaf(ldf(e, 4 * q + 0), xv.x, acc[r]);
+                                acc[r] = fmaf(ldf(e, 4 * q + 1), xv.y, acc[r]);
+                                acc[r] = fmaf(ldf(e, 4 * q + 2), xv.z, acc[r]);
+                                acc[r] = fmaf(ldf(e, 4 * q + 3), xv.w, acc[r]);
+                            }
                         }
                     }
-                    if (32 * KS * u < left) buf[u] = ld_weights(next + 32 * KS * u);
+                    if (STEP * u < left) {
+#pragma unroll
+                        for (int r = 0; r < GEMV_ROWS; ++r) buf[r][u] = ld_weights(next[r] + STEP * u);
+                    }
                 }
             }
-        } else if (KS == 1 || n < n_end) {
-            const WT* w = W + (size_t)n * K;
-            for (int k = lane + 32 * ks; k < K; k += 32 * KS) acc = fmaf(ldf(w, k), xs[k], acc);
-        }
-        acc = warp_sum(acc + acc1);
-        if constexpr (KS > 1) {      // the row's parts meet in part order
-            if (lane == 0) red[warp] = acc;
-            __syncthreads();
-            if (ks != 0 || n >= n_end) return;
+        } else {
 #pragma unroll
-            for (int q = 1; q < KS; ++q) acc += red[warp + q];
+            for (int r = 0; r < GEMV_ROWS; ++r) {
+                const WT* w = W + (size_t)min(n + r, jb.N - 1) * K;
+                for (int k = lane + 32 * ks; k < K; k += STEP) acc[r] = fmaf(ldf(w, k), xs[k], acc[r]);
+            }
         }
-        if (lane == 0) {
-            if (n < jb.conv_rows) {      // this row is a channel: its past inputs, then the tail moves on
+#pragma unroll
+        for (int r = 0; r < GEMV_ROWS; ++r) acc[r] = warp_sum(acc[r]);
+        float sum = acc[0];
+#pragma unroll
+        for (int r = 1; r < GEMV_ROWS; ++r) sum = lane == r ? acc[r] : sum;      // lane r closes row n + r
+        if constexpr (KS > 1) {      // the rows' parts meet in part order
+            if (lane < GEMV_ROWS) red[warp * GEMV_ROWS + lane] = sum;
+            __syncthreads();
+            if (ks != 0) return;
+#pragma unroll
+            for (int q = 1; q < KS; ++q) sum += red[(warp + q) * GEMV_ROWS + lane % GEMV_ROWS];
+        }
+        const int m = n + lane;
+        if (lane < GEMV_ROWS && m < n_end) {
+            if (m < jb.conv_rows) {      // this row is a channel: its past inputs, then the tail moves on
                 const int C = jb.conv_rows, taps = jb.taps;
-                const float* cw = jb.conv_w + (size_t)n * taps;
+                const float* cw = jb.conv_w + (size_t)m * taps;
                 float c = 0.f;
                 for (int t = 0; t < taps - 1; ++t) {
-                    const float u = jb.tail[(size_t)t * C + n];
+                    const float u = jb.tail[(size_t)t * C + m];
                     c = fmaf(cw[t], u, c);
-                    if (t > 0) jb.tail[(size_t)(t - 1) * C + n] = u;
+                    if (t > 0) jb.tail[(size_t)(t - 1) * C + m] = u;
                 }
-                if (taps > 1) jb.tail[(size_t)(taps - 2) * C + n] = acc;
-                acc = unit_act(fmaf(cw[taps - 1], acc, c), jb.conv_act);
+                if (taps > 1) jb.tail[(size_t)(taps - 2) * C + m] = sum;
+                sum = unit_act(fmaf(cw[taps - 1], sum, c), jb.conv_act);
             }
-            if (j == 0 && g.post.x != nullptr) bounded_row(g.post, n, acc);
-            if (jb.out != nullptr) ((float*)jb.out)[n] = acc;
+            if (j == 0 && g.post.x != nullptr) bounded_row(g.post, m, sum);
+            if (jb.out != nullptr) ((float*)jb.out)[m] = sum;
         }
         if constexpr (KS > 1) return;
     }
 }
 
-// How a launch is split: the rows of all jobs over the warps that fit the GPU at once (148 SMs x GEMV_CTAS CTAs).  Few rows:
-// two, four or eight warps share one, as long as each keeps four vectors per lane; many rows: a CTA walks several row
-// groups of 8, so that its input is staged once.
+// How a launch is split: the row pairs of all jobs over the warps that fit the GPU at once (148 SMs x GEMV_CTAS CTAs).  Few
+// rows: two, four or eight warps share a pair, as long as each keeps two vectors per lane and row; many rows: a CTA walks
+// several groups of 16 rows, so that its input is staged once.
 struct GemvSplit { int ks, rows_per_cta; };
 static GemvSplit gemv_split(const CcSeqGemvMulti* g, size_t smem, int elem) {
-    int rows = 0, kmin = 1 << 30;
+    int pairs = 0, kmin = 1 << 30;
     for (int j = 0; j < g->n_jobs; ++j) {
-        rows += g->job[j].N;
+        pairs += (g->job[j].N + GEMV_ROWS - 1) / GEMV_ROWS;
         kmin = g->job[j].K < kmin ? g->job[j].K : kmin;
     }
     const int fit = (int)(220 * 1024 / (smem + 2048));
     const int slots = 148 * 8 * (fit < 1 ? 1 : fit < GEMV_CTAS ? fit : GEMV_CTAS);
-    GemvSplit s = {1, 8};
-    while (s.ks < 8 && rows * s.ks * 2 <= slots && kmin * elem / 16 / (32 * s.ks * 2) >= 4) s.ks *= 2;
-    if (s.ks > 1) s.rows_per_cta = 8 / s.ks;
-    else s.rows_per_cta = 8 * ((rows + slots - 1) / slots);
+    GemvSplit s = {1, 8 * GEMV_ROWS};
+    while (s.ks < 8 && pairs * s.ks * 2 <= slots && kmin * elem / 16 / (32 * s.ks * 2) >= 2) s.ks *= 2;
+    if (s.ks > 1) s.rows_per_cta = 8 / s.ks * GEMV_ROWS;
+    else s.rows_per_cta = 8 * GEMV_ROWS * ((pairs + slots - 1) / slots);
     return s;
 }
 
@@ -1247,7 +1302,7 @@ int cc_seq_latent_prepare(const CcSeqLatentPrep* a, void* stream) {
         (a->q_rank > 0 && (!a->cq || !a->wq)))
         return fail(CC_SEQ_ERR_INVALID_ARG, "latent_prepare: bad argument");
     cudaStream_t st = (cudaStream_t)stream;
-#define CALL(ST) latent_prepare_kernel<ST><<<a->T, 256, 0, st>>>(*a)
+#define CALL(ST) ccs::launch_under(latent_prepare_kernel<ST>, dim3(a->T), dim3(256), 0, st, *a)
     CCM_ST(a->dtype, CALL);
 #undef CALL
     return cuda_check("latent_prepare_kernel");
@@ -1259,7 +1314,7 @@ int cc_seq_rope_heads(float* q, int64_t ld, const int32_t* input_pos, const floa
     if (!q || !input_pos || T < 1 || H < 1 || dims < 0 || (dims & 1) || dims > seg || off + seg > head_w ||
         (dims && !inv_freq))
         return fail(CC_SEQ_ERR_INVALID_ARG, "rope_heads: bad argument");
-    rope_heads_kernel<<<T, 256, 0, (cudaStream_t)stream>>>(q, ld, input_pos, inv_freq, H, head_w, off, seg, dims, tail,
+    ccs::launch_under(rope_heads_kernel, dim3(T), dim3(256), 0, (cudaStream_t)stream, q, ld, input_pos, inv_freq, H, head_w, off, seg, dims, tail,
                                                            tail_ld, tail_off, T, interleaved);
     return cuda_check("rope_heads_kernel");
 }
@@ -1291,7 +1346,7 @@ int cc_seq_head_gemv(const void* W, int32_t w_dtype, const void* x, int32_t x_dt
     cudaStream_t st = (cudaStream_t)stream;
     const int nb = (H * N + 7) / 8;
     const bool wb = w_dtype == CC_DT_BF16, xb = x_dtype == CC_DT_BF16, ob = out_dtype == CC_DT_BF16;
-#define HG(WT, XT, OT) head_gemv_kernel<WT, XT, OT><<<nb, 256, 0, st>>>((const WT*)W, (const XT*)x, sx, (OT*)out, so, gate, H, N, K)
+#define HG(WT, XT, OT) ccs::launch_under(head_gemv_kernel<WT, XT, OT>, dim3(nb), dim3(256), 0, st, (const WT*)W, (const XT*)x, sx, (OT*)out, so, gate, H, N, K)
     if (wb && xb && ob) HG(bf16, bf16, bf16);
     else if (wb && xb && !ob) HG(bf16, bf16, float);
     else if (wb && !xb && ob) HG(bf16, float, bf16);

@@ -13,6 +13,7 @@
 #include <stdint.h>
 
 #include "../../../include/cc_b200_seq.h"
+#include "launch.cuh"
 
 namespace ccs {
 int fail(int code, const char* msg);
@@ -519,6 +520,7 @@ __device__ __forceinline__ void pair_index(int i, int dims, int interleaved, int
 // A warp per (token, head) over the H query heads, the G key heads and the G value heads.
 template <typename OT>
 __global__ void qkv_rope_kernel(const CcSeqQkvRope a) {
+    ccs::pdl_wait_release();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int heads = a.H + 2 * a.G;
     const size_t th = (size_t)blockIdx.x * (blockDim.x >> 5) + warp;
@@ -767,7 +769,7 @@ int cc_seq_qkv_rope(const CcSeqQkvRope* a, void* stream) {
     cudaStream_t st = (cudaStream_t)stream;
     const size_t warps = (size_t)a->T * (a->H + 2 * a->G);
     const unsigned blocks = (unsigned)((warps + 7) / 8);
-#define CALL(OT) qkv_rope_kernel<OT><<<blocks, 256, 0, st>>>(*a)
+#define CALL(OT) ccs::launch_under(qkv_rope_kernel<OT>, dim3(blocks), dim3(256), 0, st, *a)
     CCN_ST(a->out_dtype, CALL);
 #undef CALL
     return cuda_check("qkv_rope_kernel");
