@@ -12,6 +12,7 @@
 #include <string.h>
 
 #include "../../../include/cc_b200_seq.h"
+#include "launch.cuh"
 
 namespace ccs {
 
@@ -703,6 +704,277 @@ __global__ void __launch_bounds__(DEC_THREADS) attn_decode_kernel(const CcSeqAtt
     if (a.append) append_row<CT>(a, g, 0, p, tid, DEC_THREADS);
 }
 
+// ---- the same for rows of whole 16-byte vectors and up to 8 query heads per key/value head
+// A run of 64-key tiles per CTA; the key and value rows of a tile are all requested at once (cp.async, the next tile under
+// this one) before anything is known about their slots, which are checked meanwhile.  Scores: eight lanes per key, four keys
+// at a time, the query rows read from shared memory once for the four.  Values: a thread owns a 16-byte column group and
+// every nkg-th key.  Partials and their combination as above, 16 bytes a load and 16 loads in flight.
+// Bound: the chain of dependent round trips (lookup and rows, partials, counter, combination), not the rows' bandwidth;
+// the kernel above walked every row by one thread and read the values after the scores (8 layers, 32 / 8 heads of 128, 4096
+// positions, in a graph: 32 us a layer).
+constexpr int VT = 64, VD_THREADS = 128, VD_MAX_SPLITS = 64, VD_RMAX = 8;
+
+__host__ __device__ inline int vd_splits(int L, int reach, int G) {     // runs per head: two CTAs per SM over the heads
+    const long long maxkeys = reach > 0 ? (reach < L + 1 ? reach : L + 1) : (long long)L + 1;
+    const long long tiles = (maxkeys + VT - 1) / VT;
+    long long most = 296 / G;
+    if (most < 1) most = 1;
+    if (most > VD_MAX_SPLITS) most = VD_MAX_SPLITS;
+    return (int)(tiles < most ? tiles : most);
+}
+
+__device__ __forceinline__ void cp_async16_or_zero(void* dst, const void* src, bool have) {
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(have ? 16 : 0) : "memory");
+}
+
+template <typename CT, typename YT, int RMAX>
+__global__ void __launch_bounds__(VD_THREADS) attn_decode_rows_kernel(const CcSeqAttn a, int buffers) {
+    extern __shared__ float4 smd4[];
+    constexpr int VEC = 16 / (int)sizeof(CT);
+    const int R = a.H / a.G, Dk = a.Dk, Dv = a.Dv, kc16 = Dk / VEC, vc16 = Dv / VEC;
+    const int k_row = kc16 + 1, k_tile = VT * k_row, v_tile = VT * vc16;         // 16-byte units; one of padding per key row
+    uint4* const ks = reinterpret_cast<uint4*>(smd4);                            // [buffers][VT][k_row]
+    uint4* const vs = ks + buffers * k_tile;                                     // [buffers][VT][vc16]
+    float* const qs = reinterpret_cast<float*>(vs + buffers * v_tile);           // [R][Dk]
+    float* const Ps = qs + RMAX * Dk;                                            // [RMAX][VT]
+    __shared__ int s_live[2][VT];
+    __shared__ float s_M[RMAX], s_L[RMAX], s_corr[RMAX], s_inv[RMAX];
+    __shared__ int s_last;
+
+    pdl_wait_release();
+    const int sp = blockIdx.x, g = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int p = a.input_pos[0];
+    const int j_lo = a.block > 0 ? (p / a.block) * a.block : (a.window > 0 ? max(0, p - a.window + 1) : 0);
+    const int kx = a.window > 0 ? min(a.keep_first, j_lo) : 0;
+    const int n = kx + (p - j_lo + 1);
+    const int n_tiles = (n + VT - 1) / VT, NS = vd_splits(a.L, attn_reach(a), a.G);
+    const int tiles_per = (n_tiles + NS - 1) / NS, nsplit = (n_tiles + tiles_per - 1) / tiles_per;
+    if (sp >= nsplit) return;
+    const CT* kc = (const CT*)a.k_cache + (size_t)g * a.L * Dk;
+    const CT* vc = (const CT*)a.v_cache + (size_t)g * a.L * Dv;
+    const CT* kn = (const CT*)a.k_new + (size_t)g * Dk;
+    const CT* vn = (const CT*)a.v_new + (size_t)g * Dv;
+    const int tile0 = sp * tiles_per, tile_end = min(n_tiles, tile0 + tiles_per);
+
+    auto fetch = [&](int tile) {
+        const int b = buffers > 1 ? (tile - tile0) & 1 : 0, u0 = tile * VT;
+        auto position = [&](int row) { return u0 + row < kx ? u0 + row : j_lo + (u0 + row - kx); };
+        for (int row = tid / kc16; row < VT; row += VD_THREADS / kc16) {          // kc16 divides into whole rows below
+            const int c = tid % kc16, j = position(row);
+            if (tid >= VD_THREADS / kc16 * kc16) break;
+            const bool have = u0 + row < n;
+            const CT* src = j == p ? kn : kc + (size_t)slot_of(a, j) * Dk;
+            cp_async16_or_zero(ks + b * k_tile + row * k_row + c, have ? (const void*)(src + c * VEC) : (const void*)kn, have);
+        }
+        for (int row = tid / vc16; row < VT; row += VD_THREADS / vc16) {
+            const int c = tid % vc16, j = position(row);
+            if (tid >= VD_THREADS / vc16 * vc16) break;
+            const bool have = u0 + row < n;
+            const CT* src = j == p ? vn : vc + (size_t)slot_of(a, j) * Dv;
+            cp_async16_or_zero(vs + b * v_tile + row * vc16 + c, have ? (const void*)(src + c * VEC) : (const void*)vn, have);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        if (tid < VT) {
+            const int j = position(tid);
+            s_live[(tile - tile0) & 1][tid] = u0 + tid < n && (j == p || a.pos[slot_of(a, j)] == j);
+        }
+    };
+    fetch(tile0);
+    for (int i = tid; i < R * Dk; i += VD_THREADS) qs[i] = a.q[(size_t)g * R * Dk + i];
+    if (tid < RMAX) { s_M[tid] = -INFINITY; s_L[tid] = 0.f; }
+    const int nkg = VD_THREADS / vc16, kg = tid / vc16, cg = tid - kg * vc16;     // value phase: key groups x column groups
+    float acc[RMAX][VEC];
+#pragma unroll
+    for (int r = 0; r < RMAX; ++r)
+#pragma unroll
+        for (int x = 0; x < VEC; ++x) acc[r][x] = 0.f;
+
+    for (int tile = tile0; tile < tile_end; ++tile) {
+        const int b = buffers > 1 ? (tile - tile0) & 1 : 0, u0 = tile * VT;
+        const int* live = s_live[(tile - tile0) & 1];
+        if (buffers > 1 && tile + 1 < tile_end) {
+            fetch(tile + 1);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+        }
+        __syncthreads();
+        {   // scores: keys 16 warp + 4 i + lane / 8
+            const int part = lane & 7, k0 = 16 * warp + (lane >> 3);
+            float sc[4][RMAX];
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int r = 0; r < RMAX; ++r) sc[i][r] = 0.f;
+            for (int c = part; c < kc16; c += 8) {
+                float kf[4][VEC];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const uint4 u = ks[b * k_tile + (k0 + 4 * i) * k_row + c];
+                    const CT* e = reinterpret_cast<const CT*>(&u);
+#pragma unroll
+                    for (int x = 0; x < VEC; ++x) kf[i][x] = ldf(e, x);
+                }
+#pragma unroll
+                for (int r = 0; r < RMAX; ++r)
+                    if (r < R) {
+#pragma unroll
+                        for (int x4 = 0; x4 < VEC / 4; ++x4) {
+                            const float4 qv = *reinterpret_cast<const float4*>(qs + r * Dk + c * VEC + 4 * x4);
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) {
+                                sc[i][r] = fmaf(qv.x, kf[i][4 * x4 + 0], sc[i][r]);
+                                sc[i][r] = fmaf(qv.y, kf[i][4 * x4 + 1], sc[i][r]);
+                                sc[i][r] = fmaf(qv.z, kf[i][4 * x4 + 2], sc[i][r]);
+                                sc[i][r] = fmaf(qv.w, kf[i][4 * x4 + 3], sc[i][r]);
+                            }
+                        }
+                    }
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int k = k0 + 4 * i, j = u0 + k < kx ? u0 + k : j_lo + (u0 + k - kx);
+                const bool ok = live[k] != 0;
+#pragma unroll
+                for (int r = 0; r < RMAX; ++r) {
+#pragma unroll
+                    for (int o = 4; o > 0; o >>= 1) sc[i][r] += __shfl_xor_sync(0xffffffffu, sc[i][r], o);
+                    if (r < R && part == (r & 7)) Ps[r * VT + k] = ok ? shape_score(a, sc[i][r] * a.scale, g * R + r, p - j) : -INFINITY;
+                }
+            }
+        }
+        __syncthreads();
+        for (int r = warp; r < R; r += VD_THREADS / 32) {
+            const float s0 = Ps[r * VT + lane], s1 = Ps[r * VT + lane + 32];
+            const float m_old = s_M[r], m_new = fmaxf(m_old, warp_max(fmaxf(s0, s1)));
+            const float p0 = s0 == -INFINITY ? 0.f : expf(s0 - m_new), p1 = s1 == -INFINITY ? 0.f : expf(s1 - m_new);
+            Ps[r * VT + lane] = p0;
+            Ps[r * VT + lane + 32] = p1;
+            const float sum = warp_sum(p0 + p1);
+            if (lane == 0) {
+                const float corr = m_old == -INFINITY ? 0.f : expf(m_old - m_new);
+                s_corr[r] = corr;
+                s_L[r] = s_L[r] * corr + sum;
+                s_M[r] = m_new;
+            }
+        }
+        __syncthreads();
+        if (kg < nkg) {
+#pragma unroll
+            for (int r = 0; r < RMAX; ++r)
+                if (r < R) {
+                    const float cr = s_corr[r];
+#pragma unroll
+                    for (int x = 0; x < VEC; ++x) acc[r][x] *= cr;
+                }
+#pragma unroll 4
+            for (int k = kg; k < VT; k += nkg) {
+                if (!live[k]) continue;
+                const uint4 u = vs[b * v_tile + k * vc16 + cg];
+                const CT* e = reinterpret_cast<const CT*>(&u);
+                float vf[VEC];
+#pragma unroll
+                for (int x = 0; x < VEC; ++x) vf[x] = ldf(e, x);
+#pragma unroll
+                for (int r = 0; r < RMAX; ++r)
+                    if (r < R) {
+                        const float w = Ps[r * VT + k];
+#pragma unroll
+                        for (int x = 0; x < VEC; ++x) acc[r][x] = fmaf(w, vf[x], acc[r][x]);
+                    }
+            }
+        }
+        __syncthreads();      // the tile is consumed: its buffers may be filled again
+        if (buffers == 1 && tile + 1 < tile_end) fetch(tile + 1);
+    }
+    // the key groups' sums meet in group order: red[kg][r][c], over the tiles
+    float* const red = reinterpret_cast<float*>(ks);
+    if (kg < nkg) {
+#pragma unroll
+        for (int r = 0; r < RMAX; ++r)
+            if (r < R) {
+#pragma unroll
+                for (int x = 0; x < VEC; ++x) red[((size_t)kg * R + r) * Dv + cg * VEC + x] = acc[r][x];
+            }
+    }
+    __syncthreads();
+    int* counters = (int*)a.workspace;
+    float* part_m = (float*)(counters + ((a.G + 3) & ~3));
+    float* part_l = part_m + (size_t)a.G * NS * R;
+    float* part_o = (float*)(((uintptr_t)(part_l + (size_t)a.G * NS * R) + 15) & ~(uintptr_t)15);
+    YT* y = (YT*)a.y + (size_t)g * R * Dv;
+    auto sink_of = [&](int r) { return a.sink_mode == CC_SINK_LEARNED ? a.sink[g * R + r] : a.sink_mode == CC_SINK_ZERO ? 0.f : -INFINITY; };
+    if (nsplit == 1) {
+        if (tid < R) {
+            const float sk = sink_of(tid), M = fmaxf(s_M[tid], sk);
+            const float w = s_M[tid] == -INFINITY ? 0.f : expf(s_M[tid] - M);
+            const float L = s_L[tid] * w + (a.sink_mode != CC_SINK_NONE ? expf(sk - M) : 0.f);
+            s_inv[tid] = L > 0.f ? w / L : 0.f;
+        }
+        __syncthreads();
+        for (int i = tid; i < R * Dv; i += VD_THREADS) {
+            float t = 0.f;
+            for (int q = 0; q < nkg; ++q) t += red[(size_t)q * R * Dv + i];
+            stf(y, i, t * s_inv[i / Dv]);
+        }
+        if (a.append) append_row<CT>(a, g, 0, p, tid, VD_THREADS);
+        return;
+    }
+    const size_t pbase = ((size_t)g * NS + sp) * R;
+    for (int i = tid; i < R * Dv; i += VD_THREADS) {
+        float t = 0.f;
+        for (int q = 0; q < nkg; ++q) t += red[(size_t)q * R * Dv + i];
+        part_o[pbase * Dv + i] = t;
+    }
+    if (tid < R) { part_m[pbase + tid] = s_M[tid]; part_l[pbase + tid] = s_L[tid]; }
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) s_last = atomicAdd(&counters[g], 1) == nsplit - 1;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    // the last CTA of the head: every other one has finished reading; combine in split order
+    float* const wgt = Ps;     // [R][VT] weights of the splits (at most VD_MAX_SPLITS == VT)
+    for (int r = warp; r < R; r += VD_THREADS / 32) {
+        const float sk = sink_of(r);
+        const float* pm = part_m + (size_t)g * NS * R + r;
+        const float m0 = lane < nsplit ? __ldcg(pm + (size_t)lane * R) : -INFINITY, m1 = lane + 32 < nsplit ? __ldcg(pm + (size_t)(lane + 32) * R) : -INFINITY;
+        const float* pl = part_l + (size_t)g * NS * R + r;
+        const float l0 = lane < nsplit ? __ldcg(pl + (size_t)lane * R) : 0.f, l1 = lane + 32 < nsplit ? __ldcg(pl + (size_t)(lane + 32) * R) : 0.f;
+        const float M = fmaxf(sk, warp_max(fmaxf(m0, m1)));
+        const float w0 = m0 == -INFINITY ? 0.f : expf(m0 - M), w1 = m1 == -INFINITY ? 0.f : expf(m1 - M);
+        wgt[r * VT + lane] = w0;
+        wgt[r * VT + lane + 32] = w1;
+        float L = warp_sum(l0 * w0 + l1 * w1);
+        if (a.sink_mode != CC_SINK_NONE) L += expf(sk - M);
+        if (lane == 0) s_inv[r] = L > 0.f ? 1.0f / L : 0.f;
+    }
+    __syncthreads();
+    const float4* po = reinterpret_cast<const float4*>(part_o + (size_t)g * NS * R * Dv);     // Dv is a multiple of 4
+    const int quads = R * Dv / 4;
+    for (int i = tid; i < quads; i += VD_THREADS) {
+        const int r = i / (Dv / 4);
+        const float* w = wgt + r * VT;
+        float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 16
+        for (int s = 0; s < nsplit; ++s) {
+            const float4 v = __ldcg(po + (size_t)s * quads + i);
+            t.x = fmaf(w[s], v.x, t.x);
+            t.y = fmaf(w[s], v.y, t.y);
+            t.z = fmaf(w[s], v.z, t.z);
+            t.w = fmaf(w[s], v.w, t.w);
+        }
+        const float inv = s_inv[r];
+        stf(y, 4 * i + 0, t.x * inv);
+        stf(y, 4 * i + 1, t.y * inv);
+        stf(y, 4 * i + 2, t.z * inv);
+        stf(y, 4 * i + 3, t.w * inv);
+    }
+    if (tid == 0) counters[g] = 0;
+    if (a.append) append_row<CT>(a, g, 0, p, tid, VD_THREADS);
+}
+
 template <typename CT>
 __global__ void cache_append_kernel(const CcSeqAttn a, int t_first) {
     const int t = t_first + blockIdx.x, g = blockIdx.y;
@@ -935,9 +1207,39 @@ static int launch_decode_r(const CcSeqAttn* a, cudaStream_t st) {
     return cuda_check("attn_decode_kernel");
 }
 
+// Rows of whole 16-byte vectors on 16-byte boundaries, up to 8 query heads per key/value head, tiles that fit the shared memory
+static bool decode_rows_serves(const CcSeqAttn* a) {
+    const int size = a->cache_dtype == CC_DT_BF16 ? 2 : 4;
+    const uintptr_t all = (uintptr_t)a->k_new | (uintptr_t)a->v_new | (uintptr_t)a->k_cache | (uintptr_t)a->v_cache | (uintptr_t)a->workspace;
+    return a->Dk * size % 16 == 0 && a->Dv * size % 16 == 0 && a->Dk * size <= 512 && a->Dv * size <= 512 && (all & 15) == 0 && a->H / a->G <= VD_RMAX;
+}
+
+template <typename CT, typename YT, int RMAX>
+static int launch_decode_rows(const CcSeqAttn* a, cudaStream_t st) {
+    const int NS = vd_splits(a->L, attn_reach(*a), a->G);
+    const long long reach = attn_reach(*a) > 0 && attn_reach(*a) < a->L + 1 ? attn_reach(*a) : (long long)a->L + 1;
+    const int buffers = (reach + VT - 1) / VT > NS ? 2 : 1;      // a run can be longer than one tile
+    const size_t row = sizeof(CT) * (size_t)(a->Dk + a->Dv) + 16;
+    size_t tiles = (size_t)buffers * VT * row;
+    const int vc16 = a->Dv * (int)sizeof(CT) / 16;
+    const size_t red = sizeof(float) * (size_t)(VD_THREADS / vc16) * (a->H / a->G) * a->Dv;
+    const size_t smem = (tiles > red ? tiles : red) + sizeof(float) * RMAX * (size_t)(a->Dk + VT);
+    auto kern = attn_decode_rows_kernel<CT, YT, RMAX>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return fail(CC_SEQ_ERR_CUDA, cudaGetErrorString(e));
+    launch_under(kern, dim3(NS, a->G), dim3(VD_THREADS), smem, st, *a, buffers);
+    return cuda_check("attn_decode_rows_kernel");
+}
+
 template <typename CT, typename YT>
 static int launch_decode(const CcSeqAttn* a, cudaStream_t st) {
     const int R = a->H / a->G;
+    if (decode_rows_serves(a)) {
+        if (R <= 1) return launch_decode_rows<CT, YT, 1>(a, st);
+        if (R <= 2) return launch_decode_rows<CT, YT, 2>(a, st);
+        if (R <= 4) return launch_decode_rows<CT, YT, 4>(a, st);
+        return launch_decode_rows<CT, YT, 8>(a, st);
+    }
     if (R <= 1) return launch_decode_r<CT, YT, 1>(a, st);
     if (R <= 2) return launch_decode_r<CT, YT, 2>(a, st);
     if (R <= 4) return launch_decode_r<CT, YT, 4>(a, st);
@@ -1006,8 +1308,9 @@ int cc_seq_attention(const CcSeqAttn* a, void* stream) {
 }
 
 uint64_t cc_seq_decode_workspace(int32_t H, int32_t G, int32_t Dv, int32_t L, int32_t window) {
-    const uint64_t NS = (uint64_t)decode_max_splits(L, window);
-    return sizeof(int) * (uint64_t)((G + 3) & ~3) + sizeof(float) * NS * (uint64_t)H * (2 + (uint64_t)Dv);
+    const uint64_t narrow = (uint64_t)decode_max_splits(L, window), wide = (uint64_t)vd_splits(L, window, G < 1 ? 1 : G);
+    const uint64_t NS = narrow > wide ? narrow : wide;       // either kernel may serve the call
+    return sizeof(int) * (uint64_t)((G + 3) & ~3) + sizeof(float) * NS * (uint64_t)H * (2 + (uint64_t)Dv) + 16;
 }
 
 int cc_seq_attention_decode(const CcSeqAttn* a, void* stream) {

@@ -86,3 +86,50 @@ def test_portion_matches_64_bit_attention(shape, stale):
         # mean), it enters the weight through exp, and scores here stay below 8; bf16 adds the rounding of the output
         bound = 8 * 2.0 ** -24 * math.sqrt(max(Dk, 64))
         assert err <= (bound if dtype == torch.float32 else 2.0 ** -8), (err, bound)
+
+
+# past, H, G, Dk, Dv, options: one token
+TOKEN_SHAPES = [
+    (0, 4, 2, 128, 128, dict(sink=1)),                 # the token alone
+    (62, 2, 2, 64, 64, {}), (63, 8, 2, 128, 128, {}), (64, 8, 1, 128, 128, dict(sink=2)),      # around a tile of 64 keys
+    (127, 7, 1, 72, 40, {}), (1000, 6, 2, 96, 128, {}),                                        # rows that are not powers of two
+    (4200, 32, 8, 128, 128, dict(sink=1)), (20000, 2, 1, 128, 64, {}),                         # several tiles per run
+    (3000, 4, 4, 256, 256, {}), (777, 10, 1, 128, 128, {}), (500, 4, 2, 130, 70, {}),          # widest rows; the general kernel
+    (900, 4, 2, 128, 128, dict(window=300)), (900, 4, 2, 64, 72, dict(window=65, keep=5, softcap=15.0, dist=True, sink=1)),
+    (300, 8, 2, 128, 128, dict(block=128)),
+]
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("shape", TOKEN_SHAPES, ids=lambda s: f"past{s[0]}-H{s[1]}-G{s[2]}-{s[3]}x{s[4]}" + "".join(f"-{k}{v}" for k, v in s[5].items()))
+def test_one_token_matches_64_bit_attention(shape, dtype):
+    from cold_compress_b200 import _lib
+    from cold_compress_b200.cache import get_cache_constructor
+    past, H, G, Dk, Dv, o = shape
+    dev, gen = "cuda", torch.Generator(device="cuda").manual_seed(past + H)
+    window, block, keep = o.get("window", 0), o.get("block", 0), o.get("keep", 0)
+    L = window + keep + 5 if window else block or past + 40
+    cls, _ = get_cache_constructor("recent_global" if window or block else "full")
+    cache = cls(1, G, Dk, dtype, max_cache_length=L, global_tokens=keep, max_seq_length=1 << 20, cache_bits=None, v_head_dim=Dv).to(dev)
+    randn = lambda *s: torch.randn(*s, device=dev, generator=gen)  # noqa: E731
+    k, v = randn(past + 2, G, Dk).to(dtype), randn(past + 2, G, Dv).to(dtype)
+    held = torch.full((L,), -1, dtype=torch.long)
+    for j in range(past):
+        held[j if j < keep else keep + (j - keep) % (L - keep)] = j
+    at = held >= 0
+    cache.k_cache.fill_(math.inf)      # what empty slots hold is never a key
+    cache.v_cache.fill_(math.nan)
+    cache.k_cache[0][:, at], cache.v_cache[0][:, at] = k[held[at]].transpose(0, 1), v[held[at]].transpose(0, 1)
+    cache.pos[0, 0], cache.mask[0, :, 0] = held.int().to(dev), at.to(dev)
+    sink = randn(H) if o.get("sink") == 1 else None
+    dist = (torch.rand(H, device=dev, generator=gen) * 0.5, torch.rand(H, device=dev, generator=gen)) if o.get("dist") else None
+    mode = {None: _lib.SINK_NONE, 1: _lib.SINK_LEARNED, 2: _lib.SINK_ZERO}[o.get("sink")]
+    for p in (past, past + 1):         # the second token reads the row that the first has left
+        q, y = 1.3 * randn(1, H, Dk), torch.empty(1, H, Dv, device=dev)
+        want = _reference(q, k[:p + 1], v[:p + 1], p, Dk ** -0.5, o, sink, dist)
+        cache.sequence_step(q, k[p:p + 1].contiguous(), v[p:p + 1].contiguous(), torch.full((1,), p, dtype=torch.int32, device=dev), y,
+                            window=window, sink=sink, sink_mode=mode, scale=Dk ** -0.5, softcap=o.get("softcap", 0.0), dist=dist, block=block)
+        # fp32 sums of Dk products and of up to `past` weighted values in one rounding each, scores below 8 through exp
+        assert ((y.double() - want).norm() / want.norm()).item() <= 8 * 2.0 ** -24 * math.sqrt(max(Dk, 64))
+        slot = p if p < keep else keep + (p - keep) % (L - keep)
+        assert cache.pos[0, 0, slot].item() == p and torch.equal(cache.k_cache[0, :, slot], k[p]) and torch.equal(cache.v_cache[0, :, slot], v[p])
