@@ -69,6 +69,15 @@ int cc_requantize_cache(void* k_cache, void* v_cache, int32_t n_kv_heads, int32_
                                      k_zero_points, v_scales, v_zero_points, (cudaStream_t)stream);
 }
 
+int cc_rmsnorm_rows(const void* x, const void* w, float eps, void* out, int32_t rows, int32_t dim, void* stream) {
+    return cc::rmsnorm_rows_impl(x, w, eps, out, rows, dim, (cudaStream_t)stream);
+}
+int cc_rope_rows(const void* qkv, int64_t row_stride, const void* freqs, void* q, void* k, int32_t S, int32_t n_q_heads, int32_t n_kv_heads,
+                 int32_t head_dim, void* stream) {
+    return cc::rope_rows_impl(qkv, row_stride, freqs, q, k, S, n_q_heads, n_kv_heads, head_dim, (cudaStream_t)stream);
+}
+int cc_silu_mul(const void* a, const void* b, void* out, int64_t n, void* stream) { return cc::silu_mul_impl(a, b, out, n, (cudaStream_t)stream); }
+
 uint64_t cc_prefill_attention_workspace(int32_t seq_len, int32_t n_kv_heads, int32_t q_per_kv, int32_t obs_len,
                                         int32_t n_windows) {
     return cc::prefill_attention_workspace_impl(seq_len, n_kv_heads, q_per_kv, obs_len, n_windows);

@@ -15,6 +15,10 @@ int key_norms_impl(const void* k, void* key_norm, int n_rows, int head_dim, cuda
 int prefill_gather_impl(const CcCacheState* st, const void* k_prompt, const void* v_prompt,
                         const int64_t* keep_idx, int keep_heads, int n_keep, int prompt_len,
                         cudaStream_t stream);
+int rmsnorm_rows_impl(const void* x, const void* w, float eps, void* out, int rows, int dim, cudaStream_t stream);
+int rope_rows_impl(const void* qkv, long long row_stride, const void* freqs, void* q, void* k, int S, int n_q_heads, int n_kv_heads, int head_dim,
+                   cudaStream_t stream);
+int silu_mul_impl(const void* a, const void* b, void* out, long long n, cudaStream_t stream);
 int prefill_attention_impl(const CcPrefillAttnArgs* a, cudaStream_t stream);
 unsigned long long prefill_attention_workspace_impl(int S, int Hkv, int G, int obs_len, int n_windows);
 int requantize_cache_impl(void* k_cache, void* v_cache, int H, int L, int D, int n_bit, uint8_t* k_codes, uint8_t* v_codes,

@@ -370,7 +370,14 @@ class Attention(nn.Module):
     def _project(self, x, freqs_cis):
         bsz, seqlen, _ = x.shape
         kv = self.n_local_heads * self.head_dim
-        q, k, v = self.wqkv(x).split([self.dim, kv, kv], dim=-1)
+        qkv = self.wqkv(x)
+        if bsz == 1 and self.head_dim % 8 == 0 and qkv.shape[-1] == self.dim + 2 * kv and freqs_cis.shape == (seqlen, self.head_dim // 2, 2) and freqs_cis.is_contiguous() \
+                and self.dim == self.n_head * self.head_dim and ops.plain_rows(qkv, freqs_cis.view(seqlen, self.head_dim)):
+            q = torch.empty(1, seqlen, self.n_head, self.head_dim, dtype=qkv.dtype, device=qkv.device)
+            k = torch.empty(1, seqlen, self.n_local_heads, self.head_dim, dtype=qkv.dtype, device=qkv.device)
+            ops.rope_rows(qkv[0], freqs_cis, q[0], k[0])
+            return q.transpose(1, 2), k.transpose(1, 2), qkv[..., self.dim + kv:].view(bsz, seqlen, self.n_local_heads, self.head_dim).transpose(1, 2)
+        q, k, v = qkv.split([self.dim, kv, kv], dim=-1)
         q = apply_rotary_emb(q.view(bsz, seqlen, self.n_head, self.head_dim), freqs_cis).transpose(1, 2)
         k = apply_rotary_emb(k.view(bsz, seqlen, self.n_local_heads, self.head_dim), freqs_cis).transpose(1, 2)
         v = v.view(bsz, seqlen, self.n_local_heads, self.head_dim).transpose(1, 2)
@@ -421,7 +428,13 @@ class FeedForward(nn.Module):
         self.tp_group = None
 
     def forward(self, x: Tensor) -> Tensor:
-        y = self.w2(F.silu(self.w1(x)) * self.w3(x))
+        a, b = self.w1(x), self.w3(x)
+        if ops.plain_rows(a, b):
+            gated = torch.empty_like(a)
+            ops.silu_mul(a, b, gated)
+        else:
+            gated = F.silu(a) * b
+        y = self.w2(gated)
         if self.tp_group is not None:
             torch.distributed.all_reduce(y, group=self.tp_group)
         return y
@@ -434,6 +447,10 @@ class RMSNorm(nn.Module):
         self.weight = nn.Parameter(torch.ones(dim))
 
     def forward(self, x: Tensor) -> Tensor:
+        if x.shape[-1] == self.weight.numel() <= 16384 and ops.plain_rows(x, self.weight):
+            out = torch.empty_like(x)
+            ops.rmsnorm_rows(x, self.weight, self.eps, out)
+            return out
         xf = x.float()
         return (xf * torch.rsqrt(xf.pow(2).mean(-1, keepdim=True) + self.eps)).type_as(x) * self.weight
 

@@ -31,6 +31,9 @@ _library.define("requantize_cache(Tensor(a!) k_cache, Tensor(b!) v_cache, int n_
 _library.define(
     "prefill_attention(Tensor q, Tensor k, Tensor v, Tensor(a!) y, int attn_mode, int obs_len, int[] windows, "
     "Tensor(b!)? col_sum, Tensor(c!)? obs_sum, Tensor(d!)? band_sum, Tensor(e!)? workspace) -> ()")
+_library.define("rmsnorm_rows(Tensor x, Tensor w, float eps, Tensor(a!) out) -> ()")
+_library.define("rope_rows(Tensor qkv, Tensor freqs, Tensor(a!) q, Tensor(b!) k) -> ()")
+_library.define("silu_mul(Tensor a, Tensor b, Tensor(a!) out) -> ()")
 _library.define(
     "rmsnorm_qkv_rope(Tensor x, Tensor norm_w, float eps, Tensor wqkv, Tensor? bias, Tensor freqs_cis, "
     "Tensor input_pos, Tensor(a!) q, Tensor(b!) k, Tensor(c!) v, int n_q_heads, int n_kv_heads, int head_dim, "
@@ -145,6 +148,33 @@ def _prefill_attention(q, k, v, y, attn_mode, obs_len, windows, col_sum, obs_sum
     _lib.check(_lib.load().cc_prefill_attention(C.byref(a), _stream()), "cc_prefill_attention")
 
 
+def _rmsnorm_rows(x, w, eps, out):
+    _require_cuda(x, w, out)
+    _lib.check(_lib.load().cc_rmsnorm_rows(_ptr(x), _ptr(w), float(eps), _ptr(out), x.numel() // x.shape[-1], x.shape[-1], _stream()), "cc_rmsnorm_rows")
+
+
+def _rope_rows(qkv, freqs, q, k):
+    """qkv [S, >= (Hq + Hkv) D] rows, freqs [S, D / 2, 2], q [S, Hq, D], k [S, Hkv, D]."""
+    _require_cuda(qkv, freqs, q, k)
+    _lib.check(_lib.load().cc_rope_rows(_ptr(qkv), qkv.stride(0), _ptr(freqs), _ptr(q), _ptr(k), q.shape[0], q.shape[1], k.shape[1],
+                                        q.shape[2], _stream()), "cc_rope_rows")
+
+
+def _silu_mul(a, b, out):
+    _require_cuda(a, b, out)
+    _lib.check(_lib.load().cc_silu_mul(_ptr(a), _ptr(b), _ptr(out), a.numel(), _stream()), "cc_silu_mul")
+
+
+def plain_rows(*tensors) -> bool:
+    """Whether the row kernels of a prompt layer may stand for tensor operations on these: plain contiguous bf16 CUDA tensors
+    whose last dimension is whole 16-byte vectors, on 16-byte boundaries, outside of differentiation (reverse or forward)
+    and of function transforms."""
+    return (torch._C._functorch.peek_interpreter_stack() is None and torch.autograd.forward_ad._current_level < 0
+            and all(type(t) in (torch.Tensor, torch.nn.Parameter) and t.is_cuda and t.dtype == torch.bfloat16 and t.is_contiguous()
+                    and t.numel() > 0 and t.shape[-1] % 8 == 0 and t.data_ptr() % 16 == 0 for t in tensors)
+            and not (torch.is_grad_enabled() and any(t.requires_grad for t in tensors)))
+
+
 def _optr(t):
     return None if t is None else t.data_ptr()
 
@@ -195,6 +225,9 @@ _library.impl("rmsnorm_qkv_rope", _rmsnorm_qkv_rope, "CUDA")
 _library.impl("gemv_residual", _gemv_residual, "CUDA")
 _library.impl("rmsnorm_ffn_gate", _rmsnorm_ffn_gate, "CUDA")
 _library.impl("key_norms", _key_norms, "CUDA")
+_library.impl("rmsnorm_rows", _rmsnorm_rows, "CUDA")
+_library.impl("rope_rows", _rope_rows, "CUDA")
+_library.impl("silu_mul", _silu_mul, "CUDA")
 _library.impl("prefill_gather", _prefill_gather, "CUDA")
 _library.impl("prefill_attention", _prefill_attention, "CUDA")
 _library.impl("requantize_cache", _requantize_cache, "CUDA")
@@ -204,7 +237,8 @@ def _no_cpu(*_a, **_k):
     raise _lib.CcError("cold_compress_b200 ops have no CPU implementation: the decode path is CUDA (sm_100a) only")
 
 
-for _name in ("decode_step", "key_norms", "prefill_gather", "prefill_attention", "requantize_cache", "rmsnorm_qkv_rope", "gemv_residual", "rmsnorm_ffn_gate"):
+for _name in ("decode_step", "key_norms", "prefill_gather", "prefill_attention", "requantize_cache", "rmsnorm_qkv_rope", "gemv_residual", "rmsnorm_ffn_gate",
+              "rmsnorm_rows", "rope_rows", "silu_mul"):
     _library.impl(_name, _no_cpu, "CPU")
 
 decode_step = torch.ops.cold_compress_b200.decode_step
@@ -214,4 +248,7 @@ prefill_attention = torch.ops.cold_compress_b200.prefill_attention
 requantize_cache = torch.ops.cold_compress_b200.requantize_cache
 rmsnorm_qkv_rope = torch.ops.cold_compress_b200.rmsnorm_qkv_rope
 gemv_residual = torch.ops.cold_compress_b200.gemv_residual
+rmsnorm_rows = torch.ops.cold_compress_b200.rmsnorm_rows
+rope_rows = torch.ops.cold_compress_b200.rope_rows
+silu_mul = torch.ops.cold_compress_b200.silu_mul
 rmsnorm_ffn_gate = torch.ops.cold_compress_b200.rmsnorm_ffn_gate

@@ -177,6 +177,19 @@ void cc_debug_set_trace(void* device_buffer);
 int cc_key_norms(const void* k, void* key_norm, int32_t n_rows, int32_t head_dim, void* stream);
 
 /*
+ * The element-wise work of a prompt layer (bf16 tensors, rows of whole 16-byte vectors on 16-byte boundaries;
+ * CC_ERR_UNSUPPORTED_SHAPE otherwise), with the rounding points of model.py:
+ *   cc_rmsnorm_rows  out[r] = bf16(x[r] * rsqrt(mean(x[r]^2) + eps)) * w               model.py:452-457
+ *   cc_rope_rows     q [S, n_q_heads, D], k [S, n_kv_heads, D] = the turned q and k columns of rows [q | k | ...] of stride
+ *                    row_stride; freqs [S, D / 2, 2] (cos, sin)                          model.py:507-519
+ *   cc_silu_mul      out = bf16(silu(a)) * b, n elements                                 model.py:436-443
+ */
+int cc_rmsnorm_rows(const void* x, const void* w, float eps, void* out, int32_t rows, int32_t dim, void* stream);
+int cc_rope_rows(const void* qkv, int64_t row_stride, const void* freqs, void* q, void* k, int32_t S, int32_t n_q_heads,
+                 int32_t n_kv_heads, int32_t head_dim, void* stream);
+int cc_silu_mul(const void* a, const void* b, void* out, int64_t n, void* stream);
+
+/*
  * Prompt compression gather (prompt_compression.py:82-88 + cache.py:381-401):
  * k_cache[h, j, :] = k_prompt[h, keep_idx[h or 0, j], :] for j < n_keep, same for V,
  * pos[h, j] = keep_idx[..], mask[h, j] = 1.

@@ -1,0 +1,73 @@
+"""The row kernels of a prompt layer against the tensor operations they stand for, and the calls that keep those operations."""
+import pytest
+import torch
+import torch.nn.functional as F
+
+pytestmark = pytest.mark.gpu
+
+
+def _bf16(*shape, seed=0, scale=1.0):
+    return (torch.randn(*shape, generator=torch.Generator().manual_seed(seed)) * scale).bfloat16().cuda()
+
+
+def _adjacent(got, want, share=0.02):
+    """Equal or neighbouring bf16 values, and equal almost everywhere."""
+    a, b = got.float(), want.float()
+    assert torch.all((a - b).abs() <= 2.0 ** -7 * torch.maximum(a.abs(), b.abs()))
+    assert (a != b).float().mean().item() <= share
+
+
+@pytest.mark.parametrize("rows, dim", [(1, 8), (3, 896), (7, 2048), (5, 2056), (2, 4096), (129, 3584), (2, 8200), (1, 16384)])
+def test_rms_norm_rows(rows, dim):
+    from cold_compress_b200.model import RMSNorm
+    m = RMSNorm(dim, eps=1e-5)
+    m.weight.data = 1.0 + 0.3 * torch.randn(dim)
+    m = m.to(torch.bfloat16).cuda()
+    x = _bf16(1, rows, dim, seed=dim, scale=3.0)
+    want = m(x)                      # gradients wanted: tensor operations
+    assert want.requires_grad
+    with torch.no_grad():
+        got = m(x)
+    _adjacent(got, want.detach())    # the mean of the squares is summed in another order
+
+
+@pytest.mark.parametrize("S, Hq, Hkv, D", [(1, 1, 1, 8), (5, 14, 2, 64), (33, 28, 4, 128), (130, 8, 8, 128), (7, 3, 1, 72)])
+def test_rotated_rows(S, Hq, Hkv, D):
+    from cold_compress_b200 import ops
+    from cold_compress_b200.model import apply_rotary_emb, precompute_freqs_cis
+    qkv = _bf16(S, (Hq + 2 * Hkv) * D, seed=S)
+    freqs = precompute_freqs_cis(S, D, 10000, torch.bfloat16).cuda()
+    q, k = torch.empty(S, Hq, D, dtype=torch.bfloat16, device="cuda"), torch.empty(S, Hkv, D, dtype=torch.bfloat16, device="cuda")
+    ops.rope_rows(qkv, freqs, q, k)
+    assert torch.equal(q, apply_rotary_emb(qkv[:, :Hq * D].reshape(1, S, Hq, D), freqs)[0])
+    assert torch.equal(k, apply_rotary_emb(qkv[:, Hq * D:(Hq + Hkv) * D].reshape(1, S, Hkv, D), freqs)[0])
+
+
+@pytest.mark.parametrize("n", [8, 2040, 100 * 4864])
+def test_gated_unit_rows(n):
+    from cold_compress_b200 import ops
+    a, b = _bf16(n, seed=1, scale=4.0), _bf16(n, seed=2)
+    a[:4] = torch.tensor([float("inf"), -float("inf"), -100.0, 0.0])
+    out = torch.empty_like(a)
+    ops.silu_mul(a, b, out)
+    want = F.silu(a) * b
+    finite = want.isfinite()
+    assert torch.equal(out[~finite].nan_to_num(7.0), want[~finite].nan_to_num(7.0))
+    _adjacent(out[finite], want[finite], share=1e-3)
+
+
+def test_calls_that_keep_the_tensor_operations():
+    from cold_compress_b200 import ops
+    from cold_compress_b200.model import RMSNorm
+    x = _bf16(4, 64)
+    assert ops.plain_rows(x)
+    assert not ops.plain_rows(x.float()) and not ops.plain_rows(x.t()) and not ops.plain_rows(x[:, :60]) and not ops.plain_rows(x.view(-1)[1:57].view(7, 8))
+    assert not ops.plain_rows(x.clone().requires_grad_()) and not ops.plain_rows(x[:0])
+    m = RMSNorm(64).to(torch.bfloat16).cuda().requires_grad_(False)
+    want = m(x)
+    with torch.no_grad():
+        batched = torch.vmap(m)(x.view(2, 2, 64))
+        _adjacent(batched.view(4, 64), want)
+        out, tangent = torch.func.jvp(m, (x,), (x,))
+    _adjacent(out, want)
+    assert tangent.shape == x.shape
