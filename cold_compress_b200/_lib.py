@@ -137,7 +137,7 @@ def check(rc: int, what: str = "") -> int:
 
 # --------------------------------------------------------------------------- libcc_b200_seq.so (include/cc_b200_seq.h)
 SEQ_SO_PATH = Path(os.environ.get("CC_B200_SEQ_LIB", PKG / "libcc_b200_seq.so"))
-SEQ_ABI_VERSION = 7
+SEQ_ABI_VERSION = 8
 DT_F32, DT_BF16 = 0, 1
 SINK_NONE, SINK_LEARNED, SINK_ZERO = 0, 1, 2
 
@@ -237,7 +237,7 @@ class CcSeqLatentDecode(C.Structure):
 
 
 class CcSeqWkv(C.Structure):
-    _fields_ = [(n, _vp) for n in ("r", "k", "v", "wraw", "w0", "u", "state", "o")] + [(n, _i32) for n in ("T", "H", "D")]
+    _fields_ = [(n, _vp) for n in ("r", "k", "v", "wraw", "w0", "u", "state", "o")] + [(n, _i32) for n in ("T", "H", "D", "decayed")]
 
 
 class CcSeqMoeGrouped(C.Structure):
@@ -263,6 +263,7 @@ SEQ_EXPORTS.update({
     "cc_seq_head_gate": (C.c_int, [_vp, _i32, _vp, _i64, _i32, _i32, _i32, _vp]),
     "cc_seq_head_gemv": (C.c_int, [_vp, _i32, _vp, _i32, _i64, _vp, _i32, _i64, _vp, _i32, _i32, _i32, _vp]),
     "cc_seq_wkv": (C.c_int, [C.POINTER(CcSeqWkv), _vp]),
+    "cc_seq_wkv_decay": (C.c_int, [_vp, _vp, _vp, _i32, _i32, _vp]),
     "cc_seq_head_norm_gate": (C.c_int, [_vp, _vp, _i64, _vp, _vp, _i32, _i32, _i32, _i32, _f32, _vp]),
     "cc_seq_moe_route": (C.c_int, [_vp, _i64, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _i32, _i32, _i32, _i32, _f32, _vp]),
     "cc_seq_moe_group": (C.c_int, [_vp, _i32, _i32, _i32, _vp, _vp, _vp, _vp]),

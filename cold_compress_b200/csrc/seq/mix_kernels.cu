@@ -361,18 +361,36 @@ __global__ void __launch_bounds__(256) head_gemv_kernel(const WT* W, const XT* x
 // ------------------------------------------------------------------------------------------------ matrix-state recurrence
 // Per head a state S [D, D] (key channel i, value channel j):  o_t[j] = sum_i r_t[i] (S[i][j] + u[i] k_t[i] v_t[j]),
 // then S[i][j] <- w_t[i] S[i][j] + k_t[i] v_t[j], with w_t = exp(-exp(wraw_t + w0)).  A CTA owns WKV_J value
-// channels of one head; thread (part, j) keeps WKV_CH rows of column j in registers.  Tokens are staged WKV_TB at a
+// channels of one head; thread (part, j) keeps CH rows of column j in registers.  Tokens are staged TB at a
 // time; the parts' partial outputs meet in shared memory after each batch, summed in part order, so the arithmetic of
 // a token does not depend on how the sequence was cut into launches.
-constexpr int WKV_J = 32;   // template: TB tokens per staged batch (fewer when a wide head would not fit), CH state rows per thread
+// Bound: issue slots of one warp per scheduler (a token is 32 FMA-pipe instructions and 7 reads per thread).  16 columns per
+// CTA: 32 columns left half of the SMs without work at 32 heads of 64; the decays of long steps come from a launch of their
+// own, since every column tile of a head needs them (two expf each, a quarter of the instructions).
+constexpr int WKV_J = 16;   // template: TB tokens per staged batch (fewer when a wide head would not fit), CH state rows per thread
 
 __device__ __forceinline__ void cp_async4(float* dst, const float* src) {
     const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d), "l"(src));
 }
+__device__ __forceinline__ void cp_async16(float* dst, const float* src) {
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(src));
+}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
+
+__device__ __forceinline__ float wkv_decay(float raw, float w0) { return expf(-expf(raw + w0)); }
+
+// The decays of all tokens, for steps long enough that it pays to form them once.
+__global__ void __launch_bounds__(256) wkv_decay_kernel(const float* __restrict__ wraw, const float* __restrict__ w0, float* __restrict__ w, int T, int HD) {
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= HD) return;
+    const float b = w0[c];
+#pragma unroll 4
+    for (int t = blockIdx.y; t < T; t += gridDim.y) w[(size_t)t * HD + c] = wkv_decay(wraw[(size_t)t * HD + c], b);
+}
 
 // Shared memory: two buffers of [r | k | w | v] for WKV_TB tokens (the next batch is copied in asynchronously while
 // this one is computed; rows are padded to a multiple of 4 floats so that a thread reads its 16 key channels with
@@ -396,27 +414,40 @@ __global__ void __launch_bounds__(512) wkv_kernel(const CcSeqWkv a) {
         st[c] = in ? S[(size_t)(i0 + c) * D + j] : 0.f;
         u[c] = i0 + c < D ? a.u[(size_t)h * D + i0 + c] : 0.f;
     }
-    // staging layout: with more threads than channels, thread = (token lane t0, channel ich)
-    const int tstep = nth > D ? nth / D : 1, istep = nth > D ? D : nth;
-    int t0 = nth > D ? tid / D : 0;
-    const int ich = nth > D ? tid - t0 * D : tid;
+    // staging layout: 16 bytes per copy where the rows allow it; thread = (token lane t0, column ich of the copies)
+    const bool vec = D % 4 == 0 && (((uintptr_t)a.r | (uintptr_t)a.k | (uintptr_t)a.v | (uintptr_t)a.wraw) & 15) == 0;
+    const int cols = vec ? D / 4 : D, unit = vec ? 4 : 1;
+    const int tstep = nth > cols ? nth / cols : 1, istep = nth > cols ? cols : nth;
+    int t0 = nth > cols ? tid / cols : 0;
+    const int ich = nth > cols ? tid - t0 * cols : tid;
     if (t0 >= tstep) t0 = 1 << 20;      // threads beyond the last whole token lane do not stage
     for (int idx = tid; idx < 2 * buf_floats; idx += nth) sm[idx] = 0.f;    // padding channels stay zero
     __syncthreads();
     auto fetch = [&](int tb, float* buf) {
         const int nt = min(TB, a.T - tb);
-        // thread -> (token t0 + n * tstep, channel i): every thread copies, with one division per batch
+        // thread -> (token t0 + n * tstep, column): every thread copies, with one division per launch
         for (int t = t0; t < nt; t += tstep) {
             const size_t row = (size_t)(tb + t) * HD + (size_t)h * D;
-            for (int i = ich; i < D; i += istep) {
-                cp_async4(buf + t * Dp + i, a.r + row + i);
-                cp_async4(buf + TB * Dp + t * Dp + i, a.k + row + i);
-                cp_async4(buf + 2 * TB * Dp + t * Dp + i, a.wraw + row + i);
+            for (int i = ich * unit; i < D; i += istep * unit) {
+                float* d = buf + t * Dp + i;
+                if (vec) {
+                    cp_async16(d, a.r + row + i);
+                    cp_async16(d + TB * Dp, a.k + row + i);
+                    cp_async16(d + 2 * TB * Dp, a.wraw + row + i);
+                } else {
+                    cp_async4(d, a.r + row + i);
+                    cp_async4(d + TB * Dp, a.k + row + i);
+                    cp_async4(d + 2 * TB * Dp, a.wraw + row + i);
+                }
             }
         }
-        for (int idx = tid; idx < nt * WKV_J; idx += nth) {
+        for (int idx = tid * unit; idx < nt * WKV_J; idx += nth * unit) {
             const int t = idx / WKV_J, c = idx - t * WKV_J;
-            if (j0 + c < D) cp_async4(buf + 3 * TB * Dp + idx, a.v + (size_t)(tb + t) * HD + (size_t)h * D + j0 + c);
+            if (j0 + c >= D) continue;
+            float* d = buf + 3 * TB * Dp + idx;
+            const float* s = a.v + (size_t)(tb + t) * HD + (size_t)h * D + j0 + c;
+            if (vec) cp_async16(d, s);
+            else cp_async4(d, s);
         }
         cp_async_commit();
     };
@@ -429,11 +460,13 @@ __global__ void __launch_bounds__(512) wkv_kernel(const CcSeqWkv a) {
         else cp_async_wait<0>();
         __syncthreads();
         float* ws = buf + 2 * TB * Dp;
-        for (int i = ich; i < D; i += istep) {      // decay from its raw form, in place
-            const float w0 = a.w0[(size_t)h * D + i];
-            for (int t = t0; t < nt; t += tstep) ws[t * Dp + i] = expf(-expf(ws[t * Dp + i] + w0));
+        if (!a.decayed) {
+            for (int idx = tid; idx < nt * D; idx += nth) {      // decay from its raw form, in place
+                const int t = idx / D, i = idx - t * D;
+                ws[t * Dp + i] = wkv_decay(ws[t * Dp + i], a.w0[(size_t)h * D + i]);
+            }
+            __syncthreads();
         }
-        __syncthreads();
         const float* __restrict__ vs = buf + 3 * TB * Dp;
         const float* __restrict__ rb = buf + i0;
         const float* __restrict__ kb = buf + TB * Dp + i0;
@@ -1205,7 +1238,7 @@ static int launch_wkv(const CcSeqWkv* a, cudaStream_t st) {
     return cuda_check("wkv_kernel");
 }
 
-// 8 state rows per thread up to 128-wide heads (at most 512 threads), 16 above; the token batch shrinks until two
+// 8 state rows per thread up to 128-wide heads (at most 256 threads), 16 above; the token batch shrinks until two
 // staging buffers and the partial outputs fit in 160 KB.
 template <int CH>
 static int dispatch_wkv(const CcSeqWkv* a, cudaStream_t st) {
@@ -1363,6 +1396,13 @@ int cc_seq_wkv(const CcSeqWkv* a, void* stream) {
     if (a->D > 256) return fail(CC_SEQ_ERR_UNSUPPORTED_SHAPE, "wkv: head size above 256");
     cudaStream_t st = (cudaStream_t)stream;
     return a->D <= 128 ? dispatch_wkv<8>(a, st) : dispatch_wkv<16>(a, st);
+}
+
+int cc_seq_wkv_decay(const float* wraw, const float* w0, float* w, int32_t T, int32_t HD, void* stream) {
+    if (!wraw || !w0 || !w || T < 1 || HD < 1) return fail(CC_SEQ_ERR_INVALID_ARG, "wkv_decay: bad argument");
+    const int cols = (HD + 255) / 256, rows = (148 * 8 + cols - 1) / cols;
+    wkv_decay_kernel<<<dim3(cols, T < rows ? T : rows), 256, 0, (cudaStream_t)stream>>>(wraw, w0, w, T, HD);
+    return cuda_check("wkv_decay_kernel");
 }
 
 int cc_seq_head_norm_gate(const float* o, const float* graw, int64_t ldg, const float* nw, void* out, int32_t out_dtype,

@@ -317,7 +317,16 @@ def wkv(r, k, v, wraw, w0, u, state, o, H, D):
     a.r, a.k, a.v, a.wraw, a.w0, a.u, a.state, a.o = _p(r), _p(k), _p(v), _p(wraw), _p(w0), _p(u), _p(state), _p(o)
     a.T, a.H, a.D = r.shape[0], int(H), int(D)
     assert r.shape[1] == H * D and state.numel() == H * D * D
+    if a.T >= WKV_DECAY_FROM:
+        # long steps: the decays in a launch of their own, spread over the GPU, instead of once per column tile inside the
+        # recurrence; same arithmetic, same bits
+        decays = torch.empty(a.T, H * D, dtype=torch.float32, device=o.device)
+        _lib.check_seq(_lib.load_seq().cc_seq_wkv_decay(_p(wraw), _p(w0), _p(decays), a.T, H * D, _stream()), "cc_seq_wkv_decay")
+        a.wraw, a.decayed = _p(decays), 1
     _lib.check_seq(_lib.load_seq().cc_seq_wkv(C.byref(a), _stream()), "cc_seq_wkv")
+
+
+WKV_DECAY_FROM = 64
 
 
 def head_norm_gate(o, graw, nw, out, H, D, eps):

@@ -21,7 +21,7 @@
 extern "C" {
 #endif
 
-#define CC_SEQ_ABI_VERSION 7
+#define CC_SEQ_ABI_VERSION 8
 
 #define CC_SEQ_OK                     0
 #define CC_SEQ_ERR_INVALID_ARG       -1
@@ -324,15 +324,18 @@ int cc_seq_head_gemv(const void* W, int32_t w_dtype, const void* x, int32_t x_dt
  * r, k, v and the decay w_t = exp(-exp(wraw_t + w0)):
  *   o_t[j]  = sum_i r_t[i] * (S[i][j] + u[i] * k_t[i] * v_t[j])
  *   S[i][j] = w_t[i] * S[i][j] + k_t[i] * v_t[j]
- * r, k, v, wraw, o: fp32 [T, H * D] contiguous; w0, u: [H * D]; state [H, D, D] is read and written.
+ * r, k, v, wraw, o: fp32 [T, H * D] contiguous; w0, u: [H * D]; state [H, D, D] is read and written.  decayed != 0: wraw
+ * holds the decays w_t themselves, as cc_seq_wkv_decay writes them (same bits; it pays for steps of many tokens).
  */
 typedef struct CcSeqWkv {
     const float* r;  const float* k;  const float* v;  const float* wraw;
     const float* w0;  const float* u;
     float* state;  float* o;
-    int32_t T, H, D;
+    int32_t T, H, D, decayed;
 } CcSeqWkv;
 int cc_seq_wkv(const CcSeqWkv* a, void* stream);
+/* w = exp(-exp(wraw + w0)), fp32 [T, HD] */
+int cc_seq_wkv_decay(const float* wraw, const float* w0, float* w, int32_t T, int32_t HD, void* stream);
 
 /* out[t, h, :] = o[t, h, :] / sqrt(mean(o[t, h, :]^2) + eps) * nw[h, :] * silu(graw[t, h, :])   (graw fp32 [T, ldg]) */
 int cc_seq_head_norm_gate(const float* o, const float* graw, int64_t ldg, const float* nw, void* out, int32_t out_dtype,

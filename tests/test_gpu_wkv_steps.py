@@ -1,0 +1,43 @@
+"""The matrix-state recurrence gives the same bits however a sequence is cut: below and above the length from which the decays
+come from a launch of their own, across staged batches of 32 tokens, with head sizes that are not whole column tiles or
+16-byte vectors."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("H, D", [(1, 8), (2, 16), (3, 33), (2, 64), (1, 72), (2, 128), (1, 200)])
+def test_any_cut_of_a_sequence_gives_the_same_bits(H, D):
+    from cold_compress_b200 import seq_ops
+    T = 2 * seq_ops.WKV_DECAY_FROM + 37
+    gen = torch.Generator(device="cuda").manual_seed(D)
+    randn = lambda *s: torch.randn(*s, device="cuda", generator=gen)  # noqa: E731
+    r, k, v, wraw = (randn(T, H * D) for _ in range(4))
+    w0, u = randn(H * D) - 1.5, 0.5 * randn(H * D)
+
+    def run(portions):
+        state, out, at = torch.zeros(H, D, D, device="cuda"), [], 0
+        for m in portions:
+            o = torch.empty(m, H * D, device="cuda")
+            seq_ops.wkv(*(t[at:at + m].contiguous() for t in (r, k, v, wraw)), w0, u, state, o, H, D)
+            out.append(o)
+            at += m
+        assert at == T
+        return torch.cat(out), state
+
+    whole, state = run((T,))
+    n = seq_ops.WKV_DECAY_FROM
+    for portions in ((1, n - 1, n, T - 2 * n), (n + 1, 31, T - n - 32), (33,) * (T // 33) + (T % 33,) * (T % 33 > 0)):
+        got, s = run(portions)
+        assert torch.equal(got, whole) and torch.equal(s, state)
+    w = torch.exp(-torch.exp(wraw.double() + w0.double())).view(T, H, D, 1)
+    S, want = torch.zeros(H, D, D, dtype=torch.float64, device="cuda"), []
+    rd, kd, vd, ud = (t.double().view(-1, H, D) for t in (r, k, v, u))
+    for t in range(T):
+        kv = kd[t].unsqueeze(-1) * vd[t].unsqueeze(-2)
+        want.append(torch.einsum("hij,hi->hj", S + ud[0].unsqueeze(-1) * kv, rd[t]).reshape(-1))
+        S = w[t] * S + kv
+    want = torch.stack(want)
+    # D products summed in fp32 and a state that forgets: a few roundings of the sum's size
+    assert ((whole.double() - want).norm() / want.norm()).item() <= 4 * 2.0 ** -23 and ((state.double() - S).norm() / S.norm()).item() <= 4 * 2.0 ** -23
