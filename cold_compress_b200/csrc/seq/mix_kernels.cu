@@ -364,9 +364,10 @@ __global__ void __launch_bounds__(256) head_gemv_kernel(const WT* W, const XT* x
 // channels of one head; thread (part, j) keeps CH rows of column j in registers.  Tokens are staged TB at a
 // time; the parts' partial outputs meet in shared memory after each batch, summed in part order, so the arithmetic of
 // a token does not depend on how the sequence was cut into launches.
-// Bound: issue slots of one warp per scheduler (a token is 32 FMA-pipe instructions and 7 reads per thread).  16 columns per
-// CTA: 32 columns left half of the SMs without work at 32 heads of 64; the decays of long steps come from a launch of their
-// own, since every column tile of a head needs them (two expf each, a quarter of the instructions).
+// Bound: the latencies of one warp per scheduler.  16 columns per CTA: 32 columns left half of the SMs without work at 32
+// heads of 64; the decays of long steps come from a launch of their own, since every column tile of a head needs them (two
+// expf each); the next token's operands are read while one is computed, and two rows share an instruction.  4096 tokens, 32
+// heads of 64: 808 us -> 592 (columns, decays, 16-byte staging) -> 408; 4 rows per thread and twice the warps: 406, other bits.
 constexpr int WKV_J = 16;   // template: TB tokens per staged batch (fewer when a wide head would not fit), CH state rows per thread
 
 __device__ __forceinline__ void cp_async4(float* dst, const float* src) {
@@ -380,6 +381,25 @@ __device__ __forceinline__ void cp_async16(float* dst, const float* src) {
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
+
+// pairs of fp32 values: one instruction for two operations, each rounded as the scalar one
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pair(float a, float b) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void unpair(f32x2 r, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(r)); }
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
 
 __device__ __forceinline__ float wkv_decay(float raw, float w0) { return expf(-expf(raw + w0)); }
 
@@ -396,7 +416,7 @@ __global__ void __launch_bounds__(256) wkv_decay_kernel(const float* __restrict_
 // this one is computed; rows are padded to a multiple of 4 floats so that a thread reads its 16 key channels with
 // 16-byte loads), then the parts' partial outputs.
 template <int TB, int CH>
-__global__ void __launch_bounds__(512) wkv_kernel(const CcSeqWkv a) {
+__global__ void __launch_bounds__(256) wkv_kernel(const CcSeqWkv a) {
     extern __shared__ float4 smw4[];
     float* sm = reinterpret_cast<float*>(smw4);
     const int D = a.D, P = (D + CH - 1) / CH, Dp = P * CH;
@@ -407,12 +427,20 @@ __global__ void __launch_bounds__(512) wkv_kernel(const CcSeqWkv a) {
     const int i0 = p * CH;
     const size_t HD = (size_t)a.H * D;
     float* S = a.state + (size_t)h * D * D;
-    float st[CH], u[CH];
+    f32x2 st2[CH / 2], u2[CH / 2];
+    {
+        float st[CH], u[CH];
 #pragma unroll
-    for (int c = 0; c < CH; ++c) {
-        const bool in = i0 + c < D && j < D;
-        st[c] = in ? S[(size_t)(i0 + c) * D + j] : 0.f;
-        u[c] = i0 + c < D ? a.u[(size_t)h * D + i0 + c] : 0.f;
+        for (int c = 0; c < CH; ++c) {
+            const bool in = i0 + c < D && j < D;
+            st[c] = in ? S[(size_t)(i0 + c) * D + j] : 0.f;
+            u[c] = i0 + c < D ? a.u[(size_t)h * D + i0 + c] : 0.f;
+        }
+#pragma unroll
+        for (int c = 0; c < CH / 2; ++c) {
+            st2[c] = pair(st[2 * c], st[2 * c + 1]);
+            u2[c] = pair(u[2 * c], u[2 * c + 1]);
+        }
     }
     // staging layout: 16 bytes per copy where the rows allow it; thread = (token lane t0, column ich of the copies)
     const bool vec = D % 4 == 0 && (((uintptr_t)a.r | (uintptr_t)a.k | (uintptr_t)a.v | (uintptr_t)a.wraw) & 15) == 0;
@@ -471,26 +499,41 @@ __global__ void __launch_bounds__(512) wkv_kernel(const CcSeqWkv a) {
         const float* __restrict__ rb = buf + i0;
         const float* __restrict__ kb = buf + TB * Dp + i0;
         const float* __restrict__ wb = ws + i0;
-#pragma unroll 4
-        for (int t = 0; t < nt; ++t) {
-            const float v = vs[t * WKV_J + jl];
-            const float4* r4 = reinterpret_cast<const float4*>(rb + t * Dp);
-            const float4* k4 = reinterpret_cast<const float4*>(kb + t * Dp);
-            const float4* w4 = reinterpret_cast<const float4*>(wb + t * Dp);
-            float acc[4] = {0.f, 0.f, 0.f, 0.f};
+        // the next token's operands are read while this one is computed; pairs of rows per instruction
+        float4 rv[CH / 4], kv4[CH / 4], wv[CH / 4];
+        float v;
+        auto read = [&](int t) {
 #pragma unroll
             for (int c4 = 0; c4 < CH / 4; ++c4) {
-                const float4 rv = r4[c4], kv4 = k4[c4], wv = w4[c4];
-                const float rr[4] = {rv.x, rv.y, rv.z, rv.w}, kk[4] = {kv4.x, kv4.y, kv4.z, kv4.w}, ww[4] = {wv.x, wv.y, wv.z, wv.w};
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const int c = 4 * c4 + e;
-                    const float kv = kk[e] * v;
-                    acc[e] = fmaf(rr[e], fmaf(u[c], kv, st[c]), acc[e]);
-                    st[c] = fmaf(ww[e], st[c], kv);
-                }
+                rv[c4] = reinterpret_cast<const float4*>(rb + t * Dp)[c4];
+                kv4[c4] = reinterpret_cast<const float4*>(kb + t * Dp)[c4];
+                wv[c4] = reinterpret_cast<const float4*>(wb + t * Dp)[c4];
             }
-            part[(t * P + p) * WKV_J + jl] = (acc[0] + acc[1]) + (acc[2] + acc[3]);
+            v = vs[t * WKV_J + jl];
+        };
+        read(0);
+#pragma unroll 4
+        for (int t = 0; t < nt; ++t) {
+            f32x2 r2[CH / 2], k2[CH / 2], w2[CH / 2];
+#pragma unroll
+            for (int c4 = 0; c4 < CH / 4; ++c4) {
+                r2[2 * c4] = pair(rv[c4].x, rv[c4].y); r2[2 * c4 + 1] = pair(rv[c4].z, rv[c4].w);
+                k2[2 * c4] = pair(kv4[c4].x, kv4[c4].y); k2[2 * c4 + 1] = pair(kv4[c4].z, kv4[c4].w);
+                w2[2 * c4] = pair(wv[c4].x, wv[c4].y); w2[2 * c4 + 1] = pair(wv[c4].z, wv[c4].w);
+            }
+            const f32x2 v2 = pair(v, v);
+            read(min(t + 1, nt - 1));
+            f32x2 acc[2] = {0ull, 0ull};
+#pragma unroll
+            for (int c = 0; c < CH / 2; ++c) {
+                const f32x2 kv = mul2(k2[c], v2);
+                acc[c & 1] = fma2(r2[c], fma2(u2[c], kv, st2[c]), acc[c & 1]);
+                st2[c] = fma2(w2[c], st2[c], kv);
+            }
+            float a0, a1, a2, a3;
+            unpair(acc[0], a0, a1);
+            unpair(acc[1], a2, a3);
+            part[(t * P + p) * WKV_J + jl] = (a0 + a1) + (a2 + a3);
         }
         __syncthreads();
         for (int idx = tid; idx < nt * WKV_J; idx += nth) {
@@ -502,8 +545,12 @@ __global__ void __launch_bounds__(512) wkv_kernel(const CcSeqWkv a) {
         }
     }
 #pragma unroll
-    for (int c = 0; c < CH; ++c)
-        if (i0 + c < D && j < D) S[(size_t)(i0 + c) * D + j] = st[c];
+    for (int c = 0; c < CH; c += 2) {
+        float s0, s1;
+        unpair(st2[c / 2], s0, s1);
+        if (i0 + c < D && j < D) S[(size_t)(i0 + c) * D + j] = s0;
+        if (i0 + c + 1 < D && j < D) S[(size_t)(i0 + c + 1) * D + j] = s1;
+    }
 }
 
 // out[t, h, :] = o[t, h, :] / rms(o[t, h, :]) * nw[h, :] * silu(graw[t, h, :]); a warp per (token, head).
