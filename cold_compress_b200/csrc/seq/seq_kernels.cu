@@ -705,14 +705,16 @@ __global__ void __launch_bounds__(DEC_THREADS) attn_decode_kernel(const CcSeqAtt
 }
 
 // ---- the same for rows of whole 16-byte vectors and up to 8 query heads per key/value head
-// A run of 64-key tiles per CTA; the key and value rows of a tile are all requested at once (cp.async, the next tile under
+// A run of 128-key tiles per CTA; the key and value rows of a tile are all requested at once (cp.async, the next tile under
 // this one) before anything is known about their slots, which are checked meanwhile.  Scores: eight lanes per key, four keys
 // at a time, the query rows read from shared memory once for the four.  Values: a thread owns a 16-byte column group and
-// every nkg-th key.  Partials and their combination as above, 16 bytes a load and 16 loads in flight.
-// Bound: the chain of dependent round trips (lookup and rows, partials, counter, combination), not the rows' bandwidth;
-// the kernel above walked every row by one thread and read the values after the scores (8 layers, 32 / 8 heads of 128, 4096
-// positions, in a graph: 32 us a layer).
-constexpr int VT = 64, VD_THREADS = 128, VD_MAX_SPLITS = 64, VD_RMAX = 8;
+// every nkg-th key.  Two fp32 operations per instruction in both.  Partials and their combination as above, 16 bytes a load
+// and 16 loads in flight.
+// Bound: issue slots and the chain of dependent round trips (lookup and rows, partials, counter, combination), not the rows'
+// bandwidth.  8 layers, 32 / 8 heads of 128, 4096 positions in a graph: 32 us a layer on the kernel above (a thread walks a
+// row, values are read after the scores), 27 with rows requested at once, 18 with 256 threads, 128-key tiles, paired operations and ring
+// places without a division per row.
+constexpr int VT = 128, VD_THREADS = 256, VD_MAX_SPLITS = 64, VD_RMAX = 8;
 
 __host__ __device__ inline int vd_splits(int L, int reach, int G) {     // runs per head: two CTAs per SM over the heads
     const long long maxkeys = reach > 0 ? (reach < L + 1 ? reach : L + 1) : (long long)L + 1;
@@ -728,10 +730,34 @@ __device__ __forceinline__ void cp_async16_or_zero(void* dst, const void* src, b
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(have ? 16 : 0) : "memory");
 }
 
+// pairs of fp32 values: one instruction for two operations, each rounded as the scalar one
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pair(float a, float b) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void unpair(f32x2 r, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(r)); }
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+// the elements of a 16-byte vector as pairs
+__device__ __forceinline__ void as_pairs(const uint4& u, f32x2 (&v)[2], const float*) {
+    v[0] = pair(__uint_as_float(u.x), __uint_as_float(u.y));
+    v[1] = pair(__uint_as_float(u.z), __uint_as_float(u.w));
+}
+__device__ __forceinline__ void as_pairs(const uint4& u, f32x2 (&v)[4], const __nv_bfloat16*) {
+    const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v[i] = pair(__uint_as_float(w[i] << 16), __uint_as_float(w[i] & 0xffff0000u));
+}
+
 template <typename CT, typename YT, int RMAX>
-__global__ void __launch_bounds__(VD_THREADS) attn_decode_rows_kernel(const CcSeqAttn a, int buffers) {
+__global__ void __launch_bounds__(VD_THREADS, RMAX <= 4 ? 2 : 1) attn_decode_rows_kernel(const CcSeqAttn a, int buffers) {
     extern __shared__ float4 smd4[];
-    constexpr int VEC = 16 / (int)sizeof(CT);
+    constexpr int VEC = 16 / (int)sizeof(CT), VP = VEC / 2, WARPS = VD_THREADS / 32, KEYS = VT / WARPS, KI = KEYS / 4;
     const int R = a.H / a.G, Dk = a.Dk, Dv = a.Dv, kc16 = Dk / VEC, vc16 = Dv / VEC;
     const int k_row = kc16 + 1, k_tile = VT * k_row, v_tile = VT * vc16;         // 16-byte units; one of padding per key row
     uint4* const ks = reinterpret_cast<uint4*>(smd4);                            // [buffers][VT][k_row]
@@ -751,44 +777,57 @@ __global__ void __launch_bounds__(VD_THREADS) attn_decode_rows_kernel(const CcSe
     const int n_tiles = (n + VT - 1) / VT, NS = vd_splits(a.L, attn_reach(a), a.G);
     const int tiles_per = (n_tiles + NS - 1) / NS, nsplit = (n_tiles + tiles_per - 1) / tiles_per;
     if (sp >= nsplit) return;
-    const CT* kc = (const CT*)a.k_cache + (size_t)g * a.L * Dk;
-    const CT* vc = (const CT*)a.v_cache + (size_t)g * a.L * Dv;
-    const CT* kn = (const CT*)a.k_new + (size_t)g * Dk;
-    const CT* vn = (const CT*)a.v_new + (size_t)g * Dv;
-    const int tile0 = sp * tiles_per, tile_end = min(n_tiles, tile0 + tiles_per);
+    const int tile0 = sp * tiles_per, tile_end = min(n_tiles, tile0 + tiles_per), ring = a.L - a.keep_first;
+    // copies: thread = column c of rows row, row + step, ...
+    const int k_step = VD_THREADS / kc16, k_first = tid / kc16, k_col = tid - k_first * kc16;
+    const int v_step = VD_THREADS / vc16, v_first = tid / vc16, v_col = tid - v_first * vc16;
+    const CT* const kc = (const CT*)a.k_cache + (size_t)g * a.L * Dk + k_col * VEC;
+    const CT* const vc = (const CT*)a.v_cache + (size_t)g * a.L * Dv + v_col * VEC;
+    const CT* const kn = (const CT*)a.k_new + (size_t)g * Dk + k_col * VEC;
+    const CT* const vn = (const CT*)a.v_new + (size_t)g * Dv + v_col * VEC;
 
     auto fetch = [&](int tile) {
         const int b = buffers > 1 ? (tile - tile0) & 1 : 0, u0 = tile * VT;
+        // beside the kept first positions a tile's slots are one or two runs of the ring (rings of at least a tile)
+        const int j0 = u0 < kx ? 0 : j_lo + (u0 - kx);
+        const bool plain = u0 >= kx && j0 >= a.keep_first && ring >= VT;
+        const int r0 = plain ? (j0 - a.keep_first) % ring : 0;
         auto position = [&](int row) { return u0 + row < kx ? u0 + row : j_lo + (u0 + row - kx); };
-        for (int row = tid / kc16; row < VT; row += VD_THREADS / kc16) {          // kc16 divides into whole rows below
-            const int c = tid % kc16, j = position(row);
-            if (tid >= VD_THREADS / kc16 * kc16) break;
-            const bool have = u0 + row < n;
-            const CT* src = j == p ? kn : kc + (size_t)slot_of(a, j) * Dk;
-            cp_async16_or_zero(ks + b * k_tile + row * k_row + c, have ? (const void*)(src + c * VEC) : (const void*)kn, have);
+        auto slot = [&](int row) {
+            if (!plain) return slot_of(a, position(row));
+            const int r = r0 + row;
+            return a.keep_first + (r >= ring ? r - ring : r);
+        };
+        const int rows = min(VT, n - u0), last = p - (u0 < kx ? 0 : j0);      // row of the token itself, in a tile beside the kept ones
+        if (k_first < k_step) {
+#pragma unroll 4
+            for (int row = k_first; row < VT; row += k_step) {
+                const bool have = row < rows, mine = plain ? row == last : position(row) == p;
+                cp_async16_or_zero(ks + b * k_tile + row * k_row + k_col, have && !mine ? kc + (size_t)slot(row) * Dk : kn, have);
+            }
         }
-        for (int row = tid / vc16; row < VT; row += VD_THREADS / vc16) {
-            const int c = tid % vc16, j = position(row);
-            if (tid >= VD_THREADS / vc16 * vc16) break;
-            const bool have = u0 + row < n;
-            const CT* src = j == p ? vn : vc + (size_t)slot_of(a, j) * Dv;
-            cp_async16_or_zero(vs + b * v_tile + row * vc16 + c, have ? (const void*)(src + c * VEC) : (const void*)vn, have);
+        if (v_first < v_step) {
+#pragma unroll 4
+            for (int row = v_first; row < VT; row += v_step) {
+                const bool have = row < rows, mine = plain ? row == last : position(row) == p;
+                cp_async16_or_zero(vs + b * v_tile + row * vc16 + v_col, have && !mine ? vc + (size_t)slot(row) * Dv : vn, have);
+            }
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
         if (tid < VT) {
             const int j = position(tid);
-            s_live[(tile - tile0) & 1][tid] = u0 + tid < n && (j == p || a.pos[slot_of(a, j)] == j);
+            s_live[(tile - tile0) & 1][tid] = tid < rows && (j == p || a.pos[slot(tid)] == j);
         }
     };
     fetch(tile0);
     for (int i = tid; i < R * Dk; i += VD_THREADS) qs[i] = a.q[(size_t)g * R * Dk + i];
     if (tid < RMAX) { s_M[tid] = -INFINITY; s_L[tid] = 0.f; }
-    const int nkg = VD_THREADS / vc16, kg = tid / vc16, cg = tid - kg * vc16;     // value phase: key groups x column groups
-    float acc[RMAX][VEC];
+    const int nkg = v_step, kg = v_first, cg = v_col;     // value phase: key groups x column groups
+    f32x2 acc[RMAX][VP];
 #pragma unroll
     for (int r = 0; r < RMAX; ++r)
 #pragma unroll
-        for (int x = 0; x < VEC; ++x) acc[r][x] = 0.f;
+        for (int x = 0; x < VP; ++x) acc[r][x] = 0ull;
 
     for (int tile = tile0; tile < tile_end; ++tile) {
         const int b = buffers > 1 ? (tile - tile0) & 1 : 0, u0 = tile * VT;
@@ -800,58 +839,60 @@ __global__ void __launch_bounds__(VD_THREADS) attn_decode_rows_kernel(const CcSe
             asm volatile("cp.async.wait_group 0;" ::: "memory");
         }
         __syncthreads();
-        {   // scores: keys 16 warp + 4 i + lane / 8
-            const int part = lane & 7, k0 = 16 * warp + (lane >> 3);
-            float sc[4][RMAX];
+        {   // scores: keys KEYS warp + 4 i + lane / 8
+            const int part = lane & 7, k0 = KEYS * warp + (lane >> 3);
+            f32x2 sc[KI][RMAX];
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
+            for (int i = 0; i < KI; ++i)
 #pragma unroll
-                for (int r = 0; r < RMAX; ++r) sc[i][r] = 0.f;
+                for (int r = 0; r < RMAX; ++r) sc[i][r] = 0ull;
             for (int c = part; c < kc16; c += 8) {
-                float kf[4][VEC];
+                f32x2 kf[KI][VP];
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const uint4 u = ks[b * k_tile + (k0 + 4 * i) * k_row + c];
-                    const CT* e = reinterpret_cast<const CT*>(&u);
-#pragma unroll
-                    for (int x = 0; x < VEC; ++x) kf[i][x] = ldf(e, x);
-                }
+                for (int i = 0; i < KI; ++i) as_pairs(ks[b * k_tile + (k0 + 4 * i) * k_row + c], kf[i], (const CT*)nullptr);
 #pragma unroll
                 for (int r = 0; r < RMAX; ++r)
                     if (r < R) {
 #pragma unroll
                         for (int x4 = 0; x4 < VEC / 4; ++x4) {
                             const float4 qv = *reinterpret_cast<const float4*>(qs + r * Dk + c * VEC + 4 * x4);
+                            const f32x2 q0 = pair(qv.x, qv.y), q1 = pair(qv.z, qv.w);
 #pragma unroll
-                            for (int i = 0; i < 4; ++i) {
-                                sc[i][r] = fmaf(qv.x, kf[i][4 * x4 + 0], sc[i][r]);
-                                sc[i][r] = fmaf(qv.y, kf[i][4 * x4 + 1], sc[i][r]);
-                                sc[i][r] = fmaf(qv.z, kf[i][4 * x4 + 2], sc[i][r]);
-                                sc[i][r] = fmaf(qv.w, kf[i][4 * x4 + 3], sc[i][r]);
-                            }
+                            for (int i = 0; i < KI; ++i) sc[i][r] = fma2(q1, kf[i][2 * x4 + 1], fma2(q0, kf[i][2 * x4], sc[i][r]));
                         }
                     }
             }
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
+            for (int i = 0; i < KI; ++i) {
                 const int k = k0 + 4 * i, j = u0 + k < kx ? u0 + k : j_lo + (u0 + k - kx);
                 const bool ok = live[k] != 0;
+                float mine = 0.f;      // lane `part` of the key closes query head `part`
 #pragma unroll
                 for (int r = 0; r < RMAX; ++r) {
+                    if (r >= R) break;
+                    float s0, s1;
+                    unpair(sc[i][r], s0, s1);
+                    s0 += s1;
 #pragma unroll
-                    for (int o = 4; o > 0; o >>= 1) sc[i][r] += __shfl_xor_sync(0xffffffffu, sc[i][r], o);
-                    if (r < R && part == (r & 7)) Ps[r * VT + k] = ok ? shape_score(a, sc[i][r] * a.scale, g * R + r, p - j) : -INFINITY;
+                    for (int o = 4; o > 0; o >>= 1) s0 += __shfl_xor_sync(0xffffffffu, s0, o);
+                    mine = part == r ? s0 : mine;
                 }
+                if (part < R) Ps[part * VT + k] = ok ? shape_score(a, mine * a.scale, g * R + part, p - j) : -INFINITY;
             }
         }
         __syncthreads();
-        for (int r = warp; r < R; r += VD_THREADS / 32) {
-            const float s0 = Ps[r * VT + lane], s1 = Ps[r * VT + lane + 32];
-            const float m_old = s_M[r], m_new = fmaxf(m_old, warp_max(fmaxf(s0, s1)));
-            const float p0 = s0 == -INFINITY ? 0.f : expf(s0 - m_new), p1 = s1 == -INFINITY ? 0.f : expf(s1 - m_new);
-            Ps[r * VT + lane] = p0;
-            Ps[r * VT + lane + 32] = p1;
-            const float sum = warp_sum(p0 + p1);
+        for (int r = warp; r < R; r += WARPS) {
+            float sv[VT / 32], mx = -INFINITY, sum = 0.f;
+#pragma unroll
+            for (int q = 0; q < VT / 32; ++q) mx = fmaxf(mx, sv[q] = Ps[r * VT + lane + 32 * q]);
+            const float m_old = s_M[r], m_new = fmaxf(m_old, warp_max(mx));
+#pragma unroll
+            for (int q = 0; q < VT / 32; ++q) {
+                const float w = sv[q] == -INFINITY ? 0.f : expf(sv[q] - m_new);
+                Ps[r * VT + lane + 32 * q] = w;
+                sum += w;
+            }
+            sum = warp_sum(sum);
             if (lane == 0) {
                 const float corr = m_old == -INFINITY ? 0.f : expf(m_old - m_new);
                 s_corr[r] = corr;
@@ -861,27 +902,26 @@ __global__ void __launch_bounds__(VD_THREADS) attn_decode_rows_kernel(const CcSe
         }
         __syncthreads();
         if (kg < nkg) {
+            if (tile > tile0) {
 #pragma unroll
-            for (int r = 0; r < RMAX; ++r)
-                if (r < R) {
-                    const float cr = s_corr[r];
+                for (int r = 0; r < RMAX; ++r)
+                    if (r < R) {
+                        const float cr = s_corr[r];
 #pragma unroll
-                    for (int x = 0; x < VEC; ++x) acc[r][x] *= cr;
-                }
+                        for (int x = 0; x < VP; ++x) acc[r][x] = fma2(acc[r][x], pair(cr, cr), 0ull);
+                    }
+            }
 #pragma unroll 4
             for (int k = kg; k < VT; k += nkg) {
                 if (!live[k]) continue;
-                const uint4 u = vs[b * v_tile + k * vc16 + cg];
-                const CT* e = reinterpret_cast<const CT*>(&u);
-                float vf[VEC];
-#pragma unroll
-                for (int x = 0; x < VEC; ++x) vf[x] = ldf(e, x);
+                f32x2 vf[VP];
+                as_pairs(vs[b * v_tile + k * vc16 + cg], vf, (const CT*)nullptr);
 #pragma unroll
                 for (int r = 0; r < RMAX; ++r)
                     if (r < R) {
                         const float w = Ps[r * VT + k];
 #pragma unroll
-                        for (int x = 0; x < VEC; ++x) acc[r][x] = fmaf(w, vf[x], acc[r][x]);
+                        for (int x = 0; x < VP; ++x) acc[r][x] = fma2(pair(w, w), vf[x], acc[r][x]);
                     }
             }
         }
@@ -895,7 +935,11 @@ __global__ void __launch_bounds__(VD_THREADS) attn_decode_rows_kernel(const CcSe
         for (int r = 0; r < RMAX; ++r)
             if (r < R) {
 #pragma unroll
-                for (int x = 0; x < VEC; ++x) red[((size_t)kg * R + r) * Dv + cg * VEC + x] = acc[r][x];
+                for (int x = 0; x < VP; ++x) {
+                    float s0, s1;
+                    unpair(acc[r][x], s0, s1);
+                    *reinterpret_cast<float2*>(red + ((size_t)kg * R + r) * Dv + cg * VEC + 2 * x) = make_float2(s0, s1);
+                }
             }
     }
     __syncthreads();
@@ -935,8 +979,8 @@ __global__ void __launch_bounds__(VD_THREADS) attn_decode_rows_kernel(const CcSe
     if (!s_last) return;
     __threadfence();
     // the last CTA of the head: every other one has finished reading; combine in split order
-    float* const wgt = Ps;     // [R][VT] weights of the splits (at most VD_MAX_SPLITS == VT)
-    for (int r = warp; r < R; r += VD_THREADS / 32) {
+    float* const wgt = Ps;     // [R][VT] weights of the splits (at most VD_MAX_SPLITS < VT)
+    for (int r = warp; r < R; r += WARPS) {
         const float sk = sink_of(r);
         const float* pm = part_m + (size_t)g * NS * R + r;
         const float m0 = lane < nsplit ? __ldcg(pm + (size_t)lane * R) : -INFINITY, m1 = lane + 32 < nsplit ? __ldcg(pm + (size_t)(lane + 32) * R) : -INFINITY;
@@ -1218,9 +1262,9 @@ template <typename CT, typename YT, int RMAX>
 static int launch_decode_rows(const CcSeqAttn* a, cudaStream_t st) {
     const int NS = vd_splits(a->L, attn_reach(*a), a->G);
     const long long reach = attn_reach(*a) > 0 && attn_reach(*a) < a->L + 1 ? attn_reach(*a) : (long long)a->L + 1;
-    const int buffers = (reach + VT - 1) / VT > NS ? 2 : 1;      // a run can be longer than one tile
     const size_t row = sizeof(CT) * (size_t)(a->Dk + a->Dv) + 16;
-    size_t tiles = (size_t)buffers * VT * row;
+    const int buffers = (reach + VT - 1) / VT > NS && 2 * VT * row <= 200 * 1024 ? 2 : 1;      // a run can be longer than one tile
+    const size_t tiles = (size_t)buffers * VT * row;
     const int vc16 = a->Dv * (int)sizeof(CT) / 16;
     const size_t red = sizeof(float) * (size_t)(VD_THREADS / vc16) * (a->H / a->G) * a->Dv;
     const size_t smem = (tiles > red ? tiles : red) + sizeof(float) * RMAX * (size_t)(a->Dk + VT);
