@@ -131,6 +131,15 @@ __device__ __forceinline__ uint32_t cvt_bf16x2(float lo, float hi) {
 __device__ __forceinline__ float round_bf16(float x) {
     uint32_t d; asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(x), "f"(0.0f)); return __uint_as_float(d);
 }
+// pairs of fp32 values: one instruction for two operations, each rounded as the scalar one
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pair(float a, float b) { f32x2 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b)); return r; }
+__device__ __forceinline__ void unpair(f32x2 r, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(r)); }
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) { f32x2 r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) { f32x2 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
 __device__ __forceinline__ float bf16x2_lo(uint32_t d) { return __uint_as_float(d << 16); }
 __device__ __forceinline__ float bf16x2_hi(uint32_t d) { return __uint_as_float(d & 0xffff0000u); }
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
@@ -182,19 +191,21 @@ __device__ __forceinline__ void tile_stats(const uint8_t* sP_ptr, float (*s_comb
     const bool g_pow2 = (p.G & (p.G - 1)) == 0;
 #pragma unroll
     for (int ii = 0; ii < NI; ++ii) {
-        float sum[8];
-#pragma unroll
-        for (int c = 0; c < 8; ++c) sum[c] = 0.f;
+        f32x2 sum2[4] = {0ull, 0ull, 0ull, 0ull};
 #pragma unroll
         for (int kk = 0; kk < NK; ++kk) {
             const int k = ii + NI * kk;                                  // row = lane + 32 k (same swizzle phase)
             const int g = QB >= 32 ? kk : 2 * kk + (lane >> 4);          // QB = 16: rows l + 32 k hold heads 2k, 2k + 1
             const uint4 u = *reinterpret_cast<const uint4*>(base + k * 32 * 128);
             if (g < p.G) {
-                sum[0] += bf16x2_lo(u.x); sum[1] += bf16x2_hi(u.x); sum[2] += bf16x2_lo(u.y); sum[3] += bf16x2_hi(u.y);
-                sum[4] += bf16x2_lo(u.z); sum[5] += bf16x2_hi(u.z); sum[6] += bf16x2_lo(u.w); sum[7] += bf16x2_hi(u.w);
+                const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+                for (int c = 0; c < 4; ++c) sum2[c] = add2(sum2[c], pair(bf16x2_lo(w[c]), bf16x2_hi(w[c])));
             }
         }
+        float sum[8];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) unpair(sum2[c], sum[2 * c], sum[2 * c + 1]);
         if (QB < 32) {   // the other half of the heads sits 16 lanes away
 #pragma unroll
             for (int c = 0; c < 8; ++c) sum[c] += __shfl_xor_sync(0xffffffffu, sum[c], 16);
@@ -399,10 +410,15 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         tmem_ld32(tS + lane_base + sb * BNH + ch * 32, v0);
         if (gt == 0 && n + 2 < NT) issue_k((n + 2) % T, sb);   // K[sb] is free: its MMA has completed
         __syncwarp();
+        const f32x2 scale2 = pair(scale, scale);
 #pragma unroll
-        for (int c = 0; c < 32; ++c) {
-            const float x = __uint_as_float(v0[c]);
-            l[c] = NAIVE ? round_bf16(round_bf16(x) * scale) : x * scale;
+        for (int c = 0; c < 32; c += 2) {
+            float x = __uint_as_float(v0[c]), y = __uint_as_float(v0[c + 1]);
+            if (NAIVE) { x = round_bf16(x); y = round_bf16(y); }
+            unpair(mul2(pair(x, y), scale2), x, y);
+            if (NAIVE && D != 64) { x = round_bf16(x); y = round_bf16(y); }   // D = 64: the scale is 2^-3
+            l[c] = x;
+            l[c + 1] = y;
         }
         if (t * BN + grp * BNH + BNH - 1 > i0) {   // the block reaches past the diagonal for some row
             const int kbase = t * BN + grp * BNH + ch * 32;
@@ -412,21 +428,27 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         }
     };
 
+    const f32x2 log2e2 = pair(LOG2E, LOG2E);
+
     // ---- sweep 1: softmax statistics
     for (int n = 0; n < T; ++n) {
         float l[32];
         visit(n, n, l);
-        float tmax = l[0];
+        float tm[4] = {l[0], l[1], l[2], l[3]};
 #pragma unroll
-        for (int c = 1; c < 32; ++c) tmax = fmaxf(tmax, l[c]);
-        const float m_new = fmaxf(m_run, tmax);
+        for (int c = 4; c < 32; ++c) tm[c & 3] = fmaxf(tm[c & 3], l[c]);
+        const float m_new = fmaxf(m_run, fmaxf(fmaxf(tm[0], tm[1]), fmaxf(tm[2], tm[3])));
         if (m_new > -INFINITY) {
-            float a0 = 0.f, a1 = 0.f;
+            const f32x2 off = pair(-m_new * LOG2E, -m_new * LOG2E);
+            f32x2 a[2] = {0ull, 0ull};
 #pragma unroll
             for (int c = 0; c < 32; c += 2) {
-                a0 += ex2((l[c] - m_new) * LOG2E);
-                a1 += ex2((l[c + 1] - m_new) * LOG2E);
+                float x, y;
+                unpair(fma2(pair(l[c], l[c + 1]), log2e2, off), x, y);
+                a[(c >> 1) & 1] = add2(a[(c >> 1) & 1], pair(ex2(x), ex2(y)));
             }
+            float a0, a1;
+            unpair(add2(a[0], a[1]), a0, a1);
             s_run = s_run * ex2((m_run - m_new) * LOG2E) + (a0 + a1);
             m_run = m_new;
         }
@@ -449,15 +471,17 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     }
 
     // ---- sweep 2: probabilities, P V, pooled reductions
+    const f32x2 off2 = pair(-m_fin * LOG2E, -m_fin * LOG2E), inv2 = pair(inv_s, inv_s);
     for (int t = 0; t < T; ++t) {
         float l[32];
         visit(T + t, t, l);
         uint32_t pk[16];
 #pragma unroll
         for (int c = 0; c < 32; c += 2) {
-            const float p0 = ex2((l[c] - m_fin) * LOG2E) * inv_s;
-            const float p1 = ex2((l[c + 1] - m_fin) * LOG2E) * inv_s;
-            pk[c >> 1] = cvt_bf16x2(p0, p1);
+            float x, y;
+            unpair(fma2(pair(l[c], l[c + 1]), log2e2, off2), x, y);
+            unpair(mul2(pair(ex2(x), ex2(y)), inv2), x, y);
+            pk[c >> 1] = cvt_bf16x2(x, y);
         }
         if (t > 0) mbar_wait_u32(BAR_PV, (t - 1) & 1);   // P V of the previous block done: sP and V[(t-1)&1] are free
         group_sync(grp);                                  // the group finished reading the previous P block
