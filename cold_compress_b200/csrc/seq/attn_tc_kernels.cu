@@ -7,15 +7,16 @@
 // rounds, so an accumulator lives for one tile of 128 keys only; the sum over the tiles is an fp32 FMA in registers
 // that also applies the softmax's rescaling.
 //
-// Bound: tensor pipe, 2 x 24 MMAs of 128 x 128 x 16 per 128 x 128 scores at head size 128 (3072 cycles at the nominal
-// rate) beside ~14 instructions per score on the other pipes (about 1700 cycles when all four schedulers issue).  Layout
-// that follows: the query parts stay in shared memory (96 KB) and the weight parts go to tensor memory, over the scores
-// they came from, as the A operand -- through shared memory they would cost more bandwidth than the MMAs have.
+// Bound: tensor pipe and the shared memory it reads: 2 x 24 MMAs of 128 x 128 x 16 per 128 x 128 scores at head size 128,
+// measured 107 cycles each with both operands in shared memory (scores), 74 with the weights in tensor memory (values),
+// 4350 of the 5000 cycles that a tile takes; the other pipes need ~10 instructions per score beside them.  Layout that
+// follows: the query parts stay in shared memory (96 KB) and the weight parts go to tensor memory, over the scores they came
+// from, as the A operand.  Sixteen warps of softmax, four threads per row.
 //
-// Measured on a B200: 4096 tokens, 32 / 8 heads of 128, learned sinks, 6.17 ms on the FMA kernel -> 0.464 ms (296 TFLOP/s of
-// the attention, 3 times that on the tensor pipe); 1001 tokens behind 3333 in a window of 1024, 16 / 4 heads, 0.435 ms ->
-// 0.079 ms.  What is left is latency between the steps of a tile (eight warps of softmax per SM).  Error of fp32 outputs against
-// 64 bits over shapes, masks and score ranges: 0.15-0.8e-6 relative, on the FMA kernel 0.1-2.5e-6, never larger than there.
+// Measured on a B200: 4096 tokens, 32 / 8 heads of 128, learned sinks, 6.17 ms on the FMA kernel -> 0.452 ms (304 TFLOP/s of
+// the attention, 3 times that on the tensor pipe; 0.464 with eight warps); 1001 tokens behind 3333 in a window of 1024, 16 / 4
+// heads, 0.435 ms -> 0.077 ms.  Error of fp32 outputs against 64 bits over shapes, masks and score ranges: 0.15-0.8e-6
+// relative, on the FMA kernel 0.1-2.5e-6, never larger than there.  Descriptors formed ahead of the loop changed nothing.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <math.h>
@@ -35,7 +36,7 @@ typedef __nv_bfloat16 bf16;
 
 constexpr int BM = 128, BN = 128;             // score tile: rows = (query, query head of the group) pairs, keys
 constexpr int TILE_BYTES = 128 * 128;         // 128 rows x 64 bf16, 128-byte swizzled
-constexpr int SOFT_THREADS = 256;             // two threads per row (64 keys and half of the value columns each)
+constexpr int SOFT_THREADS = 512;             // four threads per row (32 keys and a quarter of the value columns each)
 constexpr int THREADS = SOFT_THREADS + 128;   // + MMA warp, K warp, V warp, one warp without work
 constexpr int RING = 8;                       // tiles in flight, for the marks of their live keys
 constexpr int TM_O = 256, TM_P3 = 384, TM_COLS = 512;   // tensor memory: scores 2 x 128 | tile result 128 | third part 2 x 64
@@ -96,6 +97,13 @@ __device__ __forceinline__ void tmem_ld32(uint32_t t, float* v) {
           "=f"(v[10]), "=f"(v[11]), "=f"(v[12]), "=f"(v[13]), "=f"(v[14]), "=f"(v[15]), "=f"(v[16]), "=f"(v[17]), "=f"(v[18]),
           "=f"(v[19]), "=f"(v[20]), "=f"(v[21]), "=f"(v[22]), "=f"(v[23]), "=f"(v[24]), "=f"(v[25]), "=f"(v[26]), "=f"(v[27]),
           "=f"(v[28]), "=f"(v[29]), "=f"(v[30]), "=f"(v[31])
+        : "r"(t) : "memory");
+}
+__device__ __forceinline__ void tmem_ld16(uint32_t t, float* v) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n"
+        : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]), "=f"(v[8]), "=f"(v[9]),
+          "=f"(v[10]), "=f"(v[11]), "=f"(v[12]), "=f"(v[13]), "=f"(v[14]), "=f"(v[15])
         : "r"(t) : "memory");
 }
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
@@ -251,11 +259,11 @@ struct Small {
     uint64_t bars[12];          // k full[2], v full[2], scores[2], weights[2], product[2], result read, queries
     uint32_t tmem;
     int failed;
-    float max[2][2][BM], sum[BM];
+    uint16_t max[2][4][BM];     // bf16 bounds of the row maxima over a quarter of the keys; the sums' meeting place at the end
     uint32_t live[RING][BN / 32];   // bit of key u % 32 of the tile: a slot holds it
 };
 
-// NO: value columns per thread (half of the padded value width).  SHAPED: soft cap, distance penalty, or a scale that is not
+// NO: value columns per thread (a quarter of the padded value width).  SHAPED: soft cap, distance penalty, or a scale that is not
 // positive.
 template <typename YT, int NO, bool SHAPED>
 __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const CcSeqAttn a) {
@@ -307,9 +315,9 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const CcSeqAttn a) 
     const int N = (ks.n + BN - 1) / BN;
 
     if (warp >= SOFT_THREADS / 32) {
-        // 384 threads x 168 registers at launch = 256 x 224 + 128 x 56
+        // 640 threads x 96 registers at launch = 61440 >= 512 x 104 + 128 x 56
         asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
-        if (warp == 8) {
+        if (warp == SOFT_THREADS / 32) {
             if (lane == 0) {
                 const uint32_t id_s = idesc(BN, false), id_v = idesc((Dv + 15) & ~15, true);
                 auto scores = [&](int n) {
@@ -337,15 +345,15 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const CcSeqAttn a) 
                     for (int s = 2; s >= 0; --s)
 #pragma unroll
                         for (int k = 0; k < BN / 16; ++k, acc = 1) {
-                            const uint32_t half = k >> 2, kk = (k & 3) * 8;
-                            const uint32_t at = s < 2 ? tmem + b * BN + half * 64 + s * 32 + kk : tmem + TM_P3 + b * 64 + half * 32 + kk;
+                            const uint32_t part = k >> 1, kk = (k & 1) * 8;      // 16 keys of a thread's 32
+                            const uint32_t at = s < 2 ? tmem + b * BN + part * 32 + s * 16 + kk : tmem + TM_P3 + b * 64 + part * 16 + kk;
                             mma_ts(tmem + TM_O, at, smem_desc(sV + b * v_tile + k * 2048, TILE_BYTES, 1024), id_v, acc);
                         }
                     mma_commit(PV_DONE + 8 * b);
                 }
             }
             __syncwarp();
-        } else if (warp == 9) {
+        } else if (warp == SOFT_THREADS / 32 + 1) {
             for (int n = 0; n < N; ++n) {
                 const int b = n & 1;
                 const TileRows t = look_up(a, ks, n, lane);
@@ -357,7 +365,7 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const CcSeqAttn a) 
                 fence_async();
                 mbar_arrive(K_FULL + 8 * b);
             }
-        } else if (warp == 10) {
+        } else if (warp == SOFT_THREADS / 32 + 2) {
             for (int n = 0; n < N; ++n) {
                 const int b = n & 1;
                 const TileRows t = look_up(a, ks, n, lane);
@@ -369,7 +377,7 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const CcSeqAttn a) 
             }
         }
     } else {
-        asm volatile("setmaxnreg.inc.sync.aligned.u32 224;");
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
         // the query rows in three parts; columns up to the padded width and rows past the end are zero
         for (int idx = tid; idx < BM * q_chunks; idx += SOFT_THREADS) {
             const int row = idx / q_chunks, c = idx - row * q_chunks, flat = f0 + row;
@@ -391,28 +399,26 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const CcSeqAttn a) 
         }
         fence_async();
         mbar_arrive(Q_FULL);
-        const int half = warp >> 2, quarter = warp & 3, row = quarter * 32 + lane, flat = min(f0 + row, n_rows - 1);
+        const int part = warp >> 2, quarter = warp & 3, row = quarter * 32 + lane, flat = min(f0 + row, n_rows - 1);
         const int t = flat / R, h = g * R + (flat - t * R), i = ks.p0 + t;
         const uint32_t lanes = (uint32_t)(quarter * 32) << 16;
         const float c2 = SHAPED ? 1.f : a.scale * LOG2E;
         const float dist_a = SHAPED && a.dist_a != nullptr ? a.dist_a[h] : 0.f, dist_b = SHAPED && a.dist_a != nullptr ? a.dist_b[h] : 0.f;
         float m = -INFINITY, l = 0.f, corr_before = 0.f;
-        if (a.sink_mode == CC_SINK_LEARNED) { m = a.sink[h] * LOG2E; l = half == 0 ? 1.f : 0.f; }
-        else if (a.sink_mode == CC_SINK_ZERO) { m = 0.f; l = half == 0 ? 1.f : 0.f; }
+        if (a.sink_mode == CC_SINK_LEARNED) { m = a.sink[h] * LOG2E; l = part == 0 ? 1.f : 0.f; }
+        else if (a.sink_mode == CC_SINK_ZERO) { m = 0.f; l = part == 0 ? 1.f : 0.f; }
         f32x2 O[NO / 2];
 #pragma unroll
         for (int c = 0; c < NO / 2; ++c) O[c] = 0ull;
         auto add_result = [&](int n, float corr) {   // O = O corr + the product of tile n
             mbar_wait(PV_DONE + 8 * (n & 1), (n >> 1) & 1, failed);
             fence_after();
+            float v[NO];
+            if constexpr (NO == 32) tmem_ld32(tmem + lanes + TM_O + part * NO, v);
+            else tmem_ld16(tmem + lanes + TM_O + part * NO, v);
+            tmem_wait_ld();
 #pragma unroll
-            for (int c0 = 0; c0 < NO; c0 += 32) {
-                float v[32];
-                tmem_ld32(tmem + lanes + TM_O + half * NO + c0, v);
-                tmem_wait_ld();
-#pragma unroll
-                for (int c = 0; c < 32; c += 2) O[(c0 + c) / 2] = fma2(O[(c0 + c) / 2], pair(corr, corr), pair(v[c], v[c + 1]));
-            }
+            for (int c = 0; c < NO; c += 2) O[c / 2] = fma2(O[c / 2], pair(corr, corr), pair(v[c], v[c + 1]));
             fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(O_READ);
@@ -426,59 +432,57 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const CcSeqAttn a) 
                                (a.block == 0 || j0 >= (i_last / a.block) * a.block);
             mbar_wait(S_DONE + 8 * b, (n >> 1) & 1, failed);
             fence_after();
-            float s[64];
-            tmem_ld32(tmem + lanes + b * BN + half * 64, s);
-            tmem_ld32(tmem + lanes + b * BN + half * 64 + 32, s + 32);
+            float s[32];
+            tmem_ld32(tmem + lanes + b * BN + part * 32, s);
             tmem_wait_ld();
-            const uint32_t live0 = sm.live[n & (RING - 1)][2 * half], live1 = sm.live[n & (RING - 1)][2 * half + 1];
+            const uint32_t live = sm.live[n & (RING - 1)][part];
             if constexpr (SHAPED) {
 #pragma unroll
-                for (int c = 0; c < 64; ++c) {
+                for (int c = 0; c < 32; ++c) {
                     float x = s[c] * a.scale;
                     if (a.softcap > 0.f) x = a.softcap * tanhf(x / a.softcap);
-                    if (a.dist_a != nullptr) x -= dist_a * log1pf(dist_b * (float)max(0, i - ks.at(u0 + half * 64 + c)));
+                    if (a.dist_a != nullptr) x -= dist_a * log1pf(dist_b * (float)max(0, i - ks.at(u0 + part * 32 + c)));
                     s[c] = x * LOG2E;
                 }
             }
-            if (!(plain && (live0 & live1) == 0xffffffffu)) {
-                const int i_block = a.block > 0 ? (i / a.block) * a.block : 0, u = u0 + half * 64;
+            if (!(plain && live == 0xffffffffu)) {
+                const int i_block = a.block > 0 ? (i / a.block) * a.block : 0, u = u0 + part * 32;
 #pragma unroll
-                for (int c = 0; c < 64; ++c) {
+                for (int c = 0; c < 32; ++c) {
                     const int j = ks.at(u + c);
-                    const bool ok = ((c < 32 ? live0 : live1) >> (c & 31) & 1u) && j <= i && (a.window == 0 || i - j < a.window || j < a.keep_first) &&
+                    const bool ok = (live >> c & 1u) && j <= i && (a.window == 0 || i - j < a.window || j < a.keep_first) &&
                                     j >= i_block;
                     if (!ok) s[c] = -INFINITY;
                 }
             }
             float mx[4] = {s[0], s[1], s[2], s[3]};
 #pragma unroll
-            for (int c = 4; c < 64; ++c) mx[c & 3] = fmaxf(mx[c & 3], s[c]);
-            float m_new = fmaxf(m, fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * c2);
-            sm.max[b][half][row] = m_new;
-            asm volatile("bar.sync %0, 64;" ::"r"(quarter + 1) : "memory");   // the two warps of these rows
-            m_new = fmaxf(m_new, sm.max[b][half ^ 1][row]);
+            for (int c = 4; c < 32; ++c) mx[c & 3] = fmaxf(mx[c & 3], s[c]);
+            // any common bound of the row's scores serves as its maximum: bf16, rounded up
+            sm.max[b][part][row] = __bfloat16_as_ushort(__float2bfloat16_ru(fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * c2));
+            asm volatile("bar.sync %0, 128;" ::"r"(quarter + 1) : "memory");   // the four warps of these rows
+            float m_new = m;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) m_new = fmaxf(m_new, __uint_as_float((uint32_t)sm.max[b][q][row] << 16));
             const float ms = m_new == -INFINITY ? 0.f : m_new;
             const float corr = m == -INFINITY ? 0.f : ex2(m - ms);
             m = m_new;
             const f32x2 cc = pair(c2, c2), mm = pair(-ms, -ms);
             f32x2 sum[2] = {0ull, 0ull};
+            uint32_t p1[16], p2[16], p3[16];
 #pragma unroll
-            for (int c0 = 0; c0 < 64; c0 += 32) {
-                uint32_t p1[16], p2[16], p3[16];
-#pragma unroll
-                for (int c = 0; c < 32; c += 2) {
-                    float x, y;
-                    unpair(fma2(pair(s[c0 + c], s[c0 + c + 1]), cc, mm), x, y);
-                    x = ex2(x);
-                    y = ex2(y);
-                    sum[(c >> 1) & 1] = add2(sum[(c >> 1) & 1], pair(x, y));
-                    split3(x, y, p1[c >> 1], p2[c >> 1], p3[c >> 1]);
-                }
-                const uint32_t at = tmem + lanes + b * BN + half * 64 + c0 / 2;   // 32 keys = 16 columns, over scores that are in registers
-                tmem_st16(at, p1);
-                tmem_st16(at + 32, p2);
-                tmem_st16(tmem + lanes + TM_P3 + b * 64 + half * 32 + c0 / 2, p3);
+            for (int c = 0; c < 32; c += 2) {
+                float x, y;
+                unpair(fma2(pair(s[c], s[c + 1]), cc, mm), x, y);
+                x = ex2(x);
+                y = ex2(y);
+                sum[(c >> 1) & 1] = add2(sum[(c >> 1) & 1], pair(x, y));
+                split3(x, y, p1[c >> 1], p2[c >> 1], p3[c >> 1]);
             }
+            const uint32_t at = tmem + lanes + b * BN + part * 32;   // 32 keys = 16 columns a part, over scores that are in registers
+            tmem_st16(at, p1);
+            tmem_st16(at + 16, p2);
+            tmem_st16(tmem + lanes + TM_P3 + b * 64 + part * 16, p3);
             float sum_x, sum_y;
             unpair(add2(sum[0], sum[1]), sum_x, sum_y);
             l = fmaf(l, corr, sum_x + sum_y);
@@ -490,16 +494,16 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const CcSeqAttn a) 
             corr_before = corr;
         }
         add_result(N - 1, corr_before);
-        if (half == 1) sm.sum[row] = l;
-        asm volatile("bar.sync %0, 64;" ::"r"(quarter + 1) : "memory");
-        if (half == 0) { l += sm.sum[row]; sm.max[0][0][row] = l; }
-        asm volatile("bar.sync %0, 64;" ::"r"(quarter + 1) : "memory");
-        l = sm.max[0][0][row];
+        asm volatile("bar.sync 5, 512;" ::: "memory");      // the last bounds of all rows have been read
+        float* const sums = reinterpret_cast<float*>(sm.max);                 // [4][BM]
+        sums[part * BM + row] = l;
+        asm volatile("bar.sync %0, 128;" ::"r"(quarter + 1) : "memory");
+        l = (sums[row] + sums[BM + row]) + (sums[2 * BM + row] + sums[3 * BM + row]);
         if (f0 + row < n_rows) {
             float inv = l > 0.f ? 1.0f / l : 0.f;
             if (*failed) inv = NAN;
-            YT* y = (YT*)a.y + ((size_t)t * a.H + h) * Dv + half * NO;
-            const int have = min(NO, Dv - half * NO);
+            YT* y = (YT*)a.y + ((size_t)t * a.H + h) * Dv + part * NO;
+            const int have = min(NO, Dv - part * NO);
             // rows are multiples of 8 elements wide: 16-byte stores
 #pragma unroll
             for (int c = 0; c < NO; c += 8) {
@@ -537,8 +541,8 @@ int launch_tc(const CcSeqAttn* a, cudaStream_t st) {
 template <typename YT>
 int dispatch_tc(const CcSeqAttn* a, cudaStream_t st) {
     const bool shaped = a->softcap > 0.f || a->dist_a != nullptr || !(a->scale > 0.f);
-    if (a->Dv <= 64) return shaped ? launch_tc<YT, 32, true>(a, st) : launch_tc<YT, 32, false>(a, st);
-    return shaped ? launch_tc<YT, 64, true>(a, st) : launch_tc<YT, 64, false>(a, st);
+    if (a->Dv <= 64) return shaped ? launch_tc<YT, 16, true>(a, st) : launch_tc<YT, 16, false>(a, st);
+    return shaped ? launch_tc<YT, 32, true>(a, st) : launch_tc<YT, 32, false>(a, st);
 }
 
 }  // namespace
