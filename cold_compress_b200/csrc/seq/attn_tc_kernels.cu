@@ -241,10 +241,29 @@ __device__ __forceinline__ void copy_tile(uint32_t dst, const CcSeqAttn& a, cons
         return;
     }
     const int u0 = n * BN;
+    if (u0 >= ks.kx && (t.fresh || t.r0 >= 0)) {
+        // up to three runs: slots up to the ring's end, slots from its start, rows of the portion
+        const int nc = max(0, min(BN, ks.p0 - t.j0)), w1 = min(nc, t.ring - t.r0), fresh_step = a.G * width;
+        const bf16* const r1 = cb + (ptrdiff_t)(a.keep_first + t.r0) * width;
+        const bf16* const r2 = r1 - (ptrdiff_t)t.ring * width;
+        const bf16* const r3 = fb + (ptrdiff_t)(t.j0 - ks.p0) * fresh_step;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const uint32_t live = t.live[q] >> hi;
+#pragma unroll 8
+            for (int i = 0; i < 16; ++i) {
+                const int row = 32 * q + 2 * i + hi;
+                const bool have = col && (live >> (2 * i) & 1u);
+                const bf16* src = row < nc ? (row < w1 ? r1 : r2) + row * width : r3 + (ptrdiff_t)row * fresh_step;
+                cp_async16(sw[i & 3] + 256 * (16 * q + i), have ? (const void*)src : fresh, have);
+            }
+        }
+        return;
+    }
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
         const uint32_t live = t.live[q] >> hi;
-#pragma unroll 4
+#pragma unroll 1
         for (int i = 0; i < 16; ++i) {
             const int row = 32 * q + 2 * i + hi, j = ks.at(u0 + row);
             const bool have = col && (live >> (2 * i) & 1u);
