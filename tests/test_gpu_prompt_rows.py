@@ -71,3 +71,42 @@ def test_calls_that_keep_the_tensor_operations():
         out, tangent = torch.func.jvp(m, (x,), (x,))
     _adjacent(out, want)
     assert tangent.shape == x.shape
+
+
+@pytest.mark.parametrize("S, Hkv, G, windows", [(1, 1, 1, ()), (31, 2, 4, (3,)), (512, 1, 4, ()), (513, 2, 4, (65, 600)), (1055, 1, 7, (300,))])
+def test_score_reductions_add_the_tiles_in_order(S, Hkv, G, windows):
+    """15, 16, 17 and more query tiles behind a column: the sums are the tiles' partials added in order, bit for bit."""
+    from cold_compress_b200 import _lib, ops
+    gen = torch.Generator().manual_seed(S)
+    q, k, v = (torch.randn(h, S, 128, generator=gen).bfloat16().cuda() for h in (Hkv * G, Hkv, Hkv))
+    y, obs = torch.empty_like(q), min(16, S)
+    ws = torch.full((ops.prefill_attention_workspace(S, Hkv, G, obs, len(windows)) // 4 + 64,), float("nan"), device="cuda")
+    col, seen, band = (torch.empty(n, device="cuda") for n in ((Hkv, S), (Hkv, S), (max(1, len(windows)), Hkv, S)))
+    ops._prefill_attention(q, k, v, y, _lib.ATTN_NAIVE_BF16, obs, list(windows), col, seen, band if windows else None, ws)
+    QB = 1 << ((128 // G).bit_length() - 1)
+    tiles, pad = -(-S // QB), -(-S // 128) * 128
+    at = (-ws.data_ptr() % 256) // 4
+    first = (S - obs) // QB
+
+    def part(n_tiles, lead=()):
+        nonlocal at
+        n = Hkv * n_tiles * pad
+        for d in lead:
+            n *= d
+        t = ws[at:at + n].view(*lead, Hkv, n_tiles, pad)[..., :S].cpu()
+        at += n
+        return t
+
+    def in_order(p, lo, hi):       # p [.., n, S]; column j takes tiles lo[j] .. hi[j] - 1
+        acc = torch.zeros(p.shape[:-2] + p.shape[-1:])
+        for t in range(p.shape[-2]):
+            acc = torch.where((lo <= t) & (t < hi), acc + p[..., t, :], acc)
+        return acc
+
+    j = torch.arange(S)
+    assert torch.equal(col.cpu(), in_order(part(tiles), j // QB, torch.tensor(tiles)))
+    assert torch.equal(seen.cpu(), in_order(part(tiles - first), (j // QB - first).clamp(min=0), torch.tensor(tiles - first)))
+    if windows:
+        bands = part(tiles, (len(windows),))
+        for i, w in enumerate(windows):
+            assert torch.equal(band[i].cpu(), in_order(bands[i], j // QB, ((j + w - 1) // QB).clamp(max=tiles - 1) + 1))
