@@ -175,8 +175,8 @@ __device__ __forceinline__ int warp_reduce8_column(int lane) { return ((lane >> 
 // rows l, l + 32, l + 64, l + 96 (one LDS.128 each), pools over the heads (model.py:413-418), and the warp adds the
 // pooled values over the query rows.  QBL = log2(query rows per tile); row = g * QB + i.
 template <int QBL>
-__device__ __forceinline__ void tile_stats(const uint8_t* sP_ptr, float (*s_comb)[BNH], const PrefillParams& p, int ck,
-                                           int lane, int i0, int jbase, bool want_obs) {
+__device__ __forceinline__ void tile_stats(const uint8_t* sP_ptr, float* out_col, float* out_obs, float* out_band, size_t band_stride,
+                                           const PrefillParams& p, int ck, int lane, int i0, int jbase, bool want_obs) {
     constexpr int QB = 1 << QBL;
     constexpr int NI = QB >= 32 ? QB / 32 : 1;   // query rows held by one lane
     constexpr int NK = 4 / NI;                   // heads per query row held by one lane
@@ -242,18 +242,18 @@ __device__ __forceinline__ void tile_stats(const uint8_t* sP_ptr, float (*s_comb
         }
     }
     const int oc = ck * 8 + warp_reduce8_column(lane);
-    const bool writer = (lane & 3) == 0;
+    const bool writer = (lane & 3) == 0;          // eight lanes write the warp's eight columns: one 32-byte sector
     float r = warp_reduce8(col, lane);
-    if (writer) s_comb[0][oc] = r;
+    if (writer) out_col[oc] = r;
     if (want_obs) {
         r = warp_reduce8(obs, lane);
-        if (writer) s_comb[1][oc] = r;
+        if (writer) out_obs[oc] = r;
     }
 #pragma unroll
     for (int w = 0; w < MAX_WINDOWS; ++w) {
         if (w < p.n_windows) {
             r = warp_reduce8(band[w], lane);
-            if (writer) s_comb[2 + w][oc] = r;
+            if (writer) out_band[w * band_stride + oc] = r;
         }
     }
 }
@@ -265,6 +265,11 @@ __device__ __forceinline__ void tile_stats(const uint8_t* sP_ptr, float (*s_comb
 // MUFU-bound softmax overlaps the other's rounding / store / reduction phases.  In a group, thread
 // (row = t % 128, ch = t / 128) owns keys [32 ch, 32 ch + 32) of its row of every S block (TMEM lane quarter row / 32).
 // The partial accumulators Y_0 + Y_1 are added in the epilogue (fixed order: bit-reproducible).
+// Bound: latency at four warps per scheduler (issue slots 38 % busy, the largest stall the group's barrier).  A group has
+// two P blocks so that one barrier per block of sweep 2 is enough: it says that the block is written, and that everyone has
+// read the block before, which the block after it may then overwrite once its MMAs are done.  With one P block there were
+// two barriers per block and the column sums waited in shared memory: 1718 us at 7680 tokens x 32 heads of 128 (8 key/value
+// heads), 1573 now; 116.2 -> 110.7 at 1531 x 28 (4).  The two blocks take 32 KB more: 225 KB of the 227 a CTA may have.
 __device__ __forceinline__ void group_sync(int grp) { asm volatile("bar.sync %0, 256;" :: "r"(grp + 1) : "memory"); }
 
 template <int D, bool NAIVE>
@@ -275,13 +280,10 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     constexpr int Q_BYTES = DH * ATOM_BYTES;    // Q tile: 128 rows
     constexpr int HALF_ATOM = BNH * 128;        // 64 rows x 128 bytes
     constexpr int KV_BYTES = DH * HALF_ATOM;    // one K or V block of a group: 64 keys x D
-    constexpr int GROUP_BYTES = 4 * KV_BYTES + ATOM_BYTES;   // K[2], V[2], P (128 rows x 64 keys)
-    constexpr int NSTAT = 2 + MAX_WINDOWS;      // col, obs, bands
+    constexpr int GROUP_BYTES = 4 * KV_BYTES + 2 * ATOM_BYTES;   // K[2], V[2], P[2] (128 rows x 64 keys)
     extern __shared__ uint8_t smem_raw[];
-    __shared__ __align__(8) uint64_t bars[16];  // 0 q; group g at 1 + 7 g: k[2], v[2], s[2], pv
+    __shared__ __align__(8) uint64_t bars[17];  // 0 q; group g at 1 + 8 g: k[2], v[2], s[2], pv[2]
     __shared__ uint32_t s_tmem_base;
-    __shared__ float s_rowstat[4][BM][2];
-    __shared__ float s_comb[2][NSTAT][BNH];     // per-block column sums of each group, flushed one block later
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int grp = tid >> 8, gt = tid & 255, gwarp = gt >> 5;
@@ -298,15 +300,17 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     const uint32_t sG = sQ + Q_BYTES + grp * GROUP_BYTES;
     const uint32_t sK = sG, sV = sG + 2 * KV_BYTES, sP = sG + 4 * KV_BYTES;
     uint8_t* const sP_ptr = smem_raw + (sP - smem_u32(smem_raw));
+    // row statistics of the four key quarters, between the sweeps, where group 0's P blocks are afterwards
+    float (*s_rowstat)[BM][2] = reinterpret_cast<float (*)[BM][2]>(smem_raw + (sQ + Q_BYTES + 4 * KV_BYTES - smem_u32(smem_raw)));
     const uint32_t bar0 = smem_u32(bars);
-    const uint32_t BAR_Q = bar0, bG = bar0 + 8u * (1 + 7 * grp);
+    const uint32_t BAR_Q = bar0, bG = bar0 + 8u * (1 + 8 * grp);
     auto BAR_K = [&](int b) { return bG + 8u * b; };
     auto BAR_V = [&](int b) { return bG + 8u * (2 + b); };
     auto BAR_S = [&](int b) { return bG + 8u * (4 + b); };
-    const uint32_t BAR_PV = bG + 8u * 6;
+    auto BAR_PV = [&](int b) { return bG + 8u * (6 + b); };
 
     if (tid == 0) {
-        for (int i = 0; i < 15; ++i) mbar_init_u32(bar0 + 8u * i, 1);
+        for (int i = 0; i < 17; ++i) mbar_init_u32(bar0 + 8u * i, 1);
         mbar_fence_init();
     }
     if (warp == 0) {
@@ -355,9 +359,9 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     auto mma_pv = [&](int buf, bool first) {
 #pragma unroll
         for (int k = 0; k < BNH / 16; ++k)
-            umma_bf16(tY, smem_desc(sP + k * 32, 16, 1024), smem_desc(sV + buf * KV_BYTES + k * 2048, HALF_ATOM, 1024),
+            umma_bf16(tY, smem_desc(sP + buf * ATOM_BYTES + k * 32, 16, 1024), smem_desc(sV + buf * KV_BYTES + k * 2048, HALF_ATOM, 1024),
                       IDESC_PV, !(first && k == 0));
-        umma_commit(BAR_PV);
+        umma_commit(BAR_PV(buf));
     };
 
     const int NT = 2 * T;   // block visits of this group: sweep 1 then sweep 2
@@ -384,17 +388,12 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     float m_fin = 0.f, inv_s = 0.f;
     const float scale = p.scale;
 
-    // pooled-map reductions: warp = 16-byte chunk of key columns (tile_stats); the sums of block t are written to the
-    // scratch during block t + 1 (after its first barrier) so no extra barrier is needed
+    // pooled-map reductions: warp = 16-byte chunk of key columns (tile_stats), straight to this query block's partials
     const bool want_obs = qt >= p.first_obs_tile;
-    auto flush_stats = [&](int t) {   // group threads < 64: one key column of block t
-        const int j = t * BN + grp * BNH + gt;
-        const size_t slab = (size_t)p.S_pad;
-        p.part_col[((size_t)h * p.n_qtiles + qt) * slab + j] = s_comb[grp][0][gt];
-        if (want_obs) p.part_obs[((size_t)h * p.n_obs_tiles + (qt - p.first_obs_tile)) * slab + j] = s_comb[grp][1][gt];
-        for (int w = 0; w < p.n_windows; ++w)
-            p.part_band[(((size_t)w * p.Hkv + h) * p.n_qtiles + qt) * slab + j] = s_comb[grp][2 + w][gt];
-    };
+    float* const out_col = p.part_col + ((size_t)h * p.n_qtiles + qt) * p.S_pad + grp * BNH;
+    float* const out_obs = p.part_obs + ((size_t)h * p.n_obs_tiles + (want_obs ? qt - p.first_obs_tile : 0)) * p.S_pad + grp * BNH;
+    float* const out_band = p.part_band + ((size_t)h * p.n_qtiles + qt) * p.S_pad + grp * BNH;
+    const size_t band_stride = (size_t)p.Hkv * p.n_qtiles * p.S_pad;
 
     // one block visit up to the logits: l[c] = logit of key (block t, 32 ch + c), -inf past the diagonal
     auto visit = [&](int n, int t, float (&l)[32]) {
@@ -470,6 +469,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         for (int c = 0; c < 4; ++c) tot += sq[c] * ex2((mq[c] - m_fin) * LOG2E);
         inv_s = 1.0f / tot;
     }
+    __syncthreads();   // every thread has its statistics: P blocks may take their place
 
     // ---- sweep 2: probabilities, P V, pooled reductions
     const f32x2 off2 = pair(-m_fin * LOG2E, -m_fin * LOG2E), inv2 = pair(inv_s, inv_s);
@@ -484,12 +484,11 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
             unpair(mul2(pair(ex2(x), ex2(y)), inv2), x, y);
             pk[c >> 1] = cvt_bf16x2(x, y);
         }
-        if (t > 0) mbar_wait_u32(BAR_PV, (t - 1) & 1);   // P V of the previous block done: sP and V[(t-1)&1] are free
-        group_sync(grp);                                  // the group finished reading the previous P block
-        if (gt == 0 && t >= 1 && t + 1 < T) issue_v(t + 1, (t + 1) & 1);
-        if (p.stats && t > 0 && gt < BNH) flush_stats(t - 1);
+        // P[t & 1] is free: its MMAs of two blocks ago are done, and every warp had read it before the barrier of the last block
+        if (t > 1) mbar_wait_u32(BAR_PV(t & 1), ((t >> 1) - 1) & 1);
+        uint8_t* const P = sP_ptr + (t & 1) * ATOM_BYTES;
         {
-            uint8_t* prow = sP_ptr + row * 128;
+            uint8_t* prow = P + row * 128;
 #pragma unroll
             for (int c4 = 0; c4 < 4; ++c4) {
                 const int c8 = ch * 4 + c4;
@@ -505,25 +504,28 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
             mbar_wait_u32(BAR_V(t & 1), (t >> 1) & 1);
             tc_fence_after();
             mma_pv(t & 1, t == 0);
+            if (t >= 1 && t + 1 < T) {                      // V[(t + 1) & 1] is free once the last block's MMAs are done
+                mbar_wait_u32(BAR_PV((t - 1) & 1), ((t - 1) >> 1) & 1);
+                issue_v(t + 1, (t + 1) & 1);
+            }
         }
         __syncwarp();
         if (p.stats) {
-            const int jbase = t * BN + grp * BNH + gwarp * 8;
+            const int jbase = t * BN + grp * BNH + gwarp * 8, j = t * BN;
             switch (p.QB) {
-                case 128: tile_stats<7>(sP_ptr, s_comb[grp], p, gwarp, lane, i0, jbase, want_obs); break;
-                case 64:  tile_stats<6>(sP_ptr, s_comb[grp], p, gwarp, lane, i0, jbase, want_obs); break;
-                case 32:  tile_stats<5>(sP_ptr, s_comb[grp], p, gwarp, lane, i0, jbase, want_obs); break;
-                default:  tile_stats<4>(sP_ptr, s_comb[grp], p, gwarp, lane, i0, jbase, want_obs); break;
+                case 128: tile_stats<7>(P, out_col + j, out_obs + j, out_band + j, band_stride, p, gwarp, lane, i0, jbase, want_obs); break;
+                case 64:  tile_stats<6>(P, out_col + j, out_obs + j, out_band + j, band_stride, p, gwarp, lane, i0, jbase, want_obs); break;
+                case 32:  tile_stats<5>(P, out_col + j, out_obs + j, out_band + j, band_stride, p, gwarp, lane, i0, jbase, want_obs); break;
+                default:  tile_stats<4>(P, out_col + j, out_obs + j, out_band + j, band_stride, p, gwarp, lane, i0, jbase, want_obs); break;
             }
         }
     }
 
     // ---- epilogue: Y_0 + Y_1 (fp32 in TMEM) -> bf16 -> global
-    if (T > 0) mbar_wait_u32(BAR_PV, (T - 1) & 1);
+    if (T > 0) mbar_wait_u32(BAR_PV((T - 1) & 1), ((T - 1) >> 1) & 1);
     tc_fence_after();
-    __syncthreads();   // both groups' accumulators and last column sums are complete
+    __syncthreads();   // both groups' accumulators are complete
     tc_fence_after();
-    if (p.stats && T > 0 && gt < BNH) flush_stats(T - 1);
     {
         constexpr int CPT = D / 4;   // columns per thread: 32 (D = 128) or 16 (D = 64)
         const int cq = tid >> 7, orow = tid & 127;
@@ -660,7 +662,7 @@ Plan make_plan(int S, int Hkv, int G, int obs_len, int n_windows) {
 template <int D, bool NAIVE>
 int launch(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const PrefillParams& p, int grid,
            cudaStream_t stream) {
-    const int smem = 1024 + (D / 64) * ATOM_BYTES + 2 * (4 * (D / 64) * BNH * 128 + ATOM_BYTES);
+    const int smem = 1024 + (D / 64) * ATOM_BYTES + 2 * (4 * (D / 64) * BNH * 128 + 2 * ATOM_BYTES);
     static bool configured = false;
     if (!configured) {
         cudaError_t e = cudaFuncSetAttribute(prefill_attn_kernel<D, NAIVE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);

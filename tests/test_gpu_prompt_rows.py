@@ -110,3 +110,22 @@ def test_score_reductions_add_the_tiles_in_order(S, Hkv, G, windows):
         bands = part(tiles, (len(windows),))
         for i, w in enumerate(windows):
             assert torch.equal(band[i].cpu(), in_order(bands[i], j // QB, ((j + w - 1) // QB).clamp(max=tiles - 1) + 1))
+
+
+@pytest.mark.parametrize("S", [1, 64, 65, 128, 129, 192, 193, 257, 321, 449])
+@pytest.mark.parametrize("Hkv, G, D", [(2, 4, 128), (1, 7, 64)])
+def test_scores_attention_at_every_count_of_key_blocks(S, Hkv, G, D):
+    """No, one, two, three and four 64-key blocks per key half (its value and probability blocks alternate between two)."""
+    from cold_compress_b200.attention_utils import prefill_attention_stats
+    gen = torch.Generator().manual_seed(S)
+    q, k, v = (torch.randn(1, h, S, D, generator=gen).bfloat16().cuda() for h in (Hkv * G, Hkv, Hkv))
+    y, _ = prefill_attention_stats(q, k, v, obs_len=1)
+    rnd = lambda x: x.bfloat16().double()
+    kk, vv = (x.repeat_interleave(G, 1).double() for x in (k, v))
+    s = rnd(rnd((q.double() @ kk.mT).float()).float() * (1.0 / D ** 0.5))
+    s = s.masked_fill(torch.ones(S, S, dtype=torch.bool, device="cuda").triu(1), float("-inf"))
+    want = rnd(s.softmax(-1).float()) @ vv
+    y = y.reshape(want.shape).double()
+    # a logit's two roundings may fall the other way (2^-8 of |s| <= ~5, hence 2^-6 of a weight), a weight's and y's (2^-9)
+    err = (y - want).norm(dim=-1) / (rnd(s.softmax(-1).float()) @ vv.abs()).norm(dim=-1)
+    assert err.max().item() <= 2.0 ** -6 + 2.0 ** -8 and ((y - want).norm() / want.norm()).item() <= 2.0 ** -8
