@@ -269,7 +269,7 @@ __device__ __forceinline__ void tile_stats(const uint8_t* sP_ptr, float* out_col
 // two P blocks so that one barrier per block of sweep 2 is enough: it says that the block is written, and that everyone has
 // read the block before, which the block after it may then overwrite once its MMAs are done.  With one P block there were
 // two barriers per block and the column sums waited in shared memory: 1718 us at 7680 tokens x 32 heads of 128 (8 key/value
-// heads), 1573 now; 116.2 -> 110.7 at 1531 x 28 (4).  The two blocks take 32 KB more: 225 KB of the 227 a CTA may have.
+// heads), 1573 with two; 116.2 and 110.7 at 1531 x 28 (4).  The two blocks take 32 KB more: 225 KB of the 227 a CTA may have.
 __device__ __forceinline__ void group_sync(int grp) { asm volatile("bar.sync %0, 256;" :: "r"(grp + 1) : "memory"); }
 
 template <int D, bool NAIVE>
@@ -288,6 +288,9 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int grp = tid >> 8, gt = tid & 255, gwarp = gt >> 5;
     const int row = gt & 127, ch = gt >> 7;
+    // One thread each of three warps of the group issues its Q K^T products, its K loads, and its P V products and V loads:
+    // what one warp issued alone, the other seven waited for at the next barrier (1573 -> 1416 us at 7680 tokens x 32 heads).
+    const bool lead_s = gt == 0, lead_k = gt == 3 * 32, lead_v = gt == 6 * 32;
     const int h = blockIdx.x % p.Hkv;
     const int qt = p.n_qtiles - 1 - blockIdx.x / p.Hkv;
     const int i0 = qt * p.QB;
@@ -370,7 +373,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
 #pragma unroll
         for (int dh = 0; dh < DH; ++dh) tma_load_3d(sQ + dh * ATOM_BYTES, &tm_q, dh * 64, i0, h * p.G, BAR_Q);
     }
-    if (gt == 0 && T > 0) {
+    if (lead_s && T > 0) {
         issue_k(0, 0);
         issue_k(1 % T, 1);
         issue_v(0, 0);
@@ -398,7 +401,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     // one block visit up to the logits: l[c] = logit of key (block t, 32 ch + c), -inf past the diagonal
     auto visit = [&](int n, int t, float (&l)[32]) {
         const int sb = n & 1;
-        if (gt == 0 && n + 1 < NT) {   // next block's logits under this block's softmax
+        if (lead_s && n + 1 < NT) {   // next block's logits under this block's softmax
             mbar_wait_u32(BAR_K((n + 1) & 1), ((n + 1) >> 1) & 1);
             tc_fence_after();
             mma_s((n + 1) & 1);
@@ -408,7 +411,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         tc_fence_after();
         uint32_t v0[32];
         tmem_ld32(tS + lane_base + sb * BNH + ch * 32, v0);
-        if (gt == 0 && n + 2 < NT) issue_k((n + 2) % T, sb);   // K[sb] is free: its MMA has completed
+        if (lead_k && n + 2 < NT) issue_k((n + 2) % T, sb);   // K[sb] is free: its MMA has completed
         __syncwarp();
         const f32x2 scale2 = pair(scale, scale);
 #pragma unroll
@@ -499,7 +502,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         fence_proxy_async();
         tc_fence_before();
         group_sync(grp);
-        if (gt == 0) {
+        if (lead_v) {
             tc_fence_after();
             mbar_wait_u32(BAR_V(t & 1), (t >> 1) & 1);
             tc_fence_after();
