@@ -278,7 +278,7 @@ struct Small {
     uint64_t bars[12];          // k full[2], v full[2], scores[2], weights[2], product[2], result read, queries
     uint32_t tmem;
     int failed;
-    uint16_t max[2][4][BM];     // bf16 bounds of the row maxima over a quarter of the keys; the sums' meeting place at the end
+    float max[4][BM];           // row maxima over a quarter of a tile's keys; the sums' meeting place at the end
     uint32_t live[RING][BN / 32];   // bit of key u % 32 of the tile: a slot holds it
 };
 
@@ -421,10 +421,10 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const CcSeqAttn a) 
         const int part = warp >> 2, quarter = warp & 3, row = quarter * 32 + lane, flat = min(f0 + row, n_rows - 1);
         const int t = flat / R, h = g * R + (flat - t * R), i = ks.p0 + t;
         const uint32_t lanes = (uint32_t)(quarter * 32) << 16;
-        const float c2 = SHAPED ? 1.f : a.scale * LOG2E;
+        const float c2 = SHAPED ? LOG2E : a.scale * LOG2E;
         const float dist_a = SHAPED && a.dist_a != nullptr ? a.dist_a[h] : 0.f, dist_b = SHAPED && a.dist_a != nullptr ? a.dist_b[h] : 0.f;
         float m = -INFINITY, l = 0.f, corr_before = 0.f;
-        if (a.sink_mode == CC_SINK_LEARNED) { m = a.sink[h] * LOG2E; l = part == 0 ? 1.f : 0.f; }
+        if (a.sink_mode == CC_SINK_LEARNED) { m = __fmul_rn(a.sink[h], LOG2E); l = part == 0 ? ex2(fmaf(a.sink[h], LOG2E, -m)) : 0.f; }
         else if (a.sink_mode == CC_SINK_ZERO) { m = 0.f; l = part == 0 ? 1.f : 0.f; }
         f32x2 O[NO / 2];
 #pragma unroll
@@ -461,7 +461,7 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const CcSeqAttn a) 
                     float x = s[c] * a.scale;
                     if (a.softcap > 0.f) x = a.softcap * tanhf(x / a.softcap);
                     if (a.dist_a != nullptr) x -= dist_a * log1pf(dist_b * (float)max(0, i - ks.at(u0 + part * 32 + c)));
-                    s[c] = x * LOG2E;
+                    s[c] = x;
                 }
             }
             if (!(plain && live == 0xffffffffu)) {
@@ -477,12 +477,16 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const CcSeqAttn a) 
             float mx[4] = {s[0], s[1], s[2], s[3]};
 #pragma unroll
             for (int c = 4; c < 32; ++c) mx[c & 3] = fmaxf(mx[c & 3], s[c]);
-            // any common bound of the row's scores serves as its maximum: bf16, rounded up
-            sm.max[b][part][row] = __bfloat16_as_ushort(__float2bfloat16_ru(fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * c2));
-            asm volatile("bar.sync %0, 128;" ::"r"(quarter + 1) : "memory");   // the four warps of these rows
+            // The maximum itself, in fp32: the exponents below reach from 0 down, so a bound far above it would flush every
+            // weight.  The four warps of these rows meet twice per tile, as the maxima of the tile before have to be read:
+            // arriving there and waiting here are apart.
+            if (n > 0) asm volatile("bar.sync %0, 256;" ::"r"(quarter + 6) : "memory");
+            sm.max[part][row] = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * c2;
+            asm volatile("bar.sync %0, 128;" ::"r"(quarter + 1) : "memory");
             float m_new = m;
 #pragma unroll
-            for (int q = 0; q < 4; ++q) m_new = fmaxf(m_new, __uint_as_float((uint32_t)sm.max[b][q][row] << 16));
+            for (int q = 0; q < 4; ++q) m_new = fmaxf(m_new, sm.max[q][row]);
+            if (n + 1 < N) asm volatile("bar.arrive %0, 256;" ::"r"(quarter + 6) : "memory");
             const float ms = m_new == -INFINITY ? 0.f : m_new;
             const float corr = m == -INFINITY ? 0.f : ex2(m - ms);
             m = m_new;
@@ -513,11 +517,10 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const CcSeqAttn a) 
             corr_before = corr;
         }
         add_result(N - 1, corr_before);
-        asm volatile("bar.sync 5, 512;" ::: "memory");      // the last bounds of all rows have been read
-        float* const sums = reinterpret_cast<float*>(sm.max);                 // [4][BM]
-        sums[part * BM + row] = l;
+        asm volatile("bar.sync %0, 128;" ::"r"(quarter + 1) : "memory");      // the last maxima of these rows have been read
+        sm.max[part][row] = l;
         asm volatile("bar.sync %0, 128;" ::"r"(quarter + 1) : "memory");
-        l = (sums[row] + sums[BM + row]) + (sums[2 * BM + row] + sums[3 * BM + row]);
+        l = (sm.max[0][row] + sm.max[1][row]) + (sm.max[2][row] + sm.max[3][row]);
         if (f0 + row < n_rows) {
             float inv = l > 0.f ? 1.0f / l : 0.f;
             if (*failed) inv = NAN;
