@@ -280,7 +280,72 @@ struct Small {
     int failed;
     float max[4][BM];           // row maxima over a quarter of a tile's keys; the sums' meeting place at the end
     uint32_t live[RING][BN / 32];   // bit of key u % 32 of the tile: a slot holds it
+    uint32_t redo[BM / 32];         // bit of row u % 32: its sums are not finite
 };
+
+__device__ __forceinline__ float warp_max(float v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
+    return v;
+}
+__device__ __forceinline__ float warp_sum(float v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+__device__ __forceinline__ float shaped(const CcSeqAttn& a, float x, int h, int dist) {
+    if (a.softcap > 0.f) x = a.softcap * tanhf(x / a.softcap);
+    if (a.dist_a != nullptr) x -= a.dist_a[h] * log1pf(a.dist_b[h] * (float)max(0, dist));
+    return x;
+}
+
+// One (query, head) row again by a warp, key by key on the FMA pipe, for rows whose sums above are not finite: three parts of an
+// operand times an infinity give NaN where the operand itself gives an infinity, and a weight of zero times a value row that
+// this row does not see gives NaN too.  Here a key that is not seen takes no part and operands are whole, so a score of minus
+// infinity is a weight of zero and an infinity stays one.  Ends as soon as the denominator is NaN: then everything is.
+template <typename YT, bool SHAPED>
+__device__ __forceinline__ void row_again(const CcSeqAttn& a, const Keys& ks, int t, int h, int g, int lane) {
+    const int i = ks.p0 + t, Dk = a.Dk, Dv = a.Dv, ring = a.L - a.keep_first, i_block = a.block > 0 ? (i / a.block) * a.block : 0;
+    const float* const q = a.q + ((size_t)t * a.H + h) * Dk;
+    float m = -INFINITY, l = 0.f, o[4] = {0.f, 0.f, 0.f, 0.f};      // value columns 4 lane .. 4 lane + 3
+    if (a.sink_mode == CC_SINK_LEARNED) { m = a.sink[h]; l = 1.f; }
+    else if (a.sink_mode == CC_SINK_ZERO) { m = 0.f; l = 1.f; }
+#pragma unroll 1
+    for (int u0 = 0; u0 < ks.n && l == l; u0 += 32) {
+        const int j = ks.at(u0 + lane), slot = j < a.keep_first ? j : a.keep_first + (j - a.keep_first) % ring;
+        const bool seen = u0 + lane < ks.n && j <= i && (a.window == 0 || i - j < a.window || j < a.keep_first) && j >= i_block && (j >= ks.p0 || a.pos[slot] == j);
+        const size_t row = j >= ks.p0 ? (size_t)(j - ks.p0) * a.G + g : (size_t)g * a.L + slot;
+        float s = -INFINITY;
+        if (seen) {
+            const bf16* const k = (const bf16*)(j >= ks.p0 ? a.k_new : a.k_cache) + row * Dk;
+            s = 0.f;
+#pragma unroll 1
+            for (int d = 0; d < Dk; ++d) s = fmaf(q[d], __bfloat162float(k[d]), s);
+            s *= a.scale;
+            if (SHAPED) s = shaped(a, s, h, i - j);
+        }
+        const float m_new = fmaxf(m, warp_max(s)), corr = m == -INFINITY ? 0.f : expf(m - m_new), w = s == -INFINITY ? 0.f : expf(s - m_new);
+        l = l * corr + warp_sum(w);
+        m = m_new;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) o[c] *= corr;
+#pragma unroll 1
+        for (uint32_t left = __ballot_sync(0xffffffffu, seen); left != 0; left &= left - 1) {
+            const int k = __ffs(left) - 1, fresh = __shfl_sync(0xffffffffu, (int)(j >= ks.p0), k);
+            const float wk = __shfl_sync(0xffffffffu, w, k);
+            const size_t rk = __shfl_sync(0xffffffffu, (unsigned long long)row, k);
+            if (4 * lane >= Dv) continue;
+            const bf16* const v = (const bf16*)(fresh ? a.v_new : a.v_cache) + rk * Dv + 4 * lane;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) o[c] = fmaf(wk, __bfloat162float(v[c]), o[c]);
+        }
+    }
+    const float inv = l > 0.f ? 1.0f / l : 0.f;
+    if (4 * lane < Dv)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) st_out((YT*)a.y + ((size_t)t * a.H + h) * Dv, 4 * lane + c, l == l ? o[c] * inv : NAN);
+}
 
 // NO: value columns per thread (a quarter of the padded value width).  SHAPED: soft cap, distance penalty, or a scale that is not
 // positive.
@@ -301,6 +366,7 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const CcSeqAttn a) 
     const uint32_t bar = smem_u32(sm.bars);
     const uint32_t K_FULL = bar, V_FULL = bar + 16, S_DONE = bar + 32, P_DONE = bar + 48, PV_DONE = bar + 64, O_READ = bar + 80, Q_FULL = bar + 88;
 
+    if (tid < BM / 32) sm.redo[tid] = 0;
     if (tid == 0) {
         *failed = 0;
         for (int b = 0; b < 2; ++b) {
@@ -522,7 +588,7 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const CcSeqAttn a) 
         asm volatile("bar.sync %0, 128;" ::"r"(quarter + 1) : "memory");
         l = (sm.max[0][row] + sm.max[1][row]) + (sm.max[2][row] + sm.max[3][row]);
         if (f0 + row < n_rows) {
-            float inv = l > 0.f ? 1.0f / l : 0.f;
+            float inv = l > 0.f ? 1.0f / l : 0.f, zero = 0.f * l;      // 0, or NaN once something is not finite
             if (*failed) inv = NAN;
             YT* y = (YT*)a.y + ((size_t)t * a.H + h) * Dv + part * NO;
             const int have = min(NO, Dv - part * NO);
@@ -535,6 +601,7 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const CcSeqAttn a) 
                     for (int e = 0; e < 8; e += 2) {
                         float x, x1;
                         unpair(O[(c + e) / 2], x, x1);
+                        zero = fmaf(0.f, x, fmaf(0.f, x1, zero));
                         st_out(w, e, x * inv);
                         st_out(w, e + 1, x1 * inv);
                     }
@@ -542,7 +609,13 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const CcSeqAttn a) 
                     for (int v = 0; v < (int)sizeof(YT) / 2; ++v) reinterpret_cast<uint4*>(y + c)[v] = reinterpret_cast<const uint4*>(w)[v];
                 }
             }
+            if (zero != 0.f) atomicOr(&sm.redo[quarter], 1u << lane);
         }
+        asm volatile("bar.sync 5, 512;" ::: "memory");      // everyone's marks, and what this loop writes over is written
+        if (*failed == 0)
+#pragma unroll 1
+            for (int r = warp; r < BM; r += SOFT_THREADS / 32)
+                if (sm.redo[r >> 5] >> (r & 31) & 1u) row_again<YT, SHAPED>(a, ks, (f0 + r) / R, g * R + (f0 + r) % R, g, lane);
     }
     fence_before();
     __syncthreads();

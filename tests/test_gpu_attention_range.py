@@ -53,3 +53,56 @@ def test_scores_of_any_size_keep_their_softmax(scale, learned):
     for h in range(H):
         err = ((y[:, h].double() - want[:, h]).norm() / want[:, h].norm()).item()
         assert err <= 8 * 2.0 ** -24 * math.sqrt(D), (top[h].item(), err)
+
+
+def _want(q, k, v, past, scale, seen=None):
+    """64-bit attention in which a key that is not seen takes no part, whatever it holds; 0 for weights of 0."""
+    s = _scores(q, torch.nan_to_num(k.double(), 0.0, 0.0, 0.0), past, scale)
+    if seen is not None:
+        s = s.masked_fill(~seen, -math.inf)
+    return torch.matmul(torch.softmax(s, -1), torch.nan_to_num(v.double(), 0.0, 0.0, 0.0).repeat_interleave(q.shape[1] // k.shape[1], 1).transpose(0, 1)).transpose(0, 1)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("softcap", [0.0, 30.0])
+@pytest.mark.parametrize("where", [0, 77, 299, 300, 310, 429])       # a row of the cache or of the portion, first, last, between
+@pytest.mark.parametrize("kind", ["key -inf", "key +inf", "value inf", "value nan", "query inf"])
+def test_what_is_not_finite_stays_where_it_belongs(kind, where, softcap, dtype):
+    T, past, H, G, D, scale = 130, 300, 6, 2, 72, 72 ** -0.5
+    gen = torch.Generator(device="cuda").manual_seed(where)
+    q, k, v = (torch.randn(n, h, D, device="cuda", generator=gen) for n, h in ((T, H), (past + T, G), (past + T, G)))
+    k, v = k.bfloat16(), v.bfloat16()
+    q[..., 5], q[..., 9] = -q[..., 5].abs(), 0.5       # three parts of 0.5 are 0.5, 0 and 0
+    t = max(0, where - past)                           # queries t, t + 1, ... see the row
+    if kind.startswith("key"):
+        k[where, 0, 5] = math.inf if kind == "key -inf" else -math.inf
+    elif kind.startswith("value"):
+        v[where, 0, 9] = math.inf if kind == "value inf" else math.nan
+    else:
+        q[t, 1, 9] = math.inf
+    if softcap and not kind.startswith("value"):
+        pytest.skip("the cap makes these scores finite or NaN by a tanh of its own")
+    y = _portion(q, k, v, past, scale, dtype=dtype, softcap=softcap).double()
+    seen = None
+    if kind == "key -inf":     # a weight of zero: the key of head group 0 might as well not be there
+        seen = torch.ones(H, T, past + T, dtype=torch.bool, device="cuda")
+        seen[:H // G, :, where] = False
+    clean = q.nan_to_num(0.0, 0.0, 0.0)
+    if softcap:
+        s = _scores(clean, k, past, scale)
+        s = torch.where(s.isinf(), s, softcap * torch.tanh(s / softcap))
+        want = torch.matmul(torch.softmax(s, -1), torch.nan_to_num(v.double(), 0.0, 0.0, 0.0).repeat_interleave(H // G, 1).transpose(0, 1)).transpose(0, 1)
+    else:
+        want = _want(clean, k, v, past, scale, seen)
+    if kind == "key +inf":
+        want[t:, :H // G] = math.nan
+    elif kind.startswith("value"):
+        want[t:, :H // G, 9] = math.inf if kind == "value inf" else math.nan
+    elif kind == "query inf":
+        want[t, 1] = math.nan                          # infinities of both signs among the scores
+    if where == 0 and kind == "key -inf" and past == 0:
+        want[0, :H // G] = 0
+    assert torch.equal(y.isnan(), want.isnan()) and torch.equal(y.isinf(), want.isinf())
+    keep = want.isfinite()
+    err = ((y - want)[keep].norm() / want[keep].norm()).item()
+    assert err <= (8 * 2.0 ** -24 * math.sqrt(D) if dtype == torch.float32 else 2.0 ** -8), err
