@@ -113,12 +113,12 @@ __global__ void __launch_bounds__(128) bounded_sum_kernel(const CcSeqBoundedSum 
 }
 
 template <typename ST, typename AT, int VEC>
-__global__ void __launch_bounds__(128) embed_bounded_kernel(const int32_t* tokens, const ST* __restrict__ embed, const CcSeqBounded emb_p,
-                                                            float* __restrict__ x, const CcSeqBounded next_p, AT* __restrict__ h, int T, int E) {
+__global__ void __launch_bounds__(128) embed_bounded_kernel(const int32_t* tokens, const ST* embed, const CcSeqBounded emb_p, float* x, const CcSeqBounded next_p,
+                                                            AT* h, int T, int E) {
     const int c = (blockIdx.x * blockDim.x + threadIdx.x) * VEC;
+    ccs::pdl_wait_release();
     if (c >= E) return;
     const Bounded<VEC> emb(emb_p, c), next(next_p, c);
-    ccs::pdl_wait_release();
     for (int t = blockIdx.y; t < T; t += gridDim.y) {
         Pack<VEC> s = load<VEC>(embed + (size_t)tokens[t] * E + c);
 #pragma unroll

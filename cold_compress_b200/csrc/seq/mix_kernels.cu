@@ -255,7 +255,7 @@ __global__ void __launch_bounds__(256) latent_prepare_kernel(const CcSeqLatentPr
 // Rotation of one segment of every head of a fused query row, in place; optionally the rotated segment is also
 // copied to `tail` (the absorbed query layout [H, tail_ld] at column tail_off).
 __global__ void rope_heads_kernel(float* q, int64_t ld, const int32_t* input_pos,
-                                  const float* __restrict__ inv_freq, int H, int head_w, int off, int seg, int dims,
+                                  const float* inv_freq, int H, int head_w, int off, int seg, int dims,
                                   float* tail, int64_t tail_ld, int tail_off, int T, int interleaved) {
     ccs::pdl_wait_release();
     const int t = blockIdx.x, half = dims / 2;
@@ -314,7 +314,7 @@ __global__ void head_gate_kernel(ST* __restrict__ y, const float* __restrict__ g
     }
 }
 
-__device__ __forceinline__ void read8(const float* p, float* o) {     // as load8, for what a launch before has written
+__device__ __forceinline__ void read8(const float* p, float* o) {     // as load8, in kernels that start under their predecessor
     const float4 a = reinterpret_cast<const float4*>(p)[0], b = reinterpret_cast<const float4*>(p)[1];
     o[0] = a.x; o[1] = a.y; o[2] = a.z; o[3] = a.w; o[4] = b.x; o[5] = b.y; o[6] = b.z; o[7] = b.w;
 }
@@ -325,8 +325,8 @@ __device__ __forceinline__ void read8(const bf16* p, float* o) {
     for (int i = 0; i < 8; ++i) o[i] = __bfloat162float(e[i]);
 }
 
-// out[h, n] = W[h, n, :] . x[h, :]  (* sigmoid(gate[h])): a block-diagonal one-token product, a warp per row whose first
-// 256 weights are requested before the launch waits.
+// out[h, n] = W[h, n, :] . x[h, :]  (* sigmoid(gate[h])): a block-diagonal one-token product, a warp per row, which is asked
+// for in L2 before the launch waits.
 template <typename WT, typename XT, typename OT>
 __global__ void __launch_bounds__(256) head_gemv_kernel(const WT* W, const XT* x, int64_t sx, OT* out, int64_t so, const float* gate, int H, int N, int K) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -335,15 +335,15 @@ __global__ void __launch_bounds__(256) head_gemv_kernel(const WT* W, const XT* x
     const WT* w = W + ((size_t)h * N + n) * K;
     const XT* xh = x + (size_t)h * sx;
     const bool vec = K % 8 == 0 && (((uintptr_t)w | (uintptr_t)xh) & 15) == 0;
-    float a[8];
-    if (vec && lane * 8 < K) load8(w + lane * 8, a);
+    if (vec)
+        for (int k = lane * (128 / (int)sizeof(WT)); k < K; k += 32 * (128 / (int)sizeof(WT))) ccs::ask_l2(w + k);
     ccs::pdl_wait_release();
     if ((int)blockIdx.x * 8 + warp >= H * N) return;
     float acc = 0.f;
     if (vec) {
         for (int k = lane * 8; k < K; k += 256) {
-            float b[8];
-            if (k >= 256) load8(w + k, a);
+            float a[8], b[8];
+            read8(w + k, a);
             read8(xh + k, b);
 #pragma unroll
             for (int i = 0; i < 8; ++i) acc = fmaf(a[i], b[i], acc);
@@ -1103,7 +1103,7 @@ __device__ __forceinline__ void bounded_row(const CcSeqBoundedSum& p, int n, flo
 // A weight vector that is read once: past L1
 __device__ __forceinline__ uint4 ld_weights(const uint4* p) {
     uint4 u;
-    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(u.x), "=r"(u.y), "=r"(u.z), "=r"(u.w) : "l"(p));
+    asm volatile("ld.global.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(u.x), "=r"(u.y), "=r"(u.z), "=r"(u.w) : "l"(p));
     return u;
 }
 
@@ -1113,7 +1113,7 @@ constexpr int GEMV_CTAS = 4;       // CTAs per SM (64 registers per thread)
 
 // A warp takes two neighbouring rows, KS warps share them (KS == 1: a warp walks rows_per_cta / 16 pairs, 16 rows apart).  A
 // lane keeps eight weight vectors in flight across the ends of rows: a slot is requested again as soon as it is used.  The
-// first ones are on their way before the kernel waits for the one before it.
+// first ones are asked for in L2 before the kernel waits for the one before it.
 // Bound: HBM for many rows; the input's 32 bytes from shared memory per 16 bytes of weights held one row per warp below it
 // (16384 x 2048, alone in a graph: 14.4 us, without those reads 11.4, floor 10.2).  Decode step of a 4-layer model of width
 // 2048 at 4096 positions: 370 us with one row per warp, four loads in flight and every launch behind the one before it, 338
@@ -1140,13 +1140,20 @@ __global__ void __launch_bounds__(256, GEMV_CTAS) gemv_multi_kernel(const CcSeqG
     const bool vec = K % VEC == 0;
     const int nv = K / VEC, v0 = lane + 32 * ks;    // this lane's vectors of a row: v0, v0 + STEP, ...
     auto row = [&](int n) { return reinterpret_cast<const uint4*>(W + (size_t)min(n, jb.N - 1) * K); };   // rows past the end: the last one
+    if (vec && lane % 8 == 0) {      // a line of 128 bytes per request
+#pragma unroll
+        for (int u = 0; u < GEMV_AHEAD; ++u)
+#pragma unroll
+            for (int r = 0; r < GEMV_ROWS; ++r)
+                if (v0 + STEP * u < nv) ccs::ask_l2(row(n0 + r) + v0 + STEP * u);
+    }
+    ccs::pdl_wait_release();
     uint4 buf[GEMV_ROWS][GEMV_AHEAD];
 #pragma unroll
     for (int u = 0; u < GEMV_AHEAD; ++u)
 #pragma unroll
         for (int r = 0; r < GEMV_ROWS; ++r)
             buf[r][u] = vec && v0 + STEP * u < nv ? ld_weights(row(n0 + r) + v0 + STEP * u) : make_uint4(0u, 0u, 0u, 0u);
-    ccs::pdl_wait_release();
     bool shared_row = false;
     if constexpr (PRE != CC_GEMV_PRE_NONE) shared_row = jb.x == nullptr;
     if (shared_row) {
