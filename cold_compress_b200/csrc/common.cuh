@@ -162,8 +162,9 @@ __device__ __forceinline__ void fence_proxy_async() {
 // ------------------------------------------------------------------ programmatic dependent launch
 // A kernel launched with cudaLaunchAttributeProgrammaticStreamSerialization may start while its
 // predecessor in the stream is still running.  Everything before pdl_wait() must only touch memory
-// no in-flight predecessor writes (weights, the K/V cache, policy state of this layer);
-// pdl_wait() returns when the predecessor grid has completed and its writes are visible.
+// the predecessor does not write (weights; with the caller's promise the K/V cache and the policy state of this layer);
+// pdl_wait() returns when the predecessor grid has completed and its writes are visible.  Dependents are launched after
+// pdl_wait(): a kernel that reads ahead then runs beside its own predecessor alone, never beside an older kernel.
 // Without the launch attribute both are no-ops.
 __device__ __forceinline__ void pdl_launch_dependents() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

@@ -175,10 +175,10 @@ cc_decode_kernel(const __grid_constant__ DecodeParams p) {
     cluster_arrive_release();
     bool b0_waited = false;
     // Without the promise that the predecessor leaves this cache alone nothing of it is read before the predecessor has
-    // ended; the launch, the barriers and the cluster's start above run under it all the same.  Dependents are released
-    // only after this wait, so a kernel that does read ahead never meets one older than its own predecessor.
-    // (32 steps back to back in a graph: 64-slot sliding caches 8.8 -> 8.2 us a step, 1024 heavy-hitter slots 11.4 -> 10.9.)
-    if (!(p.a.flags & CC_FLAG_OVERLAP_PREDECESSOR)) pdl_wait();
+    // ended; the launch, the barriers and the cluster's start above run under it all the same.  (32 steps back to back in a
+    // graph: 64-slot sliding caches 8.8 -> 8.2 us a step, 1024 heavy-hitter slots 11.4 -> 10.9.)
+    const bool ahead = p.a.flags & CC_FLAG_OVERLAP_PREDECESSOR;
+    if (!ahead) pdl_wait();
 
     // ---- hybrid: per-head decision from scalars (every CTA of the cluster computes the same)
     int hyb_mode = kHybAppend, hyb_bits = 0, hyb_cts = 0, hyb_rw = 0;
@@ -248,7 +248,9 @@ cc_decode_kernel(const __grid_constant__ DecodeParams p) {
         maskb[lr] = (s < L) ? st.mask[(size_t)h * L + s] : 0;
     }
 
-    pdl_launch_dependents();  // the next kernel in the stream may start its own independent prologue
+    // The next kernel in the stream may start its own prologue.  Never before this kernel has waited: the one after may read
+    // ahead too, on the promise that THIS kernel leaves its cache alone, and must not meet the kernel before this one.
+    if (!ahead) pdl_launch_dependents();
 
     // ---- 1. L2 only: key_norm.max() over every head and slot (cache.py:602) = X0 exchange
     float l2_max = 0.f;
@@ -384,7 +386,10 @@ cc_decode_kernel(const __grid_constant__ DecodeParams p) {
     // Everything above reads only this layer's cache and policy state, which no kernel in flight
     // writes (CC_FLAG_OVERLAP_PREDECESSOR); q / k_new / v_new come from the projection kernel launched
     // just before this one: wait for it here, with the K/V tiles already on their way.
-    pdl_wait();
+    if (ahead) {
+        pdl_wait();
+        pdl_launch_dependents();
+    }
     // query rows of this KV group and the new value slice, in registers
     float q[G][8];
     uint4 vnew8 = make_uint4(0, 0, 0, 0);

@@ -248,8 +248,8 @@ __device__ __forceinline__ bool combine_split(float (*part)[R], float (&out)[R])
         const __nv_bfloat16* rows[R_] = ROWS_OF;                                                    \
         wd.prefetch(rows, k0, k0 + klen);                                                           \
     }                                                                                               \
-    pdl_launch_dependents();                                                                        \
     pdl_wait();                                                                                     \
+    pdl_launch_dependents();                                                                        \
     stage_input(p.x, p.norm_w, p.eps, p.K, xs, scratch, p.tp);
 
 // ---------------------------------------------------------------- attention_norm -> wqkv -> RoPE

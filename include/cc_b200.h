@@ -59,7 +59,8 @@ extern "C" {
                                           not write this layer's cache or policy state (it is the q/k/v
                                           projection, or another layer's step): cc_decode_step may then
                                           start early (programmatic dependent launch) and fetch K/V and
-                                          policy state while that kernel is still running               */
+                                          policy state while that kernel is still running.  Older kernels
+                                          have ended by then and may have written anything.              */
 
 #define CC_FLAG_VIA_TOKEN_KERNEL     2  /* tests: run this step through the attention stage of the whole-token
                                           kernel (cc_decode_token) instead of the per-layer kernel: same results,
@@ -289,6 +290,8 @@ typedef struct CcTpArgs {
  * cc_gemv_residual:   out = [residual +] W x      (wo: model.py:431,317; w2: 443,326; output head: 290-291)
  * cc_rmsnorm_ffn_gate: out = silu(w1 xn) * (w3 xn), xn = ffn_norm(x)   (model.py:442-443)
  * tp (may be NULL) fuses the tensor-parallel all-reduce into producer / consumer, see CcTpArgs.
+ * The three read their first weights while the kernel launched just before them on the stream may still be running: that
+ * kernel must not be the one that writes the weights (any launch between the two is enough).
  */
 int cc_rmsnorm_qkv_rope(const void* x, const void* norm_w, float eps, const void* wqkv, const void* bias,
                         const void* freqs_cis, const int32_t* input_pos, void* q, void* k, void* v,

@@ -40,3 +40,16 @@ def test_nothing_is_read_before_the_wait(file, name, head, body):
 def test_no_memory_is_read_through_the_read_only_path(file, name, head, body):
     assert "__restrict__" not in head.replace("__grid_constant__", "")
     assert "__ldg" not in body and "load8(" not in body and "warp_dot" not in body and ".nc." not in body
+
+
+def test_kernels_that_read_ahead_release_no_one_before_they_have_waited():
+    """A kernel may read its cache or its weights ahead because its predecessor does not write them.  That says nothing about
+    older kernels, which therefore have to be done: every kernel releases its dependents only after its own wait."""
+    gemv = (CSRC / "gemv.cu").read_text()
+    assert 0 < gemv.index("pdl_wait();") < gemv.index("pdl_launch_dependents();") and gemv.count("pdl_launch_dependents();") == 1
+    lines = [re.sub(r"//.*", "", x).strip() for x in (CSRC / "decode_step.cu").read_text().split("\n")]
+    lines = [x for x in lines if x]
+    waits, releases = ([i for i, x in enumerate(lines) if call in x] for call in ("pdl_wait();", "pdl_launch_dependents();"))
+    assert len(waits) == len(releases) == 2
+    assert lines[waits[0]] == "if (!ahead) pdl_wait();" and lines[releases[0]] == "if (!ahead) pdl_launch_dependents();" and waits[0] < releases[0]
+    assert lines[waits[1] - 1] == "if (ahead) {" and releases[1] == waits[1] + 1
