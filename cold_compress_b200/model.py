@@ -429,7 +429,7 @@ class FeedForward(nn.Module):
 
     def forward(self, x: Tensor) -> Tensor:
         a, b = self.w1(x), self.w3(x)
-        if ops.plain_rows(a, b):
+        if ops.plain_rows(a, b) and a.shape == b.shape:
             gated = torch.empty_like(a)
             ops.silu_mul(a, b, gated)
         else:
@@ -447,7 +447,7 @@ class RMSNorm(nn.Module):
         self.weight = nn.Parameter(torch.ones(dim))
 
     def forward(self, x: Tensor) -> Tensor:
-        if x.shape[-1] == self.weight.numel() <= 16384 and ops.plain_rows(x, self.weight):
+        if ops.plain_rows(x, self.weight) and x.shape[-1:] == self.weight.shape and x.shape[-1] <= 16384:
             out = torch.empty_like(x)
             ops.rmsnorm_rows(x, self.weight, self.eps, out)
             return out
