@@ -9,6 +9,7 @@
 //   * dependents are released after pdl_wait(), so a kernel that starts early meets no kernel older than its own predecessor.
 #pragma once
 #include <cuda_runtime.h>
+#include <stdlib.h>
 
 namespace ccs {
 
@@ -21,6 +22,12 @@ __device__ __forceinline__ void pdl_wait_release() {
 
 __device__ __forceinline__ void ask_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
+// CC_B200_PDL=0 turns programmatic dependent launch off, here as in the main library.
+inline bool pdl_enabled() {
+    static const bool on = [] { const char* e = getenv("CC_B200_PDL"); return !(e && e[0] == '0'); }();
+    return on;
+}
+
 template <typename... P, typename... A>
 inline cudaError_t launch_under(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
     cudaLaunchConfig_t cfg = {};
@@ -32,7 +39,7 @@ inline cudaError_t launch_under(void (*kern)(P...), dim3 grid, dim3 block, size_
     attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr.val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = &attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = pdl_enabled() ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kern, P(args)...);
 }
 
