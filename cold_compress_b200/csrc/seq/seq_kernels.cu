@@ -705,7 +705,7 @@ __global__ void __launch_bounds__(DEC_THREADS) attn_decode_kernel(const CcSeqAtt
 }
 
 // ---- the same for rows of whole 16-byte vectors and up to 8 query heads per key/value head
-// A run of 128-key tiles per CTA; the key and value rows of a tile are all requested at once (cp.async, the next tile under
+// A run of VT-key tiles per CTA; the key and value rows of a tile are all requested at once (cp.async, the next tile under
 // this one) before anything is known about their slots, which are checked meanwhile.  Scores: eight lanes per key, four keys
 // at a time, the query rows read from shared memory once for the four.  Values: a thread owns a 16-byte column group and
 // every nkg-th key.  Two fp32 operations per instruction in both.  Partials and their combination as above, 16 bytes a load
@@ -714,12 +714,15 @@ __global__ void __launch_bounds__(DEC_THREADS) attn_decode_kernel(const CcSeqAtt
 // bandwidth.  8 layers, 32 / 8 heads of 128, 4096 positions in a graph: 32 us a layer on the kernel above (a thread walks a
 // row, values are read after the scores), 27 with rows requested at once, 18 with 256 threads, 128-key tiles, paired operations and ring
 // places without a division per row.
-constexpr int VT = 128, VD_THREADS = 256, VD_MAX_SPLITS = 64, VD_RMAX = 8;
+constexpr int VD_THREADS = 256, VD_MAX_SPLITS = 64, VD_RMAX = 8;
 
-__host__ __device__ inline int vd_splits(int L, int reach, int G) {     // runs per head: two CTAs per SM over the heads
-    const long long maxkeys = reach > 0 ? (reach < L + 1 ? reach : L + 1) : (long long)L + 1;
-    const long long tiles = (maxkeys + VT - 1) / VT;
-    long long most = 296 / G;
+// tiles of VT keys that a head can have at most, and the runs they are cut into: as many CTAs over the heads as the GPU holds at once
+inline long long vd_tiles(int L, int reach, int VT) {
+    const long long maxkeys = reach > 0 && reach <= L ? reach : (long long)L + 1;
+    return (maxkeys + VT - 1) / VT;
+}
+inline int vd_splits(long long tiles, int G, int per_sm) {
+    long long most = 148 * per_sm / G;
     if (most < 1) most = 1;
     if (most > VD_MAX_SPLITS) most = VD_MAX_SPLITS;
     return (int)(tiles < most ? tiles : most);
@@ -754,8 +757,8 @@ __device__ __forceinline__ void as_pairs(const uint4& u, f32x2 (&v)[4], const __
     for (int i = 0; i < 4; ++i) v[i] = pair(__uint_as_float(w[i] << 16), __uint_as_float(w[i] & 0xffff0000u));
 }
 
-template <typename CT, typename YT, int RMAX>
-__global__ void __launch_bounds__(VD_THREADS, RMAX <= 4 ? 2 : 1) attn_decode_rows_kernel(const CcSeqAttn a, int buffers) {
+template <typename CT, typename YT, int RMAX, int VT>
+__global__ void __launch_bounds__(VD_THREADS, RMAX <= 4 ? 2 : 1) attn_decode_rows_kernel(const CcSeqAttn a, int buffers, int NS) {
     extern __shared__ float4 smd4[];
     constexpr int VEC = 16 / (int)sizeof(CT), VP = VEC / 2, WARPS = VD_THREADS / 32, KEYS = VT / WARPS, KI = KEYS / 4;
     const int R = a.H / a.G, Dk = a.Dk, Dv = a.Dv, kc16 = Dk / VEC, vc16 = Dv / VEC;
@@ -774,10 +777,9 @@ __global__ void __launch_bounds__(VD_THREADS, RMAX <= 4 ? 2 : 1) attn_decode_row
     const int j_lo = a.block > 0 ? (p / a.block) * a.block : (a.window > 0 ? max(0, p - a.window + 1) : 0);
     const int kx = a.window > 0 ? min(a.keep_first, j_lo) : 0;
     const int n = kx + (p - j_lo + 1);
-    const int n_tiles = (n + VT - 1) / VT, NS = vd_splits(a.L, attn_reach(a), a.G);
-    const int tiles_per = (n_tiles + NS - 1) / NS, nsplit = (n_tiles + tiles_per - 1) / tiles_per;
+    const int n_tiles = (n + VT - 1) / VT, nsplit = min(n_tiles, NS);      // runs of n_tiles / nsplit tiles, or of one more
     if (sp >= nsplit) return;
-    const int tile0 = sp * tiles_per, tile_end = min(n_tiles, tile0 + tiles_per), ring = a.L - a.keep_first;
+    const int tile0 = (int)((long long)sp * n_tiles / nsplit), tile_end = (int)((long long)(sp + 1) * n_tiles / nsplit), ring = a.L - a.keep_first;
     // copies: thread = column c of rows row, row + step, ...
     const int k_step = VD_THREADS / kc16, k_first = tid / kc16, k_col = tid - k_first * kc16;
     const int v_step = VD_THREADS / vc16, v_first = tid / vc16, v_col = tid - v_first * vc16;
@@ -979,7 +981,8 @@ __global__ void __launch_bounds__(VD_THREADS, RMAX <= 4 ? 2 : 1) attn_decode_row
     if (!s_last) return;
     __threadfence();
     // the last CTA of the head: every other one has finished reading; combine in split order
-    float* const wgt = Ps;     // [R][VT] weights of the splits (at most VD_MAX_SPLITS < VT)
+    static_assert(VD_MAX_SPLITS <= VT, "the weights of the splits take the place of a tile's");
+    float* const wgt = Ps;     // [R][VT]
     for (int r = warp; r < R; r += WARPS) {
         const float sk = sink_of(r);
         const float* pm = part_m + (size_t)g * NS * R + r;
@@ -1288,18 +1291,26 @@ static bool decode_rows_serves(const CcSeqAttn* a) {
 
 template <typename CT, typename YT, int RMAX>
 static int launch_decode_rows(const CcSeqAttn* a, cudaStream_t st) {
-    const int NS = vd_splits(a->L, attn_reach(*a), a->G);
-    const long long reach = attn_reach(*a) > 0 && attn_reach(*a) < a->L + 1 ? attn_reach(*a) : (long long)a->L + 1;
-    const size_t row = sizeof(CT) * (size_t)(a->Dk + a->Dv) + 16;
-    const int buffers = (reach + VT - 1) / VT > NS && 2 * VT * row <= 200 * 1024 ? 2 : 1;      // a run can be longer than one tile
-    const size_t tiles = (size_t)buffers * VT * row;
-    const int vc16 = a->Dv * (int)sizeof(CT) / 16;
+    // Two CTAs per SM, one where eight query heads' registers leave room for no more: tiles of 128 keys if one fits a CTA's share of
+    // the shared memory, of 64 otherwise, and a second buffer for runs of more than one tile only if it fits too.  Runs of 5500 /
+    // 12000 / 32000 positions with a second buffer and one CTA per SM where two were counted on, and as it is now, in us: bf16
+    // 32 / 8 heads of 128 39.0 / 52.3 / 114.1 and 26.0 / 34.7 / 73.8; fp32 45.7 / 65.2 / 141.7 and 27.9 / 48.9 / 105.1; fp32 16 / 16 of 64
+    // 39.3 / 66.2 / 145.8 and 22.0 / 39.3 / 88.6.  Two buffers of 64 keys for bf16 rows of 128 + 128: 25.5 / 39.7 / 88.1.
+    const int vc16 = a->Dv * (int)sizeof(CT) / 16, per_sm = RMAX <= 4 ? 2 : 1;
+    const size_t share = (per_sm == 2 ? 111 : 223) * 1024;
     const size_t red = sizeof(float) * (size_t)(VD_THREADS / vc16) * (a->H / a->G) * a->Dv;
-    const size_t smem = (tiles > red ? tiles : red) + sizeof(float) * RMAX * (size_t)(a->Dk + VT);
-    auto kern = attn_decode_rows_kernel<CT, YT, RMAX>;
+    auto bytes = [&](int buffers, int VT) {
+        const size_t tiles = (size_t)buffers * VT * (sizeof(CT) * (size_t)(a->Dk + a->Dv) + 16);
+        return (tiles > red ? tiles : red) + sizeof(float) * RMAX * (size_t)(a->Dk + VT);
+    };
+    const int VT = bytes(1, 128) <= share ? 128 : 64;
+    const long long tiles = vd_tiles(a->L, attn_reach(*a), VT);
+    const int NS = vd_splits(tiles, a->G, per_sm), buffers = tiles > NS && bytes(2, VT) <= share ? 2 : 1;
+    const size_t smem = bytes(buffers, VT);
+    auto kern = VT == 128 ? attn_decode_rows_kernel<CT, YT, RMAX, 128> : attn_decode_rows_kernel<CT, YT, RMAX, 64>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return fail(CC_SEQ_ERR_CUDA, cudaGetErrorString(e));
-    launch_under(kern, dim3(NS, a->G), dim3(VD_THREADS), smem, st, *a, buffers);
+    launch_under(kern, dim3(NS, a->G), dim3(VD_THREADS), smem, st, *a, buffers, NS);
     return cuda_check("attn_decode_rows_kernel");
 }
 
@@ -1380,7 +1391,7 @@ int cc_seq_attention(const CcSeqAttn* a, void* stream) {
 }
 
 uint64_t cc_seq_decode_workspace(int32_t H, int32_t G, int32_t Dv, int32_t L, int32_t window) {
-    const uint64_t narrow = (uint64_t)decode_max_splits(L, window), wide = (uint64_t)vd_splits(L, window, G < 1 ? 1 : G);
+    const uint64_t narrow = (uint64_t)decode_max_splits(L, window), wide = (uint64_t)vd_splits(vd_tiles(L, window, 64), G < 1 ? 1 : G, 2);
     const uint64_t NS = narrow > wide ? narrow : wide;       // either kernel may serve the call
     return sizeof(int) * (uint64_t)((G + 3) & ~3) + sizeof(float) * NS * (uint64_t)H * (2 + (uint64_t)Dv) + 16;
 }

@@ -106,3 +106,16 @@ def test_what_is_not_finite_stays_where_it_belongs(kind, where, softcap, dtype):
     keep = want.isfinite()
     err = ((y - want)[keep].norm() / want[keep].norm()).item()
     assert err <= (8 * 2.0 ** -24 * math.sqrt(D) if dtype == torch.float32 else 2.0 ** -8), err
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("shape", [
+    (4735, 32, 8, 128, 128, {}), (4736, 8, 8, 128, 128, {}), (5500, 32, 8, 128, 128, dict(sink=1)),      # as many tiles as runs, one more, some runs of two
+    (9000, 8, 8, 64, 64, {}), (9001, 16, 16, 64, 64, dict(sink=2)),                                      # runs that fetch ahead
+    (2400, 64, 8, 128, 128, {}), (6000, 64, 8, 64, 128, {}),                                             # eight query heads: one CTA per SM
+    (8200, 2, 1, 256, 128, {}), (5000, 6, 2, 256, 256, {}),                                              # tiles of 64 keys, more of them than runs
+    (6000, 16, 16, 128, 128, dict(window=3000, sink=1)),
+], ids=lambda s: f"past{s[0]}-H{s[1]}-G{s[2]}-{s[3]}x{s[4]}" + "".join(f"-{k}{v}" for k, v in s[5].items()))
+def test_one_token_over_runs_of_several_tiles(shape, dtype):
+    import test_gpu_attention_tiles as tiles
+    tiles.test_one_token_matches_64_bit_attention(shape, dtype)
