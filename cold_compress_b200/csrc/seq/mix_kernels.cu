@@ -360,15 +360,15 @@ __global__ void __launch_bounds__(256) head_gemv_kernel(const WT* W, const XT* x
 
 // ------------------------------------------------------------------------------------------------ matrix-state recurrence
 // Per head a state S [D, D] (key channel i, value channel j):  o_t[j] = sum_i r_t[i] (S[i][j] + u[i] k_t[i] v_t[j]),
-// then S[i][j] <- w_t[i] S[i][j] + k_t[i] v_t[j], with w_t = exp(-exp(wraw_t + w0)).  A CTA owns WKV_J value
+// then S[i][j] <- w_t[i] S[i][j] + k_t[i] v_t[j], with w_t = exp(-exp(wraw_t + w0)).  A CTA owns J value
 // channels of one head; thread (part, j) keeps CH rows of column j in registers.  Tokens are staged TB at a
 // time; the parts' partial outputs meet in shared memory after each batch, summed in part order, so the arithmetic of
 // a token does not depend on how the sequence was cut into launches.
-// Bound: the latencies of one warp per scheduler.  16 columns per CTA: 32 columns left half of the SMs without work at 32
-// heads of 64; the decays of long steps come from a launch of their own, since every column tile of a head needs them (two
+// Bound: the latencies of one warp per scheduler.  16 columns per CTA where 32 leave SMs without work (half of them at 32
+// heads of 64); the decays of long steps come from a launch of their own, since every column tile of a head needs them (two
 // expf each); the next token's operands are read while one is computed, and two rows share an instruction.  4096 tokens, 32
 // heads of 64: 808 us -> 592 (columns, decays, 16-byte staging) -> 408; 4 rows per thread and twice the warps: 406, other bits.
-constexpr int WKV_J = 16;   // template: TB tokens per staged batch (fewer when a wide head would not fit), CH state rows per thread
+// Template: TB tokens per staged batch (fewer when a wide head would not fit), CH state rows per thread, J columns per CTA.
 
 __device__ __forceinline__ void cp_async4(float* dst, const float* src) {
     const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
@@ -415,15 +415,15 @@ __global__ void __launch_bounds__(256) wkv_decay_kernel(const float* __restrict_
 // Shared memory: two buffers of [r | k | w | v] for WKV_TB tokens (the next batch is copied in asynchronously while
 // this one is computed; rows are padded to a multiple of 4 floats so that a thread reads its 16 key channels with
 // 16-byte loads), then the parts' partial outputs.
-template <int TB, int CH>
-__global__ void __launch_bounds__(256) wkv_kernel(const CcSeqWkv a) {
+template <int TB, int CH, int J>
+__global__ void __launch_bounds__(16 * J) wkv_kernel(const CcSeqWkv a) {
     extern __shared__ float4 smw4[];
     float* sm = reinterpret_cast<float*>(smw4);
     const int D = a.D, P = (D + CH - 1) / CH, Dp = P * CH;
-    const int buf_floats = TB * (3 * Dp + WKV_J);
+    const int buf_floats = TB * (3 * Dp + J);
     float* __restrict__ part = sm + 2 * buf_floats;    // [TB][P][J]
-    const int h = blockIdx.x, j0 = blockIdx.y * WKV_J;
-    const int tid = threadIdx.x, nth = blockDim.x, jl = tid % WKV_J, p = tid / WKV_J, j = j0 + jl;
+    const int h = blockIdx.x, j0 = blockIdx.y * J;
+    const int tid = threadIdx.x, nth = blockDim.x, jl = tid % J, p = tid / J, j = j0 + jl;
     const int i0 = p * CH;
     const size_t HD = (size_t)a.H * D;
     float* S = a.state + (size_t)h * D * D;
@@ -469,8 +469,8 @@ __global__ void __launch_bounds__(256) wkv_kernel(const CcSeqWkv a) {
                 }
             }
         }
-        for (int idx = tid * unit; idx < nt * WKV_J; idx += nth * unit) {
-            const int t = idx / WKV_J, c = idx - t * WKV_J;
+        for (int idx = tid * unit; idx < nt * J; idx += nth * unit) {
+            const int t = idx / J, c = idx - t * J;
             if (j0 + c >= D) continue;
             float* d = buf + 3 * TB * Dp + idx;
             const float* s = a.v + (size_t)(tb + t) * HD + (size_t)h * D + j0 + c;
@@ -509,7 +509,7 @@ __global__ void __launch_bounds__(256) wkv_kernel(const CcSeqWkv a) {
                 kv4[c4] = reinterpret_cast<const float4*>(kb + t * Dp)[c4];
                 wv[c4] = reinterpret_cast<const float4*>(wb + t * Dp)[c4];
             }
-            v = vs[t * WKV_J + jl];
+            v = vs[t * J + jl];
         };
         read(0);
 #pragma unroll 4
@@ -533,14 +533,14 @@ __global__ void __launch_bounds__(256) wkv_kernel(const CcSeqWkv a) {
             float a0, a1, a2, a3;
             unpair(acc[0], a0, a1);
             unpair(acc[1], a2, a3);
-            part[(t * P + p) * WKV_J + jl] = (a0 + a1) + (a2 + a3);
+            part[(t * P + p) * J + jl] = (a0 + a1) + (a2 + a3);
         }
         __syncthreads();
-        for (int idx = tid; idx < nt * WKV_J; idx += nth) {
-            const int t = idx / WKV_J, c = idx - t * WKV_J;
+        for (int idx = tid; idx < nt * J; idx += nth) {
+            const int t = idx / J, c = idx - t * J;
             if (j0 + c >= D) continue;
             float o = 0.f;
-            for (int q = 0; q < P; ++q) o += part[(t * P + q) * WKV_J + c];
+            for (int q = 0; q < P; ++q) o += part[(t * P + q) * J + c];
             a.o[(size_t)(tb + t) * HD + (size_t)h * D + j0 + c] = o;
         }
     }
@@ -1277,32 +1277,43 @@ static GemvSplit gemv_split(const CcSeqGemvMulti* g, size_t smem, int elem) {
     return s;
 }
 
-template <int TB, int CH>
+template <int TB, int CH, int J>
 static int launch_wkv(const CcSeqWkv* a, cudaStream_t st) {
     const int P = (a->D + CH - 1) / CH;
-    const size_t smem = sizeof(float) * (2 * (size_t)TB * (3 * P * CH + WKV_J) + (size_t)TB * P * WKV_J);
+    const size_t smem = sizeof(float) * (2 * (size_t)TB * (3 * P * CH + J) + (size_t)TB * P * J);
     static size_t configured = 48 * 1024;
     if (smem > configured) {
         configured = smem;
-        if (cudaFuncSetAttribute(wkv_kernel<TB, CH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+        if (cudaFuncSetAttribute(wkv_kernel<TB, CH, J>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
             return cuda_check("wkv: shared memory");
     }
-    dim3 grid(a->H, (a->D + WKV_J - 1) / WKV_J);
-    wkv_kernel<TB, CH><<<grid, P * WKV_J, smem, st>>>(*a);
+    dim3 grid(a->H, (a->D + J - 1) / J);
+    wkv_kernel<TB, CH, J><<<grid, P * J, smem, st>>>(*a);
     return cuda_check("wkv_kernel");
 }
 
-// 8 state rows per thread up to 128-wide heads (at most 256 threads), 16 above; the token batch shrinks until two
+// 8 state rows per thread up to 128-wide heads (at most 16 J threads), 16 above; the token batch shrinks until two
 // staging buffers and the partial outputs fit in 160 KB.
-template <int CH>
+template <int CH, int J>
 static int dispatch_wkv(const CcSeqWkv* a, cudaStream_t st) {
     const int P = (a->D + CH - 1) / CH;
-    auto bytes = [&](int tb) { return sizeof(float) * (2 * (size_t)tb * (3 * P * CH + WKV_J) + (size_t)tb * P * WKV_J); };
-    if (bytes(32) <= 160 * 1024) return launch_wkv<32, CH>(a, st);
-    if (bytes(16) <= 160 * 1024) return launch_wkv<16, CH>(a, st);
-    return launch_wkv<8, CH>(a, st);
+    auto bytes = [&](int tb) { return sizeof(float) * (2 * (size_t)tb * (3 * P * CH + J) + (size_t)tb * P * J); };
+    if (bytes(32) <= 160 * 1024) return launch_wkv<32, CH, J>(a, st);
+    if (bytes(16) <= 160 * 1024) return launch_wkv<16, CH, J>(a, st);
+    return launch_wkv<8, CH, J>(a, st);
 }
 
+// Columns per CTA: 16 as long as that gives every CTA an SM of its own, and beyond that where the fullest SM then has fewer
+// columns to walk and the decays come ready-made (each column tile of a head forms them otherwise); else 32.  Heads up to 32
+// wide are one tile.  Measured, 16 / 32 columns in us: 32 heads of 64, 4096 tokens 405 / 496, 1 token 3.7 / 3.6; 16 heads of 128,
+// 4096 tokens 518 / 816; 64 heads of 64 534 / 515 and 4.0 / 3.8; 96 of 64 740 / 873 and 4.3 / 4.1; 128 of 64 1031 / 854 and 6.5 / 4.2;
+// 32 of 128 1031 / 835 and 6.5 / 4.2; 32 of 32 461 / 432.
+template <int CH>
+static int dispatch_wkv_columns(const CcSeqWkv* a, cudaStream_t st) {
+    const long long narrow = (long long)a->H * ((a->D + 15) / 16), wide = (long long)a->H * ((a->D + 31) / 32);
+    const bool use_narrow = a->D > 32 && (narrow <= 148 || (a->decayed && (narrow + 147) / 148 * 16 < (wide + 147) / 148 * 32));
+    return use_narrow ? dispatch_wkv<CH, 16>(a, st) : dispatch_wkv<CH, 32>(a, st);
+}
 
 }  // namespace ccm
 
@@ -1449,7 +1460,7 @@ int cc_seq_wkv(const CcSeqWkv* a, void* stream) {
         return fail(CC_SEQ_ERR_INVALID_ARG, "wkv: bad argument");
     if (a->D > 256) return fail(CC_SEQ_ERR_UNSUPPORTED_SHAPE, "wkv: head size above 256");
     cudaStream_t st = (cudaStream_t)stream;
-    return a->D <= 128 ? dispatch_wkv<8>(a, st) : dispatch_wkv<16>(a, st);
+    return a->D <= 128 ? dispatch_wkv_columns<8>(a, st) : dispatch_wkv_columns<16>(a, st);
 }
 
 int cc_seq_wkv_decay(const float* wraw, const float* w0, float* w, int32_t T, int32_t HD, void* stream) {

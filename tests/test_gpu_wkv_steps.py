@@ -41,3 +41,32 @@ def test_any_cut_of_a_sequence_gives_the_same_bits(H, D):
     want = torch.stack(want)
     # D products summed in fp32 and a state that forgets: a few roundings of the sum's size
     assert ((whole.double() - want).norm() / want.norm()).item() <= 4 * 2.0 ** -23 and ((state.double() - S).norm() / S.norm()).item() <= 4 * 2.0 ** -23
+
+
+@pytest.mark.parametrize("H, D", [(3, 24), (9, 256), (10, 200), (46, 64), (49, 40), (80, 64), (33, 128)])
+def test_column_tiles_of_both_widths_give_the_same_bits(H, D):
+    """More heads than one wave of CTAs takes: short portions walk tiles of 32 columns, a long one 16 or 32 by the number of
+    heads, a few heads at a time always 16 (or a single tile of narrow heads)."""
+    from cold_compress_b200 import seq_ops
+    T = seq_ops.WKV_DECAY_FROM + 5
+    gen = torch.Generator(device="cuda").manual_seed(D + H)
+    randn = lambda *s: torch.randn(*s, device="cuda", generator=gen)  # noqa: E731
+    r, k, v, wraw = (randn(T, H, D) for _ in range(4))
+    w0, u = randn(H, D) - 1.5, 0.5 * randn(H, D)
+
+    def run(heads, portions):
+        n, state, out, at = heads.stop - heads.start, torch.zeros(heads.stop - heads.start, D, D, device="cuda"), [], 0
+        for m in portions:
+            o = torch.empty(m, n * D, device="cuda")
+            seq_ops.wkv(*(t[at:at + m, heads].reshape(m, n * D).contiguous() for t in (r, k, v, wraw)), w0[heads].reshape(-1).contiguous(),
+                        u[heads].reshape(-1).contiguous(), state, o, n, D)
+            out.append(o.view(m, n, D))
+            at += m
+        return torch.cat(out), state
+
+    whole, state = run(slice(0, H), (T,))
+    cut, cut_state = run(slice(0, H), (1, 30, T - 31))
+    assert torch.equal(cut, whole) and torch.equal(cut_state, state)
+    for h in range(0, H, 2):
+        some, s = run(slice(h, min(h + 2, H)), (T,))
+        assert torch.equal(some, whole[:, h:h + 2]) and torch.equal(s, state[h:h + 2])
