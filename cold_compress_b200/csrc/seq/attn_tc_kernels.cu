@@ -611,11 +611,14 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const CcSeqAttn a) 
             }
             if (zero != 0.f) atomicOr(&sm.redo[quarter], 1u << lane);
         }
-        asm volatile("bar.sync 5, 512;" ::: "memory");      // everyone's marks, and what this loop writes over is written
-        if (*failed == 0)
+        // the marks of these rows are there, and what row_again writes over is written
+        asm volatile("bar.sync %0, 128;" ::"r"(quarter + 1) : "memory");
+        if (sm.redo[quarter] != 0 && *failed == 0)
 #pragma unroll 1
-            for (int r = warp; r < BM; r += SOFT_THREADS / 32)
-                if (sm.redo[r >> 5] >> (r & 31) & 1u) row_again<YT, SHAPED>(a, ks, (f0 + r) / R, g * R + (f0 + r) % R, g, lane);
+            for (int r = part; r < 32; r += 4) {
+                const int flat = f0 + quarter * 32 + r;
+                if (sm.redo[quarter] >> r & 1u) row_again<YT, SHAPED>(a, ks, flat / R, g * R + flat % R, g, lane);
+            }
     }
     fence_before();
     __syncthreads();
