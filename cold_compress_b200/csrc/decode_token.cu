@@ -2,7 +2,7 @@
 //
 // Replaces the per-token launch chain of the reference's decode_one_token (generation_utils.py:163-178 ->
 // Transformer.forward model.py:268-292 -> 32 x TransformerBlock.forward model.py:307-327 -> greedy sampling
-// generation_utils.py:136-142), which round 1 ran as 5 launches per layer.  A decoded token streams 15 GB of bf16
+// generation_utils.py:136-142), otherwise 5 launches per layer.  A decoded token streams 15 GB of bf16
 // weights plus the live K/V rows exactly once; the only way to keep HBM busy across the ~160 dependent stages of a
 // token is to never stop the stream at a stage boundary.  Design:
 //

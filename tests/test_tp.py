@@ -1,5 +1,5 @@
 """Tensor-parallel tests.  CPU: world_size-2 gloo run of the sharding + all-reduce host logic.
-GPU (needs >= 2 devices, `gpurun --gpus 2`): head-sharded decode reproduces the unsharded run."""
+GPU (needs >= 2 devices): head-sharded decode reproduces the unsharded run."""
 import os
 import subprocess
 import sys
@@ -38,7 +38,7 @@ def test_tp_host_logic_gloo(world):
                                       "heavy_hitter_fused", "recent_global_fused", "heavy_hitter_nccl"])
 def test_tp_decode_world2(strategy):
     if torch.cuda.device_count() < 2:
-        pytest.skip("needs 2 GPUs (gpurun --gpus 2)")
+        pytest.skip("needs 2 GPUs")
     r = _torchrun(2, strategy)
     assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-3000:]
     assert r.stdout.count("tp decode ok") == 2
@@ -49,7 +49,7 @@ def test_tp_decode_world2(strategy):
 def test_tp_decode_world4(strategy):
     """The whole-token kernel with 4 ranks (one KV head per rank): all-reduces inside the kernel over NVLink."""
     if torch.cuda.device_count() < 4:
-        pytest.skip("needs 4 GPUs (gpurun --gpus 4)")
+        pytest.skip("needs 4 GPUs")
     r = _torchrun(4, strategy)
     assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-3000:]
     assert r.stdout.count("tp decode ok") == 4
@@ -59,11 +59,10 @@ def test_tp_decode_world4(strategy):
 @pytest.mark.parametrize("strategy", ["heavy_hitter", "recent_global"])
 def test_tp_decode_world8(strategy):
     """Eight ranks, one KV head each (the BASELINE tensor-parallel layout of Llama-3-8B): the whole-token kernel's
-    second round of partial-vector reads (ranks 4-7) and its 64-CTA-per-head attention stage.  Needs an 8-GPU box
-    (`gpurun --gpus 8`); written after the round's GPU budget was spent, so this test has not run yet -- the tp8 bench
-    line under profiles/r2/ is the only evidence at this world size."""
+    second round of partial-vector reads (ranks 4-7) and its 64-CTA-per-head attention stage.  Needs 8 GPUs; not run yet:
+    the tp8 bench line under profiles/r2/ is the only evidence at this world size."""
     if torch.cuda.device_count() < 8:
-        pytest.skip("needs 8 GPUs (gpurun --gpus 8)")
+        pytest.skip("needs 8 GPUs")
     r = _torchrun(8, strategy)
     assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-3000:]
     assert r.stdout.count("tp decode ok") == 8
