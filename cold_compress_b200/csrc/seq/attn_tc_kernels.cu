@@ -8,15 +8,18 @@
 // that also applies the softmax's rescaling.
 //
 // Bound: tensor pipe and the shared memory it reads: 2 x 24 MMAs of 128 x 128 x 16 per 128 x 128 scores at head size 128,
-// measured 107 cycles each with both operands in shared memory (scores), 74 with the weights in tensor memory (values),
-// 4350 of the 5000 cycles that a tile takes; the other pipes need ~10 instructions per score beside them.  Layout that
+// 107 cycles each with both operands in shared memory (scores) and 74 with the weights in tensor memory (values) by stamps of the
+// SM's clock, where the pipe itself needs 64 (ncu: tensor pipe 49 % active, issue slots 38 %, profiles/rows); together 4350 of the
+// 5000 cycles that a tile takes; the other pipes need ~10 instructions per score beside them.  Layout that
 // follows: the query parts stay in shared memory (96 KB) and the weight parts go to tensor memory, over the scores they came
 // from, as the A operand.  Sixteen warps of softmax, four threads per row.
 //
-// Measured on a B200: 4096 tokens, 32 / 8 heads of 128, learned sinks, 6.17 ms on the FMA kernel -> 0.452 ms (304 TFLOP/s of
-// the attention, 3 times that on the tensor pipe; 0.464 with eight warps); 1001 tokens behind 3333 in a window of 1024, 16 / 4
-// heads, 0.435 ms -> 0.077 ms.  Error of fp32 outputs against 64 bits over shapes, masks and score ranges: 0.15-0.8e-6
-// relative, on the FMA kernel 0.1-2.5e-6, never larger than there.  Descriptors formed ahead of the loop changed nothing.
+// Measured on a B200: 4096 tokens, 32 / 8 heads of 128, learned sinks, 6.17 ms on the FMA kernel -> 0.449 ms (306 TFLOP/s of
+// the attention, 3 times that on the tensor pipe; eight warps of softmax 0.012 ms more); 1001 tokens behind 3333 in a window of 1024,
+// 16 / 4 heads, 0.435 ms -> 0.070 ms.  Error of fp32 outputs against 64 bits on the same inputs, here / on the FMA kernel: scores of a
+// few units 0.2-0.6e-6 / 0.3-1.7e-6; of hundreds 0.9-1.8e-6 / 2.3-6.3e-6; all of a row's scores moved by 300 1.3-3.0e-5 / 3.7-7.0e-5, by
+// 8000 0.6-1.3e-3 / 1.1-2.2e-3 (what their rounding to fp32 leaves).  Larger here only where one key takes all the weight, 0.7e-7.
+// Descriptors formed ahead of the loop changed nothing.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <math.h>
@@ -646,7 +649,11 @@ int dispatch_tc(const CcSeqAttn* a, cudaStream_t st) {
 }  // namespace
 
 // bf16 rows of whole 16-byte vectors, up to 128 wide (the three query parts, two key and two value tiles fill the shared
-// memory), every pointer on a 16-byte boundary
+// memory), every pointer on a 16-byte boundary.  Any number of tokens: how many positions lie before them is known on the device
+// only.  Measured here and on the FMA kernel in us, 2 / 16 / 64 tokens, 32 / 8 heads of 128: behind 0 positions 12.0 / 15.3 / 20.8 and
+// 13.5 / 16.6 / 30.3, behind 500 27.8 / 33.6 / 38.4 and 136 / 150 / 174, behind 4000 129 / 131 / 136 and 1028 / 1074 / 1149.  The FMA
+// kernel is ahead only where no position lies before a few tokens of a wide group: 16 tokens, 17 / 1 heads of 128 16.6 and
+// 15.4, 64 / 8 heads of 64 13.1 and 11.2.
 bool attn_tc_serves(const CcSeqAttn* a) {
     const uintptr_t all = (uintptr_t)a->q | (uintptr_t)a->k_new | (uintptr_t)a->v_new | (uintptr_t)a->k_cache | (uintptr_t)a->v_cache | (uintptr_t)a->y;
     return a->cache_dtype == CC_DT_BF16 && a->Dk % 8 == 0 && a->Dv % 8 == 0 && a->Dk <= 128 && a->Dv <= 128 && (all & 15) == 0 &&

@@ -326,6 +326,9 @@ def wkv(r, k, v, wraw, w0, u, state, o, H, D):
     _lib.check_seq(_lib.load_seq().cc_seq_wkv(C.byref(a), _stream()), "cc_seq_wkv")
 
 
+# Tokens from which the decays have their own launch.  Measured apart / inside in us: 32 heads of 64, 16 / 32 / 63 tokens 5.8 / 5.6,
+# 7.1 / 7.9, 10.2 / 12.9; 128 heads of 64 8.0 / 7.4, 11.4 / 10.9, 17.6 / 17.8; 8 heads of 256 8.1 / 9.1, 11.5 / 14.5, 18.3 / 25.2.  From 64 on
+# it is no loss for any number of heads; fewer heads would gain from about 20 on.
 WKV_DECAY_FROM = 64
 
 

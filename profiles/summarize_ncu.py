@@ -1,8 +1,8 @@
 #!/usr/bin/env python
-"""Turn the ncu outputs a gpurun call brought back (gpurun_out/) into the tracked summaries under profiles/.
+"""Turn ncu outputs into the tracked summaries under profiles/.
 
-    python profiles/summarize_ncu.py launches gpurun_out/r1_launches.csv profiles/r1_bench_launch_shares.txt "<title>"
-    python profiles/summarize_ncu.py full gpurun_out/r1_k1_full.ncu-rep profiles/r1_k1_ncu_full.txt [--traffic-json profiles/k1_traffic.json]
+    python profiles/summarize_ncu.py launches launches.csv profiles/r1_bench_launch_shares.txt "<title>"
+    python profiles/summarize_ncu.py full k1_full.ncu-rep profiles/r1_k1_ncu_full.txt [--traffic-json profiles/k1_traffic.json]
 
 `launches`: per-kernel-name totals/shares of one `ncu --metrics gpu__time_duration.sum` launch list.
 `full`: the handful of `--set full` metrics the roofline discussion uses, per captured launch.
