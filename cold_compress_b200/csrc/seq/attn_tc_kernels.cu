@@ -323,8 +323,16 @@ __device__ __forceinline__ void row_again(const CcSeqAttn& a, const Keys& ks, in
         if (seen) {
             const bf16* const k = (const bf16*)(j >= ks.p0 ? a.k_new : a.k_cache) + row * Dk;
             s = 0.f;
-#pragma unroll 1
-            for (int d = 0; d < Dk; ++d) s = fmaf(q[d], __bfloat162float(k[d]), s);
+#pragma unroll 4
+            for (int d = 0; d < Dk; d += 8) {      // rows are whole 16-byte vectors
+                const uint4 u = *reinterpret_cast<const uint4*>(k + d);
+                const bf16* const e = reinterpret_cast<const bf16*>(&u);
+                float qv[8];
+                *reinterpret_cast<float4*>(qv) = *reinterpret_cast<const float4*>(q + d);
+                *reinterpret_cast<float4*>(qv + 4) = *reinterpret_cast<const float4*>(q + d + 4);
+#pragma unroll
+                for (int x = 0; x < 8; ++x) s = fmaf(qv[x], __bfloat162float(e[x]), s);
+            }
             s *= a.scale;
             if (SHAPED) s = shaped(a, s, h, i - j);
         }
@@ -333,13 +341,15 @@ __device__ __forceinline__ void row_again(const CcSeqAttn& a, const Keys& ks, in
         m = m_new;
 #pragma unroll
         for (int c = 0; c < 4; ++c) o[c] *= corr;
-#pragma unroll 1
-        for (uint32_t left = __ballot_sync(0xffffffffu, seen); left != 0; left &= left - 1) {
-            const int k = __ffs(left) - 1, fresh = __shfl_sync(0xffffffffu, (int)(j >= ks.p0), k);
+        const uint32_t all = __ballot_sync(0xffffffffu, seen);
+        const unsigned long long mine = (unsigned long long)((const bf16*)(j >= ks.p0 ? a.v_new : a.v_cache) + row * Dv);
+#pragma unroll 8
+        for (int k = 0; k < 32; ++k) {
             const float wk = __shfl_sync(0xffffffffu, w, k);
-            const size_t rk = __shfl_sync(0xffffffffu, (unsigned long long)row, k);
-            if (4 * lane >= Dv) continue;
-            const bf16* const v = (const bf16*)(fresh ? a.v_new : a.v_cache) + rk * Dv + 4 * lane;
+            const bf16* const vr = (const bf16*)__shfl_sync(0xffffffffu, mine, k);
+            uint2 u = make_uint2(0u, 0u);      // a key that is not seen: zero times zero
+            if ((all >> k & 1u) && 4 * lane < Dv) u = *reinterpret_cast<const uint2*>(vr + 4 * lane);
+            const bf16* const v = reinterpret_cast<const bf16*>(&u);
 #pragma unroll
             for (int c = 0; c < 4; ++c) o[c] = fmaf(wk, __bfloat162float(v[c]), o[c]);
         }
