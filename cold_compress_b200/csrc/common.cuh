@@ -154,6 +154,10 @@ __device__ __forceinline__ void tma_load_1d_hint(void* smem_dst, const void* gme
 __device__ __forceinline__ void l2_prefetch_bulk(const void* ptr, uint32_t bytes) {
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" :: "l"(ptr), "r"(bytes) : "memory");
 }
+// the same for the line that holds `ptr`
+__device__ __forceinline__ void l2_prefetch_line(const void* ptr) {
+    asm volatile("prefetch.global.L2 [%0];" :: "l"(ptr));
+}
 // order earlier generic-proxy accesses to shared memory before later async-proxy (TMA) writes
 __device__ __forceinline__ void fence_proxy_async() {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -229,13 +233,35 @@ __device__ __forceinline__ float group_reduce_multi(const float (&v)[G], int li,
     return w[0];
 }
 
-__device__ __forceinline__ uint64_t warp_min_u64(uint64_t k) {
+// the query head whose sum group_reduce_multi leaves in lane `li` of a row group
+template <int LPR, int G>
+__device__ __forceinline__ int group_reduce_head(int li) {
+    int g = 0, held = G <= 1 ? 1 : G <= 2 ? 2 : G <= 4 ? 4 : 8;
 #pragma unroll
-    for (int d = 16; d >= 1; d >>= 1) {
-        uint64_t o = __shfl_xor_sync(0xffffffffu, k, d);
-        k = o < k ? o : k;
+    for (int d = LPR / 2; d >= 1 && held > 1; d >>= 1) {
+        held /= 2;
+        if (li & d) g += held;
     }
-    return k;
+    return g;
+}
+
+// Over a whole warp, with the warp reduction instruction: one instruction where a butterfly has five dependent shuffles.
+__device__ __forceinline__ uint64_t warp_min_u64(uint64_t k) {
+    const uint32_t hi = (uint32_t)(k >> 32), top = __reduce_min_sync(0xffffffffu, hi);
+    const uint32_t low = __reduce_min_sync(0xffffffffu, hi == top ? (uint32_t)k : 0xffffffffu);
+    return ((uint64_t)top << 32) | low;
+}
+// three parts of 24 bits, whose sums over 32 lanes stay below 2^29
+__device__ __forceinline__ unsigned long long warp_sum_u64(unsigned long long v) {
+    const uint32_t a = __reduce_add_sync(0xffffffffu, (uint32_t)v & 0xffffffu), b = __reduce_add_sync(0xffffffffu, (uint32_t)(v >> 24) & 0xffffffu);
+    const uint32_t c = __reduce_add_sync(0xffffffffu, (uint32_t)(v >> 48));
+    return a + ((unsigned long long)b << 24) + ((unsigned long long)c << 48);
+}
+// as fmaxf: a NaN counts only if there is nothing else
+__device__ __forceinline__ float warp_max_f32(float v) {
+    float r;
+    asm("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
 }
 
 }  // namespace cc

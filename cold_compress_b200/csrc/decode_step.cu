@@ -18,6 +18,11 @@
 //     {P.V partials}; the first one carries both the eviction decision and the softmax max, so
 //     the evicted slot's old logit is excluded / the new token's logit included without a
 //     second pass over K;
+//   * what bounds it is the chain of dependent waits, not bytes, so the chain is kept short: rows and policy state are in L2
+//     when the launch may read them (asked for before griddepcontrol.wait), all loads of the first phases are requested
+//     together, warps reduce with the warp reduction instruction instead of butterflies, every softmax warp owns one query
+//     head and sends its own sums, and the P.V phase adds nothing up across lanes.  32 steps in a graph, us a step, before and
+//     with all of it: 64 sliding slots 8.2 and 5.7, 1024 heavy-hitter slots 10.9 and 8.1, 512 l2 slots 15.2 and 8.5;
 //   * arithmetic order is the bit-reproducible definition in common.cuh (canonical dot tree,
 //     det_expf, 2^-40 fixed-point sum), so eviction indices do not depend on C, CH or the
 //     thread count.
@@ -44,7 +49,7 @@ constexpr int kRecWords = 2 + 2 * kMaxG;  // X1 record: key64, lmax[G], candlogi
 constexpr uint64_t kNoKey = ~0ull;
 
 struct SmemLayout {
-    uint32_t kring, vring, lg, red, yx, rec, sums, ssum, x0, maskb, bars, misc, total;
+    uint32_t kring, vring, lg, red, yx, rec, sums, x0, maskb, bars, misc, total;
 };
 
 struct DecodeParams {
@@ -60,6 +65,15 @@ struct DecodeParams {
     unsigned long long* trace;  // diagnostics: [gridDim.x][16] globaltimer stamps (NULL = off)
 };
 
+// misc area, indices in 4-byte words
+enum : int {
+    kMiscNewLg = 0,     // [kMaxG] logits of the new token
+    kMiscWarpKey = 8,   // [kWarps] u64
+    kMiscWarpMax = 24,  // [kWarps] largest key norm
+    kMiscRowMax = 32,   // [kWarps][kMaxG] largest logit of a warp's rows, without the candidate's
+    kMiscWords = 96,
+};
+
 __host__ __device__ inline uint32_t align_up(uint32_t x, uint32_t a) { return (x + a - 1) / a * a; }
 
 __host__ __device__ inline SmemLayout make_layout(int D, int G, int chunk_rows, int local_rows, int n_stages, int lg_stride) {
@@ -73,27 +87,13 @@ __host__ __device__ inline SmemLayout make_layout(int D, int G, int chunk_rows, 
     s.yx = off;    off += G * D * 4;
     s.rec = off;   off += kMaxCluster * kRecWords * 4;
     s.sums = off;  off += kMaxCluster * kMaxG * 8;
-    s.ssum = off;  off += kMaxG * 8;
     s.x0 = off;    off += 128;
     s.maskb = off; off += align_up(local_rows, 128);
     s.bars = off;  off += align_up((2 * n_stages + 4) * 8, 128);  // K ring, V ring, 4 exchange barriers
-    s.misc = off;  off += 512;
+    s.misc = off;  off += kMiscWords * 4;
     s.total = off;
     return s;
 }
-
-// misc area, indices in 4-byte words
-enum : int {
-    kMiscNewLg = 0,     // [kMaxG] logits of the new token
-    kMiscLmax = 8,      // [kMaxG]
-    kMiscCandLg = 16,   // [kMaxG]
-    kMiscGmax = 24,     // [kMaxG]
-    kMiscSumF = 32,     // [kMaxG]
-    kMiscMyRec = 40,    // [kRecWords]
-    kMiscWarpKey = 64,  // [kWarps] u64 (32 words)
-    kMiscWarpMax = 96,  // [kWarps]
-    kMiscWords = 128,
-};
 
 // hybrid per-head decision (reference cache.py:896-950)
 enum : int { kHybAppend = 0, kHybEvict = 1, kHybDrop = 2 };
@@ -107,11 +107,12 @@ __device__ __forceinline__ void stamp(const DecodeParams& p, int k) {
 }
 
 template <int D, int G, int POLICY, bool NAIVE>
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(kThreads, 2)
 cc_decode_kernel(const __grid_constant__ DecodeParams p) {
     constexpr int LPR = D / 8;           // lanes per cache row (16-byte slice each)
     constexpr int RPW = 32 / LPR;        // rows per warp iteration
-    constexpr int NRG = kThreads / LPR;  // row groups in the P.V phase
+    constexpr int CPL = D / 32;          // P.V phase: value columns per lane
+    constexpr int WPG = kWarps / G;      // softmax: warps that share a query head's rows (one head per warp)
     constexpr uint32_t kRowBytes = D * 2;
     constexpr bool hybrid = POLICY == CC_POLICY_HYBRID;
 
@@ -119,6 +120,7 @@ cc_decode_kernel(const __grid_constant__ DecodeParams p) {
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int li = lane % LPR, sub = lane / LPR;
     const int csh = p.c_shift, C = 1 << csh, rank = (int)cluster_ctarank();
+    const bool solo = C == 1;            // the head's rows in one CTA: nothing to exchange
     const int h = blockIdx.x >> csh;
     const CcCacheState& st = p.st;
     const int L = st.max_cache_length, H = st.n_kv_heads;
@@ -155,7 +157,6 @@ cc_decode_kernel(const __grid_constant__ DecodeParams p) {
     uint64_t* xbar = vbar + NS;  // [0] X0 (L2 max), [1] X1, [2] X2, [3] X3: single-use exchange barriers
     float* misc = reinterpret_cast<float*>(smem + lay.misc);
     uint32_t* miscu = reinterpret_cast<uint32_t*>(misc);
-    unsigned long long* ssum = reinterpret_cast<unsigned long long*>(smem + lay.ssum);  // [kMaxG] local fixed-point sums
 
     stamp(p, 0);
     constexpr int NW = 2 + 2 * G;  // words of an X1 record
@@ -164,20 +165,52 @@ cc_decode_kernel(const __grid_constant__ DecodeParams p) {
         mbar_fence_init();
         // every exchange delivers a known number of bytes into this CTA: arm the barriers right away
         // (only the exchanges this launch performs: an armed barrier nobody completes is a synccheck finding)
-        if (POLICY == CC_POLICY_L2 && do_evict) mbar_expect_tx(&xbar[0], (uint32_t)C * 4);
-        mbar_expect_tx(&xbar[1], (uint32_t)C * NW * 4);
-        if (do_attend) {
-            mbar_expect_tx(&xbar[2], (uint32_t)C * G * 8);
-            mbar_expect_tx(&xbar[3], (uint32_t)G * D * 4);
+        if (!solo) {
+            if (POLICY == CC_POLICY_L2 && do_evict) mbar_expect_tx(&xbar[0], (uint32_t)C * 4);
+            mbar_expect_tx(&xbar[1], (uint32_t)C * NW * 4);
+            if (do_attend) {
+                mbar_expect_tx(&xbar[2], (uint32_t)C * G * WPG * 8);
+                mbar_expect_tx(&xbar[3], (uint32_t)G * D * 4);
+            }
         }
     }
     // B0: this CTA has started and its exchange barriers exist; peers wait for this before they send
-    cluster_arrive_release();
-    bool b0_waited = false;
+    if (!solo) cluster_arrive_release();
+    bool b0_waited = solo;
     // Without the promise that the predecessor leaves this cache alone nothing of it is read before the predecessor has
-    // ended; the launch, the barriers and the cluster's start above run under it all the same.  (32 steps back to back in a
-    // graph: 64-slot sliding caches 8.8 -> 8.2 us a step, 1024 heavy-hitter slots 11.4 -> 10.9.)
+    // ended; the launch, the barriers and the cluster's start above run under it all the same.
     const bool ahead = p.a.flags & CC_FLAG_OVERLAP_PREDECESSOR;
+    const uint16_t* kc = reinterpret_cast<const uint16_t*>(st.k_cache) + (size_t)h * L * D;
+    const uint16_t* vc = reinterpret_cast<const uint16_t*>(st.v_cache) + (size_t)h * L * D;
+    auto chunk_rows_valid = [&](int j) { return min(CH, L - ((((j << csh) + rank)) << chs)); };
+    auto chunk_at = [&](const uint16_t* base, int j) { return base + ((size_t)((j << csh) + rank) << chs) * D; };
+    const int pos_row = (st.pos_heads == 1) ? 0 : h;
+    const int32_t* posp = st.pos + (size_t)pos_row * L;
+    const double* hist = reinterpret_cast<const double*>(st.attn_history_num) + (size_t)h * L;   // heavy hitter with W = 1
+    const int32_t* den = st.attn_history_denom + (size_t)h * L;
+    const bool hh_sum = POLICY == CC_POLICY_HEAVY_HITTER && !hh_ring;
+    const int s0 = slot_of(tid);         // this thread's first row
+    const bool in0 = tid < local_rows && s0 < L;
+    const uint16_t* qp = reinterpret_cast<const uint16_t*>(p.a.q) + (size_t)h * G * D + li * 8;
+    const uint16_t* knp = reinterpret_cast<const uint16_t*>(p.a.k_new) + (size_t)h * D + li * 8;
+    const uint16_t* vrow_new = reinterpret_cast<const uint16_t*>(p.a.v_new) + (size_t)h * D;
+    if (!ahead) {
+        // What will be read is asked for in L2: a hint, which takes no value, so that after the wait the chain below meets
+        // L2 and not DRAM.  (Rows of a hybrid head that are live are known from memory only.)
+        if constexpr (!hybrid) {
+            const int pre = do_attend ? min(NS, nlc) : 0;
+            if (tid < 2 * pre) l2_prefetch_bulk(chunk_at(tid & 1 ? vc : kc, tid >> 1), chunk_rows_valid(tid >> 1) * kRowBytes);
+        }
+        if (in0) {
+            l2_prefetch_line(posp + s0);
+            l2_prefetch_line(st.mask + (size_t)h * L + s0);
+            if (POLICY == CC_POLICY_L2 && do_evict) l2_prefetch_line(reinterpret_cast<const uint16_t*>(st.key_norm) + (size_t)h * L + s0);
+            if (hh_sum) {
+                l2_prefetch_line(hist + s0);
+                l2_prefetch_line(den + s0);
+            }
+        }
+    }
     if (!ahead) pdl_wait();
 
     // ---- hybrid: per-head decision from scalars (every CTA of the cluster computes the same)
@@ -214,10 +247,6 @@ cc_decode_kernel(const __grid_constant__ DecodeParams p) {
     const int nlc_live = do_attend ? (live_chunks_total > rank ? (live_chunks_total - rank + C - 1) >> csh : 0) : 0;
     const int live_rows = nlc_live << chs;
 
-    const uint16_t* kc = reinterpret_cast<const uint16_t*>(st.k_cache) + (size_t)h * L * D;
-    const uint16_t* vc = reinterpret_cast<const uint16_t*>(st.v_cache) + (size_t)h * L * D;
-    auto chunk_rows_valid = [&](int j) { return min(CH, L - ((((j << csh) + rank)) << chs)); };
-
     // ---- 0. barriers + as many K/V chunks in flight as the ring holds
     if (tid == 0) {
         fence_proxy_async();
@@ -225,25 +254,54 @@ cc_decode_kernel(const __grid_constant__ DecodeParams p) {
         for (int j = 0; j < pre; ++j) {
             const uint32_t bytes = chunk_rows_valid(j) * kRowBytes;
             mbar_expect_tx(&kbar[j], bytes);
-            tma_load_1d(kring + j * chunk_bytes, kc + ((size_t)((j << csh) + rank) << chs) * D, bytes, &kbar[j]);
+            tma_load_1d(kring + j * chunk_bytes, chunk_at(kc, j), bytes, &kbar[j]);
         }
         for (int j = 0; j < pre; ++j) {
             const uint32_t bytes = chunk_rows_valid(j) * kRowBytes;
             mbar_expect_tx(&vbar[j], bytes);
-            tma_load_1d(vring + j * chunk_bytes, vc + ((size_t)((j << csh) + rank) << chs) * D, bytes, &vbar[j]);
+            tma_load_1d(vring + j * chunk_bytes, chunk_at(vc, j), bytes, &vbar[j]);
         }
     }
-    if (tid < kMaxG) ssum[tid] = 0ull;
     stamp(p, 1);
     // generation of the cross-cluster "shared reads done" barrier, read by the thread that may
     // later have to wait on it (lane 0 of the last warp) BEFORE this cluster arrives
     int32_t gen = 0;
     if (needs_epoch && tid == kThreads - 32) gen = ld_acquire_gpu(&st.sync_words[1]);
 
+    // Everything the first phases take from global memory is requested here together: one round trip instead of one per phase.
     const int ipos = p.a.input_pos[0];
-    const int pos_row = (st.pos_heads == 1) ? 0 : h;
-    const int32_t* posp = st.pos + (size_t)pos_row * L;
-    for (int lr = tid; lr < local_rows; lr += kThreads) {
+    uint4 qraw[G], knew8 = make_uint4(0, 0, 0, 0), vnew8 = make_uint4(0, 0, 0, 0);   // the new rows: the last warp stores them
+    uint32_t vnew[CPL / 2];                                                          // this lane's columns of the value row
+#pragma unroll
+    for (int i = 0; i < CPL / 2; ++i) vnew[i] = 0;
+    auto load_new = [&] {
+        if (do_attend) {
+#pragma unroll
+            for (int g = 0; g < G; ++g) qraw[g] = *reinterpret_cast<const uint4*>(qp + g * D);
+        }
+        if (do_evict) {
+#pragma unroll
+            for (int i = 0; i < CPL / 2; ++i) vnew[i] = reinterpret_cast<const uint32_t*>(vrow_new)[lane * (CPL / 2) + i];
+            if (warp == kWarps - 1) {
+                knew8 = *reinterpret_cast<const uint4*>(knp);
+                vnew8 = *reinterpret_cast<const uint4*>(vrow_new + li * 8);
+            }
+        }
+    };
+    int ps0 = 0, den0 = 0;
+    double hist0 = 0.0;
+    uint8_t mask0 = 0;
+    if (in0) {
+        mask0 = st.mask[(size_t)h * L + s0];
+        if (do_evict) ps0 = posp[s0];
+        if (hh_sum) {
+            hist0 = hist[s0];
+            den0 = den[s0];
+        }
+    }
+    if (!ahead) load_new();
+    if (tid < local_rows) maskb[tid] = mask0;
+    for (int lr = tid + kThreads; lr < local_rows; lr += kThreads) {
         const int s = slot_of(lr);
         maskb[lr] = (s < L) ? st.mask[(size_t)h * L + s] : 0;
     }
@@ -258,25 +316,25 @@ cc_decode_kernel(const __grid_constant__ DecodeParams p) {
         if (do_evict) {
             const uint16_t* kn = reinterpret_cast<const uint16_t*>(st.key_norm);
             float m = -CUDART_INF_F;
-            for (int hh = 0; hh < H; ++hh)
-                for (int lr = tid; lr < local_rows; lr += kThreads) {
+            for (int hh = warp; hh < H; hh += kWarps)     // a warp per head: its loads are all under way at once
+#pragma unroll 4
+                for (int lr = lane; lr < local_rows; lr += 32) {
                     const int s = slot_of(lr);
                     if (s < L) m = fmaxf(m, bf16_bits_to_float(kn[(size_t)hh * L + s]));
                 }
-#pragma unroll
-            for (int d = 16; d >= 1; d >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, d));
+            m = warp_max_f32(m);
             if (lane == 0) misc[kMiscWarpMax + warp] = m;
             __syncthreads();
-            cluster_wait_acquire();
-            b0_waited = true;
-            if (tid < C) {
-                float mm = misc[kMiscWarpMax];
-                for (int w = 1; w < kWarps; ++w) mm = fmaxf(mm, misc[kMiscWarpMax + w]);
-                st_async_u32(map_to_rank(smem_u32(&x0[rank]), tid), __float_as_uint(mm), map_to_rank(smem_u32(&xbar[0]), tid));
+            l2_max = misc[kMiscWarpMax];
+            for (int w = 1; w < kWarps; ++w) l2_max = fmaxf(l2_max, misc[kMiscWarpMax + w]);
+            if (!solo) {
+                cluster_wait_acquire();
+                b0_waited = true;
+                if (tid < C) st_async_u32(map_to_rank(smem_u32(&x0[rank]), tid), __float_as_uint(l2_max), map_to_rank(smem_u32(&xbar[0]), tid));
+                mbar_wait(&xbar[0], 0);
+                l2_max = x0[0];
+                for (int r = 1; r < C; ++r) l2_max = fmaxf(l2_max, x0[r]);
             }
-            mbar_wait(&xbar[0], 0);
-            l2_max = x0[0];
-            for (int r = 1; r < C; ++r) l2_max = fmaxf(l2_max, x0[r]);
         }
     }
 
@@ -284,16 +342,16 @@ cc_decode_kernel(const __grid_constant__ DecodeParams p) {
     uint64_t ckey = kNoKey;
     if (do_evict) {
         if constexpr (POLICY == CC_POLICY_HEAVY_HITTER) {
-            const double* num = reinterpret_cast<const double*>(st.attn_history_num) + (size_t)h * L;
-            const int32_t* den = st.attn_history_denom + (size_t)h * L;
+#pragma unroll 1
             for (int lr = tid; lr < local_rows; lr += kThreads) {
                 const int s = slot_of(lr);
                 if (s >= L) continue;
-                const int ps = posp[s];
+                const bool first = lr == tid;
+                const int ps = first ? ps0 : posp[s];
                 // cache.py:727-749: mean accumulated attention; globals & recent -> 1.0; unfilled -> 0.0
                 float avg;
                 if (!hh_ring) {
-                    avg = __fdiv_rn(__double2float_rn(num[s]), (float)max(den[s], 1));
+                    avg = __fdiv_rn(__double2float_rn(first ? hist0 : hist[s]), (float)max(first ? den0 : den[s], 1));
                 } else {
                     // sum of the slot's ring (kept as an exact fp64 running sum): bf16 ring -> bf16(fp32 sum),
                     // thresholded (bool) ring -> integer count; / clamp(denom, 1, W)   (cache.py:727-738)
@@ -307,10 +365,11 @@ cc_decode_kernel(const __grid_constant__ DecodeParams p) {
             }
         } else if constexpr (POLICY == CC_POLICY_L2) {
             const uint16_t* kn = reinterpret_cast<const uint16_t*>(st.key_norm) + (size_t)h * L;
+#pragma unroll 1
             for (int lr = tid; lr < local_rows; lr += kThreads) {
                 const int s = slot_of(lr);
                 if (s >= L) continue;
-                const int ps = posp[s];
+                const int ps = lr == tid ? ps0 : posp[s];
                 // cache.py:597-605 then 366-379: bf16(max - norm); recent -> +inf; first g slots -> +inf; unfilled -> -inf
                 float sc = bf16_round(__fsub_rn(l2_max, bf16_bits_to_float(kn[s])));
                 if (ps >= ipos - st.recent_window) sc = CUDART_INF_F;
@@ -321,10 +380,11 @@ cc_decode_kernel(const __grid_constant__ DecodeParams p) {
             }
         } else if constexpr (POLICY == CC_POLICY_RECENT_GLOBAL) {
             // cache.py:552-556: oldest position among slots >= g (unfilled = -1 first)
+#pragma unroll 1
             for (int lr = tid; lr < local_rows; lr += kThreads) {
                 const int s = slot_of(lr);
                 if (s >= L || s < st.global_tokens) continue;
-                const uint64_t k = ((uint64_t)((uint32_t)posp[s] ^ 0x80000000u) << 32) | (uint32_t)s;
+                const uint64_t k = ((uint64_t)((uint32_t)(lr == tid ? ps0 : posp[s]) ^ 0x80000000u) << 32) | (uint32_t)s;
                 ckey = k < ckey ? k : ckey;
             }
         } else if constexpr (hybrid) {
@@ -332,7 +392,6 @@ cc_decode_kernel(const __grid_constant__ DecodeParams p) {
                 // cache.py:844-894 over the live prefix [0, cts): mean ring attention (or position for
                 // window-only heads); first g slots, special, punctuation and the recent window are saved
                 const int W = st.history_window;
-                const int32_t* den = st.attn_history_denom + (size_t)h * L;
                 const double* hsum = st.attn_history_sum + (size_t)h * L;
                 for (int lr = tid; lr < local_rows; lr += kThreads) {
                     const int s = slot_of(lr);
@@ -389,19 +448,7 @@ cc_decode_kernel(const __grid_constant__ DecodeParams p) {
     if (ahead) {
         pdl_wait();
         pdl_launch_dependents();
-    }
-    // query rows of this KV group and the new value slice, in registers
-    float q[G][8];
-    uint4 vnew8 = make_uint4(0, 0, 0, 0);
-    if (do_attend) {
-#pragma unroll
-        for (int g = 0; g < G; ++g) {
-            const uint4 v = *reinterpret_cast<const uint4*>(
-                reinterpret_cast<const uint16_t*>(p.a.q) + (size_t)(h * G + g) * D + li * 8);
-            unpack8(v, q[g]);
-        }
-        if (do_evict)
-            vnew8 = *reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(p.a.v_new) + (size_t)h * D + li * 8);
+        load_new();
     }
     // local row of this CTA's candidate (it owns the slot by construction)
     int cand_local = -1;
@@ -412,13 +459,14 @@ cc_decode_kernel(const __grid_constant__ DecodeParams p) {
     // a dropped token does not take part in attention (its slot's mask stays as it was)
     const bool attend_new = do_evict && !(hybrid && hyb_mode == kHybDrop);
 
-    // ---- 3. logits over the K ring (canonical dot tree), new-token logits by the last warp
+    // ---- 3. logits over the K ring (canonical dot tree), new-token logits by the last warp while the rows arrive
     if (do_attend) {
-        if (attend_new && warp == kWarps - 1) {
-            float kf[8];
-            const uint4 kv = *reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(p.a.k_new) + (size_t)h * D + li * 8);
-            unpack8(kv, kf);
-            float part[G];
+        float q[G][8];
+#pragma unroll
+        for (int g = 0; g < G; ++g) unpack8(qraw[g], q[g]);
+        auto dots = [&](const uint4& row, int* gsel) {
+            float kf[8], part[G];
+            unpack8(row, kf);
 #pragma unroll
             for (int g = 0; g < G; ++g) {
                 float acc = 0.f;
@@ -426,104 +474,96 @@ cc_decode_kernel(const __grid_constant__ DecodeParams p) {
                 for (int i = 0; i < 8; ++i) acc = __fmaf_rn(q[g][i], kf[i], acc);
                 part[g] = acc;
             }
-            int gsel;
-            const float dot = group_reduce_multi<LPR, G>(part, li, &gsel);
-            const float v = NAIVE ? bf16_round(__fmul_rn(bf16_round(dot), p.scale)) : __fmul_rn(dot, p.scale);
+            const float dot = group_reduce_multi<LPR, G>(part, li, gsel);
+            // naive path rounds q@k^T to bf16, then * scale to bf16 (attention_utils.py:37)
+            return NAIVE ? bf16_round(__fmul_rn(bf16_round(dot), p.scale)) : __fmul_rn(dot, p.scale);
+        };
+        int gsel = group_reduce_head<LPR, G>(li);   // the query head whose sums this lane ends up with
+        if (attend_new && warp == kWarps - 1) {
+            const float v = dots(knew8, &gsel);
             if (sub == 0 && gsel < G) misc[kMiscNewLg + gsel] = v;  // replicated lanes write the same value
         }
         // rows of chunks that cannot be live
         for (int lr = live_rows + tid; lr < local_rows; lr += kThreads)
 #pragma unroll
             for (int g = 0; g < G; ++g) lg[g * stride + lr] = -CUDART_INF_F;
-        __syncthreads();  // maskb visible
-        for (int j = 0; j < nlc_live; ++j) {
-            const int stage = j % NS;
-            mbar_wait(&kbar[stage], (j / NS) & 1);
+        if (!do_evict) __syncthreads();  // maskb visible
+        float m = -CUDART_INF_F;         // of this lane's head over its rows, without the candidate's
+        // chunks that are all in the ring are walked as one run of rows
+        const int per = nlc_live <= NS ? nlc_live : 1;
+        for (int j = 0; j < nlc_live; j += per) {
+            const int stage = j % NS, run = per << chs;
+            for (int i = 0; i < per; ++i) mbar_wait(&kbar[stage + i], (j / NS) & 1);
             if (j == 0) stamp(p, 3);
-            const int rows_c = chunk_rows_valid(j);
             const uint8_t* kbase = kring + stage * chunk_bytes;
-            // up to 4 row pairs per warp per pass, all fetched before the dependent math (ILP)
-            constexpr int UR = 4;
-            for (int r0 = warp * RPW; r0 < CH; r0 += UR * kWarps * RPW) {
+            // up to UR row pairs per warp per pass, all fetched before the dependent math (ILP)
+            constexpr int UR = G >= 7 ? 2 : 4;     // (registers: two CTAs per SM, so that the next launch fits beside this one)
+#pragma unroll 1
+            for (int r0 = warp * RPW; r0 < run; r0 += UR * kWarps * RPW) {
                 uint4 kv[UR];
 #pragma unroll
                 for (int u = 0; u < UR; ++u) {
                     const int r = r0 + u * kWarps * RPW + sub;
-                    kv[u] = (r < rows_c) ? *reinterpret_cast<const uint4*>(kbase + r * kRowBytes + li * 16)
-                                         : make_uint4(0, 0, 0, 0);
+                    if (u == 0 || r0 + u * kWarps * RPW < run) kv[u] = *reinterpret_cast<const uint4*>(kbase + r * kRowBytes + li * 16);
                 }
 #pragma unroll
                 for (int u = 0; u < UR; ++u) {
-                    const int r = r0 + u * kWarps * RPW + sub;
-                    float kf[8];
-                    unpack8(kv[u], kf);
-                    float part[G];
-#pragma unroll
-                    for (int g = 0; g < G; ++g) {
-                        float acc = 0.f;
-#pragma unroll
-                        for (int i = 0; i < 8; ++i) acc = __fmaf_rn(q[g][i], kf[i], acc);
-                        part[g] = acc;
-                    }
-                    int gsel;
-                    const float dot = group_reduce_multi<LPR, G>(part, li, &gsel);
-                    // naive path rounds q@k^T to bf16, then * scale to bf16 (attention_utils.py:37)
-                    const float v = NAIVE ? bf16_round(__fmul_rn(bf16_round(dot), p.scale)) : __fmul_rn(dot, p.scale);
-                    const int lr = (j << chs) + r;
-                    if (gsel < G && r < CH) lg[gsel * stride + lr] = (r < rows_c && maskb[lr]) ? v : -CUDART_INF_F;
+                    const int r = r0 + u * kWarps * RPW + sub, lr = (j << chs) + r;
+                    if (u > 0 && r0 + u * kWarps * RPW >= run) break;
+                    float v = dots(kv[u], &gsel);
+                    if (!maskb[lr]) v = -CUDART_INF_F;      // rows beyond the cache are masked too
+                    if (gsel < G) lg[gsel * stride + lr] = v;
+                    if (lr != cand_local) m = fmaxf(m, v);
                 }
             }
-            __syncthreads();
-            if (tid == 0 && j + NS < nlc_live) {
-                fence_proxy_async();
-                const int jn = j + NS;
-                const uint32_t bytes = chunk_rows_valid(jn) * kRowBytes;
-                mbar_expect_tx(&kbar[stage], bytes);
-                tma_load_1d(kring + stage * chunk_bytes, kc + ((size_t)((jn << csh) + rank) << chs) * D, bytes, &kbar[stage]);
+            if (j + NS < nlc_live) {  // ring slot is refilled: everyone must be done with it
+                __syncthreads();
+                if (tid == 0) {
+                    fence_proxy_async();
+                    const int jn = j + NS;
+                    const uint32_t bytes = chunk_rows_valid(jn) * kRowBytes;
+                    mbar_expect_tx(&kbar[stage], bytes);
+                    tma_load_1d(kring + stage * chunk_bytes, chunk_at(kc, jn), bytes, &kbar[stage]);
+                }
             }
         }
-        // ---- 4. row max without the local candidate, and the candidate's own logits -> my X1 record
-        for (int g = warp; g < G; g += kWarps) {
-            float m = -CUDART_INF_F;
-            for (int lr = lane; lr < live_rows; lr += 32)
-                if (lr != cand_local) m = fmaxf(m, lg[g * stride + lr]);
 #pragma unroll
-            for (int d = 16; d >= 1; d >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, d));
-            if (lane == 0) {
-                misc[kMiscMyRec + 2 + g] = m;
-                misc[kMiscMyRec + 2 + G + g] = cand_local >= 0 ? lg[g * stride + cand_local] : -CUDART_INF_F;
-            }
-        }
-    } else if (tid < 2 * G) {
-        misc[kMiscMyRec + 2 + tid] = -CUDART_INF_F;
+        for (int d = 16; d >= LPR; d >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, d));
+        if (sub == 0 && gsel < G) misc[kMiscRowMax + warp * kMaxG + gsel] = m;
     }
+    __syncthreads();  // logits and row maxima visible
     stamp(p, 4);
-    // ---- 5. X1: every CTA learns every candidate and every partial max
-    if (tid == 0) {
-        miscu[kMiscMyRec + 0] = (uint32_t)(ckey & 0xffffffffu);
-        miscu[kMiscMyRec + 1] = (uint32_t)(ckey >> 32);
+    // ---- 4./5. X1: every CTA learns every candidate, every row maximum without the local candidate, and the candidate's logits
+    if (!solo) {
+        if (!b0_waited) cluster_wait_acquire();
+        for (int idx = tid; idx < C * NW; idx += kThreads) {
+            const int dest = idx / NW, w = idx % NW;
+            uint32_t word = __float_as_uint(-CUDART_INF_F);
+            if (w < 2) {
+                word = w == 0 ? (uint32_t)(ckey & 0xffffffffu) : (uint32_t)(ckey >> 32);
+            } else if (do_attend) {
+                if (w < 2 + G) {
+                    float m = misc[kMiscRowMax + w - 2];
+#pragma unroll
+                    for (int k = 1; k < kWarps; ++k) m = fmaxf(m, misc[kMiscRowMax + k * kMaxG + w - 2]);
+                    word = __float_as_uint(m);
+                } else if (cand_local >= 0) {
+                    word = __float_as_uint(lg[(w - 2 - G) * stride + cand_local]);
+                }
+            }
+            st_async_u32(map_to_rank(smem_u32(&rec[rank * kRecWords + w]), dest), word, map_to_rank(smem_u32(&xbar[1]), dest));
+        }
+        mbar_wait(&xbar[1], 0);
     }
-    __syncthreads();
-    if (!b0_waited) cluster_wait_acquire();
-    for (int idx = tid; idx < C * NW; idx += kThreads) {
-        const int dest = idx / NW, w = idx % NW;
-        st_async_u32(map_to_rank(smem_u32(&rec[rank * kRecWords + w]), dest), miscu[kMiscMyRec + w],
-                     map_to_rank(smem_u32(&xbar[1]), dest));
-    }
-    mbar_wait(&xbar[1], 0);
     stamp(p, 5);
 
-    // ---- 6. winner + global max per query head (every warp redundantly: no block barrier needed).
-    // Lane l looks at record r = l & 15; the two half-warps split the query heads (even / odd).
-    const int rl = lane & 15, gh = lane >> 4;
-    uint64_t wkey = kNoKey;
-    if (rl < C) wkey = (uint64_t)rec[rl * kRecWords] | ((uint64_t)rec[rl * kRecWords + 1] << 32);
-    const bool lane_has_cand = wkey != kNoKey;
-#pragma unroll
-    for (int d = 8; d >= 1; d >>= 1) {
-        const uint64_t o = __shfl_xor_sync(0xffffffffu, wkey, d);
-        wkey = o < wkey ? o : wkey;
+    // ---- 6. winner, and the maximum of the query head whose softmax this warp takes (WPG warps share a head's rows)
+    uint64_t wkey = ckey;
+    if (!solo) {
+        wkey = lane < C ? (uint64_t)rec[lane * kRecWords] | ((uint64_t)rec[lane * kRecWords + 1] << 32) : kNoKey;
     }
+    const bool lane_has_cand = wkey != kNoKey && lane < C;
+    if (!solo) wkey = warp_min_u64(wkey);
     const bool has_slot = do_evict && wkey != kNoKey;  // a slot is overwritten this step
     const int widx = has_slot ? (int)(uint32_t)(wkey & 0xffffffffu) : -1;
     const int owner = has_slot ? (widx >> chs) & (C - 1) : -1;
@@ -531,108 +571,106 @@ cc_decode_kernel(const __grid_constant__ DecodeParams p) {
     const int widx_local = has_slot ? (((widx >> chs) >> csh) << chs) + (widx & (CH - 1)) : -1;
     const bool has_new = has_slot && attend_new;  // ... and the new token attends to itself there
     if (needs_epoch && rank == 0 && tid == 0) red_release_gpu_add(&st.sync_words[0], 1);  // shared reads done
-    float gmax[G], newlg[G];
+    const int wg = warp % G, wpart = warp / G;
+    const bool softmax_warp = wpart < WPG;
+    float gm = -CUDART_INF_F, nl = -CUDART_INF_F;
     if (do_attend) {
-        constexpr int GH = (G + 1) / 2;  // query heads per half-warp
-        float part[GH];
-#pragma unroll
-        for (int j = 0; j < GH; ++j) {
-            const int g = 2 * j + gh;
-            float m = -CUDART_INF_F;
-            if (rl < C && g < G) {
-                m = __uint_as_float(rec[rl * kRecWords + 2 + g]);
-                // a candidate that is not overwritten keeps its logit; the overwritten one only if the new
-                // token does not replace it in attention (hybrid drop: slot L-1 stays as it was)
-                if (lane_has_cand && (rl != owner || !has_new))
-                    m = fmaxf(m, __uint_as_float(rec[rl * kRecWords + 2 + G + g]));
-            }
-            part[j] = m;
+        float m = -CUDART_INF_F;
+        // a candidate that is not overwritten keeps its logit; the overwritten one only if the new
+        // token does not replace it in attention (hybrid drop: slot L-1 stays as it was)
+        const bool cand_stays = lane_has_cand && (lane != owner || !has_new);
+        if (solo) {
+            if (lane < kWarps) m = misc[kMiscRowMax + lane * kMaxG + wg];
+            if (cand_stays) m = fmaxf(m, lg[wg * stride + cand_local]);
+        } else if (lane < C) {
+            m = __uint_as_float(rec[lane * kRecWords + 2 + wg]);
+            if (cand_stays) m = fmaxf(m, __uint_as_float(rec[lane * kRecWords + 2 + G + wg]));
         }
-#pragma unroll
-        for (int d = 8; d >= 1; d >>= 1)
-#pragma unroll
-            for (int j = 0; j < GH; ++j) part[j] = fmaxf(part[j], __shfl_xor_sync(0xffffffffu, part[j], d));
-#pragma unroll
-        for (int g = 0; g < G; ++g) {
-            newlg[g] = has_new ? misc[kMiscNewLg + g] : -CUDART_INF_F;
-            gmax[g] = fmaxf(__shfl_sync(0xffffffffu, part[g / 2], (g & 1) * 16), newlg[g]);
-        }
+        nl = has_new ? misc[kMiscNewLg + wg] : -CUDART_INF_F;
+        gm = fmaxf(warp_max_f32(m), nl);
     }
     const int patch_row = (i_own && has_new) ? widx_local : -1;  // this row now holds the new token
     stamp(p, 6);
 
     if (do_attend) {
-        // ---- 8. exp and the exact fixed-point softmax denominator = X2.  Items are (g, row) pairs laid
-        // out g-major with the row count padded to a warp multiple, so a warp never straddles two g.
-        const int rows_pad = (live_rows + 31) & ~31;
-        for (int it = tid; it < G * rows_pad; it += kThreads) {
-            const int g = it / rows_pad, lr = it - g * rows_pad;
+        // ---- 8. exp and the exact fixed-point softmax denominator = X2: every warp sends its partial sum to every CTA itself;
+        // integers, so their order does not matter.
+        float* lgw = lg + wg * stride;
+        if (softmax_warp) {
             long long part = 0;
-            if (lr < live_rows) {
-                float gm = gmax[0], nl = newlg[0];
-#pragma unroll
-                for (int gg = 1; gg < G; ++gg) if (g == gg) { gm = gmax[gg]; nl = newlg[gg]; }
-                const float l = lr == patch_row ? nl : lg[g * stride + lr];
+            for (int lr = wpart * 32 + lane; lr < live_rows; lr += WPG * 32) {
+                const float l = lr == patch_row ? nl : lgw[lr];
                 const float e = det_expf(__fsub_rn(l, gm));
-                lg[g * stride + lr] = e;
-                part = __float2ll_rz(__fmul_rn(e, 1099511627776.0f));
+                lgw[lr] = e;
+                part += __float2ll_rz(__fmul_rn(e, 1099511627776.0f));
             }
-#pragma unroll
-            for (int d = 16; d >= 1; d >>= 1) part += __shfl_xor_sync(0xffffffffu, part, d);
-            if (lane == 0 && part) atomicAdd(&ssum[g], (unsigned long long)part);  // integers: order independent
+            part = (long long)warp_sum_u64((unsigned long long)part);
+            unsigned long long* mine = &sums[wg * (kMaxCluster * WPG) + rank * WPG + wpart];
+            if (solo) {
+                if (lane == 0) *mine = (unsigned long long)part;
+            } else if (lane < C) {
+                st_async_u64(map_to_rank(smem_u32(mine), lane), (unsigned long long)part, map_to_rank(smem_u32(&xbar[2]), lane));
+            }
         }
-        __syncthreads();
         stamp(p, 7);
-        for (int idx = tid; idx < C * G; idx += kThreads) {
-            const int dest = idx / G, g = idx % G;
-            st_async_u64(map_to_rank(smem_u32(&sums[rank * kMaxG + g]), dest), ssum[g], map_to_rank(smem_u32(&xbar[2]), dest));
-        }
-        mbar_wait(&xbar[2], 0);
+        if (solo) __syncthreads();
+        else mbar_wait(&xbar[2], 0);
         stamp(p, 8);
-        // ---- 9a. probabilities (every warp sums the C partial denominators itself)
-        float sumf[G];
-#pragma unroll
-        for (int g = 0; g < G; ++g) {
-            long long t = lane < C ? (long long)sums[lane * kMaxG + g] : 0ll;
-#pragma unroll
-            for (int d = 16; d >= 1; d >>= 1) t += __shfl_xor_sync(0xffffffffu, t, d);
-            sumf[g] = __fmul_rn(__ll2float_rn(t), 9.094947017729282e-13f);  // 2^-40
-        }
-        for (int it = tid; it < G * live_rows; it += kThreads) {
-            const int g = it / live_rows, lr = it - g * live_rows;
-            float sf = sumf[0];
-#pragma unroll
-            for (int gg = 1; gg < G; ++gg) if (g == gg) sf = sumf[gg];
-            float pr = __fdiv_rn(lg[g * stride + lr], sf);
-            if (NAIVE) pr = bf16_round(pr);
-            lg[g * stride + lr] = pr;
+        // ---- 9a. probabilities: every warp adds the partial denominators of its head and goes over its own rows again
+        if (softmax_warp) {
+            unsigned long long t = 0;
+            for (int i = lane; i < C * WPG; i += 32) t += sums[wg * (kMaxCluster * WPG) + i];
+            const float sf = __fmul_rn(__ll2float_rn((long long)warp_sum_u64(t)), 9.094947017729282e-13f);  // 2^-40
+            for (int lr = wpart * 32 + lane; lr < live_rows; lr += WPG * 32) {
+                float pr = __fdiv_rn(lgw[lr], sf);
+                if (NAIVE) pr = bf16_round(pr);
+                lgw[lr] = pr;
+            }
         }
         __syncthreads();
         stamp(p, 9);
 
         // ---- 10. y = P.V over the V ring, cluster-wide reduction = X3
-        float acc[G][8];
+        // A warp has CH / 8 neighbouring rows of a chunk and all their columns, CPL a lane: nothing to add up across lanes.
+        float acc[G][CPL];
 #pragma unroll
         for (int g = 0; g < G; ++g)
 #pragma unroll
-            for (int i = 0; i < 8; ++i) acc[g][i] = 0.f;
-        const int rg = tid / LPR;
+            for (int i = 0; i < CPL; ++i) acc[g][i] = 0.f;
+        const int rw = CH / kWarps;
         for (int j = 0; j < nlc_live; ++j) {
             const int stage = j % NS;
             mbar_wait(&vbar[stage], (j / NS) & 1);
-            const int rows_c = chunk_rows_valid(j);
-            const uint8_t* vbase = vring + stage * chunk_bytes;
-            for (int r = rg; r < rows_c; r += NRG) {
+            const int r_end = min(chunk_rows_valid(j), (warp + 1) * rw);
+            const uint8_t* vbase = vring + stage * chunk_bytes + lane * (CPL * 2);
+#pragma unroll 2
+            for (int r = warp * rw; r < r_end; r += 2) {
                 const int lr = (j << chs) + r;
-                uint4 vv = *reinterpret_cast<const uint4*>(vbase + r * kRowBytes + li * 16);
-                if (lr == patch_row) vv = vnew8;
-                float vf[8];
-                unpack8(vv, vf);
+                uint32_t vv[2][CPL / 2];
+#pragma unroll
+                for (int x = 0; x < 2; ++x) {
+                    if constexpr (CPL == 4) {
+                        const uint2 u = *reinterpret_cast<const uint2*>(vbase + (r + x) * kRowBytes);
+                        vv[x][0] = u.x;
+                        vv[x][1] = u.y;
+                    } else {
+                        vv[x][0] = *reinterpret_cast<const uint32_t*>(vbase + (r + x) * kRowBytes);
+                    }
+#pragma unroll
+                    for (int i = 0; i < CPL / 2; ++i) {
+                        if (lr + x == patch_row) vv[x][i] = vnew[i];
+                        if (r + x >= r_end) vv[x][i] = 0;      // not loaded: no number
+                    }
+                }
 #pragma unroll
                 for (int g = 0; g < G; ++g) {
-                    const float pr = lg[g * stride + lr];
+                    const float2 pr = *reinterpret_cast<const float2*>(lg + g * stride + lr);
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) acc[g][i] = fmaf(pr, vf[i], acc[g][i]);
+                    for (int i = 0; i < CPL; ++i) {
+                        const float v0 = __uint_as_float(i & 1 ? vv[0][i / 2] & 0xffff0000u : vv[0][i / 2] << 16);
+                        const float v1 = __uint_as_float(i & 1 ? vv[1][i / 2] & 0xffff0000u : vv[1][i / 2] << 16);
+                        acc[g][i] = fmaf(pr.y, v1, fmaf(pr.x, v0, acc[g][i]));
+                    }
                 }
             }
             if (j + NS < nlc_live) {  // ring slot is refilled: everyone must be done with it
@@ -642,27 +680,16 @@ cc_decode_kernel(const __grid_constant__ DecodeParams p) {
                     const int jn = j + NS;
                     const uint32_t bytes = chunk_rows_valid(jn) * kRowBytes;
                     mbar_expect_tx(&vbar[stage], bytes);
-                    tma_load_1d(vring + stage * chunk_bytes, vc + ((size_t)((jn << csh) + rank) << chs) * D, bytes, &vbar[stage]);
+                    tma_load_1d(vring + stage * chunk_bytes, chunk_at(vc, jn), bytes, &vbar[stage]);
                 }
             }
         }
         stamp(p, 10);
 #pragma unroll
-        for (int g = 0; g < G; ++g)
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                float v = acc[g][i];
-#pragma unroll
-                for (int d = 16; d >= LPR; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
-                acc[g][i] = v;
-            }
-        if (lane < LPR) {
-#pragma unroll
-            for (int g = 0; g < G; ++g) {
-                float4* dst = reinterpret_cast<float4*>(&red[warp * G * D + g * D + lane * 8]);
-                dst[0] = make_float4(acc[g][0], acc[g][1], acc[g][2], acc[g][3]);
-                dst[1] = make_float4(acc[g][4], acc[g][5], acc[g][6], acc[g][7]);
-            }
+        for (int g = 0; g < G; ++g) {
+            float* dst = &red[warp * G * D + g * D + lane * CPL];
+            if constexpr (CPL == 4) *reinterpret_cast<float4*>(dst) = make_float4(acc[g][0], acc[g][1], acc[g][2], acc[g][3]);
+            else *reinterpret_cast<float2*>(dst) = make_float2(acc[g][0], acc[g][1]);
         }
         __syncthreads();
         const int SL = (G * D) >> csh;  // outputs reduced by each CTA of the cluster (a multiple of 4)
@@ -674,6 +701,11 @@ cc_decode_kernel(const __grid_constant__ DecodeParams p) {
                 const float4 t = *reinterpret_cast<const float4*>(&red[w * G * D + o]);
                 s.x += t.x; s.y += t.y; s.z += t.z; s.w += t.w;
             }
+            if (solo) {
+                __nv_bfloat162 y2[2] = {__floats2bfloat162_rn(s.x, s.y), __floats2bfloat162_rn(s.z, s.w)};
+                *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(p.a.y) + (size_t)h * G * D + o) = *reinterpret_cast<uint2*>(y2);
+                continue;
+            }
             const int dest = o / SL, off = o - dest * SL;
             st_async_v4f32(map_to_rank(smem_u32(&yx[rank * SL + off]), dest), s, map_to_rank(smem_u32(&xbar[3]), dest));
         }
@@ -684,19 +716,16 @@ cc_decode_kernel(const __grid_constant__ DecodeParams p) {
     // ---- 7. owner CTA: in-place slot overwrite (cache.py:390-401 / 460-490) + policy state
     if (i_own && warp == kWarps - 1) {
         if (lane < LPR) {
-            const uint16_t* ks = reinterpret_cast<const uint16_t*>(p.a.k_new) + (size_t)h * D + lane * 8;
-            const uint16_t* vs = reinterpret_cast<const uint16_t*>(p.a.v_new) + (size_t)h * D + lane * 8;
             uint16_t* kd = reinterpret_cast<uint16_t*>(st.k_cache) + ((size_t)h * L + widx) * D + lane * 8;
             uint16_t* vd = reinterpret_cast<uint16_t*>(st.v_cache) + ((size_t)h * L + widx) * D + lane * 8;
-            *reinterpret_cast<uint4*>(kd) = *reinterpret_cast<const uint4*>(ks);
-            *reinterpret_cast<uint4*>(vd) = *reinterpret_cast<const uint4*>(vs);
+            *reinterpret_cast<uint4*>(kd) = knew8;     // lane == li
+            *reinterpret_cast<uint4*>(vd) = vnew8;
         }
         float knorm = 0.f;
         if constexpr (POLICY == CC_POLICY_L2) {
             // key_norm[idx] = ||k_new||_2 (cache.py:592-593), canonical tree, correctly rounded sqrt
             float kf[8];
-            const uint4 kv = *reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(p.a.k_new) + (size_t)h * D + li * 8);
-            unpack8(kv, kf);
+            unpack8(knew8, kf);
             float acc = 0.f;
 #pragma unroll
             for (int i = 0; i < 8; ++i) acc = __fmaf_rn(kf[i], kf[i], acc);
@@ -777,18 +806,17 @@ cc_decode_kernel(const __grid_constant__ DecodeParams p) {
                     pooled = __bfloat162float(probs[(size_t)h * L + s]);
                 }
                 if (hh_score) {
-                    double* num = reinterpret_cast<double*>(st.attn_history_num) + (size_t)h * L;
-                    int32_t* den = st.attn_history_denom + (size_t)h * L;
-                    const bool fresh = has_slot && s == widx;  // evicted slot's history restarts (cache.py:753-763)
-                    num[s] = (fresh ? 0.0 : num[s]) + (double)pooled;
-                    den[s] = (fresh ? 0 : den[s]) + 1;
+                    const bool first = lr == tid, fresh = has_slot && s == widx;  // evicted slot's history restarts (cache.py:753-763)
+                    const double was = first ? hist0 : hist[s];
+                    const int seen = first ? den0 : den[s];
+                    reinterpret_cast<double*>(st.attn_history_num)[(size_t)h * L + s] = (fresh ? 0.0 : was) + (double)pooled;
+                    st.attn_history_denom[(size_t)h * L + s] = (fresh ? 0 : seen) + 1;
                 } else if (hhr_score) {
                     // ring[s][counter % W] = pooled (or its indicator), denominators + 1; the evicted slot starts
                     // from a cleared ring (cache.py:716-723, 753-763).  hsum = exact running sum of the ring.
-                    int32_t* den = st.attn_history_denom + (size_t)h * L;
                     double* hs = st.attn_history_sum + (size_t)h * L + s;
                     const bool fresh = has_slot && s == widx;
-                    den[s] = (fresh ? 0 : den[s]) + 1;
+                    st.attn_history_denom[(size_t)h * L + s] = (fresh ? 0 : den[s]) + 1;
                     if (st.attn_thresholding) {
                         uint8_t* cell = reinterpret_cast<uint8_t*>(st.attn_history_num) + ((size_t)h * L + s) * W + wslot;
                         const float v = pooled >= thr ? 1.f : 0.f;
@@ -804,8 +832,7 @@ cc_decode_kernel(const __grid_constant__ DecodeParams p) {
                 } else if (ring_score) {
                     // ring[s][counter % W] = pooled; the evicted slot keeps its ring (the reference's reset is a
                     // silent no-op, cache.py:993-996).  Only live slots can hold non-zero history.
-                    int32_t* den = st.attn_history_denom + (size_t)h * L;
-                    den[s] += 1;
+                    st.attn_history_denom[(size_t)h * L + s] = den[s] + 1;
                     if (s < live_limit || pooled != 0.f) {
                         __nv_bfloat16* cell = reinterpret_cast<__nv_bfloat16*>(st.attn_history_num) + ((size_t)h * L + s) * W + wslot;
                         const float old = __bfloat162float(*cell);
@@ -821,7 +848,7 @@ cc_decode_kernel(const __grid_constant__ DecodeParams p) {
         if (hh_score && h == 0 && rank == 0 && tid == 0) st.attn_counter[0] += 1;
     }
 
-    if (do_attend) {
+    if (do_attend && !solo) {
         mbar_wait(&xbar[3], 0);
         stamp(p, 12);
         const int SL = (G * D) >> csh;
@@ -926,13 +953,18 @@ static int make_plan(const CcCacheState* st, bool needs_epoch, LaunchPlan* out) 
         cudaGetLastError();
         return set_error(CC_ERR_CUDA, "cannot raise the dynamic shared memory limit");
     }
-    // chunk size: the largest of 64/32/16 rows that still gives every CTA of a 16-cluster a chunk
-    int chs = 6;
-    while (chs > 4 && ((L + (1 << chs) - 1) >> chs) < kMaxCluster) --chs;
-    const int n_chunks = (L + (1 << chs) - 1) >> chs;
     int c_max = kMaxCluster;
     if (const char* e = getenv("CC_B200_MAX_CLUSTER")) c_max = atoi(e) > 0 ? atoi(e) : c_max;  // experiments only
+    // 16 CTAs per head from 1024 slots, or from 257 if they take at most half of the SMs; else up to 8: an exchange among 16 costs more
+    // than the shorter rows give.  32 steps in a graph, 16 / 8 / 4 CTAs, us a step: 8 heads of group 4, 256 slots 7.0 / 6.5 / 6.9, 512
+    // slots 7.4 / 7.0 / 8.3, 1024 slots of heavy hitters 8.5 / 8.7 / 11.4; 4 heads of group 7, 256 slots 7.0 / 7.2 / 7.8, 512 slots
+    // 7.5 / 7.9 / 9.5.  Up to 128 slots 4 and 8 are alike; one CTA without exchanges loses to both from 64 slots on (6.7 / 6.3).
+    if (L < 1024 && (L <= 256 || H * kMaxCluster > g_num_sms / 2) && c_max > 8) c_max = 8;
     for (int C = c_max; C >= 1; C >>= 1) {
+        // chunk size: the largest of 64/32/16 rows that still gives every CTA of the cluster a chunk
+        int chs = 6;
+        while (chs > 4 && ((L + (1 << chs) - 1) >> chs) < C) --chs;
+        const int n_chunks = (L + (1 << chs) - 1) >> chs;
         if (C > 1 && (H * C > g_num_sms || C > n_chunks)) continue;
         const int mlc = (n_chunks + C - 1) / C;
         const int stride = ((mlc << chs) + 31) / 32 * 32;
