@@ -137,7 +137,7 @@ def check(rc: int, what: str = "") -> int:
 
 # --------------------------------------------------------------------------- libcc_b200_seq.so (include/cc_b200_seq.h)
 SEQ_SO_PATH = Path(os.environ.get("CC_B200_SEQ_LIB", PKG / "libcc_b200_seq.so"))
-SEQ_ABI_VERSION = 8
+SEQ_ABI_VERSION = 9
 DT_F32, DT_BF16 = 0, 1
 SINK_NONE, SINK_LEARNED, SINK_ZERO = 0, 1, 2
 
@@ -264,6 +264,8 @@ SEQ_EXPORTS.update({
     "cc_seq_head_gemv": (C.c_int, [_vp, _i32, _vp, _i32, _i64, _vp, _i32, _i64, _vp, _i32, _i32, _i32, _vp]),
     "cc_seq_wkv": (C.c_int, [C.POINTER(CcSeqWkv), _vp]),
     "cc_seq_wkv_decay": (C.c_int, [_vp, _vp, _vp, _i32, _i32, _vp]),
+    "cc_seq_wkv_segments_workspace": (C.c_uint64, [_i32, _i32, _i32]),
+    "cc_seq_wkv_segments": (C.c_int, [C.POINTER(CcSeqWkv), _vp, C.c_uint64, _vp]),
     "cc_seq_head_norm_gate": (C.c_int, [_vp, _vp, _i64, _vp, _vp, _i32, _i32, _i32, _i32, _f32, _vp]),
     "cc_seq_moe_route": (C.c_int, [_vp, _i64, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _i32, _i32, _i32, _i32, _f32, _vp]),
     "cc_seq_moe_group": (C.c_int, [_vp, _i32, _i32, _i32, _vp, _vp, _vp, _vp]),

@@ -317,6 +317,13 @@ def wkv(r, k, v, wraw, w0, u, state, o, H, D):
     a.r, a.k, a.v, a.wraw, a.w0, a.u, a.state, a.o = _p(r), _p(k), _p(v), _p(wraw), _p(w0), _p(u), _p(state), _p(o)
     a.T, a.H, a.D = r.shape[0], int(H), int(D)
     assert r.shape[1] == H * D and state.numel() == H * D * D
+    lib = _lib.load_seq()
+    if a.T >= WKV_SEGMENTS_FROM and not (a.r | a.k | a.v | a.wraw | a.state) & 15:
+        nbytes = lib.cc_seq_wkv_segments_workspace(a.T, a.H, a.D)
+        if nbytes:
+            ws = torch.empty(nbytes, dtype=torch.uint8, device=o.device)
+            _lib.check_seq(lib.cc_seq_wkv_segments(C.byref(a), _p(ws), nbytes, _stream()), "cc_seq_wkv_segments")
+            return
     if a.T >= WKV_DECAY_FROM:
         # long steps: the decays in a launch of their own, spread over the GPU, instead of once per column tile inside the
         # recurrence; same arithmetic, same bits
@@ -330,6 +337,11 @@ def wkv(r, k, v, wraw, w0, u, state, o, H, D):
 # 7.1 / 7.9, 10.2 / 12.9; 128 heads of 64 8.0 / 7.4, 11.4 / 10.9, 17.6 / 17.8; 8 heads of 256 8.1 / 9.1, 11.5 / 14.5, 18.3 / 25.2.  From 64 on
 # it is no loss for any number of heads; fewer heads would gain from about 20 on.
 WKV_DECAY_FROM = 64
+
+# Tokens from which segments of a step go side by side, where the library serves the head size (other roundings than token after
+# token: steps below it give the same bits however they are cut).  Measured segments / one after another in us: 256 tokens of 1, 16, 32,
+# 128 heads of 64 20 / 28, 20 / 29, 21 / 29, 51 / 56, of 16 and 64 heads of 128 33 / 36 and 95 / 108; 192 tokens of 32 heads of 64 20 / 23.
+WKV_SEGMENTS_FROM = 256
 
 
 def head_norm_gate(o, graw, nw, out, H, D, eps):

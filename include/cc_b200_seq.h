@@ -21,7 +21,7 @@
 extern "C" {
 #endif
 
-#define CC_SEQ_ABI_VERSION 8
+#define CC_SEQ_ABI_VERSION 9
 
 #define CC_SEQ_OK                     0
 #define CC_SEQ_ERR_INVALID_ARG       -1
@@ -336,6 +336,13 @@ typedef struct CcSeqWkv {
 int cc_seq_wkv(const CcSeqWkv* a, void* stream);
 /* w = exp(-exp(wraw + w0)), fp32 [T, HD] */
 int cc_seq_wkv_decay(const float* wraw, const float* w0, float* w, int32_t T, int32_t HD, void* stream);
+/*
+ * The same recurrence for steps of many tokens, segments of them side by side (decayed == 0).  Serves heads of multiples of 4 up to
+ * 128 whose r, k, v, wraw, state and workspace start on 16-byte boundaries.  cc_seq_wkv_segments_workspace: bytes that a step
+ * needs, 0 where it is not cut (too few tokens for the heads, other head sizes).
+ */
+uint64_t cc_seq_wkv_segments_workspace(int32_t T, int32_t H, int32_t D);
+int cc_seq_wkv_segments(const CcSeqWkv* a, void* workspace, uint64_t workspace_bytes, void* stream);
 
 /* out[t, h, :] = o[t, h, :] / sqrt(mean(o[t, h, :]^2) + eps) * nw[h, :] * silu(graw[t, h, :])   (graw fp32 [T, ldg]) */
 int cc_seq_head_norm_gate(const float* o, const float* graw, int64_t ldg, const float* nw, void* out, int32_t out_dtype,
