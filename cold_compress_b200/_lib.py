@@ -137,7 +137,7 @@ def check(rc: int, what: str = "") -> int:
 
 # --------------------------------------------------------------------------- libcc_b200_seq.so (include/cc_b200_seq.h)
 SEQ_SO_PATH = Path(os.environ.get("CC_B200_SEQ_LIB", PKG / "libcc_b200_seq.so"))
-SEQ_ABI_VERSION = 9
+SEQ_ABI_VERSION = 10
 DT_F32, DT_BF16 = 0, 1
 SINK_NONE, SINK_LEARNED, SINK_ZERO = 0, 1, 2
 
@@ -193,7 +193,7 @@ GEMV_MAX_JOBS = 6
 
 class CcSeqGemvJob(C.Structure):
     _fields_ = [("x", _vp), ("W", _vp), ("out", _vp)] + [(n, _i32) for n in ("x_dtype", "kind", "off_gate", "off_up", "N", "K")] + [
-        ("conv_w", _vp), ("tail", _vp)] + [(n, _i32) for n in ("conv_rows", "taps", "conv_act")]
+        ("conv_w", _vp), ("tail", _vp)] + [(n, _i32) for n in ("conv_rows", "taps", "conv_act", "pair", "pair_act")]
 
 
 GEMV_PRE_NONE, GEMV_PRE_OUTPUT_NORM, GEMV_PRE_GATED_HEADS = range(3)

@@ -1117,7 +1117,9 @@ constexpr int GEMV_CTAS = 4;       // CTAs per SM (64 registers per thread)
 // Bound: HBM for many rows; the input's 32 bytes from shared memory per 16 bytes of weights held one row per warp below it
 // (16384 x 2048, alone in a graph: 14.4 us, without those reads 11.4, floor 10.2).  Decode step of a 4-layer model of width
 // 2048 at 4096 positions: 370 us with one row per warp, four loads in flight and every launch behind the one before it, 338
-// with eight loads across rows and launches under their predecessor, 312 with pairs and the small launches alike.
+// with eight loads across rows and launches under their predecessor, 312 with pairs and the small launches alike.  The way in of a
+// down product that formed act(gate) * up itself was 512 CTAs times 8192 units read 4 bytes at a time (2048 x 8192: 33 us, 13 with
+// the units on the way out of the product before, each formed once, and 16 bytes an access): 307 -> 273.
 template <typename WT, int PRE, int KS>
 __global__ void __launch_bounds__(256, GEMV_CTAS) gemv_multi_kernel(const CcSeqGemvMulti g, int rows_per_cta) {
     extern __shared__ float4 smg4[];
@@ -1139,13 +1141,17 @@ __global__ void __launch_bounds__(256, GEMV_CTAS) gemv_multi_kernel(const CcSeqG
     constexpr int VEC = 16 / (int)sizeof(WT);
     const bool vec = K % VEC == 0;
     const int nv = K / VEC, v0 = lane + 32 * ks;    // this lane's vectors of a row: v0, v0 + STEP, ...
-    auto row = [&](int n) { return reinterpret_cast<const uint4*>(W + (size_t)min(n, jb.N - 1) * K); };   // rows past the end: the last one
+    // rows past the end: the last one.  With a unit on the way out a warp's pair is a gate row and its up row.
+    auto row = [&](int n, int r) {
+        const int m = jb.pair > 0 ? (min(n, jb.N - 2) >> 1) + r * jb.pair : min(n + r, jb.N - 1);
+        return reinterpret_cast<const uint4*>(W + (size_t)m * K);
+    };
     if (vec && lane % 8 == 0) {      // a line of 128 bytes per request
 #pragma unroll
         for (int u = 0; u < GEMV_AHEAD; ++u)
 #pragma unroll
             for (int r = 0; r < GEMV_ROWS; ++r)
-                if (v0 + STEP * u < nv) ccs::ask_l2(row(n0 + r) + v0 + STEP * u);
+                if (v0 + STEP * u < nv) ccs::ask_l2(row(n0, r) + v0 + STEP * u);
     }
     ccs::pdl_wait_release();
     uint4 buf[GEMV_ROWS][GEMV_AHEAD];
@@ -1153,7 +1159,7 @@ __global__ void __launch_bounds__(256, GEMV_CTAS) gemv_multi_kernel(const CcSeqG
     for (int u = 0; u < GEMV_AHEAD; ++u)
 #pragma unroll
         for (int r = 0; r < GEMV_ROWS; ++r)
-            buf[r][u] = vec && v0 + STEP * u < nv ? ld_weights(row(n0 + r) + v0 + STEP * u) : make_uint4(0u, 0u, 0u, 0u);
+            buf[r][u] = vec && v0 + STEP * u < nv ? ld_weights(row(n0, r) + v0 + STEP * u) : make_uint4(0u, 0u, 0u, 0u);
     bool shared_row = false;
     if constexpr (PRE != CC_GEMV_PRE_NONE) shared_row = jb.x == nullptr;
     if (shared_row) {
@@ -1165,19 +1171,55 @@ __global__ void __launch_bounds__(256, GEMV_CTAS) gemv_multi_kernel(const CcSeqG
             gemv_gated_heads_row<WT>(g.pre, xs, K, W);
         }
     } else if (jb.kind != CC_ACT_NONE || jb.off_up >= 0) {
-        const float* src = (const float*)jb.x;
+        const float* src = (const float*)jb.x + jb.off_gate;
+        const float* up = (const float*)jb.x + jb.off_up;
+        const bool two = jb.off_up >= 0;
+        if (K % 4 == 0 && (((uintptr_t)src | (two ? (uintptr_t)up : 0)) & 15) == 0) {
 #pragma unroll 4
-        for (int k = tid; k < K; k += 256) {
-            float v = unit_act(src[jb.off_gate + k], jb.kind);
-            if (jb.off_up >= 0) v *= src[jb.off_up + k];
-            xs[k] = round_to(v, W);
+            for (int k = 4 * tid; k < K; k += 1024) {
+                const float4 a = *reinterpret_cast<const float4*>(src + k);
+                float4 u = make_float4(1.f, 1.f, 1.f, 1.f);
+                if (two) u = *reinterpret_cast<const float4*>(up + k);
+                float4 v = make_float4(unit_act(a.x, jb.kind), unit_act(a.y, jb.kind), unit_act(a.z, jb.kind), unit_act(a.w, jb.kind));
+                if (two) v = make_float4(v.x * u.x, v.y * u.y, v.z * u.z, v.w * u.w);
+                *reinterpret_cast<float4*>(xs + k) = make_float4(round_to(v.x, W), round_to(v.y, W), round_to(v.z, W), round_to(v.w, W));
+            }
+        } else {
+#pragma unroll 4
+            for (int k = tid; k < K; k += 256) {
+                float v = unit_act(src[k], jb.kind);
+                if (two) v *= up[k];
+                xs[k] = round_to(v, W);
+            }
         }
     } else if (jb.x_dtype == CC_DT_F32) {
+        const float* src = (const float*)jb.x;
+        if (K % 4 == 0 && ((uintptr_t)src & 15) == 0) {
+#pragma unroll 8
+            for (int k = 4 * tid; k < K; k += 1024) {
+                const float4 v = *reinterpret_cast<const float4*>(src + k);
+                *reinterpret_cast<float4*>(xs + k) = make_float4(round_to(v.x, W), round_to(v.y, W), round_to(v.z, W), round_to(v.w, W));
+            }
+        } else {
 #pragma unroll 4
-        for (int k = tid; k < K; k += 256) xs[k] = round_to(((const float*)jb.x)[k], W);
+            for (int k = tid; k < K; k += 256) xs[k] = round_to(src[k], W);
+        }
     } else {
+        const bf16* src = (const bf16*)jb.x;
+        if (K % 8 == 0 && ((uintptr_t)src & 15) == 0) {
 #pragma unroll 4
-        for (int k = tid; k < K; k += 256) xs[k] = __bfloat162float(((const bf16*)jb.x)[k]);
+            for (int k = 8 * tid; k < K; k += 2048) {
+                const uint4 v = *reinterpret_cast<const uint4*>(src + k);
+                const uint32_t e[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                for (int q = 0; q < 2; ++q)
+                    *reinterpret_cast<float4*>(xs + k + 4 * q) = make_float4(__uint_as_float(e[2 * q] << 16), __uint_as_float(e[2 * q] & 0xffff0000u),
+                                                                             __uint_as_float(e[2 * q + 1] << 16), __uint_as_float(e[2 * q + 1] & 0xffff0000u));
+            }
+        } else {
+#pragma unroll 4
+            for (int k = tid; k < K; k += 256) xs[k] = __bfloat162float(src[k]);
+        }
     }
     __syncthreads();
     if (KS == 1 && n0 >= n_end) return;
@@ -1194,7 +1236,7 @@ __global__ void __launch_bounds__(256, GEMV_CTAS) gemv_multi_kernel(const CcSeqG
                 const int left = last && !more ? 0 : nv - from;
                 const uint4* next[GEMV_ROWS];
 #pragma unroll
-                for (int r = 0; r < GEMV_ROWS; ++r) next[r] = row(last ? n + RW + r : n + r) + from;
+                for (int r = 0; r < GEMV_ROWS; ++r) next[r] = row(last ? n + RW : n, r) + from;
 #pragma unroll
                 for (int u = 0; u < GEMV_AHEAD; ++u) {
                     if (c + STEP * u < nv) {
@@ -1221,7 +1263,7 @@ __global__ void __launch_bounds__(256, GEMV_CTAS) gemv_multi_kernel(const CcSeqG
         } else {
 #pragma unroll
             for (int r = 0; r < GEMV_ROWS; ++r) {
-                const WT* w = W + (size_t)min(n + r, jb.N - 1) * K;
+                const WT* w = reinterpret_cast<const WT*>(row(n, r));
                 for (int k = lane + 32 * ks; k < K; k += STEP) acc[r] = fmaf(ldf(w, k), xs[k], acc[r]);
             }
         }
@@ -1238,7 +1280,10 @@ __global__ void __launch_bounds__(256, GEMV_CTAS) gemv_multi_kernel(const CcSeqG
             for (int q = 1; q < KS; ++q) sum += red[(warp + q) * GEMV_ROWS + lane % GEMV_ROWS];
         }
         const int m = n + lane;
-        if (lane < GEMV_ROWS && m < n_end) {
+        if (jb.pair > 0) {
+            const float up = __shfl_sync(0xffffffffu, sum, 1);
+            if (lane == 0 && n < n_end) stf((WT*)jb.out, n >> 1, unit_act(sum, jb.pair_act) * up);
+        } else if (lane < GEMV_ROWS && m < n_end) {
             if (m < jb.conv_rows) {      // this row is a channel: its past inputs, then the tail moves on
                 const int C = jb.conv_rows, taps = jb.taps;
                 const float* cw = jb.conv_w + (size_t)m * taps;
@@ -1561,6 +1606,8 @@ int cc_seq_gemv_multi(const CcSeqGemvMulti* g, void* stream) {
         if (!b.W || (!b.out && !(j == 0 && g->post.x)) || b.N < 1 || b.K < 1 || b.kind < CC_ACT_NONE || b.kind > CC_ACT_LAST ||
             ((b.kind != CC_ACT_NONE || b.off_up >= 0) && b.x_dtype != CC_DT_F32))
             return fail(CC_SEQ_ERR_INVALID_ARG, "gemv_multi: bad job");
+        if (b.pair && (b.pair < 0 || b.N != 2 * b.pair || b.conv_rows || (j == 0 && g->post.x) || b.pair_act < CC_ACT_NONE || b.pair_act > CC_ACT_LAST))
+            return fail(CC_SEQ_ERR_INVALID_ARG, "gemv_multi: bad unit on the way out");
         if (b.conv_rows < 0 || b.conv_rows > b.N || (b.conv_rows > 0 && (!b.conv_w || b.taps < 1 || (b.taps > 1 && !b.tail) ||
                                                                          b.conv_act < CC_ACT_NONE || b.conv_act > CC_ACT_LAST)))
             return fail(CC_SEQ_ERR_INVALID_ARG, "gemv_multi: bad convolution");

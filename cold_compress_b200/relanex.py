@@ -229,16 +229,15 @@ class Stream:
         self.first = x if keep else None      # the embedding output, when later passes add it
 
     def close(self, inp: Optional[Tensor], w: Tensor, out_norm: BoundedNorm, next_norm: BoundedNorm, one_token: bool, pre=None,
-              built=(), add_first: bool = False, rows: Optional[Tensor] = None):
+              add_first: bool = False, rows: Optional[Tensor] = None):
         """x += mult * out_norm(w inp) (+ the embedding output); h = next_norm(x).  One token: `inp` None takes the shared row
-        `pre`, `built` = (activation, gate column, up column) forms the input of a gated unit.  `rows`: only these rows are
-        wanted and x ends here."""
+        `pre`.  `rows`: only these rows are wanted and x ends here."""
         x, add = self.x, (self.first if add_first else None)
         if one_token:
             h = torch.empty_like(self.h)
             x_out = torch.empty_like(x) if x is self.first else x
             post = seq_ops.bounded_way_out(x, out_norm.parts, self.mult, x_out, next_norm.parts, h, add)
-            seq_ops.gemv_multi([(inp, w, None, *built)], pre=pre, post=post)
+            seq_ops.gemv_multi([(inp, w, None)], pre=pre, post=post)
             self.x, self.h = x_out, h
             return
         y = _mm(inp, w)
@@ -295,13 +294,12 @@ class RelanexBlock(nn.Module):
         if self.mlp is None:
             return
         f = self.mlp
-        gu = _product(s.h, self.w_gu, one_token)
+        act = torch.empty(s.h.shape[0], f.ff, dtype=f.w_down.dtype, device=s.h.device)
         if one_token:
-            s.close(gu, f.w_down, self.norm2b, next_norm, True, built=(f.act, 0, f.ff), **last)
-            return
-        act = torch.empty(gu.shape[0], f.ff, dtype=f.w_down.dtype, device=gu.device)
-        seq_ops.gated_unit(gu, 0, f.ff, act, f.act)
-        s.close(act, f.w_down, self.norm2b, next_norm, False, **last)
+            seq_ops.gemv_multi([(s.h, self.w_gu, act)], unit=f.act)
+        else:
+            seq_ops.gated_unit(_product(s.h, self.w_gu, False), 0, f.ff, act, f.act)
+        s.close(act, f.w_down, self.norm2b, next_norm, one_token, **last)
 
     def kernels_per_token(self) -> int:
         return self.mixer.kernels_per_token + (2 if self.mlp is not None else 0)

@@ -490,13 +490,13 @@ def latent_decode(q, k_new, k_cache, pos, mask, cache_cts, input_pos, y, scale, 
     _lib.check_seq(_lib.load_seq().cc_seq_latent_decode(C.byref(a), _stream()), "cc_seq_latent_decode")
 
 
-def gemv_multi(jobs, pre=None, conv=None, post=None):
+def gemv_multi(jobs, pre=None, conv=None, post=None, unit=None):
     """Up to six one-token products in one launch.  jobs: (x, w, out) or (src, w, out, kind, off_gate, off_up) where the
     input is built from the fp32 row `src` as act(src[off_gate + k]) * src[off_up + k]; out fp32 [1, N].  x = None: the
     launch's shared row `pre` (output_norm_row or gated_heads_row), which every CTA forms for itself.  conv = (table
     [C, taps], tail [taps - 1, C], act): the first C rows of job 0 pass that short convolution, whose tail moves on.
     post = bounded_way_out(...): job 0's rows are a sublayer's result and join the stream on their way out (its out may be
-    None)."""
+    None).  unit = an activation: job 0's rows are gate | up rows, its out [1, N / 2] in the weights' type is act(gate) * up."""
     g = _lib.CcSeqGemvMulti()
     g.n_jobs = len(jobs)
     assert 1 <= len(jobs) <= _lib.GEMV_MAX_JOBS
@@ -504,13 +504,16 @@ def gemv_multi(jobs, pre=None, conv=None, post=None):
     for j, job in enumerate(jobs):
         x, w, out = job[:3]
         kind, off_gate, off_up = job[3:] if len(job) > 3 else (_lib.ACT_NONE, 0, -1)
-        _need(("x", x, None), ("w", w, jobs[0][1].dtype), ("out", out, torch.float32))
+        paired = j == 0 and unit is not None
+        _need(("x", x, None), ("w", w, jobs[0][1].dtype), ("out", out, w.dtype if paired else torch.float32))
         N, K = w.shape
         built = kind != _lib.ACT_NONE or off_up >= 0
-        assert (out is None if j == 0 and post is not None and out is None else out.numel() == N) and (pre.length == K if x is None else x.numel() >= max(off_gate, off_up) + K if built else x.numel() == K)
+        assert (out is None if j == 0 and post is not None and out is None else out.numel() * (2 if paired else 1) == N) and (pre.length == K if x is None else x.numel() >= max(off_gate, off_up) + K if built else x.numel() == K)
         b = g.job[j]
         b.x, b.W, b.out = _p(x), _p(w), _p(out)
         b.x_dtype, b.kind, b.off_gate, b.off_up, b.N, b.K = _dt(x) if x is not None else _lib.DT_F32, int(kind), int(off_gate), int(off_up), N, K
+        if paired:
+            b.pair, b.pair_act = N // 2, int(unit)
     if pre is not None:
         g.pre = pre
     if post is not None:

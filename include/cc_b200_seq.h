@@ -21,7 +21,7 @@
 extern "C" {
 #endif
 
-#define CC_SEQ_ABI_VERSION 9
+#define CC_SEQ_ABI_VERSION 10
 
 #define CC_SEQ_OK                     0
 #define CC_SEQ_ERR_INVALID_ARG       -1
@@ -271,6 +271,8 @@ int cc_seq_latent_decode(const CcSeqLatentDecode* a, void* stream);
  *                            (part_len 0 = w_len)
  * conv_rows > 0: rows n < conv_rows of the job then pass a causal convolution over time (a channel per row, the taps
  * before the current one from `tail` fp32 [taps - 1, conv_rows], which is moved on) and the activation conv_act.
+ * pair > 0: the job's N = 2 pair rows are the gate and up rows of a gated unit; `out` [pair], in the weights' type, is
+ * pair_act(row n) * (row n + pair), formed in fp32.
  * post.x set: row n of job 0 is the sublayer's result for channel n and passes cc_seq_bounded_sum's arithmetic on its
  * way out (post.y, T, E and rows are not used; post.x_out may be post.x; job 0's `out` may then be NULL).
  */
@@ -282,7 +284,7 @@ typedef struct CcSeqGemvJob {
     const void* x;  const void* W;  void* out;
     int32_t x_dtype, kind, off_gate, off_up, N, K;
     const float* conv_w;  float* tail;
-    int32_t conv_rows, taps, conv_act;
+    int32_t conv_rows, taps, conv_act, pair, pair_act;
 } CcSeqGemvJob;
 typedef struct CcSeqGemvPre {
     int32_t kind, top, w_len, gate_act;
