@@ -264,6 +264,7 @@ SEQ_EXPORTS.update({
     "cc_seq_head_gemv": (C.c_int, [_vp, _i32, _vp, _i32, _i64, _vp, _i32, _i64, _vp, _i32, _i32, _i32, _vp]),
     "cc_seq_wkv": (C.c_int, [C.POINTER(CcSeqWkv), _vp]),
     "cc_seq_wkv_decay": (C.c_int, [_vp, _vp, _vp, _i32, _i32, _vp]),
+    "cc_seq_greedy": (C.c_int, [_vp, _i32, _vp, _vp, _vp]),
     "cc_seq_wkv_segments_workspace": (C.c_uint64, [_i32, _i32, _i32]),
     "cc_seq_wkv_segments": (C.c_int, [C.POINTER(CcSeqWkv), _vp, C.c_uint64, _vp]),
     "cc_seq_head_norm_gate": (C.c_int, [_vp, _vp, _i64, _vp, _vp, _i32, _i32, _i32, _i32, _f32, _vp]),

@@ -14,6 +14,7 @@ from typing import Optional, Tuple
 import torch
 import yaml
 
+from . import ops
 from .model import Transformer, find_multiple
 
 default_device = "cuda" if torch.cuda.is_available() else "cpu"
@@ -89,6 +90,11 @@ def device_sync(device):
 # --------------------------------------------------------------------------- sampling / steps
 
 def greedy(logits, next_token):
+    row = logits[0, -1]
+    if ops.plain_tensors(torch.float32, row) and 1 < row.numel() < 1 << 30:
+        from . import seq_ops
+        token, probs = seq_ops.greedy(row)
+        return (token if next_token is None else next_token), probs
     probs = torch.nn.functional.softmax(logits[0, -1], dim=-1)
     if next_token is None:
         return torch.argmax(probs, keepdim=True).to(dtype=torch.int), probs

@@ -165,17 +165,21 @@ def _silu_mul(a, b, out):
     _lib.check(_lib.load().cc_silu_mul(_ptr(a), _ptr(b), _ptr(out), a.numel(), _stream()), "cc_silu_mul")
 
 
-def plain_rows(*tensors) -> bool:
-    """Whether the row kernels of a prompt layer may stand for tensor operations on these: plain contiguous bf16 CUDA tensors
-    whose last dimension is whole 16-byte vectors, on 16-byte boundaries, on the current device (where the kernels are
-    launched), outside of differentiation (reverse or forward), of function transforms and of everything that records
-    operations to run them again on other tensors."""
+def plain_tensors(dtype, *tensors) -> bool:
+    """Whether kernels may stand for tensor operations on these: plain contiguous CUDA tensors of this type on 16-byte
+    boundaries, on the current device (where the kernels are launched), outside of differentiation (reverse or forward), of
+    function transforms and of everything that records operations to run them again on other tensors."""
     return (not torch.compiler.is_compiling() and torch._C._get_tracing_state() is None and torch._C._len_torch_dispatch_stack() == 0
             and torch._C._functorch.peek_interpreter_stack() is None and torch.autograd.forward_ad._current_level < 0
-            and all(type(t) in (torch.Tensor, torch.nn.Parameter) and t.is_cuda and t.dtype == torch.bfloat16 and t.is_contiguous()
-                    and t.dim() > 0 and t.numel() > 0 and t.shape[-1] % 8 == 0 and t.data_ptr() % 16 == 0 for t in tensors)
+            and all(type(t) in (torch.Tensor, torch.nn.Parameter) and t.is_cuda and t.dtype == dtype and t.is_contiguous()
+                    and t.dim() > 0 and t.numel() > 0 and t.data_ptr() % 16 == 0 for t in tensors)
             and all(t.device.index == torch.cuda.current_device() for t in tensors)
             and not (torch.is_grad_enabled() and any(t.requires_grad for t in tensors)))
+
+
+def plain_rows(*tensors) -> bool:
+    """The same for the row kernels of a prompt layer: bf16 rows of whole 16-byte vectors."""
+    return plain_tensors(torch.bfloat16, *tensors) and all(t.shape[-1] % 8 == 0 for t in tensors)
 
 
 def _optr(t):

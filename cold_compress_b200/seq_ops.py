@@ -344,6 +344,14 @@ WKV_DECAY_FROM = 64
 WKV_SEGMENTS_FROM = 256
 
 
+def greedy(logits):
+    """(token int32 [1], probs fp32 [V]) of one row of fp32 logits [V]: the softmax and the first index of its largest entry."""
+    _need(("logits", logits, torch.float32))
+    token, probs = torch.empty(1, dtype=torch.int32, device=logits.device), torch.empty_like(logits)
+    _lib.check_seq(_lib.load_seq().cc_seq_greedy(_p(logits), logits.numel(), _p(probs), _p(token), _stream()), "cc_seq_greedy")
+    return token, probs
+
+
 def head_norm_gate(o, graw, nw, out, H, D, eps):
     _need(("o", o, torch.float32), ("nw", nw, torch.float32), ("out", out, None))
     ptr, ld = _cols(_f32("graw", graw))

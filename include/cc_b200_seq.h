@@ -346,6 +346,9 @@ int cc_seq_wkv_decay(const float* wraw, const float* w0, float* w, int32_t T, in
 uint64_t cc_seq_wkv_segments_workspace(int32_t T, int32_t H, int32_t D);
 int cc_seq_wkv_segments(const CcSeqWkv* a, void* workspace, uint64_t workspace_bytes, void* stream);
 
+/* probs = softmax(logits), fp32 [V] on 16-byte boundaries; *token = the first index of the largest probability. */
+int cc_seq_greedy(const float* logits, int32_t V, float* probs, int32_t* token, void* stream);
+
 /* out[t, h, :] = o[t, h, :] / sqrt(mean(o[t, h, :]^2) + eps) * nw[h, :] * silu(graw[t, h, :])   (graw fp32 [T, ldg]) */
 int cc_seq_head_norm_gate(const float* o, const float* graw, int64_t ldg, const float* nw, void* out, int32_t out_dtype,
                           int32_t T, int32_t H, int32_t D, float eps, void* stream);
