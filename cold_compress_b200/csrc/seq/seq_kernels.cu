@@ -1022,6 +1022,418 @@ __global__ void __launch_bounds__(VD_THREADS, RMAX <= 4 ? 2 : 1) attn_decode_row
     if (a.append) append_row<CT>(a, g, 0, p, tid, VD_THREADS);
 }
 
+// ---- bf16 rows of that kind: both products on the tensor cores (mma.sync), fp32 queries and weights in three exact bf16 parts
+// Truncation takes 8 of the 24 significant bits at a time, so the three parts of a number add up to it exactly and every product
+// of a part with a bf16 key or value is exact; the sums are fp32.  An MMA cuts off what it adds below the last bit of the largest
+// term, so those of the large part start from zero and are added up, rounded, outside.  Scores: 16 keys x 8 query heads per MMA, the three parts of q
+// into one accumulator.  Values: 8 columns per MMA, two parts of the weights in the two halves of its 16 rows, the third in a
+// second one; a warp owns columns, so no sums meet across warps.  Sums that are not finite (an infinite key or value meets parts
+// that are zero) are formed again key by key with fp32 multiplications, where such operands give what they give.
+// The keys of a tile are waited for alone, its values land under the scores and the softmax.  The last CTA of a head asks for all
+// partial sums before it knows their weights, and stores the new row under them.
+// Bound: the chain of dependent waits (position 0.5 us, rows 3.6 = the HBM rate, partials and counter 1.3, combination 3) around
+// 3.3 us of work; 8 layers of 32 / 8 heads of 128, 4096 positions in a graph: 143 us on the kernel above, 109 here.  Against 64 bits
+// (fp32 results, scores of size 4): 2.1e-7 of the norm, 2.4e-7 above.
+constexpr int MD_THREADS = 256, MD_WARPS = MD_THREADS / 32, MD_AHEAD = 17, MD_KEYS = 128;      // MD_KEYS: keys of a tile
+
+__device__ __forceinline__ uint32_t smem_at(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void ldsm4(uint32_t (&r)[4], const void* p) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_at(p)) : "memory");
+}
+__device__ __forceinline__ void ldsm4_t(uint32_t (&r)[4], const void* p) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_at(p)) : "memory");
+}
+__device__ __forceinline__ void ldsm2(uint32_t (&r)[2], const void* p) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0, %1}, [%2];" : "=r"(r[0]), "=r"(r[1]) : "r"(smem_at(p)) : "memory");
+}
+__device__ __forceinline__ void mma16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+// the parts of x, largest first
+__device__ __forceinline__ void three_parts(float x, __nv_bfloat16 (&o)[3]) {
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        const uint32_t top = __float_as_uint(x) & 0xffff0000u;
+        o[i] = __ushort_as_bfloat16((unsigned short)(top >> 16));
+        x -= __uint_as_float(top);
+    }
+}
+__device__ __forceinline__ void md_bar_init(uint64_t* bar, uint32_t count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_at(bar)), "r"(count) : "memory");
+}
+__device__ __forceinline__ void md_bar_expect(uint64_t* bar, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_at(bar)), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void md_bar_arrive(uint64_t* bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_at(bar)) : "memory"); }
+// a row of whole 16-byte vectors into shared memory; the barrier counts its bytes
+__device__ __forceinline__ void md_copy_row(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_at(dst)), "l"(src), "r"(bytes),
+                 "r"(smem_at(bar)) : "memory");
+}
+// bounded: a copy that does not arrive ends the wait, not the kernel; what it leaves is then no number
+__device__ __forceinline__ bool md_bar_wait(uint64_t* bar, uint32_t parity) {
+    for (uint32_t n = 0; n < (1u << 22); ++n) {
+        uint32_t done;
+        asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(done) : "r"(smem_at(bar)), "r"(parity) : "memory");
+        if (done) return true;
+    }
+    return false;
+}
+__device__ __forceinline__ bool finite(float x) { return fabsf(x) <= 3.402823466e38f; }
+
+struct MdLayout {
+    int KU, k_row, v_row;                                   // 16-byte units: padded key row, strides (odd: rows on different banks)
+    size_t vs, qs, qb, ps, pb, total;                       // byte offsets
+};
+__host__ __device__ inline MdLayout md_layout(int R, int Dk, int Dv, int buffers) {
+    constexpr int VT = MD_KEYS;
+    MdLayout l;
+    l.KU = 2 * ((Dk + 15) / 16);
+    l.k_row = l.KU + 1;
+    l.v_row = (Dv / 8) | 1;
+    l.vs = (size_t)buffers * VT * l.k_row * 16;
+    l.qs = l.vs + ((size_t)buffers * VT * l.v_row + 1) * 16;        // one more: the second half of an odd last tile is read
+    l.qb = l.qs + ((size_t)R * Dk * 4 + 15) / 16 * 16;
+    l.ps = l.qb + (size_t)3 * 8 * (l.KU + 1) * 16;
+    l.pb = l.ps + (size_t)8 * VT * 4;
+    l.total = l.pb + (size_t)3 * 8 * (VT + 8) * 2;
+    const size_t combine = (size_t)MD_THREADS * 16;                 // the groups' sums of the combination take the keys' place
+    if (l.vs < combine) l.total += combine;
+    return l;
+}
+
+template <typename YT>
+__global__ void __launch_bounds__(MD_THREADS, 2) attn_decode_mma_kernel(const CcSeqAttn a, int buffers, int NS) {
+    extern __shared__ float4 smd4[];
+    typedef __nv_bfloat16 CT;
+    constexpr int VT = MD_KEYS;
+    uint8_t* const sm = reinterpret_cast<uint8_t*>(smd4);
+    const int R = a.H / a.G, Dk = a.Dk, Dv = a.Dv, kc16 = Dk / 8, vc16 = Dv / 8;
+    const MdLayout lay = md_layout(R, Dk, Dv, buffers);
+    const int KU = lay.KU, k_row = lay.k_row, v_row = lay.v_row, qb_row = 8 * (KU + 1);      // qb_row in elements
+    uint4* const ks = reinterpret_cast<uint4*>(sm);                                 // [buffers][VT][k_row]
+    uint4* const vs = reinterpret_cast<uint4*>(sm + lay.vs);                        // [buffers][VT][v_row]
+    float* const qs = reinterpret_cast<float*>(sm + lay.qs);                        // [R][Dk]
+    CT* const qb = reinterpret_cast<CT*>(sm + lay.qb);                              // [3][8][qb_row] parts of q, zero beyond R and Dk
+    float* const Ps = reinterpret_cast<float*>(sm + lay.ps);                        // [8][VT]
+    CT* const pb = reinterpret_cast<CT*>(sm + lay.pb);                              // [3][8][VT + 8] parts of the weights, zero beyond R
+    __shared__ int s_live[2][VT];
+    __shared__ float s_M[8], s_L[8], s_corr[8], s_inv[8];
+    __shared__ int s_last;
+    __shared__ __align__(8) uint64_t bars[2][2];      // [buffer][keys, values]
+
+    const int sp = blockIdx.x, g = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (tid == 0) {
+        for (int i = 0; i < 4; ++i) md_bar_init(&bars[i >> 1][i & 1], MD_THREADS / 2);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    for (int i = tid; i < 3 * 8 * (VT + 8) / 8; i += MD_THREADS) reinterpret_cast<uint4*>(pb)[i] = make_uint4(0, 0, 0, 0);
+    if (KU > kc16)
+        for (int i = tid; i < buffers * VT; i += MD_THREADS) ks[i * k_row + kc16] = make_uint4(0, 0, 0, 0);
+    if (tid < 8) { s_M[tid] = -INFINITY; s_L[tid] = 0.f; s_corr[tid] = 0.f; s_inv[tid] = 0.f; }
+    pdl_wait_release();
+    const int p = a.input_pos[0];
+    const int j_lo = a.block > 0 ? (p / a.block) * a.block : (a.window > 0 ? max(0, p - a.window + 1) : 0);
+    const int kx = a.window > 0 ? min(a.keep_first, j_lo) : 0;
+    const int n = kx + (p - j_lo + 1);
+    const int n_tiles = (n + VT - 1) / VT, nsplit = min(n_tiles, NS);      // runs of n_tiles / nsplit tiles, or of one more
+    if (sp >= nsplit) return;
+    const int tile0 = (int)((long long)sp * n_tiles / nsplit), tile_end = (int)((long long)(sp + 1) * n_tiles / nsplit);
+    __syncthreads();      // the barriers and the zeros stand
+    // The first half of the CTA asks for keys, the second for values, a thread per row: a whole tile is under way at once, where 16
+    // copies of 16 bytes per thread waited for one another (8 layers of 8 heads x 4096 positions of 128 + 128: 117 us, 109).
+    static_assert(MD_THREADS == 2 * 128 && VT <= 128, "a thread per row");
+    const bool value = tid >= MD_THREADS / 2;
+    const int ht = tid & (MD_THREADS / 2 - 1), D = value ? Dv : Dk, stride = value ? v_row : k_row;
+    const CT* const fresh_row = value ? (const CT*)a.v_new + (size_t)g * Dv : (const CT*)a.k_new + (size_t)g * Dk;
+    const CT* const cached = (value ? (const CT*)a.v_cache : (const CT*)a.k_cache) + (size_t)g * a.L * D;
+    auto fetch = [&](int tile) {
+        const int b = buffers > 1 ? (tile - tile0) & 1 : 0, u0 = tile * VT, rows = min(VT, n - u0);
+        uint64_t* const bar = &bars[b][value];
+        uint4* const dst = (value ? vs : ks) + b * VT * stride;
+        auto position = [&](int row) { return u0 + row < kx ? u0 + row : j_lo + (u0 + row - kx); };
+        auto source = [&](int row) {
+            const int j = position(row);
+            return j == p ? fresh_row : cached + (size_t)slot_of(a, j) * D;
+        };
+        if (ht < rows) {
+            md_bar_expect(bar, (uint32_t)D * 2);
+            md_copy_row(dst + ht * stride, source(ht), (uint32_t)D * 2, bar);
+        } else {
+            md_bar_arrive(bar);
+        }
+        if (ht >= VT) return;
+        if (value) {      // no position: whatever lay there must not meet a weight of zero
+            if (ht >= rows)
+                for (int c = 0; c < vc16; ++c) dst[ht * stride + c] = make_uint4(0, 0, 0, 0);
+        } else {
+            const int j = position(ht);
+            s_live[(tile - tile0) & 1][ht] = ht < rows && (j == p || a.pos[slot_of(a, j)] == j);
+        }
+    };
+    fetch(tile0);
+    for (int i = tid; i < 8 * KU * 8; i += MD_THREADS) {
+        const int r = i / (KU * 8), d = i - r * (KU * 8);
+        float x = 0.f;
+        if (r < R && d < Dk) qs[r * Dk + d] = x = a.q[((size_t)g * R + r) * Dk + d];
+        CT part[3];
+        three_parts(x, part);
+#pragma unroll
+        for (int q = 0; q < 3; ++q) qb[(q * 8 + r) * qb_row + d] = part[q];
+    }
+    const int row_r = lane >> 2, col2 = (lane & 3) * 2;      // of an accumulator
+    float acc[2][2][2];                                      // [pair of column tiles][tile][column]: head row_r
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int t = 0; t < 2; ++t) acc[i][t][0] = acc[i][t][1] = 0.f;
+
+    for (int tile = tile0; tile < tile_end; ++tile) {
+        const int b = buffers > 1 ? (tile - tile0) & 1 : 0, u0 = tile * VT;
+        const int* live = s_live[(tile - tile0) & 1];
+        const uint32_t turn = (buffers > 1 ? (tile - tile0) >> 1 : tile - tile0) & 1;
+        if (buffers > 1 && tile + 1 < tile_end) fetch(tile + 1);
+        bool landed = md_bar_wait(&bars[b][0], turn);
+        __syncthreads();
+        const uint4* const kt = ks + b * VT * k_row;
+        for (int mt = warp; mt < VT / 16; mt += MD_WARPS) {
+            float d[2][4], small[2][4];      // sums of even and odd steps; of the two smaller parts
+#pragma unroll
+            for (int e = 0; e < 4; ++e) d[0][e] = d[1][e] = small[0][e] = small[1][e] = 0.f;
+#pragma unroll 4
+            for (int k = 0; k < KU / 2; ++k) {
+                uint32_t ka[4];
+                ldsm4(ka, kt + (16 * mt + (lane & 15)) * k_row + 2 * k + (lane >> 4));
+                float step[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                for (int q = 2; q >= 0; --q) {
+                    uint32_t bq[2];
+                    ldsm2(bq, qb + (q * 8 + (lane & 7)) * qb_row + 16 * k + ((lane >> 3) & 1) * 8);
+                    mma16816(q > 0 ? small[q - 1] : step, ka[0], ka[1], ka[2], ka[3], bq[0], bq[1]);
+                }
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    if (k & 1) d[1][e] += step[e];
+                    else d[0][e] += step[e];
+                }
+            }
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const int k = 16 * mt + row_r + 8 * (e >> 1), r = col2 + (e & 1), j = u0 + k < kx ? u0 + k : j_lo + (u0 + k - kx);
+                if (r >= R) continue;
+                float s = (d[0][e] + d[1][e]) + (small[0][e] + small[1][e]);
+                if (!finite(s) && live[k]) {
+                    const CT* kr = reinterpret_cast<const CT*>(kt + k * k_row);
+                    s = 0.f;
+                    for (int c = 0; c < Dk; ++c) s = fmaf(qs[r * Dk + c], __bfloat162float(kr[c]), s);
+                }
+                Ps[r * VT + k] = live[k] ? shape_score(a, s * a.scale, g * R + r, p - j) : -INFINITY;
+            }
+        }
+        __syncthreads();
+        if (warp < R) {
+            const int r = warp;
+            float sv[VT / 32], mx = -INFINITY, sum = 0.f;
+#pragma unroll
+            for (int q = 0; q < VT / 32; ++q) mx = fmaxf(mx, sv[q] = Ps[r * VT + lane + 32 * q]);
+            const float m_old = s_M[r], m_new = fmaxf(m_old, warp_max(mx));
+#pragma unroll
+            for (int q = 0; q < VT / 32; ++q) {
+                const float w = sv[q] == -INFINITY ? 0.f : expf(sv[q] - m_new);
+                CT part[3];
+                three_parts(w, part);
+                Ps[r * VT + lane + 32 * q] = w;
+#pragma unroll
+                for (int i = 0; i < 3; ++i) pb[(i * 8 + r) * (VT + 8) + lane + 32 * q] = part[i];
+                sum += w;
+            }
+            sum = warp_sum(sum);
+            if (lane == 0) {
+                const float corr = m_old == -INFINITY ? 0.f : expf(m_old - m_new);
+                s_corr[r] = corr;
+                s_L[r] = s_L[r] * corr + sum;
+                s_M[r] = m_new;
+            }
+        }
+        landed = md_bar_wait(&bars[b][1], turn) && landed;
+        __syncthreads();
+        const uint4* const vt = vs + b * VT * v_row;
+        const float corr = s_corr[row_r];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int np = warp + MD_WARPS * i;
+            if (16 * np >= Dv) break;
+            float d[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}}, odd[2][2] = {{0.f, 0.f}, {0.f, 0.f}}, small[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+#pragma unroll 4
+            for (int k = 0; k < VT / 16; ++k) {
+                uint32_t pa[4], pc[2], vb[4];
+                ldsm4(pa, pb + (((lane >> 3) & 1) * 8 + (lane & 7)) * (VT + 8) + 16 * k + (lane >> 4) * 8);
+                ldsm2(pc, pb + (16 + (lane & 7)) * (VT + 8) + 16 * k + ((lane >> 3) & 1) * 8);
+                ldsm4_t(vb, vt + (16 * k + (lane & 15)) * v_row + 2 * np + (lane >> 4));
+#pragma unroll
+                for (int t = 0; t < 2; ++t) {
+                    float step[4] = {0.f, 0.f, 0.f, 0.f};
+                    mma16816(small[t], pc[0], 0u, pc[1], 0u, vb[2 * t], vb[2 * t + 1]);
+                    mma16816(step, pa[0], pa[1], pa[2], pa[3], vb[2 * t], vb[2 * t + 1]);
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        if (k & 1) odd[t][e] += step[e];
+                        else d[t][e] += step[e];
+                        d[t][2 + e] += step[2 + e];
+                    }
+                }
+            }
+#pragma unroll
+            for (int t = 0; t < 2; ++t)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const int c = 16 * np + 8 * t + col2 + e;
+                    float sum = (d[t][e] + odd[t][e]) + (d[t][2 + e] + small[t][e]);
+                    if (!finite(sum) && row_r < R && c < Dv) {
+                        sum = 0.f;
+                        for (int k = 0; k < VT; ++k)
+                            if (live[k]) sum = fmaf(Ps[row_r * VT + k], __bfloat162float(reinterpret_cast<const CT*>(vt + k * v_row)[c]), sum);
+                    }
+                    if (!landed) sum = NAN;
+                    acc[i][t][e] = tile > tile0 ? fmaf(acc[i][t][e], corr, sum) : sum;
+                }
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // reads before the copies that follow
+        __syncthreads();      // the tile is consumed: its buffers may be filled again
+        if (buffers == 1 && tile + 1 < tile_end) fetch(tile + 1);
+    }
+    int* counters = (int*)a.workspace;
+    float* part_m = (float*)(counters + ((a.G + 3) & ~3));
+    float* part_l = part_m + (size_t)a.G * NS * R;
+    float* part_o = (float*)(((uintptr_t)(part_l + (size_t)a.G * NS * R) + 15) & ~(uintptr_t)15);
+    YT* y = (YT*)a.y + (size_t)g * R * Dv;
+    auto sink_of = [&](int r) { return a.sink_mode == CC_SINK_LEARNED ? a.sink[g * R + r] : a.sink_mode == CC_SINK_ZERO ? 0.f : -INFINITY; };
+    // this thread's values: f(head, column, value, value of the next column)
+    auto each_pair = [&](auto&& f) {
+        if (row_r >= R) return;
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int t = 0; t < 2; ++t) {
+                const int c = 16 * (warp + MD_WARPS * i) + 8 * t + col2;
+                if (c < Dv) f(row_r, c, acc[i][t][0], acc[i][t][1]);
+            }
+    };
+    if (nsplit == 1) {
+        if (tid < R) {
+            const float sk = sink_of(tid), M = fmaxf(s_M[tid], sk);
+            const float w = s_M[tid] == -INFINITY ? 0.f : expf(s_M[tid] - M);
+            const float L = s_L[tid] * w + (a.sink_mode != CC_SINK_NONE ? expf(sk - M) : 0.f);
+            s_inv[tid] = L > 0.f ? w / L : 0.f;
+        }
+        __syncthreads();
+        each_pair([&](int r, int c, float v0, float v1) {
+            stf(y, (size_t)r * Dv + c, v0 * s_inv[r]);
+            stf(y, (size_t)r * Dv + c + 1, v1 * s_inv[r]);
+        });
+        if (a.append) append_row<CT>(a, g, 0, p, tid, MD_THREADS);
+        return;
+    }
+    const size_t pbase = ((size_t)g * NS + sp) * R;
+    each_pair([&](int r, int c, float v0, float v1) { *reinterpret_cast<float2*>(part_o + (pbase + r) * Dv + c) = make_float2(v0, v1); });
+    if (tid < R) { part_m[pbase + tid] = s_M[tid]; part_l[pbase + tid] = s_L[tid]; }
+    __syncthreads();
+    if (tid == 0) {      // releases what the whole CTA stored before the barrier, and acquires what the others did
+        int before;
+        asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], 1;" : "=r"(before) : "l"(counters + g) : "memory");
+        s_last = before == nsplit - 1;
+    }
+    __syncthreads();
+    if (!s_last) return;
+    // the last CTA of the head: every other one has finished reading
+    static_assert(VD_MAX_SPLITS <= VT, "the weights of the splits take the place of a tile's");
+    float* const wgt = Ps;     // [R][VT]
+    const float4* po = reinterpret_cast<const float4*>(part_o + (size_t)g * NS * R * Dv);     // Dv is a multiple of 8
+    const int quads = R * Dv / 4, groups = quads >= MD_THREADS ? 1 : min(8, MD_THREADS / quads);
+    const int grp = groups > 1 ? tid / quads : 0, first = groups > 1 ? tid - grp * quads : tid;
+    // asked for together: maxima and sums, the new row and its slot, the first partial sums
+    const int hr = min(warp, R - 1);
+    const float* pm = part_m + (size_t)g * NS * R + hr;
+    const float* pl = part_l + (size_t)g * NS * R + hr;
+    const float m0 = lane < nsplit ? __ldcg(pm + (size_t)lane * R) : -INFINITY, m1 = lane + 32 < nsplit ? __ldcg(pm + (size_t)(lane + 32) * R) : -INFINITY;
+    const float l0 = lane < nsplit ? __ldcg(pl + (size_t)lane * R) : 0.f, l1 = lane + 32 < nsplit ? __ldcg(pl + (size_t)(lane + 32) * R) : 0.f;
+    const int at = slot_of(a, p);
+    const bool stores = a.append && tid < kc16 + vc16, key = tid < kc16;
+    uint4 fresh = make_uint4(0, 0, 0, 0);
+    int old = 0;
+    if (stores) fresh = key ? reinterpret_cast<const uint4*>((const CT*)a.k_new + (size_t)g * Dk)[tid] : reinterpret_cast<const uint4*>((const CT*)a.v_new + (size_t)g * Dv)[tid - kc16];
+    if (a.append && tid == 0 && g == 0) old = a.pos[at];
+    float4 v[MD_AHEAD];
+#pragma unroll
+    for (int u = 0; u < MD_AHEAD; ++u)
+        if (grp < groups && first < quads && grp + u * groups < nsplit) v[u] = __ldcg(po + (size_t)(grp + u * groups) * quads + first);
+    if (warp < R) {
+        const float sk = sink_of(hr), M = fmaxf(sk, warp_max(fmaxf(m0, m1)));
+        const float w0 = m0 == -INFINITY ? 0.f : expf(m0 - M), w1 = m1 == -INFINITY ? 0.f : expf(m1 - M);
+        wgt[hr * VT + lane] = w0;
+        wgt[hr * VT + lane + 32] = w1;
+        float L = warp_sum(l0 * w0 + l1 * w1);
+        if (a.sink_mode != CC_SINK_NONE) L += expf(sk - M);
+        if (lane == 0) s_inv[hr] = L > 0.f ? 1.0f / L : 0.f;
+    }
+    if (stores) {      // every CTA of the head has read its rows, and none of another head reads these
+        if (key) reinterpret_cast<uint4*>((CT*)a.k_cache + ((size_t)g * a.L + at) * Dk)[tid] = fresh;
+        else reinterpret_cast<uint4*>((CT*)a.v_cache + ((size_t)g * a.L + at) * Dv)[tid - kc16] = fresh;
+        if (tid == 0) {
+            if (a.mask != nullptr) a.mask[(size_t)g * a.L + at] = 1;
+            if (g == 0) {
+                a.pos[at] = p;
+                if (old < 0 && a.cache_cts != nullptr) atomicAdd(a.cache_cts, 1);
+            }
+        }
+    }
+    if (tid == 0) counters[g] = 0;
+    __syncthreads();
+    // splits of a group in order, then the groups in order
+    float4* const met = reinterpret_cast<float4*>(sm);      // [groups][quads], over the keys
+    for (int i = first; i < quads && grp < groups; i += MD_THREADS) {
+        const float* w = wgt + (i / (Dv / 4)) * VT;
+        float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
+        auto add = [&](int s, const float4& x) {
+            t.x = fmaf(w[s], x.x, t.x);
+            t.y = fmaf(w[s], x.y, t.y);
+            t.z = fmaf(w[s], x.z, t.z);
+            t.w = fmaf(w[s], x.w, t.w);
+        };
+        if (i == first) {
+#pragma unroll
+            for (int u = 0; u < MD_AHEAD; ++u)
+                if (grp + u * groups < nsplit) add(grp + u * groups, v[u]);
+        }
+#pragma unroll 16
+        for (int s = grp + (i == first ? MD_AHEAD * groups : 0); s < nsplit; s += groups) add(s, __ldcg(po + (size_t)s * quads + i));
+        if (groups == 1) {
+            const float inv = s_inv[i / (Dv / 4)];
+            stf(y, 4 * i + 0, t.x * inv);
+            stf(y, 4 * i + 1, t.y * inv);
+            stf(y, 4 * i + 2, t.z * inv);
+            stf(y, 4 * i + 3, t.w * inv);
+        } else {
+            met[grp * quads + i] = t;
+        }
+    }
+    if (groups == 1) return;
+    __syncthreads();
+    if (tid < quads) {
+        float4 t = met[tid];
+        for (int q = 1; q < groups; ++q) {
+            const float4 x = met[q * quads + tid];
+            t.x += x.x; t.y += x.y; t.z += x.z; t.w += x.w;
+        }
+        const float inv = s_inv[tid / (Dv / 4)];
+        stf(y, 4 * tid + 0, t.x * inv);
+        stf(y, 4 * tid + 1, t.y * inv);
+        stf(y, 4 * tid + 2, t.z * inv);
+        stf(y, 4 * tid + 3, t.w * inv);
+    }
+}
+
 template <typename CT>
 __global__ void cache_append_kernel(const CcSeqAttn a, int t_first) {
     const int t = t_first + blockIdx.x, g = blockIdx.y;
@@ -1314,10 +1726,40 @@ static int launch_decode_rows(const CcSeqAttn* a, cudaStream_t st) {
     return cuda_check("attn_decode_rows_kernel");
 }
 
+// One query head per key head leaves seven of an MMA's eight columns empty: where narrow rows make the tiles' work count (more than a
+// tile per CTA), the kernel above is ahead.  16 heads of 64 + 64, us a layer, this kernel and that one: 300 positions 10.6 / 10.5,
+// 1000 10.8 / 12.3, 4096 17.2 / 16.9, 8000 26.6 / 25.5, 12000 35.8 / 33.9; of 96 + 128 13.5 / 13.8 at 2000, 31.2 / 32.2 at 8000.
+static bool decode_mma_serves(const CcSeqAttn* a) {
+    const long long tiles = vd_tiles(a->L, attn_reach(*a), MD_KEYS);
+    return a->H > a->G || a->Dk > 64 || a->Dv > 64 || tiles <= vd_splits(tiles, a->G, 2);
+}
+template <typename YT>
+static int launch_decode_mma(const CcSeqAttn* a, cudaStream_t st) {
+    const int reach = attn_reach(*a), R = a->H / a->G;
+    auto bytes = [&](int buffers) { return md_layout(R, a->Dk, a->Dv, buffers).total; };
+    const size_t half = 111 * 1024, all = 223 * 1024;
+    // Two CTAs per SM where a tile fits half of the shared memory, one otherwise (rows of 256 + 256 fit it whole).  8 / 2 heads of
+    // 256, 300 / 2000 / 4096 / 8000 positions, us a layer: two CTAs with tiles of 64 keys 12.0 / 16.3 / 27.2 / 29.3, one of 128
+    // 13.0 / 13.4 / 17.9 / 25.2.
+    const int per_sm = bytes(1) <= half ? 2 : 1;
+    const long long tiles = vd_tiles(a->L, reach, MD_KEYS);
+    const int NS = vd_splits(tiles, a->G, per_sm), buffers = tiles > NS && bytes(2) <= (per_sm == 2 ? half : all) ? 2 : 1;
+    const size_t smem = bytes(buffers);
+    auto kern = attn_decode_mma_kernel<YT>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return fail(CC_SEQ_ERR_CUDA, cudaGetErrorString(e));
+    launch_under(kern, dim3(NS, a->G), dim3(MD_THREADS), smem, st, *a, buffers, NS);
+    return cuda_check("attn_decode_mma_kernel");
+}
+
 template <typename CT, typename YT>
 static int launch_decode(const CcSeqAttn* a, cudaStream_t st) {
     const int R = a->H / a->G;
     if (decode_rows_serves(a)) {
+        if constexpr (sizeof(CT) == 2) {
+            if (decode_mma_serves(a)) return launch_decode_mma<YT>(a, st);
+            return launch_decode_rows<CT, YT, 1>(a, st);
+        }
         if (R <= 1) return launch_decode_rows<CT, YT, 1>(a, st);
         if (R <= 2) return launch_decode_rows<CT, YT, 2>(a, st);
         if (R <= 4) return launch_decode_rows<CT, YT, 4>(a, st);
