@@ -22,7 +22,7 @@
 //     when the launch may read them (asked for before griddepcontrol.wait), all loads of the first phases are requested
 //     together, warps reduce with the warp reduction instruction instead of butterflies, every softmax warp owns one query
 //     head and sends its own sums, and the P.V phase adds nothing up across lanes.  32 steps in a graph, us a step, before and
-//     with all of it: 64 sliding slots 8.2 and 5.7, 1024 heavy-hitter slots 10.9 and 8.1, 512 l2 slots 15.2 and 8.5;
+//     with all of it: 64 sliding slots 8.2 and 5.4, 1024 heavy-hitter slots 10.9 and 7.8, 512 l2 slots 15.2 and 8.2;
 //   * arithmetic order is the bit-reproducible definition in common.cuh (canonical dot tree,
 //     det_expf, 2^-40 fixed-point sum), so eviction indices do not depend on C, CH or the
 //     thread count.
@@ -248,10 +248,14 @@ cc_decode_kernel(const __grid_constant__ DecodeParams p) {
     const int live_rows = nlc_live << chs;
 
     // ---- 0. barriers + as many K/V chunks in flight as the ring holds
+    // (The keys of a CTA with one short chunk go straight to registers below: they are there when the candidate is, half a
+    // microsecond before a bulk copy of the same rows.  32 steps in a graph: 64 sliding slots 185 -> 174 us, 1024 heavy-hitter slots 260 -> 251.)
+    constexpr int UR = G >= 7 ? 2 : 4;     // row pairs of a warp per pass (registers: two CTAs per SM, so that the next launch fits beside this one)
+    const bool direct = !ahead && nlc_live == 1 && CH <= UR * kWarps * RPW;
     if (tid == 0) {
         fence_proxy_async();
         const int pre = min(NS, nlc_live);
-        for (int j = 0; j < pre; ++j) {
+        for (int j = 0; j < pre && !direct; ++j) {
             const uint32_t bytes = chunk_rows_valid(j) * kRowBytes;
             mbar_expect_tx(&kbar[j], bytes);
             tma_load_1d(kring + j * chunk_bytes, chunk_at(kc, j), bytes, &kbar[j]);
@@ -297,6 +301,14 @@ cc_decode_kernel(const __grid_constant__ DecodeParams p) {
         if (hh_sum) {
             hist0 = hist[s0];
             den0 = den[s0];
+        }
+    }
+    uint4 kdir[UR];      // this lane's parts of the warp's key rows
+    if (direct) {
+#pragma unroll
+        for (int u = 0; u < UR; ++u) {
+            const int r = (warp + u * kWarps) * RPW + sub;
+            kdir[u] = r < chunk_rows_valid(0) ? *reinterpret_cast<const uint4*>(chunk_at(kc, 0) + (size_t)r * D + li * 8) : make_uint4(0, 0, 0, 0);
         }
     }
     if (!ahead) load_new();
@@ -489,15 +501,27 @@ cc_decode_kernel(const __grid_constant__ DecodeParams p) {
             for (int g = 0; g < G; ++g) lg[g * stride + lr] = -CUDART_INF_F;
         if (!do_evict) __syncthreads();  // maskb visible
         float m = -CUDART_INF_F;         // of this lane's head over its rows, without the candidate's
+        auto row_logits = [&](const uint4& row, int lr) {
+            float v = dots(row, &gsel);
+            if (!maskb[lr]) v = -CUDART_INF_F;      // rows beyond the cache are masked too
+            if (gsel < G) lg[gsel * stride + lr] = v;
+            if (lr != cand_local) m = fmaxf(m, v);
+        };
+        if (direct) {
+#pragma unroll
+            for (int u = 0; u < UR; ++u) {
+                const int r0 = (warp + u * kWarps) * RPW;
+                if (r0 < CH) row_logits(kdir[u], r0 + sub);
+            }
+        }
         // chunks that are all in the ring are walked as one run of rows
         const int per = nlc_live <= NS ? nlc_live : 1;
-        for (int j = 0; j < nlc_live; j += per) {
+        for (int j = 0; j < nlc_live && !direct; j += per) {
             const int stage = j % NS, run = per << chs;
             for (int i = 0; i < per; ++i) mbar_wait(&kbar[stage + i], (j / NS) & 1);
             if (j == 0) stamp(p, 3);
             const uint8_t* kbase = kring + stage * chunk_bytes;
             // up to UR row pairs per warp per pass, all fetched before the dependent math (ILP)
-            constexpr int UR = G >= 7 ? 2 : 4;     // (registers: two CTAs per SM, so that the next launch fits beside this one)
 #pragma unroll 1
             for (int r0 = warp * RPW; r0 < run; r0 += UR * kWarps * RPW) {
                 uint4 kv[UR];
@@ -510,10 +534,7 @@ cc_decode_kernel(const __grid_constant__ DecodeParams p) {
                 for (int u = 0; u < UR; ++u) {
                     const int r = r0 + u * kWarps * RPW + sub, lr = (j << chs) + r;
                     if (u > 0 && r0 + u * kWarps * RPW >= run) break;
-                    float v = dots(kv[u], &gsel);
-                    if (!maskb[lr]) v = -CUDART_INF_F;      // rows beyond the cache are masked too
-                    if (gsel < G) lg[gsel * stride + lr] = v;
-                    if (lr != cand_local) m = fmaxf(m, v);
+                    row_logits(kv[u], lr);
                 }
             }
             if (j + NS < nlc_live) {  // ring slot is refilled: everyone must be done with it
