@@ -71,7 +71,8 @@ enum : int {
     kMiscWarpKey = 8,   // [kWarps] u64
     kMiscWarpMax = 24,  // [kWarps] largest key norm
     kMiscRowMax = 32,   // [kWarps][kMaxG] largest logit of a warp's rows, without the candidate's
-    kMiscWords = 96,
+    kMiscCandLg = 96,   // [kMaxG] logits of the candidate: a copy, the softmax overwrites the row's own while others still read
+    kMiscWords = 104,
 };
 
 __host__ __device__ inline uint32_t align_up(uint32_t x, uint32_t a) { return (x + a - 1) / a * a; }
@@ -437,6 +438,7 @@ cc_decode_kernel(const __grid_constant__ DecodeParams p) {
         }
         ckey = warp_min_u64(ckey);
         if (lane == 0) reinterpret_cast<unsigned long long*>(miscu + kMiscWarpKey)[warp] = ckey;
+        if (tid < kMaxG) misc[kMiscCandLg + tid] = -CUDART_INF_F;
         __syncthreads();
         ckey = lane < kWarps ? reinterpret_cast<unsigned long long*>(miscu + kMiscWarpKey)[lane] : kNoKey;
         ckey = warp_min_u64(ckey);
@@ -506,6 +508,7 @@ cc_decode_kernel(const __grid_constant__ DecodeParams p) {
             if (!maskb[lr]) v = -CUDART_INF_F;      // rows beyond the cache are masked too
             if (gsel < G) lg[gsel * stride + lr] = v;
             if (lr != cand_local) m = fmaxf(m, v);
+            else if (gsel < G) misc[kMiscCandLg + gsel] = v;      // replicated lanes write the same value
         };
         if (direct) {
 #pragma unroll
@@ -569,7 +572,7 @@ cc_decode_kernel(const __grid_constant__ DecodeParams p) {
                     for (int k = 1; k < kWarps; ++k) m = fmaxf(m, misc[kMiscRowMax + k * kMaxG + w - 2]);
                     word = __float_as_uint(m);
                 } else if (cand_local >= 0) {
-                    word = __float_as_uint(lg[(w - 2 - G) * stride + cand_local]);
+                    word = __float_as_uint(misc[kMiscCandLg + w - 2 - G]);
                 }
             }
             st_async_u32(map_to_rank(smem_u32(&rec[rank * kRecWords + w]), dest), word, map_to_rank(smem_u32(&xbar[1]), dest));
