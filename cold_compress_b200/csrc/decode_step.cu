@@ -605,7 +605,7 @@ cc_decode_kernel(const __grid_constant__ DecodeParams p) {
         const bool cand_stays = lane_has_cand && (lane != owner || !has_new);
         if (solo) {
             if (lane < kWarps) m = misc[kMiscRowMax + lane * kMaxG + wg];
-            if (cand_stays) m = fmaxf(m, lg[wg * stride + cand_local]);
+            if (cand_stays) m = fmaxf(m, misc[kMiscCandLg + wg]);
         } else if (lane < C) {
             m = __uint_as_float(rec[lane * kRecWords + 2 + wg]);
             if (cand_stays) m = fmaxf(m, __uint_as_float(rec[lane * kRecWords + 2 + G + wg]));

@@ -15,3 +15,9 @@ def test_the_exchange_of_candidates_sends_no_logit_from_the_rows():
     sending this CTA's record to its peers then, so what they send must lie where the softmax does not write."""
     sent = _between("__syncthreads();  // logits and row maxima visible", "mbar_wait(&xbar[1], 0);")
     assert "st_async_u32(" in sent and not re.search(r"\blg(w)?\s*\[", sent)
+
+
+def test_the_maximum_of_one_cta_takes_no_logit_from_the_rows():
+    """The same where one CTA holds a head: the warps of a query head find its maximum one by one, and the first may be storing."""
+    found = _between("mbar_wait(&xbar[1], 0);", "float* lgw = lg + wg * stride;")
+    assert "gm = fmaxf(" in found and not re.search(r"\blg\s*\[", found)
