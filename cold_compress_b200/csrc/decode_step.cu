@@ -402,13 +402,13 @@ cc_decode_kernel(const __grid_constant__ DecodeParams p) {
             }
         } else if constexpr (hybrid) {
             if (hyb_mode == kHybEvict) {
-                // cache.py:844-894 over the live prefix [0, cts): mean ring attention (or position for
+                // cache.py:844-894 over the live prefix [0, min(cts, L)): mean ring attention (or position for
                 // window-only heads); first g slots, special, punctuation and the recent window are saved
                 const int W = st.history_window;
                 const double* hsum = st.attn_history_sum + (size_t)h * L;
                 for (int lr = tid; lr < local_rows; lr += kThreads) {
                     const int s = slot_of(lr);
-                    if (s >= hyb_cts) continue;
+                    if (s >= live_limit) continue;      // a head that only appends counts on beyond its last slot
                     const int ps = posp[s];
                     float sc;
                     if (hyb_bits & CC_HYB_HEAVY_HITTER) {

@@ -224,7 +224,7 @@ static int64_t hybrid_select(const CcCacheState* st, int h, int32_t input_pos, i
     float best = 0;
     int64_t bi = -1;
     int best_nan = 0;
-    for (int s = 0; s < cts; ++s) {
+    for (int s = 0; s < cts && s < L; ++s) { /* the count of a head that appends goes on beyond L */
         float sc;
         if (bits & CC_HYB_HEAVY_HITTER) {
             int32_t d = den[s] > W ? W : den[s];
