@@ -218,6 +218,7 @@ cc_decode_kernel(const __grid_constant__ DecodeParams p) {
     int hyb_mode = kHybAppend, hyb_bits = 0, hyb_cts = 0, hyb_rw = 0;
     int64_t hyb_counter = 0;
     int live_limit = L;  // slots >= live_limit cannot be live: their chunks are never loaded
+    bool last_live = false;
     const bool is_punc = hybrid && (p.a.is_punc_dev ? p.a.is_punc_dev[0] != 0 : p.a.is_punc != 0);
     if constexpr (hybrid) {
         hyb_bits = st.hyb_strategy_bits[h];
@@ -238,6 +239,7 @@ cc_decode_kernel(const __grid_constant__ DecodeParams p) {
             }
         }
         live_limit = min(L, hyb_cts + ((do_evict && hyb_mode == kHybAppend) ? 1 : 0));
+        last_live = live_limit == L && st.mask[(size_t)h * L + L - 1] != 0;
     }
     int32_t hh_cts = 0;   // cache_cts before this step (thresholded history compares against 1 / cache_cts)
     if (hh_ring) {
@@ -470,8 +472,8 @@ cc_decode_kernel(const __grid_constant__ DecodeParams p) {
         const int s = (int)(uint32_t)(ckey & 0xffffffffu);
         cand_local = (((s >> chs) >> csh) << chs) + (s & (CH - 1));
     }
-    // a dropped token does not take part in attention (its slot's mask stays as it was)
-    const bool attend_new = do_evict && !(hybrid && hyb_mode == kHybDrop);
+    // a dropped token is stored in the last slot, whose mask stays as it was: it takes part in attention only if that slot was live
+    const bool attend_new = do_evict && !(hybrid && hyb_mode == kHybDrop && !last_live);
 
     // ---- 3. logits over the K ring (canonical dot tree), new-token logits by the last warp while the rows arrive
     if (do_attend) {

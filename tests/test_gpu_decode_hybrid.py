@@ -54,6 +54,17 @@ def _steps(cache, oc, Hkv, G, D, nxt, gen, punc, steps):
             assert torch.equal(a.cpu().reshape(b.shape).to(b.dtype), b), f"final {n} differs"
 
 
+SHAPES = [(80, 2, 64, 100, 100), (80, 4, 64, 100, 70), (76, 1, 128, 47, 47), (8, 4, 128, 300, 300), (8, 4, 128, 300, 200), (3, 7, 64, 130, 130),
+          (8, 8, 128, 1024, 1000), (6, 2, 128, 600, 600)]
+
+
+@pytest.mark.parametrize("Hkv,G,D,L,filled", SHAPES)
+@pytest.mark.parametrize("heavy", [True, False])
+def test_heads_that_append_evict_and_drop(Hkv, G, D, L, filled, heavy):
+    cache, oc, nxt, gen = _cache(Hkv, G, D, L, filled, heavy)
+    _steps(cache, oc, Hkv, G, D, nxt, gen, lambda t: t % 5 == 4, 12)
+
+
 @pytest.mark.parametrize("Hkv,G,D,L", [(76, 1, 128, 47), (8, 4, 128, 300), (4, 7, 64, 64), (8, 2, 128, 1024)])
 def test_counts_that_go_on_beyond_the_last_slot(Hkv, G, D, L):
     """A head that appends counts on when its cache is full (a punctuation token takes the last slot again); when it next evicts, it
