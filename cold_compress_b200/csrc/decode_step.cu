@@ -657,24 +657,28 @@ cc_decode_kernel(const __grid_constant__ DecodeParams p) {
         stamp(p, 9);
 
         // ---- 10. y = P.V over the V ring, cluster-wide reduction = X3
-        // A warp has CH / 8 neighbouring rows of a chunk and all their columns, CPL a lane: nothing to add up across lanes.
-        float acc[G][CPL];
+        // A warp has RPW neighbouring rows out of every kWarps * RPW and all their columns, CPL a lane: nothing to add up across
+        // lanes.  Each of the RPW rows has sums of its own, which meet at the end: the order of the additions is part of the result
+        // (a bf16 rounding of y), so it stays what it is however rows are dealt to lanes.  (One sum per column for all rows of a
+        // warp is no faster: 32 steps in a graph, 64 sliding slots 189.3 and 189.4 us, 1024 heavy-hitter slots 257.0 and 256.9, L2 flushed.)
+        float acc[RPW][G][CPL];
 #pragma unroll
-        for (int g = 0; g < G; ++g)
+        for (int x = 0; x < RPW; ++x)
 #pragma unroll
-            for (int i = 0; i < CPL; ++i) acc[g][i] = 0.f;
-        const int rw = CH / kWarps;
+            for (int g = 0; g < G; ++g)
+#pragma unroll
+                for (int i = 0; i < CPL; ++i) acc[x][g][i] = 0.f;
         for (int j = 0; j < nlc_live; ++j) {
             const int stage = j % NS;
             mbar_wait(&vbar[stage], (j / NS) & 1);
-            const int r_end = min(chunk_rows_valid(j), (warp + 1) * rw);
+            const int r_end = chunk_rows_valid(j);
             const uint8_t* vbase = vring + stage * chunk_bytes + lane * (CPL * 2);
-#pragma unroll 2
-            for (int r = warp * rw; r < r_end; r += 2) {
+#pragma unroll (G >= 7 ? 1 : 2)
+            for (int r = warp * RPW; r < r_end; r += kWarps * RPW) {
                 const int lr = (j << chs) + r;
-                uint32_t vv[2][CPL / 2];
+                uint32_t vv[RPW][CPL / 2];
 #pragma unroll
-                for (int x = 0; x < 2; ++x) {
+                for (int x = 0; x < RPW; ++x) {
                     if constexpr (CPL == 4) {
                         const uint2 u = *reinterpret_cast<const uint2*>(vbase + (r + x) * kRowBytes);
                         vv[x][0] = u.x;
@@ -690,13 +694,19 @@ cc_decode_kernel(const __grid_constant__ DecodeParams p) {
                 }
 #pragma unroll
                 for (int g = 0; g < G; ++g) {
-                    const float2 pr = *reinterpret_cast<const float2*>(lg + g * stride + lr);
-#pragma unroll
-                    for (int i = 0; i < CPL; ++i) {
-                        const float v0 = __uint_as_float(i & 1 ? vv[0][i / 2] & 0xffff0000u : vv[0][i / 2] << 16);
-                        const float v1 = __uint_as_float(i & 1 ? vv[1][i / 2] & 0xffff0000u : vv[1][i / 2] << 16);
-                        acc[g][i] = fmaf(pr.y, v1, fmaf(pr.x, v0, acc[g][i]));
+                    float pr[RPW];
+                    if constexpr (RPW == 4) {
+                        const float4 t = *reinterpret_cast<const float4*>(lg + g * stride + lr);
+                        pr[0] = t.x; pr[1] = t.y; pr[2] = t.z; pr[3] = t.w;
+                    } else {
+                        const float2 t = *reinterpret_cast<const float2*>(lg + g * stride + lr);
+                        pr[0] = t.x; pr[1] = t.y;
                     }
+#pragma unroll
+                    for (int x = 0; x < RPW; ++x)
+#pragma unroll
+                        for (int i = 0; i < CPL; ++i)
+                            acc[x][g][i] = fmaf(pr[x], __uint_as_float(i & 1 ? vv[x][i / 2] & 0xffff0000u : vv[x][i / 2] << 16), acc[x][g][i]);
                 }
             }
             if (j + NS < nlc_live) {  // ring slot is refilled: everyone must be done with it
@@ -714,8 +724,14 @@ cc_decode_kernel(const __grid_constant__ DecodeParams p) {
 #pragma unroll
         for (int g = 0; g < G; ++g) {
             float* dst = &red[warp * G * D + g * D + lane * CPL];
-            if constexpr (CPL == 4) *reinterpret_cast<float4*>(dst) = make_float4(acc[g][0], acc[g][1], acc[g][2], acc[g][3]);
-            else *reinterpret_cast<float2*>(dst) = make_float2(acc[g][0], acc[g][1]);
+            float sum[CPL];
+#pragma unroll
+            for (int i = 0; i < CPL; ++i) {
+                if constexpr (RPW == 4) sum[i] = (acc[0][g][i] + acc[2][g][i]) + (acc[1][g][i] + acc[3][g][i]);
+                else sum[i] = acc[0][g][i] + acc[1][g][i];
+            }
+            if constexpr (CPL == 4) *reinterpret_cast<float4*>(dst) = make_float4(sum[0], sum[1], sum[2], sum[3]);
+            else *reinterpret_cast<float2*>(dst) = make_float2(sum[0], sum[1]);
         }
         __syncthreads();
         const int SL = (G * D) >> csh;  // outputs reduced by each CTA of the cluster (a multiple of 4)
