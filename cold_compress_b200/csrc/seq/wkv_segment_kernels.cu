@@ -6,6 +6,8 @@
 //      at a time.  No decay is ever divided by: every factor is a product of numbers in (0, 1];
 //   2. the states at the segments' starts, one after another over the segments and beside each other over the elements;
 //   3. the recurrence inside every segment from its own start.
+// Where a start or a sum is not finite, 2. goes token after token (a product of decays may underflow where no decay is zero) and 3. walks
+// its segment again with the bonus per row, so that infinities and NaN come out as they do token after token (the checks: 1 %).
 // One multiplication and addition per state element and token more than the plain recurrence, for segments times the parallelism:
 // 4096 tokens of 32 heads of 64 go from 405 us to 152 (60 + 7 + 96), of 4 heads from 387 to 37, of 64 heads of 128 from 1663 to 1190.
 // Now bound by the fp32 pipe (63 % busy in 3., 42 % in 1.; 9 warps of 168 registers an SM).  Against 64 bits the outputs are as
@@ -171,6 +173,20 @@ __global__ void __launch_bounds__(STATE_THREADS, 8) wkv_segment_state_kernel(con
     }
 }
 
+// The states at the segments' starts for four elements, through the tokens one after another.
+__device__ __forceinline__ void again_one_by_one(const CcSeqWkv& a, const Segments& g, size_t e, size_t n4, size_t hi, float4 x) {
+    const size_t HD = (size_t)a.H * a.D, col = hi / a.D * a.D + e * 4 % a.D;
+    const int last = (g.n - 1) * g.len;
+#pragma unroll 4
+    for (int t = 0; t < last; ++t) {
+        const size_t row = (size_t)t * HD;
+        const float w = g.w[row + hi], k = a.k[row + hi];
+        const float* v = a.v + row + col;
+        x = make_float4(fmaf(w, x.x, k * v[0]), fmaf(w, x.y, k * v[1]), fmaf(w, x.z, k * v[2]), fmaf(w, x.w, k * v[3]));
+        if ((t + 1) % g.len == 0) reinterpret_cast<float4*>(g.X)[(size_t)((t + 1) / g.len) * n4 + e] = x;
+    }
+}
+
 // State at every segment's start, thread = four elements of a state row; the loads of sixteen segments are under way together.
 __global__ void __launch_bounds__(128) wkv_segment_starts_kernel(const CcSeqWkv a, const Segments g) {
     const size_t n4 = (size_t)a.H * a.D * a.D / 4, e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -195,6 +211,8 @@ __global__ void __launch_bounds__(128) wkv_segment_starts_kernel(const CcSeqWkv 
                 X[(size_t)(s0 + q + 1) * n4 + e] = x;
             }
     }
+    // what is not finite stays so: all of it again, token after token
+    if (!(fabsf(x.x) + fabsf(x.y) + fabsf(x.z) + fabsf(x.w) < INFINITY)) again_one_by_one(a, g, e, n4, hi, reinterpret_cast<const float4*>(a.state)[e]);
 }
 
 // The recurrence inside a segment, 64 columns of a head.  Thread = 16 rows x 4 columns: lane % P holds rows 4 P q + 4 p .. + 3 of
@@ -253,6 +271,7 @@ __global__ void __launch_bounds__(Dp, Dp == 64 ? 6 : 3) wkv_segment_scan_kernel(
     const bool up2 = p & 2, up1 = p & 1;
     float* out = a.o + (size_t)first * HD + (size_t)h * a.D + j + (up2 ? 2 : 0) + (up1 ? 1 : 0);
     const bool writes = p < 4 && j < a.D;
+    float none = 0.f;      // NaN from the first sum on that is not finite
     int cur = 0;
     for (int t0 = 0; t0 < count; t0 += TB, cur ^= 1) {
         const float* const buf = sm + cur * BUF;
@@ -299,8 +318,40 @@ __global__ void __launch_bounds__(Dp, Dp == 64 ? 6 : 3) wkv_segment_scan_kernel(
             a0 = (up1 ? a1 : a0) + __shfl_xor_sync(0xffffffffu, up1 ? a0 : a1, 1);
             if (P == 8) a0 += __shfl_xor_sync(0xffffffffu, a0, 4);
             if (writes) *out = a0;
+            none = fmaf(0.f, a0, none);
         }
         __syncthreads();
+    }
+    const size_t at = (size_t)first * HD + (size_t)h * a.D;
+    const bool again = __syncthreads_or(none != none);
+    if (again) {
+        // the segment again from memory, with the bonus per row; the state stands in X, where nobody else reads this tile
+        float* const mine = g.X + ((size_t)s * a.H + h) * a.D * a.D + j;
+#pragma unroll 1
+        for (int t = 0; t < count; ++t) {
+            const size_t row = at + (size_t)t * HD;
+            float sum[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+            for (int r = 0; r < 16; ++r) {
+                const int i = 4 * P * (r / 4) + 4 * p + r % 4;
+                if (i >= a.D || j >= a.D) continue;
+                const float rv = a.r[row + i], k = a.k[row + i], w = g.w[row + i], u = a.u[(size_t)h * a.D + i];
+                float4* const x4 = reinterpret_cast<float4*>(mine + (size_t)i * a.D);
+                const float4 x = *x4;
+                const float kv[4] = {k * a.v[row + j], k * a.v[row + j + 1], k * a.v[row + j + 2], k * a.v[row + j + 3]};
+                sum[0] = fmaf(rv, fmaf(u, kv[0], x.x), sum[0]);
+                sum[1] = fmaf(rv, fmaf(u, kv[1], x.y), sum[1]);
+                sum[2] = fmaf(rv, fmaf(u, kv[2], x.z), sum[2]);
+                sum[3] = fmaf(rv, fmaf(u, kv[3], x.w), sum[3]);
+                *x4 = make_float4(fmaf(w, x.x, kv[0]), fmaf(w, x.y, kv[1]), fmaf(w, x.z, kv[2]), fmaf(w, x.w, kv[3]));
+            }
+#pragma unroll
+            for (int x = 0; x < 4; ++x) {
+#pragma unroll
+                for (int d = 1; d < P; d <<= 1) sum[x] += __shfl_xor_sync(0xffffffffu, sum[x], d);
+                if (p == x && j < a.D) a.o[row + j + x] = sum[x];
+            }
+        }
     }
     if (s + 1 < g.n) return;
     float* const S = a.state + (size_t)h * a.D * a.D;
