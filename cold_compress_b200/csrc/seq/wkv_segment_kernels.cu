@@ -8,6 +8,7 @@
 //   3. the recurrence inside every segment from its own start.
 // Where a start or a sum is not finite, 2. goes token after token (a product of decays may underflow where no decay is zero) and 3. walks
 // its segment again with the bonus per row, so that infinities and NaN come out as they do token after token (the checks: 1 %).
+// Rows on other than 16-byte boundaries are staged 4 bytes at a time: the same sums, so the same bits.
 // One multiplication and addition per state element and token more than the plain recurrence, for segments times the parallelism:
 // 4096 tokens of 32 heads of 64 go from 405 us to 152 (60 + 7 + 96), of 4 heads from 387 to 37, of 64 heads of 128 from 1663 to 1190.
 // Now bound by the fp32 pipe (63 % busy in 3., 42 % in 1.; 9 warps of 168 registers an SM).  Against 64 bits the outputs are as
@@ -53,6 +54,20 @@ __device__ __forceinline__ void cp_async16_or_zero(void* dst, const void* src, b
     const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(have ? 16 : 0) : "memory");
 }
+__device__ __forceinline__ void cp_async4_or_zero(void* dst, const void* src, bool have) {
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d), "l"(src), "r"(have ? 4 : 0) : "memory");
+}
+// four floats of a row, on any boundary of a float unless VEC
+template <bool VEC>
+__device__ __forceinline__ void stage4(float* dst, const float* src, bool have) {
+    if constexpr (VEC) {
+        cp_async16_or_zero(dst, src, have);
+    } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) cp_async4_or_zero(dst + i, src + i, have);
+    }
+}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
@@ -68,6 +83,7 @@ constexpr int TILE = 64, STATE_THREADS = 64, TB = 16;      // state tile, thread
 
 // Decays of a segment's tokens, their product, and (but for the last segment, whose end nobody starts from) what the segment adds
 // to a 64 x 64 tile of the state.  A thread first takes a channel of a batch of tokens, then 16 rows x 4 columns of the tile.
+template <bool VEC>
 __global__ void __launch_bounds__(STATE_THREADS, 8) wkv_segment_state_kernel(const CcSeqWkv a, const Segments g) {
     __shared__ float4 smw4[2 * 3 * TB * TILE / 4];
     __shared__ float4 decay4[TILE / 4];
@@ -86,10 +102,10 @@ __global__ void __launch_bounds__(STATE_THREADS, 8) wkv_segment_state_kernel(con
         for (int t = tid / (TILE / 4); t < TB; t += STATE_THREADS / (TILE / 4)) {
             const size_t row = (size_t)(first + b * TB + (t < nt ? t : 0)) * HD + (size_t)h * a.D;
             float* const d = buf + t * TILE + x;
-            cp_async16_or_zero(d, a.wraw + row + (in ? i0 + x : 0), t < nt && in);
+            stage4<VEC>(d, a.wraw + row + (in ? i0 + x : 0), t < nt && in);
             if (!add) continue;
-            cp_async16_or_zero(d + ROWS, a.k + row + (in ? i0 + x : 0), t < nt && in);
-            cp_async16_or_zero(d + 2 * ROWS, a.v + row + (inv ? j0 + x : 0), t < nt && inv);
+            stage4<VEC>(d + ROWS, a.k + row + (in ? i0 + x : 0), t < nt && in);
+            stage4<VEC>(d + 2 * ROWS, a.v + row + (inv ? j0 + x : 0), t < nt && inv);
         }
         cp_async_commit();
     };
@@ -192,7 +208,11 @@ __global__ void __launch_bounds__(128) wkv_segment_starts_kernel(const CcSeqWkv 
     const size_t n4 = (size_t)a.H * a.D * a.D / 4, e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= n4) return;
     const size_t hi = e * 4 / a.D;      // head and row
-    float4 x = reinterpret_cast<const float4*>(a.state)[e];
+    auto begin = [&] {
+        if (((uintptr_t)a.state & 15) == 0) return reinterpret_cast<const float4*>(a.state)[e];
+        return make_float4(a.state[4 * e], a.state[4 * e + 1], a.state[4 * e + 2], a.state[4 * e + 3]);
+    };
+    float4 x = begin();
     float4* X = reinterpret_cast<float4*>(g.X);
     X[e] = x;
     for (int s0 = 0; s0 + 1 < g.n; s0 += 16) {
@@ -212,13 +232,13 @@ __global__ void __launch_bounds__(128) wkv_segment_starts_kernel(const CcSeqWkv 
             }
     }
     // what is not finite stays so: all of it again, token after token
-    if (!(fabsf(x.x) + fabsf(x.y) + fabsf(x.z) + fabsf(x.w) < INFINITY)) again_one_by_one(a, g, e, n4, hi, reinterpret_cast<const float4*>(a.state)[e]);
+    if (!(fabsf(x.x) + fabsf(x.y) + fabsf(x.z) + fabsf(x.w) < INFINITY)) again_one_by_one(a, g, e, n4, hi, begin());
 }
 
 // The recurrence inside a segment, 64 columns of a head.  Thread = 16 rows x 4 columns: lane % P holds rows 4 P q + 4 p .. + 3 of
 // P = Dp / 16 row groups, the rest of the thread number the columns.  A token's operands are 13 16-byte reads of shared memory for
 // 124 pairs of fp32 operations; the row groups of a column meet by shuffles, so that tokens need no barrier.
-template <int Dp>
+template <int Dp, bool VEC>
 __global__ void __launch_bounds__(Dp, Dp == 64 ? 6 : 3) wkv_segment_scan_kernel(const CcSeqWkv a, const Segments g) {
     extern __shared__ float4 smw4[];
     float* const sm = reinterpret_cast<float*>(smw4);
@@ -237,16 +257,16 @@ __global__ void __launch_bounds__(Dp, Dp == 64 ? 6 : 3) wkv_segment_scan_kernel(
                 const bool in = t < nt && x < a.D;
                 const size_t src = at + (in ? (size_t)t * HD + x : 0);
                 float* const d = buf + t * Dp + x;
-                cp_async16_or_zero(d, a.r + src, in);
-                cp_async16_or_zero(d + ROWS, a.k + src, in);
-                cp_async16_or_zero(d + 2 * ROWS, g.w + src, in);
+                stage4<VEC>(d, a.r + src, in);
+                stage4<VEC>(d + ROWS, a.k + src, in);
+                stage4<VEC>(d + 2 * ROWS, g.w + src, in);
             }
         }
         const int x = 4 * (tid % (TILE / 4));
 #pragma unroll
         for (int t = tid / (TILE / 4); t < TB; t += THREADS / (TILE / 4)) {
             const bool in = t < nt && j0 + x < a.D;
-            cp_async16_or_zero(buf + 3 * ROWS + t * TILE + x, a.v + at + (in ? (size_t)t * HD + j0 + x : 0), in);
+            stage4<VEC>(buf + 3 * ROWS + t * TILE + x, a.v + at + (in ? (size_t)t * HD + j0 + x : 0), in);
         }
         cp_async_commit();
     };
@@ -362,8 +382,17 @@ __global__ void __launch_bounds__(Dp, Dp == 64 ? 6 : 3) wkv_segment_scan_kernel(
         float lo[4], hi[4];
 #pragma unroll
         for (int x = 0; x < 4; ++x) unpair(st[r][x], lo[x], hi[x]);
-        *reinterpret_cast<float4*>(S + (size_t)i * a.D + j) = make_float4(lo[0], lo[1], lo[2], lo[3]);
-        *reinterpret_cast<float4*>(S + (size_t)(i + 1) * a.D + j) = make_float4(hi[0], hi[1], hi[2], hi[3]);
+        float* const row = S + (size_t)i * a.D + j;
+        if (((uintptr_t)S & 15) == 0) {      // D is a multiple of 4
+            *reinterpret_cast<float4*>(row) = make_float4(lo[0], lo[1], lo[2], lo[3]);
+            *reinterpret_cast<float4*>(row + a.D) = make_float4(hi[0], hi[1], hi[2], hi[3]);
+        } else {
+#pragma unroll
+            for (int x = 0; x < 4; ++x) {
+                row[x] = lo[x];
+                row[a.D + x] = hi[x];
+            }
+        }
     }
 }
 
@@ -383,14 +412,14 @@ static uint64_t workspace_floats(const Segments& g, int T, int H, int D) {
     return ((uint64_t)T * H * D + 3) / 4 * 4 + (uint64_t)g.n * H * D * D + (uint64_t)g.n * H * D;
 }
 
-template <int Dp>
+template <int Dp, bool VEC>
 static int launch_scan(const CcSeqWkv* a, const Segments& g, cudaStream_t st) {
     const size_t smem = 2 * sizeof(float) * (3 * TB * Dp + TB * TILE);
     if (smem > 48 * 1024) {
-        const cudaError_t e = cudaFuncSetAttribute(wkv_segment_scan_kernel<Dp>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        const cudaError_t e = cudaFuncSetAttribute(wkv_segment_scan_kernel<Dp, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return cuda_check("wkv_segments: shared memory");
     }
-    wkv_segment_scan_kernel<Dp><<<dim3(g.n, a->H, (a->D + TILE - 1) / TILE), Dp, smem, st>>>(*a, g);
+    wkv_segment_scan_kernel<Dp, VEC><<<dim3(g.n, a->H, (a->D + TILE - 1) / TILE), Dp, smem, st>>>(*a, g);
     return cuda_check("wkv_segment_scan_kernel");
 }
 
@@ -412,22 +441,25 @@ int cc_seq_wkv_segments(const CcSeqWkv* a, void* workspace, uint64_t workspace_b
     const uint64_t need = cc_seq_wkv_segments_workspace(a->T, a->H, a->D);
     if (need == 0) return fail(CC_SEQ_ERR_UNSUPPORTED_SHAPE, "wkv_segments: heads of multiples of 4 up to 128, at least two segments");
     if (!workspace || workspace_bytes < need) return fail(CC_SEQ_ERR_INVALID_ARG, "wkv_segments: workspace too small");
-    if (((uintptr_t)a->r | (uintptr_t)a->k | (uintptr_t)a->v | (uintptr_t)a->wraw | (uintptr_t)a->state | (uintptr_t)workspace) & 15)
-        return fail(CC_SEQ_ERR_INVALID_ARG, "wkv_segments: rows, state and workspace start on 16-byte boundaries");
+    if ((uintptr_t)workspace & 15) return fail(CC_SEQ_ERR_INVALID_ARG, "wkv_segments: the workspace starts on a 16-byte boundary");
     cudaStream_t st = (cudaStream_t)stream;
     Segments g = plan(a->T, a->H, a->D);
     g.w = (float*)workspace;
     g.X = g.w + ((uint64_t)a->T * a->H * a->D + 3) / 4 * 4;
     g.P = g.X + (uint64_t)g.n * a->H * a->D * a->D;
     const int tiles = (a->D + TILE - 1) / TILE;
-    wkv_segment_state_kernel<<<dim3(g.n, a->H, tiles * tiles), STATE_THREADS, 0, st>>>(*a, g);
+    const bool vec = (((uintptr_t)a->r | (uintptr_t)a->k | (uintptr_t)a->v | (uintptr_t)a->wraw) & 15) == 0;
+    const dim3 grid(g.n, a->H, tiles * tiles);
+    if (vec) wkv_segment_state_kernel<true><<<grid, STATE_THREADS, 0, st>>>(*a, g);
+    else wkv_segment_state_kernel<false><<<grid, STATE_THREADS, 0, st>>>(*a, g);
     int rc = cuda_check("wkv_segment_state_kernel");
     if (rc) return rc;
     const uint64_t n4 = (uint64_t)a->H * a->D * a->D / 4;
     wkv_segment_starts_kernel<<<(unsigned)((n4 + 127) / 128), 128, 0, st>>>(*a, g);
     rc = cuda_check("wkv_segment_starts_kernel");
     if (rc) return rc;
-    return a->D <= 64 ? launch_scan<64>(a, g, st) : launch_scan<128>(a, g, st);
+    if (vec) return a->D <= 64 ? launch_scan<64, true>(a, g, st) : launch_scan<128, true>(a, g, st);
+    return a->D <= 64 ? launch_scan<64, false>(a, g, st) : launch_scan<128, false>(a, g, st);
 }
 
 }  // extern "C"

@@ -318,7 +318,7 @@ def wkv(r, k, v, wraw, w0, u, state, o, H, D):
     a.T, a.H, a.D = r.shape[0], int(H), int(D)
     assert r.shape[1] == H * D and state.numel() == H * D * D
     lib = _lib.load_seq()
-    if a.T >= WKV_SEGMENTS_FROM and not (a.r | a.k | a.v | a.wraw | a.state) & 15:
+    if a.T >= WKV_SEGMENTS_FROM:
         nbytes = lib.cc_seq_wkv_segments_workspace(a.T, a.H, a.D)
         if nbytes:
             ws = torch.empty(nbytes, dtype=torch.uint8, device=o.device)

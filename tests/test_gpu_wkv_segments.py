@@ -61,3 +61,27 @@ def test_what_is_not_served_goes_token_after_token():
         assert ((a - b).norm() / b.norm()).item() <= 2e-6
     w = _lib.CcSeqWkv()
     assert lib.cc_seq_wkv_segments(w, None, 0, None) < 0 and b"wkv_segments" in lib.cc_seq_last_error()
+
+
+@pytest.mark.parametrize("T, H, D", [(257, 3, 64), (400, 2, 100), (300, 5, 20)])
+def test_rows_and_a_state_on_any_boundary_of_a_float_give_the_same_bits(T, H, D):
+    from cold_compress_b200 import _lib, seq_ops
+    assert _lib.load_seq().cc_seq_wkv_segments_workspace(T, H, D) > 0 and T >= seq_ops.WKV_SEGMENTS_FROM
+    gen = torch.Generator(device="cuda").manual_seed(D)
+    rows = [torch.randn(T, H * D, device="cuda", generator=gen) for _ in range(4)]
+    base, u, S0 = torch.randn(H * D, device="cuda", generator=gen) - 2, torch.randn(H * D, device="cuda", generator=gen), torch.randn(H, D, D, device="cuda", generator=gen)
+
+    def at(t, floats):
+        held = torch.empty(t.numel() + 4, device="cuda")
+        held[floats:floats + t.numel()] = t.reshape(-1)
+        return held[floats:floats + t.numel()].view(t.shape)
+
+    def run(*floats):
+        args, state, o = [at(t, n) for t, n in zip(rows, floats)], at(S0, floats[4]), at(torch.zeros(T, H * D, device="cuda"), floats[5])
+        seq_ops.wkv(*args, base, u, state, o, H, D)
+        return o, state
+
+    want = run(0, 0, 0, 0, 0, 0)
+    for floats in ((1, 0, 0, 0, 0, 0), (0, 2, 0, 0, 0, 0), (0, 0, 3, 0, 0, 0), (0, 0, 0, 1, 0, 0), (0, 0, 0, 0, 1, 0), (1, 2, 3, 1, 2, 3)):
+        for a, b in zip(run(*floats), want):
+            assert torch.equal(a, b), floats
