@@ -408,6 +408,17 @@ static Segments plan(int T, int H, int D) {
     if (len < MIN_LEN) len = MIN_LEN;
     return {nullptr, nullptr, nullptr, len, (T + len - 1) / len};
 }
+// Whether segments side by side are the faster way.  They work on whole tiles of 64 rows and columns, the other way on 8 x 16 or 32
+// columns, so heads that leave much of a tile empty gain only while the GPU is not full.  Measured, this / token after token in us:
+//   filled tiles (56 to 64, 100 to 128 wide), any number of heads: 256 tokens of 64 30 / 36 (64 heads), 131 / 144 (300), 141 / 177
+//   (444), of 56 96 / 124 (296); 1024 of 60 482 / 578 (370), of 100 884 / 1189 (222); 256 of 104 62 / 60 (40), 300 70 / 69, 512 97 / 112;
+//   others up to 74 tiles of the state: 256 tokens of 16 29 / 45 (74 heads), 37 / 45 (96), 48 / 45 (128); of 32 29 / 32, 37 / 32, 48 / 33;
+//   of 48 30 / 42 (74), 61 / 55 (160); of 72 30 / 39 (18), 45 / 39 (28), 66 / 47 (48); of 96 31 / 38 (18), 39 / 38 (20), 68 / 45 (48).
+static bool pays(int T, int H, int D) {
+    const int tiles = (D + TILE - 1) / TILE;
+    if (D <= TILE ? D >= 56 : D >= 100) return D <= TILE || D == 2 * TILE || T >= 384;
+    return (long long)H * tiles * tiles <= 74;
+}
 static uint64_t workspace_floats(const Segments& g, int T, int H, int D) {
     return ((uint64_t)T * H * D + 3) / 4 * 4 + (uint64_t)g.n * H * D * D + (uint64_t)g.n * H * D;
 }
@@ -432,7 +443,7 @@ extern "C" {
 uint64_t cc_seq_wkv_segments_workspace(int32_t T, int32_t H, int32_t D) {
     if (T < 1 || H < 1 || D < 1 || D > 128 || D % 4 != 0) return 0;
     const Segments g = plan(T, H, D);
-    return g.n < 2 ? 0 : sizeof(float) * workspace_floats(g, T, H, D);
+    return g.n < 2 || !pays(T, H, D) ? 0 : sizeof(float) * workspace_floats(g, T, H, D);
 }
 
 int cc_seq_wkv_segments(const CcSeqWkv* a, void* workspace, uint64_t workspace_bytes, void* stream) {

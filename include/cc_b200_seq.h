@@ -341,7 +341,7 @@ int cc_seq_wkv_decay(const float* wraw, const float* w0, float* w, int32_t T, in
 /*
  * The same recurrence for steps of many tokens, segments of them side by side (decayed == 0).  Serves heads of multiples of 4 up to
  * 128; the workspace starts on a 16-byte boundary.  cc_seq_wkv_segments_workspace: bytes that a step needs, 0 where it is not cut
- * (too few tokens for the heads, other head sizes).
+ * (too few tokens for the heads, heads that leave much of a tile of 64 empty while they fill the GPU, other head sizes).
  */
 uint64_t cc_seq_wkv_segments_workspace(int32_t T, int32_t H, int32_t D);
 int cc_seq_wkv_segments(const CcSeqWkv* a, void* workspace, uint64_t workspace_bytes, void* stream);
