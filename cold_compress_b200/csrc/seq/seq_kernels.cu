@@ -1726,12 +1726,22 @@ static int launch_decode_rows(const CcSeqAttn* a, cudaStream_t st) {
     return cuda_check("attn_decode_rows_kernel");
 }
 
-// One query head per key head leaves seven of an MMA's eight columns empty: where narrow rows make the tiles' work count (more than a
-// tile per CTA), the kernel above is ahead.  16 heads of 64 + 64, us a layer, this kernel and that one: 300 positions 10.6 / 10.5,
-// 1000 10.8 / 12.3, 4096 17.2 / 16.9, 8000 26.6 / 25.5, 12000 35.8 / 33.9; of 96 + 128 13.5 / 13.8 at 2000, 31.2 / 32.2 at 8000.
+// One or two query heads per key head leave most of an MMA's eight columns empty: where narrow rows make the tiles' work count (several
+// tiles per CTA), the kernel above is ahead.  us a layer, this kernel and that one, tiles per run in brackets:
+//   one query head of 64 + 64, 16 heads: [1] 10.6 / 10.5 and 10.8 / 12.3, [1.8] 17.2 / 16.9, [3.5] 26.6 / 25.5, [5.2] 35.8 / 33.9;
+//   of 72 + 72: [1.8] 16.6 / 16.9, [2.6] 22.3 / 22.2, [5.2] 37.6 / 36.7; 32 heads [3.6] 27.8 / 28.8, [10] 63.7 / 62.8; of 80 + 80 [5.2]
+//   38.1 / 38.2, of 96 + 96 40.0 / 41.0;
+//   two of 32 + 32, 16 key heads: [1.8] 15.8 / 15.8, [2.6] 20.0 / 19.2, [5.2] 33.8 / 31.5; 32 key heads [10] 58.3 / 53.4;
+//   of 24 + 40: 32 key heads [3.6] 24.6 / 25.6, [5.2] 33.8 / 34.2, [10] 58.2 / 56.0; of 48 + 32 [5.2] 35.4 / 33.4; of 48 + 48 36.2 / 40.0,
+//   of 64 + 64 [2.6] 21.5 / 22.2, [5.2] 37.9 / 37.3;
+//   three of 32 + 32, 32 key heads [10] 58.6 / 61.6; four 58.7 / 65.9.
 static bool decode_mma_serves(const CcSeqAttn* a) {
-    const long long tiles = vd_tiles(a->L, attn_reach(*a), MD_KEYS);
-    return a->H > a->G || a->Dk > 64 || a->Dv > 64 || tiles <= vd_splits(tiles, a->G, 2);
+    const long long tiles = vd_tiles(a->L, attn_reach(*a), MD_KEYS), runs = vd_splits(tiles, a->G, 2);
+    const int R = a->H / a->G, D = a->Dk + a->Dv, widest = a->Dk > a->Dv ? a->Dk : a->Dv;
+    if (R == 1 && widest <= 64) return tiles <= runs;
+    if (R == 2 && widest <= 32) return tiles <= 2 * runs;
+    if ((R == 1 && D <= 144) || (R == 2 && D <= 80)) return tiles <= 4 * runs;
+    return true;
 }
 template <typename YT>
 static int launch_decode_mma(const CcSeqAttn* a, cudaStream_t st) {
@@ -1758,7 +1768,6 @@ static int launch_decode(const CcSeqAttn* a, cudaStream_t st) {
     if (decode_rows_serves(a)) {
         if constexpr (sizeof(CT) == 2) {
             if (decode_mma_serves(a)) return launch_decode_mma<YT>(a, st);
-            return launch_decode_rows<CT, YT, 1>(a, st);
         }
         if (R <= 1) return launch_decode_rows<CT, YT, 1>(a, st);
         if (R <= 2) return launch_decode_rows<CT, YT, 2>(a, st);

@@ -65,6 +65,15 @@ def test_rows_and_edges(H, G, Dk, Dv, past):
     assert ((y.double() - want).abs().max() / want.abs().max()).item() <= 2 * tol
 
 
+@pytest.mark.parametrize("H,G,Dk,Dv", [(32, 16, 32, 32), (32, 16, 8, 24), (32, 16, 48, 32), (16, 16, 72, 72), (16, 16, 64, 80), (16, 16, 64, 64), (48, 16, 32, 32)])
+@pytest.mark.parametrize("past", [2290, 2310, 4590, 4620, 9200, 9300])
+def test_narrow_rows_of_few_query_heads(H, G, Dk, Dv, past):
+    """Around the numbers of tiles from which one or two query heads leave the tensor cores (18 runs a head of 128 keys a tile)."""
+    y, want, s = _run(H, G, Dk, Dv, past)
+    tol = 2.0 ** -24 * (2 * (Dk / 16 + 8) * max(s.abs().max().item(), 1.0) + past / 32 + 32)      # as above
+    assert ((y.double() - want).norm() / want.norm()).item() <= tol
+
+
 @pytest.mark.parametrize("past,window,keep", [(10, 64, 0), (500, 64, 0), (1000, 129, 4), (3000, 1000, 7), (70, 64, 4)])
 @pytest.mark.parametrize("sink,softcap", [(0, 0.0), (1, 30.0), (2, 0.0)])
 def test_rings_kept_positions_sinks_and_caps(past, window, keep, sink, softcap):
