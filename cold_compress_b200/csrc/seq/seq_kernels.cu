@@ -1098,8 +1098,7 @@ __host__ __device__ inline MdLayout md_layout(int R, int Dk, int Dv, int buffers
     l.ps = l.qb + (size_t)3 * 8 * (l.KU + 1) * 16;
     l.pb = l.ps + (size_t)8 * VT * 4;
     l.total = l.pb + (size_t)3 * 8 * (VT + 8) * 2;
-    const size_t combine = (size_t)MD_THREADS * 16;                 // the groups' sums of the combination take the keys' place
-    if (l.vs < combine) l.total += combine;
+    static_assert(MD_KEYS * 3 >= MD_THREADS, "the groups' sums of the combination take the keys' place, three units a row at least");
     return l;
 }
 
@@ -1143,7 +1142,7 @@ __global__ void __launch_bounds__(MD_THREADS, 2) attn_decode_mma_kernel(const Cc
     __syncthreads();      // the barriers and the zeros stand
     // The first half of the CTA asks for keys, the second for values, a thread per row: a whole tile is under way at once, where 16
     // copies of 16 bytes per thread waited for one another (8 layers of 8 heads x 4096 positions of 128 + 128: 117 us, 109).
-    static_assert(MD_THREADS == 2 * 128 && VT <= 128, "a thread per row");
+    static_assert(MD_THREADS == 2 * VT, "a thread per row");
     const bool value = tid >= MD_THREADS / 2;
     const int ht = tid & (MD_THREADS / 2 - 1), D = value ? Dv : Dk, stride = value ? v_row : k_row;
     const CT* const fresh_row = value ? (const CT*)a.v_new + (size_t)g * Dv : (const CT*)a.k_new + (size_t)g * Dk;
@@ -1163,7 +1162,6 @@ __global__ void __launch_bounds__(MD_THREADS, 2) attn_decode_mma_kernel(const Cc
         } else {
             md_bar_arrive(bar);
         }
-        if (ht >= VT) return;
         if (value) {      // no position: whatever lay there must not meet a weight of zero
             if (ht >= rows)
                 for (int c = 0; c < vc16; ++c) dst[ht * stride + c] = make_uint4(0, 0, 0, 0);
@@ -1704,10 +1702,10 @@ static bool decode_rows_serves(const CcSeqAttn* a) {
 template <typename CT, typename YT, int RMAX>
 static int launch_decode_rows(const CcSeqAttn* a, cudaStream_t st) {
     // Two CTAs per SM, one where eight query heads' registers leave room for no more: tiles of 128 keys if one fits a CTA's share of
-    // the shared memory, of 64 otherwise, and a second buffer for runs of more than one tile only if it fits too.  Runs of 5500 /
-    // 12000 / 32000 positions with a second buffer and one CTA per SM where two were counted on, and as it is now, in us: bf16
-    // 32 / 8 heads of 128 39.0 / 52.3 / 114.1 and 26.0 / 34.7 / 73.8; fp32 45.7 / 65.2 / 141.7 and 27.9 / 48.9 / 105.1; fp32 16 / 16 of 64
-    // 39.3 / 66.2 / 145.8 and 22.0 / 39.3 / 88.6.  Two buffers of 64 keys for bf16 rows of 128 + 128: 25.5 / 39.7 / 88.1.
+    // the shared memory (the bf16 rows that come here, of at most 144 columns, always do), of 64 otherwise, and a second buffer for runs
+    // of more than one tile only if it fits too.  Runs of 5500 / 12000 / 32000 positions with a second buffer and one CTA per SM
+    // where two were counted on, and as it is now, in us: fp32 32 / 8 heads of 128 45.7 / 65.2 / 141.7 and 27.9 / 48.9 / 105.1; fp32 16 / 16
+    // of 64 39.3 / 66.2 / 145.8 and 22.0 / 39.3 / 88.6.
     const int vc16 = a->Dv * (int)sizeof(CT) / 16, per_sm = RMAX <= 4 ? 2 : 1;
     const size_t share = (per_sm == 2 ? 111 : 223) * 1024;
     const size_t red = sizeof(float) * (size_t)(VD_THREADS / vc16) * (a->H / a->G) * a->Dv;
@@ -1715,11 +1713,14 @@ static int launch_decode_rows(const CcSeqAttn* a, cudaStream_t st) {
         const size_t tiles = (size_t)buffers * VT * (sizeof(CT) * (size_t)(a->Dk + a->Dv) + 16);
         return (tiles > red ? tiles : red) + sizeof(float) * RMAX * (size_t)(a->Dk + VT);
     };
-    const int VT = bytes(1, 128) <= share ? 128 : 64;
+    const int VT = sizeof(CT) == 2 || bytes(1, 128) <= share ? 128 : 64;
     const long long tiles = vd_tiles(a->L, attn_reach(*a), VT);
     const int NS = vd_splits(tiles, a->G, per_sm), buffers = tiles > NS && bytes(2, VT) <= share ? 2 : 1;
     const size_t smem = bytes(buffers, VT);
-    auto kern = VT == 128 ? attn_decode_rows_kernel<CT, YT, RMAX, 128> : attn_decode_rows_kernel<CT, YT, RMAX, 64>;
+    auto kern = attn_decode_rows_kernel<CT, YT, RMAX, 128>;
+    if constexpr (sizeof(CT) == 4) {
+        if (VT == 64) kern = attn_decode_rows_kernel<CT, YT, RMAX, 64>;
+    }
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return fail(CC_SEQ_ERR_CUDA, cudaGetErrorString(e));
     launch_under(kern, dim3(NS, a->G), dim3(VD_THREADS), smem, st, *a, buffers, NS);
@@ -1768,11 +1769,13 @@ static int launch_decode(const CcSeqAttn* a, cudaStream_t st) {
     if (decode_rows_serves(a)) {
         if constexpr (sizeof(CT) == 2) {
             if (decode_mma_serves(a)) return launch_decode_mma<YT>(a, st);
+            return R <= 1 ? launch_decode_rows<CT, YT, 1>(a, st) : launch_decode_rows<CT, YT, 2>(a, st);
+        } else {
+            if (R <= 1) return launch_decode_rows<CT, YT, 1>(a, st);
+            if (R <= 2) return launch_decode_rows<CT, YT, 2>(a, st);
+            if (R <= 4) return launch_decode_rows<CT, YT, 4>(a, st);
+            return launch_decode_rows<CT, YT, 8>(a, st);
         }
-        if (R <= 1) return launch_decode_rows<CT, YT, 1>(a, st);
-        if (R <= 2) return launch_decode_rows<CT, YT, 2>(a, st);
-        if (R <= 4) return launch_decode_rows<CT, YT, 4>(a, st);
-        return launch_decode_rows<CT, YT, 8>(a, st);
     }
     if (R <= 1) return launch_decode_r<CT, YT, 1>(a, st);
     if (R <= 2) return launch_decode_r<CT, YT, 2>(a, st);
