@@ -119,3 +119,36 @@ def test_a_slot_without_its_position_counts_for_nothing():
     K, V = (torch.cat([t[:, :gone], t[:, gone + 1:], n.transpose(0, 1)], 1).double() for t, n in ((k, k1), (v, v1)))
     w = torch.softmax(torch.einsum("grd,gnd->grn", q[0].double().view(2, 4, 64), K) * 0.125, -1)
     assert ((y[0].double() - torch.einsum("grn,gnd->grd", w, V).reshape(8, 64)).abs() <= 1e-5).all()
+
+
+def _two_keys(q, keys, values, scale):
+    """y [8, 64] of eight query heads over two positions, keys and values [2, 64]."""
+    from cold_compress_b200 import _lib
+    cache, _, _, _, _ = _layer(1, 64, 64, 1)
+    cache.k_cache[0, 0, 0], cache.v_cache[0, 0, 0] = keys[0], values[0]
+    y, ip = torch.empty(1, 8, 64, device=DEV), torch.ones(1, dtype=torch.int32, device=DEV)
+    cache.sequence_step(q.view(1, 8, 64), keys[1].view(1, 1, 64), values[1].view(1, 1, 64), ip, y, sink_mode=_lib.SINK_NONE, scale=scale)
+    return y[0].double()
+
+
+def test_all_three_parts_of_a_query_count():
+    """Queries whose first and second part cancel between two channels: the score is what the third one holds."""
+    j = torch.arange(1, 9, device=DEV)
+    q, keys, values = torch.zeros(8, 64, device=DEV), torch.zeros(2, 64, device=DEV).bfloat16(), torch.zeros(2, 64, device=DEV).bfloat16()
+    q[:, 0], q[:, 1] = 1 + 2.0 ** -9 + j * 2.0 ** -20, 1 + 2.0 ** -9
+    keys[0, 0], keys[0, 1], values[0] = 1, -1, 1
+    # scores j / 4 and 0, exact in fp32; the exponentials and the quotient are a few roundings
+    y = _two_keys(q, keys, values, 2.0 ** 18)
+    assert ((y - torch.sigmoid(j.double() / 4).view(8, 1)).abs() <= 8 * 2.0 ** -24).all()
+
+
+def test_all_three_parts_of_a_weight_count():
+    """Weights of 1 and of almost 1 on values of opposite sign: the sum is what the third part of the second one holds."""
+    j = torch.arange(1, 9, device=DEV)
+    q, keys, values = torch.zeros(8, 64, device=DEV), torch.zeros(2, 64, device=DEV).bfloat16(), torch.ones(2, 64, device=DEV).bfloat16()
+    q[:, 0] = j * 2.0 ** -18
+    keys[1, 0], values[1] = -1, -1
+    w = torch.exp(-j.double() * 2.0 ** -18)
+    # the smaller weight is one rounding of a number just below 1 and an exponential's error (2 units of 2^-24), the sum exact
+    y = _two_keys(q, keys, values, 1.0)
+    assert ((y - ((1 - w) / (1 + w)).view(8, 1)).abs() <= 3 * 2.0 ** -24).all()

@@ -42,3 +42,24 @@ def test_greedy_ties_and_what_is_no_number():
         assert p.dtype == row.dtype and int(tok) == int(torch.argmax(p.detach()))
     tok, p = greedy(x.view(1, 1, -1), torch.tensor([5], dtype=torch.int32, device=DEV))
     assert int(tok) == 5 and p.shape == x.shape
+
+
+def test_greedy_under_tracing_vmap_and_capture():
+    from cold_compress_b200.generation_utils import greedy
+    gen = torch.Generator(device=DEV).manual_seed(2)
+    a, b = (torch.randn(1, 1, 5000, device=DEV, generator=gen) * 4 for _ in range(2))
+    traced = torch.jit.trace(lambda x: greedy(x, None), (a,), check_trace=False)
+    tok, p = traced(b)                                 # what was recorded runs on other logits
+    assert int(tok) == int(b.argmax()) and torch.allclose(p, torch.softmax(b[0, -1], -1), rtol=1e-5, atol=0)
+    many = torch.vmap(lambda x: greedy(x, None)[1])(torch.stack([a, b]))
+    assert torch.equal(many, torch.softmax(torch.stack([a, b])[:, 0, -1], -1))
+    held = a.clone()
+    greedy(held, None)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        tok, p = greedy(held, None)
+    for x in (a, b):
+        held.copy_(x)
+        graph.replay()
+        want_tok, want = greedy(x, None)
+        assert torch.equal(tok, want_tok) and torch.equal(p, want)
