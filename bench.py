@@ -1,10 +1,10 @@
 #!/usr/bin/env python
-"""bench.py -- decode tokens/sec of the compressed-KV decode path on B200 (see DESIGN.md section 5).
+"""bench.py -- decode tokens/sec of the compressed-KV decode path on B200.
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--config 1..5] [--impl ours|reference]
     python -m torch.distributed.run --nnodes=1 --nproc-per-node N ... bench.py --gpus N ...
 
-Workloads = the five BASELINE.json configs (random-init bf16 weights, synthetic token ids):
+Workloads (random-init bf16 weights, synthetic token ids):
   1  Llama-3-8B-shape, recent_global, 64 slots, 128-token prompt                       (the reference's CPU plumbing case)
   2  Llama-3-8B-shape, heavy_hitter + SnapKV compression, 1024 slots, 7680-token prompt = "8k ctx"   (default at N = 1)
   3  Llama-3-8B-shape, l2, 512 slots, 4096-token prompt
@@ -16,8 +16,8 @@ step is ONE persistent kernel, or a CUDA graph of per-layer kernels for config 4
 token and the position, both on the device); `e2e` = the same through the public decode loop with the token id coming
 from pinned host memory and the sampled token read back to the host every step.
 
-`--impl reference` runs the UNMODIFIED reference (installed into baseline/_ref by tools/install_reference.sh, see
-DESIGN.md) on the host cores: its own Transformer / KVCache classes and its own decode_one_token, caches in a
+`--impl reference` runs the UNMODIFIED reference (installed into baseline/_ref by tools/install_reference.sh)
+on the host cores: its own Transformer / KVCache classes and its own decode_one_token, caches in a
 synthetic full post-prefill state (the reference's O(S^2) CPU prefill of an 8k prompt takes ~20 minutes).  Without
 baseline/_ref it falls back to the port (torch CPU GEMVs + oracle/ for cache and attention) and says so.
 """
@@ -40,7 +40,7 @@ ROOT = Path(__file__).resolve().parent
 sys.path.insert(0, str(ROOT))
 
 LLAMA, QWEN = "Meta-Llama-3-8B-Instruct", "Qwen2-7B-Instruct"
-HYBRID_STRATEGIES = [   # ~2048 live slots per head of 17408 allocated
+HYBRID_STRATEGIES = [   # ~2048 live slots per head of 17408 allocated (workload 4)
     {"strategy": "window", "recent_window": 0.1176},
     {"strategy": "window_heavy_hitter", "recent_window": 0.0588, "heavy_hitter_frac": 0.0588},
     {"strategy": "full"},
@@ -58,8 +58,7 @@ CONFIGS = {
             what="heavy_hitter + SnapKV compression, pyramid cache lengths (2036 ... 256, sum 33128 slots), 7680-token "
                  "synthetic prompt, decode @ 8k ctx"),
 }
-METRIC = "decode tokens/sec @ 8k ctx, 1024-slot heavy-hitter"   # BASELINE.json's metric (configs 2 and 5)
-PROMPT_LEN, MAX_NEW = CONFIGS[2]["prompt"], CONFIGS[2]["max_new"]   # (profiles/ scripts)
+METRIC = "decode tokens/sec @ 8k ctx, 1024-slot heavy-hitter"   # of workloads 2 and 5
 
 
 def workload_config(cfg_id, world):
@@ -162,7 +161,7 @@ def build_gpu_model(device, world, model_name=LLAMA):
                 p.normal_(0.0, 0.02, generator=gen)
     fake = int(os.environ.get("CC_TP_FAKE", "0"))
     if world == 1 and fake > 1:
-        # diagnostics (profiles/): rank 0's shard of a `fake`-way split on ONE GPU with the exchanges skipped, i.e. the
+        # diagnostics: rank 0's shard of a `fake`-way split on ONE GPU with the exchanges skipped, i.e. the
         # compute-only time of a tensor-parallel rank; the number it prints is NOT a bench value
         from cold_compress_b200.tp import apply_tp
         os.environ["LOCAL_RANK"], os.environ["LOCAL_WORLD_SIZE"] = "0", str(fake)
@@ -185,11 +184,11 @@ def peaks():
     if f.exists():
         d = json.loads(f.read_text())
         return d.get("hbm_gbs", 6650.0), "measured (MEASURED_PEAKS.json)"
-    return 6650.0, "fallback (B200_PROFILING.md)"
+    return 6650.0, "fallback"
 
 
 def live_kv_bytes(model):
-    """Algorithmic bytes of the cache stage per token on this rank (SURVEY 8d): live K and V rows, bf16."""
+    """Algorithmic bytes of the cache stage per token on this rank: live K and V rows, bf16."""
     total = 0
     for b in model.layers:
         c = b.attention.kv_cache
@@ -1430,7 +1429,7 @@ def main():
     ap.add_argument("--warmup", type=int, default=16)
     ap.add_argument("--impl", default="ours", choices=["ours", "reference"])
     ap.add_argument("--config", type=int, default=0, choices=[0, 1, 2, 3, 4, 5],
-                    help="BASELINE.json config (default: 2 on one GPU, 5 = pyramid lengths under head sharding on several)")
+                    help="workload (default: 2 on one GPU, 5 = pyramid lengths under head sharding on several)")
     ap.add_argument("--k1", action="store_true", help="also time the per-layer decode kernel (cc_decode_step) alone")
     ap.add_argument("--design", default="", metavar="SIZES",
                     help="instead of the headline workload: Tidelorn beside the Llama-family model at equal layer shape, "

@@ -15,7 +15,7 @@ from pathlib import Path
 PKG = Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 SO = PKG / "libcc_b200.so"
-# CC_NVCC_DEFS="-DCC_TOKEN_PRODUCER=0 ...": A/B builds (python -m cold_compress_b200.build --out=profiles/libcc_x.so)
+# CC_NVCC_DEFS="-DCC_TOKEN_PRODUCER=0 ...": A/B builds (python -m cold_compress_b200.build --out=libcc_x.so)
 NVCC_FLAGS = [*(["-DCC_TOKEN_MICROTRACE"] if __import__("os").environ.get("CC_TOKEN_MICROTRACE") else []),
               *__import__("os").environ.get("CC_NVCC_DEFS", "").split(), "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", "-std=c++17",
               "--shared", "-Xcompiler", "-fPIC", "-Xptxas", "-v"]

@@ -1,6 +1,6 @@
 """KV-cache policy layer: host-side mirror of the reference's cache.py surface.
 
-Drop-in boundary (SURVEY.md section 8b): `get_cache_constructor(strategy) -> (cls, relevant_kwargs)`,
+Drop-in boundary: `get_cache_constructor(strategy) -> (cls, relevant_kwargs)`,
 `cls(max_batch_size, n_heads, head_dim, dtype, **kwargs)`, `.update_kv / .update_state /
 .return_attn / .reset / .compute_statistics`, `add_cache_arguments`, `cache_compatibility`
 (reference cache.py:13-139, 152-346, 1444-1478).  Buffers carry the reference's names, shapes and
@@ -352,7 +352,7 @@ class KVCacheHeadSpecific(KVCache):
 
 # --------------------------------------------------------------------------- host-side (EXTERNAL) policies
 # Their slot choice is a handful of integer ops on `pos`; the kernel takes the index and does the
-# overwrite + attention.  Not in BASELINE configs.
+# overwrite + attention.
 
 
 def _base_eviction_idx(scores, pos_row, global_tokens):
@@ -634,10 +634,10 @@ class KVCacheHybrid(KVCacheHeavyHitter):
     def profile_and_update(self, input_pos, k_val, v_val, attn, **kwargs):
         """Choose a strategy per head from the prompt's attention (FastGen), lay the prompt out with the
         kept tokens first, seed masks / counts / history.  `attn` is a PrefillAttnStats with band sums
-        (or the reference's full [1,H,S,S] map, reduced here).  Deviations from the reference, both
-        documented in DESIGN.md: recovered mass is computed from column and band sums (same value up to
+        (or the reference's full [1,H,S,S] map, reduced here).  Two deviations from the
+        reference: recovered mass is computed from column and band sums (same value up to
         bf16 rounding of the reference's row sums), and kept tokens are laid out in ascending position
-        (the reference's order comes from an unstable argsort, SURVEY 8 a19)."""
+        (the reference's order comes from an unstable argsort)."""
         from .prompt_compression import PrefillAttnStats
         input_ids = kwargs["input_ids"].reshape(-1)
         S, H, dev = input_ids.numel(), self.n_heads, self.pos.device

@@ -452,7 +452,7 @@ __device__ void producer_loop(const TokParams& P, const DescWindow* W, uint8_t* 
     uint32_t par = 0xffffffffu;   // a fresh barrier passes a wait on the phase "before the first": every stage starts free
     // (a second cursor prefetching the tiles beyond the ring into L2 -- cp.async.bulk.prefetch.L2, 2 / 4 / 8 / 16 tiles
     // per warp whenever the ring is full -- was measured 0.4 / 0.7 / 1.8 / 3.9 % SLOWER than none: the bulk
-    // prefetches queue in front of the demand copies in the SM's TMA unit; profiles/r2/notes.md)
+    // prefetches queue in front of the demand copies in the SM's TMA unit)
     while (it.op < P.n_ops) {
         if (mbar_test(&eb[ps], (par >> ps) & 1u)) {
             iter_issue(it, lane, stages + (size_t)ps * kStage, &fb[ps], policy);
@@ -636,7 +636,7 @@ __device__ void stage_input(const TokParams& P, const TokOp& op, __nv_bfloat16* 
 // of an MMA can hold any 16 elements as long as A and B agree): 256 weight elements per MMA.  In every round the
 // lanes of a quarter-warp read one contiguous 128-byte run of a row and the warp reads S * 64 contiguous bytes of
 // the input: conflict free without padding, 12 (R = 2) or 10 (R = 4) shared-memory wavefronts per KiB of weights.
-// (Round 2, first version: 8 A rows duplicated into 16 = half the weights per MMA and 16 wavefronts per KiB; a
+// (First version: 8 A rows duplicated into 16 = half the weights per MMA and 16 wavefronts per KiB; a
 // hand-written FFMA loop costs 10x the instructions.  Both left the warps barely faster than the HBM stream.)
 __device__ __forceinline__ void mma_bf16_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
@@ -1341,7 +1341,7 @@ __global__ void __launch_bounds__(kLaunchThreads, 1) cc_token_kernel(const __gri
     ring.win = &win;
     // the weight / cache stream starts before anything else: fill the whole ring
     // (an L2 prefetch cursor running further ahead -- cp.async.bulk.prefetch.L2 of the tiles after the ring -- was
-    // measured SLOWER: 301 -> 273 tokens/s at 2 tiles per warp, 240 at 6; profiles/r2/notes.md)
+    // measured SLOWER: 301 -> 273 tokens/s at 2 tiles per warp, 240 at 6)
     if (kProducer) {
         if (warp >= kTW) {
             asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" :: "n"(kProducerRegs));

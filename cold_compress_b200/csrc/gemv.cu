@@ -1,4 +1,4 @@
-// gemv.cu -- the rest of the decode layer around the cache kernel (SURVEY.md 8f/f2):
+// gemv.cu -- the rest of the decode layer around the cache kernel:
 // one-token matrix-vector products over bf16 weights with the elementwise work fused in, so a
 // decoded token is 5 launches per layer instead of ~60 ATen kernels:
 //
@@ -443,7 +443,7 @@ static int launch_split(K1 k1, K2 k2, K4 k4, K8 k8, const P& p, int n_pairs, int
     const int cap = sm_count() * 8;
     if (grid > cap) grid = cap;
     // (sharing the input staging between the CTAs of a cluster over DSMEM was measured 5-8 us per launch SLOWER:
-    // gang scheduling + two cluster barriers, profiles/r1_notes.md)
+    // gang scheduling + two cluster barriers)
     auto go = [&](auto kernel) -> int {
         static thread_local const void* raised[16] = {};
         if (smem > 48 * 1024) {  // raise the per-function cap once, to the device limit

@@ -266,7 +266,7 @@ __device__ __forceinline__ void tile_stats(const uint8_t* sP_ptr, float* out_col
 // (row = t % 128, ch = t / 128) owns keys [32 ch, 32 ch + 32) of its row of every S block (TMEM lane quarter row / 32).
 // The partial accumulators Y_0 + Y_1 are added in the epilogue (fixed order: bit-reproducible).
 // Bound: latency at four warps per scheduler (issue slots 48 % busy, tensor pipe 23 %, the largest stalls fixed latencies and the
-// group's barrier: profiles/rows).  A group has
+// group's barrier).  A group has
 // two P blocks so that one barrier per block of sweep 2 is enough: it says that the block is written, and that everyone has
 // read the block before, which the block after it may then overwrite once its MMAs are done.  With one P block there were
 // two barriers per block and the column sums waited in shared memory: 1718 us at 7680 tokens x 32 heads of 128 (8 key/value

@@ -290,7 +290,7 @@ class Transformer(nn.Module):
         return b["logits"].view(1, 1, -1)
 
     # Optional L2 warm-up: bytes of w1 / w3 rows (plus all of wo) the cache step asks L2 to pre-load while it
-    # waits on its own latencies (cc_decode_step prefetch hints).  Measured on B200 (profiles/r1_notes.md):
+    # waits on its own latencies (cc_decode_step prefetch hints).  Measured on B200:
     # 333 tok/s without, 332 / 331 / 329 / 325 tok/s with wo / +10 / +24 / +40 MB -- no gain, so it is off.
     warm_l2_ffn_bytes = -1
 

@@ -168,7 +168,7 @@ int cc_decode_step(const CcCacheState* state, const CcDecodeArgs* args, void* st
 int cc_decode_cluster_size(const CcCacheState* state);
 
 /* Diagnostics: device buffer of [n_CTAs][16] u64 that later cc_decode_step launches fill with
-   %globaltimer stamps at their phase boundaries (profiles/trace_k1.py); NULL turns it off. */
+   %globaltimer stamps at their phase boundaries ; NULL turns it off. */
 void cc_debug_set_trace(void* device_buffer);
 
 /*

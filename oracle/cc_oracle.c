@@ -6,9 +6,9 @@
  * attention layer.  Only tests/, __graft_entry__.smoke() and bench.py's
  * cpu_baseline / --impl reference legs may load it; the product path never does.
  *
- * Parity pin: the reference ships no tests or golden vectors (SURVEY.md section 4), so the
- * oracle is pinned against outputs of the reference itself, executed unmodified in
- * the build container by tests/golden/make_golden.py; the fixtures are committed
+ * Parity pin: the reference ships no tests or golden vectors, so the
+ * oracle is pinned against outputs of the reference itself, executed unmodified
+ * by tests/golden/make_golden.py; the fixtures are committed
  * under tests/golden/ and checked by tests/test_oracle_golden.py.
  *
  * The arithmetic lives in PyTorch (un-vendored dependency, reference pins

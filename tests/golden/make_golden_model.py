@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""Whole-model trace of BASELINE config 1, recorded by EXECUTING THE UNMODIFIED REFERENCE on CPU (build container
+"""Whole-model trace of benchmark workload 1, recorded by EXECUTING THE UNMODIFIED REFERENCE on CPU (build container
 only, needs /root/reference and ~40 GB of RAM):
 
     python tests/golden/make_golden_model.py            # writes tests/golden/model_cfg1.npz

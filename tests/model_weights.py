@@ -1,4 +1,4 @@
-"""Seeded weights that the reference (CPU, build container) and this package (GPU box) can both build in seconds:
+"""Seeded weights that the reference (on CPU) and this package (on a GPU) can both build in seconds:
 every parameter is a window-tiling of one seeded normal block of PRIME elements.  PRIME is prime and larger than any
 row count, so no two rows of a matrix see the same window of the block (no duplicated rows, no arg-max ties by
 construction), and filling 8 B parameters is a memcpy rather than 8 B normal draws."""

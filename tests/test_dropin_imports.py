@@ -103,7 +103,7 @@ def test_abi_exports_every_declared_symbol():
 
 def test_kernel_register_budgets():
     """Occupancy guard on the build log (ptxas -v): the one-token projection kernels must stay at <= 80 registers
-    (3 CTAs of 256 threads per SM -- at 128 they drop to 2 and lose 10-15 % of their bandwidth, profiles/r1_notes.md),
+    (3 CTAs of 256 threads per SM -- at 128 they drop to 2 and lose 10-15 % of their bandwidth),
     the prefill kernel at <= 128 (512 threads), and nothing may spill more than a few bytes."""
     import re
     from pathlib import Path

@@ -86,7 +86,7 @@ def test_hybrid_decode_trace_matches_reference_and_oracle(name):
 
 SHAPES = [
     # strategy, Hkv, G, D, L, n_filled, steps
-    ("heavy_hitter", 8, 4, 128, 1024, 1024, 48),   # BASELINE config 2 shape, cache full
+    ("heavy_hitter", 8, 4, 128, 1024, 1024, 48),   # benchmark workload 2 shape, cache full
     ("heavy_hitter", 8, 4, 128, 2036, 2000, 60),   # pyramid layer length (ragged tail, 2 chunks, fill then evict)
     ("heavy_hitter", 4, 7, 128, 556, 556, 40),     # Qwen2-7B grouping, ragged length
     ("heavy_hitter", 1, 4, 128, 1024, 1024, 24),   # one local head (tp.py world size 8)
@@ -94,9 +94,9 @@ SHAPES = [
     ("heavy_hitter:w16", 8, 4, 128, 1024, 1000, 60),  # bounded history window (bf16 ring), fill then evict
     ("heavy_hitter:w4", 2, 2, 64, 200, 60, 80),
     ("heavy_hitter:w8t", 4, 4, 128, 256, 200, 120),    # thresholded (bool) history; oracle-pinned only (the reference raises)
-    ("l2", 8, 4, 128, 512, 512, 48),               # BASELINE config 3 shape
+    ("l2", 8, 4, 128, 512, 512, 48),               # benchmark workload 3 shape
     ("l2", 2, 6, 128, 200, 64, 40),
-    ("recent_global", 8, 4, 128, 64, 64, 40),      # BASELINE config 1 shape
+    ("recent_global", 8, 4, 128, 64, 64, 40),      # benchmark workload 1 shape
     ("recent_global", 8, 4, 128, 4096, 4090, 24),
     ("full", 8, 4, 128, 8192, 5000, 12),           # full cache: 8 chunks per CTA through a 4-stage ring
     ("keep_it_odd", 2, 4, 128, 128, 128, 30),
@@ -171,7 +171,7 @@ def test_three_call_surface_equals_fused_step(W):
 
 
 def test_full_size_properties():
-    """BASELINE config-2 size, no oracle: invariants of the step that hold at any size."""
+    """The headline workload's size, no oracle: invariants of the step that hold at any size."""
     from device_utils import make_device_cache, synthetic_fill
     Hkv, G, D, L = 8, 4, 128, 1024
     c = make_device_cache("heavy_hitter", Hkv, D, L)

@@ -1,6 +1,6 @@
 """GPU: the tcgen05 prefill attention kernel (cc_prefill_attention through the product API
 cold_compress_b200.attention_utils.prefill_attention_stats) against the vectors recorded from the unmodified
-reference (tests/golden/prefill_*.npz), against the restatement in oracle/prefill.py, and -- at BASELINE sizes --
+reference (tests/golden/prefill_*.npz), against the restatement in oracle/prefill.py, and -- at the benchmark's sizes --
 through size-independent properties."""
 import pytest
 import torch
@@ -80,7 +80,7 @@ def test_prefill_kernel_matches_oracle_bands_and_layouts(name):
 
 @pytest.mark.parametrize("Hkv,G,D,S,W", [(8, 4, 128, 8192, 819), (4, 7, 128, 16384, 1638), (2, 2, 64, 4096, 0)])
 def test_prefill_full_size_properties(Hkv, G, D, S, W):
-    """BASELINE-size prompts (configs 2-4 head shapes): rows of the pooled map sum to 1, so the column sums add up
+    """Prompts of the benchmark's sizes (configs 2-4 head shapes): rows of the pooled map sum to 1, so the column sums add up
     to S and the observation-window sums to obs_len; y is a convex combination of the values; y and the
     reductions agree with the torch restatement evaluated on the same device (checker only)."""
     from oracle.prefill import blockwise_stats

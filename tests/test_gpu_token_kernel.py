@@ -31,13 +31,13 @@ def test_attention_stage_matches_reference_and_oracle(name):
 
 
 SHAPES = [
-    ("heavy_hitter", 8, 4, 128, 1024, 1024, 24),   # BASELINE config 2 shape
+    ("heavy_hitter", 8, 4, 128, 1024, 1024, 24),   # benchmark workload 2 shape
     ("heavy_hitter", 8, 4, 128, 2036, 2000, 50),   # pyramid layer length: ragged 128-row chunks, fill then evict
     ("heavy_hitter", 4, 7, 128, 556, 556, 24),     # Qwen2-7B grouping, ragged length
     ("heavy_hitter", 1, 4, 128, 1024, 1024, 16),   # one local head (tp.py world size 8): 64 CTAs on one head
     ("heavy_hitter", 2, 8, 64, 300, 120, 30),      # D=64, G=8
-    ("l2", 8, 4, 128, 512, 512, 24),               # BASELINE config 3 shape
-    ("recent_global", 8, 4, 128, 64, 64, 24),      # BASELINE config 1 shape
+    ("l2", 8, 4, 128, 512, 512, 24),               # benchmark workload 3 shape
+    ("recent_global", 8, 4, 128, 64, 64, 24),      # benchmark workload 1 shape
     ("recent_global", 8, 4, 128, 4096, 4090, 12),  # two chunks per CTA through the ring
 ]
 

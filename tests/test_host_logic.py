@@ -21,7 +21,7 @@ def test_cache_length_normalisation_and_patterns_recorded_values():
     assert gu.apply_pattern([64, 128], 8, "repeat", 8192) == [64, 128, 64, 128, 64, 128, 64, 128]
     assert gu.apply_pattern([1024], 8, "pyramid", 8192) == [2023, 1535, 1287, 1039, 791, 543, 295, 256]
     assert gu.apply_pattern([1024], 8, "funnel", 8192) == [256, 295, 543, 791, 1039, 1287, 1535, 2023]
-    lens = gu.apply_pattern([1024], 32, "pyramid", 8192)
+    lens = gu.apply_pattern([1024], 32, "pyramid", 8192)   # the benchmark's pyramid workload
     assert lens == PYRAMID_1024_8192_32 and sum(lens) == 33128
     with pytest.raises(AssertionError):
         gu.apply_pattern([512, 1024], 32, "funnel", 8192)

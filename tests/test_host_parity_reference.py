@@ -2,7 +2,7 @@
 seeded `pos` states (CPU): the index rule of reference cache.py:366-379 with the `_token_importances` of cache.py:519-524
 (random) and 1437-1441 (keep_it_odd), and KVCacheFull's first-unfilled rule (cache.py:500-502).  The GPU parity tests
 hand this index to the kernel and to the oracle, so the rule itself is pinned here.  Needs the reference checkout
-(/root/reference in the build container, baseline/_ref on the GPU box)."""
+(/root/reference or baseline/_ref)."""
 import importlib.util
 import sys
 from pathlib import Path
@@ -101,6 +101,6 @@ def test_cache_statistics_match_reference(strategy, bits):
         if bits is None:
             assert got["cache_memory_gb"] == pytest.approx(want["cache_memory_gb"], rel=1e-6)
         else:
-            # --cache_bits here keeps the packed codes AND the bf16 working copy the decode kernel streams (DESIGN.md
-            # section 7: the semantics of the quantised cache, not yet its footprint); the number reported is ours
+            # --cache_bits here keeps the packed codes AND the bf16 working copy the decode kernel streams (the
+            # semantics of the quantised cache, not yet its footprint); the number reported is ours
             assert got["cache_memory_gb"] >= want["cache_memory_gb"]

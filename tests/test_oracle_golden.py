@@ -1,7 +1,7 @@
 """Pins oracle/cc_oracle.c against traces recorded from the UNMODIFIED reference
 (tests/golden/make_golden.py).  CPU only.
 
-Bars (also quoted in DESIGN.md):
+Bars:
   * eviction slot indices, `pos`, `mask`, `cache_cts`, denominators: bit-exact on every step;
   * GQA-pooled probabilities (the values that feed the eviction scores): bitwise equal except
     for a <= 2e-4 fraction of elements that may be 1 bf16 ulp off (the reference's Sleef exp and
@@ -102,7 +102,7 @@ def test_exp_matches_libm_to_one_ulp():
 
 
 def test_oracle_reproduces_the_whole_model_eviction_trace():
-    """tests/golden/model_cfg1.npz (the reference's generate() on the 32-layer model): every layer's
+    """tests/golden/model_cfg1.npz (the reference's generate() on the 32-layer model, benchmark workload 1): every layer's
     recent_global cache starts from the compressed 128-token prompt (4 global tokens + the 60 most recent) and the
     oracle, stepped with arbitrary q / k / v, overwrites the slots the reference overwrote and ends with its `pos`."""
     from pathlib import Path

@@ -40,7 +40,7 @@ def test_blockwise_restatement_matches_reference(name):
 @pytest.mark.parametrize("name", [n for n in PREFILL_FIXTURES if "math" not in n and "short" not in n])
 def test_compressor_on_stats_matches_reference_keep_set(name):
     """Host logic: the SnapKV compressor fed with the two reductions picks the reference's tokens (up to ties
-    at the cut-off, SURVEY 8 appendix B) and seeds the same cumulative attention."""
+    at the cut-off) and seeds the same cumulative attention."""
     from cold_compress_b200.prompt_compression import PrefillAttnStats, get_prompt_compressor_constructor
     g = PrefillGolden(name)
     q, k, v = g.qkv()

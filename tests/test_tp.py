@@ -58,9 +58,9 @@ def test_tp_decode_world4(strategy):
 @pytest.mark.gpu
 @pytest.mark.parametrize("strategy", ["heavy_hitter", "recent_global"])
 def test_tp_decode_world8(strategy):
-    """Eight ranks, one KV head each (the BASELINE tensor-parallel layout of Llama-3-8B): the whole-token kernel's
+    """Eight ranks, one KV head each (the tensor-parallel layout of Llama-3-8B): the whole-token kernel's
     second round of partial-vector reads (ranks 4-7) and its 64-CTA-per-head attention stage.  Needs 8 GPUs; not run yet:
-    the tp8 bench line under profiles/r2/ is the only evidence at this world size."""
+    a recorded line of the benchmark with 8 ranks is the only evidence at this world size."""
     if torch.cuda.device_count() < 8:
         pytest.skip("needs 8 GPUs")
     r = _torchrun(8, strategy)

@@ -1,5 +1,5 @@
-"""BASELINE config 4's per-layer cache shape through the per-layer decode kernel (cc_decode_step), against the oracle.
-(The file sorts late on purpose: the driver runs the suite with -x.)"""
+"""The benchmark's hybrid workload's per-layer cache shape through the per-layer decode kernel (cc_decode_step), against the oracle.
+(The file sorts late on purpose: the suite is run with -x.)"""
 import numpy as np
 import pytest
 import torch
@@ -10,7 +10,7 @@ pytestmark = pytest.mark.gpu
 
 
 def test_hybrid_decode_at_the_baseline_config4_shape():
-    """BASELINE config 4's per-layer shape: Qwen2-7B grouping (Hkv = 4, G = 7, D = 128), 17408 slots per head (17
+    """The benchmark's hybrid workload's per-layer shape: Qwen2-7B grouping (Hkv = 4, G = 7, D = 128), 17408 slots per head (17
     chunks per CTA through the 4-stage shared-memory ring), the 400-entry bf16 history ring, per-head FastGen
     strategies of bench.py's config 4 (window | window + heavy hitter | full).  Synthetic state: head 0 (window) at
     its budget -> evicts from the first step; head 1 (window + heavy hitter) at its budget -> evicts by ring score;

@@ -1,4 +1,4 @@
-"""Whole-model parity against the unmodified reference: Llama-3-8B shape,
+"""Whole-model parity against the unmodified reference (the benchmark's workload 1): Llama-3-8B shape,
 32 layers, recent_global with 64 slots per layer, 128-token prompt, 16 generated tokens.  tests/golden/model_cfg1.npz
 was recorded from the reference's own generate() on CPU by tests/golden/make_golden_model.py; both sides build the
 same weights from tests/model_weights.py.  Checked on the GPU, through this package's prefill and the whole-token
@@ -11,7 +11,7 @@ legitimate flip):
     our arg-max must be one of the reference's top-64 tokens with a reference probability of at least 0.6 of the
     reference's maximum, and our probabilities of the reference's top-64 tokens must agree with the reference's to
     35 % (a dropped row, a wrong rotation or a wrong residual scrambles the top-64 set altogether).
-(The file sorts last on purpose: the driver runs the suite with -x.)"""
+(The file sorts last on purpose: the suite is run with -x.)"""
 from pathlib import Path
 
 import numpy as np

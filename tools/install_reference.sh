@@ -1,7 +1,6 @@
 #!/bin/bash
 # Installs the UNMODIFIED reference (AnswerDotAI/cold-compress, mounted read-only at /root/reference) into
-# baseline/_ref so that `bench.py --impl reference` can run its own CPU path on the GPU box (baseline/_ref is
-# git-ignored but travels with the gpurun snapshot).  The reference's setup.py calls find_packages() on a flat
+# baseline/_ref so that `bench.py --impl reference` can run its own CPU path (baseline/_ref is git-ignored).  The reference's setup.py calls find_packages() on a flat
 # directory of modules, so a plain `pip install` produces an empty wheel; the copy under /tmp gets a setup.py that
 # lists the top-level modules (py_modules) -- the .py files themselves are installed byte for byte.
 set -e
