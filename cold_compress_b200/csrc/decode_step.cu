@@ -673,7 +673,7 @@ cc_decode_kernel(const __grid_constant__ DecodeParams p) {
             mbar_wait(&vbar[stage], (j / NS) & 1);
             const int r_end = chunk_rows_valid(j);
             const uint8_t* vbase = vring + stage * chunk_bytes + lane * (CPL * 2);
-#pragma unroll (G >= 7 ? 1 : 2)
+#pragma unroll (G >= 7 ? 1 : 2)        // two at a time would spill with 64 sums in 128 registers
             for (int r = warp * RPW; r < r_end; r += kWarps * RPW) {
                 const int lr = (j << chs) + r;
                 uint32_t vv[RPW][CPL / 2];

@@ -1031,9 +1031,10 @@ __global__ void __launch_bounds__(VD_THREADS, RMAX <= 4 ? 2 : 1) attn_decode_row
 // that are zero) are formed again key by key with fp32 multiplications, where such operands give what they give.
 // The keys of a tile are waited for alone, its values land under the scores and the softmax.  The last CTA of a head asks for all
 // partial sums before it knows their weights, and stores the new row under them.
-// Bound: the chain of dependent waits (position 0.5 us, rows 3.6 = the HBM rate, partials and counter 1.3, combination 3) around
-// 3.3 us of work; 8 layers of 32 / 8 heads of 128, 4096 positions in a graph: 143 us on the kernel above, 109 here.  Against 64 bits
-// (fp32 results, scores of size 4): 2.1e-7 of the norm, 2.4e-7 above.
+// Bound: the chain of dependent waits.  Clock stamps after the wait, us: position known 0.5, keys there 4.9 (16.8 MB of rows, asked for
+// up to 4.1, at 0.6 of the HBM rate), scores 6.4, values 8.2, partials out 8.7, counter 9.5, weights of the splits 12.7, end 13.6.
+// 8 layers of 32 / 8 heads of 128, 4096 positions in a graph: 143 us on the kernel above, 109 here.  Against 64 bits (fp32 results,
+// scores of size 4): 2.1e-7 of the norm, 2.4e-7 above.
 constexpr int MD_THREADS = 256, MD_WARPS = MD_THREADS / 32, MD_AHEAD = 17, MD_KEYS = 128;      // MD_KEYS: keys of a tile
 
 __device__ __forceinline__ uint32_t smem_at(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }

@@ -10,9 +10,9 @@
 // its segment again with the bonus per row, so that infinities and NaN come out as they do token after token (the checks: 1 %).
 // Rows on other than 16-byte boundaries are staged 4 bytes at a time: the same sums, so the same bits.
 // One multiplication and addition per state element and token more than the plain recurrence, for segments times the parallelism:
-// 4096 tokens of 32 heads of 64 go from 405 us to 152 (60 + 7 + 96), of 4 heads from 387 to 37, of 64 heads of 128 from 1663 to 1190.
-// Now bound by the fp32 pipe (63 % busy in 3., 42 % in 1.; 9 warps of 168 registers an SM).  Against 64 bits the outputs are as
-// far off as token after token (1.31e-7 and 1.34e-7 of their norm), with other roundings.
+// Back to back in a graph, 4096 tokens of 32 heads of 64 go from 405 us to 155 (57 + 5 + 95 alone), of 4 heads from 387 to 38, of 64
+// heads of 128 from 1663 to 1198.  Now bound by the fp32 pipe (63 % busy in 3., 42 % in 1.; 9 warps of up to 168 registers an SM).
+// Against 64 bits the outputs are as far off as token after token (1.31e-7 and 1.34e-7 of their norm), with other roundings.
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
@@ -397,8 +397,10 @@ __global__ void __launch_bounds__(Dp, Dp == 64 ? 6 : 3) wkv_segment_scan_kernel(
 }
 
 // Segments: as many as give an SM six CTAs (what the scan's registers allow) over heads and column tiles, of at least 32 tokens.
-// 4096 tokens of 32 heads of 64 with 4 / 5 / 6 / 7 / 8: 204 / 177 / 152 / 162 / 153 us.  The three launches follow one another in
-// full: started under each other (programmatic launch) 256 tokens of 16 heads take 32 us instead of 20.
+// With 4 / 5 / 6 / 7 / 8, back to back in a graph: 4096 tokens of 32 heads of 64 166 / 178 / 155 / 166 / 149 us, 2000 of 16 heads 49 / 52
+// / 50 / 51 / 51, 4096 of 64 heads of 128 1157 / 1152 / 1198 / 1033 / 1026 (two waves of shorter segments balance better there; not
+// measured over the range, and more segments are more work for the launch between).  The three launches follow one another in full:
+// started under each other (programmatic launch) 256 tokens of 16 heads take 32 us instead of 20.
 constexpr int MIN_LEN = 32, CTAS = 6;
 static Segments plan(int T, int H, int D) {
     const long long per = (long long)H * ((D + TILE - 1) / TILE);

@@ -311,6 +311,9 @@ def head_gemv(w, x, sx, out, so, gate=None):
 
 
 def wkv(r, k, v, wraw, w0, u, state, o, H, D):
+    """The matrix-state recurrence over T tokens; `state` [H, D, D] moves on, o [T, H * D].  Calls of fewer than WKV_SEGMENTS_FROM
+    tokens, and of heads that the library does not cut into segments, go token after token: however a sequence is cut into such calls,
+    the bits are the same.  Longer calls add the same terms in another order and agree with them to rounding."""
     _need(*[(n, t, torch.float32) for n, t in (("r", r), ("k", k), ("v", v), ("wraw", wraw), ("w0", w0), ("u", u),
                                                ("state", state), ("o", o))])
     a = _lib.CcSeqWkv()
@@ -338,9 +341,9 @@ def wkv(r, k, v, wraw, w0, u, state, o, H, D):
 # it is no loss for any number of heads; fewer heads would gain from about 20 on.
 WKV_DECAY_FROM = 64
 
-# Tokens from which segments of a step go side by side, where the library serves the head size (other roundings than token after
-# token: steps below it give the same bits however they are cut).  Measured segments / one after another in us: 256 tokens of 1, 16, 32,
-# 128 heads of 64 20 / 28, 20 / 29, 21 / 29, 51 / 56, of 16 and 64 heads of 128 33 / 36 and 95 / 108; 192 tokens of 32 heads of 64 20 / 23.
+# Tokens from which segments of a step go side by side, where the library cuts heads of this size and number.  Measured segments / one
+# after another in us: 256 tokens of 1, 16, 32, 128 heads of 64 20 / 28, 20 / 29, 21 / 29, 51 / 56, of 16 and 64 heads of 128 33 / 36 and
+# 95 / 108; 192 tokens of 32 heads of 64 20 / 23.
 WKV_SEGMENTS_FROM = 256
 
 
