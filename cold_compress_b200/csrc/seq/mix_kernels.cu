@@ -1120,7 +1120,10 @@ constexpr int GEMV_CTAS = 4;       // CTAs per SM (64 registers per thread)
 // with eight loads across rows and launches under their predecessor, 312 with pairs and the small launches alike.  The way in of a
 // down product that formed act(gate) * up itself was 512 CTAs times 8192 units read 4 bytes at a time (2048 x 8192: 33 us, 13 with
 // the units on the way out of the product before, each formed once, and 16 bytes an access): 307 -> 273.
-template <typename WT, int PRE, int KS>
+// PAIR: 0 no job's rows are a gated unit's, 1 all jobs' are, 2 some are.  The choice is not left to the run: with a job's row rule
+// read from memory, or staging loops unrolled further, weight vectors under way are spilled and wait for one another (4096 x 14336
+// alone in a graph: 26 us, 41 so; as a unit 26, 41; 14336 x 4096 21 and 28).
+template <typename WT, int PRE, int KS, int PAIR>
 __global__ void __launch_bounds__(256, GEMV_CTAS) gemv_multi_kernel(const CcSeqGemvMulti g, int rows_per_cta) {
     extern __shared__ float4 smg4[];
     float* xs = reinterpret_cast<float*>(smg4);
@@ -1143,7 +1146,7 @@ __global__ void __launch_bounds__(256, GEMV_CTAS) gemv_multi_kernel(const CcSeqG
     const int nv = K / VEC, v0 = lane + 32 * ks;    // this lane's vectors of a row: v0, v0 + STEP, ...
     // rows past the end: the last one.  With a unit on the way out a warp's pair is a gate row and its up row.
     auto row = [&](int n, int r) {
-        const int m = jb.pair > 0 ? (min(n, jb.N - 2) >> 1) + r * jb.pair : min(n + r, jb.N - 1);
+        const int m = PAIR == 1 || (PAIR == 2 && jb.pair > 0) ? (min(n, jb.N - 2) + r * jb.N) >> 1 : min(n + r, jb.N - 1);
         return reinterpret_cast<const uint4*>(W + (size_t)m * K);
     };
     if (vec && lane % 8 == 0) {      // a line of 128 bytes per request
@@ -1175,7 +1178,7 @@ __global__ void __launch_bounds__(256, GEMV_CTAS) gemv_multi_kernel(const CcSeqG
         const float* up = (const float*)jb.x + jb.off_up;
         const bool two = jb.off_up >= 0;
         if (K % 4 == 0 && (((uintptr_t)src | (two ? (uintptr_t)up : 0)) & 15) == 0) {
-#pragma unroll 4
+#pragma unroll 2
             for (int k = 4 * tid; k < K; k += 1024) {
                 const float4 a = *reinterpret_cast<const float4*>(src + k);
                 float4 u = make_float4(1.f, 1.f, 1.f, 1.f);
@@ -1195,7 +1198,7 @@ __global__ void __launch_bounds__(256, GEMV_CTAS) gemv_multi_kernel(const CcSeqG
     } else if (jb.x_dtype == CC_DT_F32) {
         const float* src = (const float*)jb.x;
         if (K % 4 == 0 && ((uintptr_t)src & 15) == 0) {
-#pragma unroll 8
+#pragma unroll 2
             for (int k = 4 * tid; k < K; k += 1024) {
                 const float4 v = *reinterpret_cast<const float4*>(src + k);
                 *reinterpret_cast<float4*>(xs + k) = make_float4(round_to(v.x, W), round_to(v.y, W), round_to(v.z, W), round_to(v.w, W));
@@ -1207,7 +1210,7 @@ __global__ void __launch_bounds__(256, GEMV_CTAS) gemv_multi_kernel(const CcSeqG
     } else {
         const bf16* src = (const bf16*)jb.x;
         if (K % 8 == 0 && ((uintptr_t)src & 15) == 0) {
-#pragma unroll 4
+#pragma unroll 1
             for (int k = 8 * tid; k < K; k += 2048) {
                 const uint4 v = *reinterpret_cast<const uint4*>(src + k);
                 const uint32_t e[4] = {v.x, v.y, v.z, v.w};
@@ -1280,7 +1283,7 @@ __global__ void __launch_bounds__(256, GEMV_CTAS) gemv_multi_kernel(const CcSeqG
             for (int q = 1; q < KS; ++q) sum += red[(warp + q) * GEMV_ROWS + lane % GEMV_ROWS];
         }
         const int m = n + lane;
-        if (jb.pair > 0) {
+        if (PAIR == 1 || (PAIR == 2 && jb.pair > 0)) {
             const float up = __shfl_sync(0xffffffffu, sum, 1);
             if (lane == 0 && n < n_end) stf((WT*)jb.out, n >> 1, unit_act(sum, jb.pair_act) * up);
         } else if (lane < GEMV_ROWS && m < n_end) {
@@ -1600,7 +1603,7 @@ int cc_seq_latent_decode(const CcSeqLatentDecode* a, void* stream) {
 int cc_seq_gemv_multi(const CcSeqGemvMulti* g, void* stream) {
     if (!g || g->n_jobs < 1 || g->n_jobs > CC_GEMV_MAX_JOBS) return fail(CC_SEQ_ERR_INVALID_ARG, "gemv_multi: bad job count");
     const CcSeqGemvPre& p = g->pre;
-    int kmax = 0;
+    int kmax = 0, paired = 0;
     for (int j = 0; j < g->n_jobs; ++j) {
         const CcSeqGemvJob& b = g->job[j];
         if (!b.W || (!b.out && !(j == 0 && g->post.x)) || b.N < 1 || b.K < 1 || b.kind < CC_ACT_NONE || b.kind > CC_ACT_LAST ||
@@ -1621,6 +1624,7 @@ int cc_seq_gemv_multi(const CcSeqGemvMulti* g, void* stream) {
                 return fail(CC_SEQ_ERR_INVALID_ARG, "gemv_multi: bad shared input row");
         }
         kmax = b.K > kmax ? b.K : kmax;
+        paired += b.pair > 0;
     }
     const CcSeqBoundedSum& q = g->post;
     if (q.x && (!q.out_norm.w || !q.out_norm.b || !q.out_norm.alpha || (!q.x_out && !q.h) ||
@@ -1633,9 +1637,9 @@ int cc_seq_gemv_multi(const CcSeqGemvMulti* g, void* stream) {
     const GemvSplit split = gemv_split(g, smem, g->w_dtype == CC_DT_BF16 ? 2 : 4);
     int blocks = 0;
     for (int j = 0; j < g->n_jobs; ++j) blocks += (g->job[j].N + split.rows_per_cta - 1) / split.rows_per_cta;
-#define CALL2(ST, PRE, KS)                                                                                         \
+#define CALL3(ST, PRE, KS, PAIR)                                                                                   \
     {                                                                                                              \
-        auto kern = gemv_multi_kernel<ST, PRE, KS>;                                                                \
+        auto kern = gemv_multi_kernel<ST, PRE, KS, PAIR>;                                                          \
         static size_t configured = 48 * 1024;                                                                      \
         if (smem > configured) {                                                                                   \
             configured = smem;                                                                                     \
@@ -1643,6 +1647,12 @@ int cc_seq_gemv_multi(const CcSeqGemvMulti* g, void* stream) {
                 return cuda_check("gemv_multi: shared memory");                                                    \
         }                                                                                                          \
         ccs::launch_under(kern, dim3(blocks), dim3(256), smem, st, *g, split.rows_per_cta);                        \
+    }
+#define CALL2(ST, PRE, KS)                                                                                         \
+    {                                                                                                              \
+        if (paired == 0) CALL3(ST, PRE, KS, 0)                                                                     \
+        else if (PRE == CC_GEMV_PRE_NONE && paired == g->n_jobs) CALL3(ST, CC_GEMV_PRE_NONE, KS, 1)                \
+        else CALL3(ST, PRE, KS, 2)                                                                                 \
     }
 #define CALL1(ST, PRE)                                  \
     {                                                   \
@@ -1661,6 +1671,7 @@ int cc_seq_gemv_multi(const CcSeqGemvMulti* g, void* stream) {
 #undef CALL
 #undef CALL1
 #undef CALL2
+#undef CALL3
     return cuda_check("gemv_multi_kernel");
 }
 
