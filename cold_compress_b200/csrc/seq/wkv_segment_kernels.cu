@@ -6,12 +6,13 @@
 //      at a time.  No decay is ever divided by: every factor is a product of numbers in (0, 1];
 //   2. the states at the segments' starts, one after another over the segments and beside each other over the elements;
 //   3. the recurrence inside every segment from its own start.
-// Where a start or a sum is not finite, 2. goes token after token (a product of decays may underflow where no decay is zero) and 3. walks
-// its segment again with the bonus per row, so that infinities and NaN come out as they do token after token (the checks: 1 %).
+// Where a start is not finite, 2. looks at the tokens (a product of decays may underflow where no decay is zero), and where a sum is not,
+// 3. walks its segment again with the bonus per row, so that infinities and NaN come out as they do token after token (4096 tokens of
+// 32 heads of 64 with keys that are all NaN: 330 us).
 // Rows on other than 16-byte boundaries are staged 4 bytes at a time: the same sums, so the same bits.
 // One multiplication and addition per state element and token more than the plain recurrence, for segments times the parallelism:
-// Back to back in a graph, 4096 tokens of 32 heads of 64 go from 405 us to 155 (57 + 5 + 95 alone), of 4 heads from 387 to 38, of 64
-// heads of 128 from 1663 to 1198.  Now bound by the fp32 pipe (63 % busy in 3., 42 % in 1.; 9 warps of up to 168 registers an SM).
+// Back to back in a graph, 4096 tokens of 32 heads of 64 go from 405 us to 152 (57 + 6 + 92 alone), of 4 heads from 387 to 38, of 64
+// heads of 128 from 1663 to 1215.  Now bound by the fp32 pipe (63 % busy in 3., 42 % in 1.; 9 warps of up to 168 registers an SM).
 // Against 64 bits the outputs are as far off as token after token (1.31e-7 and 1.34e-7 of their norm), with other roundings.
 #include <cuda_runtime.h>
 #include <math.h>
@@ -189,18 +190,34 @@ __global__ void __launch_bounds__(STATE_THREADS, 8) wkv_segment_state_kernel(con
     }
 }
 
-// The states at the segments' starts for four elements, through the tokens one after another.
-__device__ __forceinline__ void again_one_by_one(const CcSeqWkv& a, const Segments& g, size_t e, size_t n4, size_t hi, float4 x) {
-    const size_t HD = (size_t)a.H * a.D, col = hi / a.D * a.D + e * 4 % a.D;
-    const int last = (g.n - 1) * g.len;
-#pragma unroll 4
-    for (int t = 0; t < last; ++t) {
-        const size_t row = (size_t)t * HD;
-        const float w = g.w[row + hi], k = a.k[row + hi];
-        const float* v = a.v + row + col;
-        x = make_float4(fmaf(w, x.x, k * v[0]), fmaf(w, x.y, k * v[1]), fmaf(w, x.z, k * v[2]), fmaf(w, x.w, k * v[3]));
-        if ((t + 1) % g.len == 0) reinterpret_cast<float4*>(g.X)[(size_t)((t + 1) / g.len) * n4 + e] = x;
+__device__ __forceinline__ bool finite(float x) { return fabsf(x) <= 3.402823466e38f; }
+__device__ __forceinline__ bool finite(const float4& x) { return finite(x.x) && finite(x.y) && finite(x.z) && finite(x.w); }
+__device__ __forceinline__ bool none_left(const float4& x) { return x.x != x.x && x.y != x.y && x.z != x.z && x.w != x.w; }
+__device__ __forceinline__ float4 fma4(float p, const float4& x, const float4& y) {
+    return make_float4(fmaf(p, x.x, y.x), fmaf(p, x.y, y.y), fmaf(p, x.z, y.z), fmaf(p, x.w, y.w));
+}
+// Four elements of a state row through segment s, where that meets numbers that are not finite: NaN stay, a sum that is not finite is
+// formed again token after token, and an infinite element stays through decays whose product underflows if none of them is zero.
+__device__ __forceinline__ float4 through_segment(const CcSeqWkv& a, const Segments& g, int s, size_t hi, size_t col, float4 x, const float4& add) {
+    if (none_left(x)) return x;
+    const size_t HD = (size_t)a.H * a.D, at = (size_t)s * g.len * HD;
+    if (!finite(add)) {
+#pragma unroll 8
+        for (int t = 0; t < g.len; ++t) {
+            const size_t row = at + (size_t)t * HD;
+            const float* v = a.v + row + col;
+            const float k = a.k[row + hi];
+            x = fma4(g.w[row + hi], x, make_float4(k * v[0], k * v[1], k * v[2], k * v[3]));
+        }
+        return x;
     }
+    const float p = g.P[(size_t)s * HD + hi];
+    if (p != 0.f || finite(x)) return fma4(p, x, add);
+    float least = 1.f;
+#pragma unroll 16
+    for (int t = 0; t < g.len; ++t) least = fminf(least, g.w[at + (size_t)t * HD + hi]);
+    if (least == 0.f) return fma4(p, x, add);
+    return make_float4(finite(x.x) ? add.x : x.x, finite(x.y) ? add.y : x.y, finite(x.z) ? add.z : x.z, finite(x.w) ? add.w : x.w);
 }
 
 // State at every segment's start, thread = four elements of a state row; the loads of sixteen segments are under way together.
@@ -208,15 +225,13 @@ __global__ void __launch_bounds__(128) wkv_segment_starts_kernel(const CcSeqWkv 
     const size_t n4 = (size_t)a.H * a.D * a.D / 4, e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= n4) return;
     const size_t hi = e * 4 / a.D;      // head and row
-    auto begin = [&] {
-        if (((uintptr_t)a.state & 15) == 0) return reinterpret_cast<const float4*>(a.state)[e];
-        return make_float4(a.state[4 * e], a.state[4 * e + 1], a.state[4 * e + 2], a.state[4 * e + 3]);
-    };
-    float4 x = begin();
+    float4 x;
+    if (((uintptr_t)a.state & 15) == 0) x = reinterpret_cast<const float4*>(a.state)[e];
+    else x = make_float4(a.state[4 * e], a.state[4 * e + 1], a.state[4 * e + 2], a.state[4 * e + 3]);
     float4* X = reinterpret_cast<float4*>(g.X);
     X[e] = x;
     for (int s0 = 0; s0 + 1 < g.n; s0 += 16) {
-        float4 add[16];
+        float4 add[16], from = x;
         float p[16];
 #pragma unroll
         for (int q = 0; q < 16; ++q)
@@ -226,20 +241,90 @@ __global__ void __launch_bounds__(128) wkv_segment_starts_kernel(const CcSeqWkv 
             }
 #pragma unroll
         for (int q = 0; q < 16; ++q)
-            if (s0 + q + 1 < g.n) {
-                x = make_float4(fmaf(p[q], x.x, add[q].x), fmaf(p[q], x.y, add[q].y), fmaf(p[q], x.z, add[q].z), fmaf(p[q], x.w, add[q].w));
-                X[(size_t)(s0 + q + 1) * n4 + e] = x;
+            if (s0 + q + 1 < g.n) add[q] = x = fma4(p[q], x, add[q]);
+        if (finite(x)) {      // what is not finite stays so: then all of them were
+#pragma unroll
+            for (int q = 0; q < 16; ++q)
+                if (s0 + q + 1 < g.n) X[(size_t)(s0 + q + 1) * n4 + e] = add[q];
+        } else {
+            x = from;
+#pragma unroll 1
+            for (int s = s0; s < s0 + 16 && s + 1 < g.n; ++s) {
+                float4* const at = X + (size_t)(s + 1) * n4 + e;
+                *at = x = through_segment(a, g, s, hi, hi / a.D * a.D + e * 4 % a.D, x, *at);
             }
+        }
     }
-    // what is not finite stays so: all of it again, token after token
-    if (!(fabsf(x.x) + fabsf(x.y) + fabsf(x.z) + fabsf(x.w) < INFINITY)) again_one_by_one(a, g, e, n4, hi, begin());
+}
+
+// A segment whose sums are not all finite, with the bonus meeting the value row by row: the outputs again, the state is the same.  Only
+// the order of loading is simpler than below: one batch of tokens at a time.
+template <int Dp>
+__device__ __forceinline__ void wkv_segment_again(const CcSeqWkv& a, const Segments& g, float* sm) {
+    constexpr int THREADS = Dp, P = Dp / 16, ROWS = TB * Dp;
+    const int tid = threadIdx.x, s = blockIdx.x, h = blockIdx.y, j0 = blockIdx.z * TILE, p = tid % P, cg = tid / P, j = j0 + 4 * cg;
+    const size_t HD = (size_t)a.H * a.D;
+    const int first = s * g.len, count = min(g.len, a.T - first);
+    const float* X = g.X + ((size_t)s * a.H + h) * a.D * a.D;
+    float st[16][4];
+    float* const us = sm + 3 * ROWS + TB * TILE;      // in the place of the second buffer
+    for (int i = tid; i < Dp; i += THREADS) us[i] = i < a.D ? a.u[(size_t)h * a.D + i] : 0.f;
+#pragma unroll
+    for (int r = 0; r < 16; ++r) {
+        const int i = 4 * P * (r / 4) + 4 * p + r % 4;
+        const bool in = i < a.D;
+        float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (in && j < a.D) x = *reinterpret_cast<const float4*>(X + (size_t)i * a.D + j);
+        st[r][0] = x.x; st[r][1] = x.y; st[r][2] = x.z; st[r][3] = x.w;
+    }
+    for (int t0 = 0; t0 < count; t0 += TB) {
+        const int nt = min(TB, count - t0);
+        const size_t at = (size_t)(first + t0) * HD + (size_t)h * a.D;
+        for (int n = tid; n < TB * Dp; n += THREADS) {
+            const int t = n / Dp, x = n % Dp;
+            const bool in = t < nt && x < a.D;
+            const size_t src = at + (in ? (size_t)t * HD + x : 0);
+            sm[n] = in ? a.r[src] : 0.f;
+            sm[ROWS + n] = in ? a.k[src] : 0.f;
+            sm[2 * ROWS + n] = in ? g.w[src] : 0.f;
+        }
+        for (int n = tid; n < TB * TILE; n += THREADS) {
+            const int t = n / TILE, x = n % TILE;
+            sm[3 * ROWS + n] = t < nt && j0 + x < a.D ? a.v[at + (size_t)t * HD + j0 + x] : 0.f;
+        }
+        __syncthreads();
+#pragma unroll 1
+        for (int t = 0; t < nt; ++t) {
+            const float* const row = sm + t * Dp;
+            const float4 v = reinterpret_cast<const float4*>(sm + 3 * ROWS + t * TILE)[cg];
+            float o[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+            for (int r = 0; r < 16; ++r) {
+                const int i = 4 * P * (r / 4) + 4 * p + r % 4;
+                const float rv = row[i], k = row[ROWS + i], w = row[2 * ROWS + i], kv[4] = {k * v.x, k * v.y, k * v.z, k * v.w};
+#pragma unroll
+                for (int x = 0; x < 4; ++x) {
+                    o[x] = fmaf(rv, fmaf(us[i], kv[x], st[r][x]), o[x]);
+                    st[r][x] = fmaf(w, st[r][x], kv[x]);
+                }
+            }
+#pragma unroll
+            for (int x = 0; x < 4; ++x) {
+#pragma unroll
+                for (int d = 1; d < P; d <<= 1) o[x] += __shfl_xor_sync(0xffffffffu, o[x], d);
+                if (p == x && j < a.D) a.o[at + (size_t)t * HD + j + x] = o[x];
+            }
+        }
+        __syncthreads();
+    }
 }
 
 // The recurrence inside a segment, 64 columns of a head.  Thread = 16 rows x 4 columns: lane % P holds rows 4 P q + 4 p .. + 3 of
 // P = Dp / 16 row groups, the rest of the thread number the columns.  A token's operands are 13 16-byte reads of shared memory for
 // 124 pairs of fp32 operations; the row groups of a column meet by shuffles, so that tokens need no barrier.
+// (168 registers, six CTAs an SM of 64 threads; asked for that many CTAs the compiler schedules the walk 3 us slower.)
 template <int Dp, bool VEC>
-__global__ void __launch_bounds__(Dp, Dp == 64 ? 6 : 3) wkv_segment_scan_kernel(const CcSeqWkv a, const Segments g) {
+__global__ void __launch_bounds__(Dp) wkv_segment_scan_kernel(const CcSeqWkv a, const Segments g) {
     extern __shared__ float4 smw4[];
     float* const sm = reinterpret_cast<float*>(smw4);
     constexpr int THREADS = Dp, P = Dp / 16, ROWS = TB * Dp, BUF = 3 * ROWS + TB * TILE;
@@ -342,41 +427,9 @@ __global__ void __launch_bounds__(Dp, Dp == 64 ? 6 : 3) wkv_segment_scan_kernel(
         }
         __syncthreads();
     }
-    const size_t at = (size_t)first * HD + (size_t)h * a.D;
-    const bool again = __syncthreads_or(none != none);
-    if (again) {
-        // the segment again from memory, with the bonus per row; the state stands in X, where nobody else reads this tile
-        float* const mine = g.X + ((size_t)s * a.H + h) * a.D * a.D + j;
-#pragma unroll 1
-        for (int t = 0; t < count; ++t) {
-            const size_t row = at + (size_t)t * HD;
-            float sum[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 4
-            for (int r = 0; r < 16; ++r) {
-                const int i = 4 * P * (r / 4) + 4 * p + r % 4;
-                if (i >= a.D || j >= a.D) continue;
-                const float rv = a.r[row + i], k = a.k[row + i], w = g.w[row + i], u = a.u[(size_t)h * a.D + i];
-                float4* const x4 = reinterpret_cast<float4*>(mine + (size_t)i * a.D);
-                const float4 x = *x4;
-                const float kv[4] = {k * a.v[row + j], k * a.v[row + j + 1], k * a.v[row + j + 2], k * a.v[row + j + 3]};
-                sum[0] = fmaf(rv, fmaf(u, kv[0], x.x), sum[0]);
-                sum[1] = fmaf(rv, fmaf(u, kv[1], x.y), sum[1]);
-                sum[2] = fmaf(rv, fmaf(u, kv[2], x.z), sum[2]);
-                sum[3] = fmaf(rv, fmaf(u, kv[3], x.w), sum[3]);
-                *x4 = make_float4(fmaf(w, x.x, kv[0]), fmaf(w, x.y, kv[1]), fmaf(w, x.z, kv[2]), fmaf(w, x.w, kv[3]));
-            }
-#pragma unroll
-            for (int x = 0; x < 4; ++x) {
-#pragma unroll
-                for (int d = 1; d < P; d <<= 1) sum[x] += __shfl_xor_sync(0xffffffffu, sum[x], d);
-                if (p == x && j < a.D) a.o[row + j + x] = sum[x];
-            }
-        }
-    }
-    if (s + 1 < g.n) return;
     float* const S = a.state + (size_t)h * a.D * a.D;
 #pragma unroll
-    for (int r = 0; r < 8; ++r) {
+    for (int r = 0; r < 8 && s + 1 == g.n; ++r) {
         const int i = 4 * P * (r / 2) + 4 * p + 2 * (r % 2);
         if (i >= a.D || j >= a.D) continue;
         float lo[4], hi[4];
@@ -394,6 +447,7 @@ __global__ void __launch_bounds__(Dp, Dp == 64 ? 6 : 3) wkv_segment_scan_kernel(
             }
         }
     }
+    if (__syncthreads_or(none != none)) wkv_segment_again<Dp>(a, g, sm);
 }
 
 // Segments: as many as give an SM six CTAs (what the scan's registers allow) over heads and column tiles, of at least 32 tokens.
