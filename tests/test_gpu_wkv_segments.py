@@ -46,7 +46,7 @@ def test_what_is_not_served_goes_token_after_token():
     from cold_compress_b200 import _lib, seq_ops
     lib = _lib.load_seq()
     assert [lib.cc_seq_wkv_segments_workspace(*s) for s in ((400, 2, 33), (400, 2, 132), (32, 2, 64), (400, 900, 64))] == [0] * 4
-    T, H, D = 400, 2, 64
+    T, H, D = 400, 2, 33                                     # not a multiple of 4: never cut
     gen = torch.Generator(device="cuda").manual_seed(1)
     rows = [torch.randn(T * H * D + 1, device="cuda", generator=gen) for _ in range(4)]
     base, u = torch.randn(H * D, device="cuda", generator=gen) - 2, torch.randn(H * D, device="cuda", generator=gen)
@@ -58,7 +58,7 @@ def test_what_is_not_served_goes_token_after_token():
         return o, state
 
     for a, b in zip(run(True), run(False)):
-        assert ((a - b).norm() / b.norm()).item() <= 2e-6
+        assert torch.equal(a, b)
     w = _lib.CcSeqWkv()
     assert lib.cc_seq_wkv_segments(w, None, 0, None) < 0 and b"wkv_segments" in lib.cc_seq_last_error()
 
