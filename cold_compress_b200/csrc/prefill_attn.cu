@@ -14,12 +14,12 @@
 // stacked into the M = 128 rows of the MMA (row = g * QB + i), so a K/V tile is read once per group.
 // Two sweeps over the key tiles (BN = 128 keys):
 //   sweep 1  S = Q K^T (tcgen05.mma, fp32 in TMEM) -> row max and sum of exp      (softmax statistics)
-//   sweep 2  S again -> P = bf16(exp(l - max) / sum), rounded where the reference rounds -> shared memory
-//            -> Y += P V (tcgen05.mma); the same P tile is read column-wise for the pooled reductions.
+//   sweep 2  S again -> P = bf16(exp(l - max) / sum), rounded where the reference rounds -> tensor memory
+//            -> Y += P V (tcgen05.mma); the same P, added up over the heads of a query, goes into the pooled reductions.
 // The reference's rounding points are kept (NAIVE: bf16 after q.k, after *scale, after softmax, after the
 // GQA mean; MATH: fp32 logits, one rounding of P for the tensor core).
-// Operands are staged by TMA (cp.async.bulk.tensor, 128-byte swizzle) into a double-buffered ring; the S
-// accumulator is double-buffered in TMEM so the next tile's Q K^T runs under the current tile's softmax.
+// K and V are staged by TMA (cp.async.bulk.tensor, 128-byte swizzle) through a ring of tiles; the logits of the next tiles are formed
+// under the current tile's softmax.
 // Per-tile partial column sums go to a scratch buffer and are added in a fixed order by a second small
 // kernel: results are bit-reproducible run to run (no floating-point atomics).
 #include <cuda.h>
@@ -29,6 +29,8 @@
 #include <stdio.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 #include "common.cuh"
 #include "internal.h"
 
@@ -36,12 +38,12 @@ namespace cc {
 namespace {
 
 constexpr int BM = 128;                 // MMA rows of a query tile (G * QB, padded)
-constexpr int BN = 128;                 // keys per tile visit of a CTA ...
-constexpr int BNH = 64;                 // ... split between the two key-half groups of 8 warps
+constexpr int BN = 128;                 // keys of a tile
 constexpr int ATOM_BYTES = 128 * 128;   // one 128-byte-swizzled sub-tile: 128 rows x 64 bf16
-constexpr int NTHREADS = 512;          // 16 warps: warp w owns TMEM lane quarter w % 4 and column quarter w / 4
+constexpr int SOFT_WARPS = 16, NTHREADS = 32 * SOFT_WARPS + 128;   // + a warp each for MMAs and loads, two for column sums
 constexpr int MAX_WINDOWS = 4;
-constexpr int TMEM_COLS = 512;          // group g: S[b] at 128 g + 64 b, Y at 256 + 128 g
+constexpr int TMEM_COLS = 512;
+constexpr uint32_t WAIT_LIMIT = 1u << 22;
 constexpr int RED_THREADS = 64, RED_AHEAD = 16;   // the reduction: columns of a CTA, loads under way per column
 constexpr float LOG2E = 1.4426950408889634f;
 
@@ -72,16 +74,25 @@ __device__ __forceinline__ void mbar_init_u32(uint32_t bar, uint32_t count) {
 __device__ __forceinline__ void mbar_expect_tx_u32(uint32_t bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(bar), "r"(bytes) : "memory");
 }
-__device__ __forceinline__ void mbar_wait_u32(uint32_t bar, uint32_t parity) {
+__device__ __forceinline__ void mbar_arrive_u32(uint32_t bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(bar) : "memory");
+}
+__device__ __forceinline__ bool mbar_try_u32(uint32_t bar, uint32_t parity) {
+    uint32_t done;
     asm volatile(
-        "{\n"
-        ".reg .pred p;\n"
-        "WAIT_%=:\n"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%0], %1;\n"
-        "@p bra DONE_%=;\n"
-        "bra WAIT_%=;\n"
-        "DONE_%=:\n"
-        "}\n" :: "r"(bar), "r"(parity) : "memory");
+        "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
+        : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+    return done != 0;
+}
+// Bounded: a wait that runs out raises `failed`; every later wait of the CTA then gives up at once, the kernel runs to its
+// end and stores NaN.
+__device__ __forceinline__ void mbar_wait_u32(uint32_t bar, uint32_t parity, volatile int* failed) {
+    if (mbar_try_u32(bar, parity)) return;
+    for (uint32_t n = 0; !mbar_try_u32(bar, parity); ++n)
+        if (n >= WAIT_LIMIT || *failed) { *failed = 1; return; }
+}
+__device__ __forceinline__ void mbar_wait_out(uint32_t bar, uint32_t parity) {
+    for (uint32_t n = 0; n < WAIT_LIMIT && !mbar_try_u32(bar, parity); ++n) {}
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
@@ -96,30 +107,82 @@ __host__ __device__ constexpr uint32_t make_idesc(int M, int N, bool b_mn_major)
     return (1u << 4) | (1u << 7) | (1u << 10) | ((b_mn_major ? 1u : 0u) << 16) | ((uint32_t)(N >> 3) << 17) |
            ((uint32_t)(M >> 4) << 24);
 }
-__device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                          uint32_t accumulate) {
+// One lane of a whole warp.  What issues MMAs is a warp in step: its operands then lie in uniform registers, where the instruction
+// wants them.  One thread on its own took 70 to 110 cycles for an MMA that the pipe does in 64.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t one;
+    asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(one));
+    return one != 0;
+}
+// A in tensor memory, B in shared memory
+__device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
         "{\n"
         ".reg .pred p;\n"
         "setp.ne.b32 p, %4, 0;\n"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
-        "}\n" :: "r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n"
+        "}\n" :: "r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
 }
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(bar) : "memory");
 }
-// 32 lanes x 32 consecutive fp32 columns of this warp's TMEM lane quarter -> registers (and wait)
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
+// 32 lanes x 32 consecutive fp32 columns of this warp's TMEM lane quarter -> registers; the caller waits with tmem_wait_ld
+__device__ __forceinline__ void tmem_ld_row(uint32_t taddr, uint32_t (&v)[32]) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
         "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
         "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];\n"
-        "tcgen05.wait::ld.sync.aligned;\n"
         : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
           "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]),
           "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]),
           "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
         : "r"(taddr) : "memory");
+}
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+// The warp's 32 lanes x 32 fp32 columns, four rows of eight values per thread; the caller waits with tmem_wait_ld: v[16 h + 4 k + 2 j + e] = lane
+// 16 h + 8 j + thread / 4, column 8 k + 2 (thread % 4) + e
+__device__ __forceinline__ void tmem_ld_4rows(uint32_t taddr, uint32_t (&v)[32]) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        uint32_t* const r = v + 16 * h;
+        asm volatile(
+            "tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n"
+            : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+              "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+            : "r"(taddr + ((uint32_t)(16 * h) << 16)) : "memory");
+    }
+}
+// The loads' values go through the wait, so that nothing reads one before it (an asm takes 30 operands at most).
+__device__ __forceinline__ void tmem_wait_ld(uint32_t (&v)[32]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+        : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]), "+r"(v[8]), "+r"(v[9]),
+          "+r"(v[10]), "+r"(v[11]), "+r"(v[12]), "+r"(v[13]), "+r"(v[14]) :: "memory");
+    asm volatile(""
+        : "+r"(v[15]), "+r"(v[16]), "+r"(v[17]), "+r"(v[18]), "+r"(v[19]), "+r"(v[20]), "+r"(v[21]), "+r"(v[22]), "+r"(v[23]), "+r"(v[24]),
+          "+r"(v[25]), "+r"(v[26]), "+r"(v[27]), "+r"(v[28]), "+r"(v[29]) :: "memory");
+    asm volatile("" : "+r"(v[30]), "+r"(v[31]) :: "memory");
+}
+// ... and their bf16 pairs into the first 16 columns: x[j][k] = lane 8 j + thread / 4, column 4 k + thread % 4
+__device__ __forceinline__ void tmem_st_4rows(uint32_t taddr, const uint32_t (&x)[4][4]) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+        asm volatile(
+            "tcgen05.st.sync.aligned.16x128b.x4.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};\n"
+            :: "r"(taddr + ((uint32_t)(16 * h) << 16)), "r"(x[2 * h][0]), "r"(x[2 * h + 1][0]), "r"(x[2 * h][1]), "r"(x[2 * h + 1][1]),
+               "r"(x[2 * h][2]), "r"(x[2 * h + 1][2]), "r"(x[2 * h][3]), "r"(x[2 * h + 1][3]) : "memory");
+}
+// one row per thread, N columns
+template <int N>
+__device__ __forceinline__ void tmem_st_row(uint32_t taddr, const uint32_t (&x)[N]) {
+    static_assert(N == 8 || N == 16, "");
+    if constexpr (N == 16)
+        asm volatile(
+            "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};\n"
+            :: "r"(taddr), "r"(x[0]), "r"(x[1]), "r"(x[2]), "r"(x[3]), "r"(x[4]), "r"(x[5]), "r"(x[6]), "r"(x[7]), "r"(x[8]), "r"(x[9]),
+               "r"(x[10]), "r"(x[11]), "r"(x[12]), "r"(x[13]), "r"(x[14]), "r"(x[15]) : "memory");
+    else
+        asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};\n"
+            :: "r"(taddr), "r"(x[0]), "r"(x[1]), "r"(x[2]), "r"(x[3]), "r"(x[4]), "r"(x[5]), "r"(x[6]), "r"(x[7]) : "memory");
 }
 __device__ __forceinline__ float ex2(float x) {
     float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y;
@@ -127,10 +190,6 @@ __device__ __forceinline__ float ex2(float x) {
 // two fp32 -> packed bf16x2 (round to nearest even), and back
 __device__ __forceinline__ uint32_t cvt_bf16x2(float lo, float hi) {
     uint32_t d; asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(hi), "f"(lo)); return d;
-}
-// fp32 value of bf16(x): the high half of the packed pair {x, 0}
-__device__ __forceinline__ float round_bf16(float x) {
-    uint32_t d; asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(x), "f"(0.0f)); return __uint_as_float(d);
 }
 // pairs of fp32 values: one instruction for two operations, each rounded as the scalar one
 typedef unsigned long long f32x2;
@@ -148,414 +207,559 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
     return *reinterpret_cast<uint32_t*>(&p);
 }
 
-// Sum v[0..7] over the 32 lanes of a warp; every lane returns the total of column
-// 4 * bit4(lane) + 2 * bit3(lane) + bit2(lane)  (transpose-reduce: 4 + 2 + 1 + 1 + 1 shuffles).
-__device__ __forceinline__ float warp_reduce8(const float (&v)[8], int lane) {
-    const bool b4 = lane & 16, b3 = lane & 8, b2 = lane & 4;
-    float w[4], x[2];
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-        const float keep = b4 ? v[c + 4] : v[c], send = b4 ? v[c] : v[c + 4];
-        w[c] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
-    }
-#pragma unroll
-    for (int c = 0; c < 2; ++c) {
-        const float keep = b3 ? w[c + 2] : w[c], send = b3 ? w[c] : w[c + 2];
-        x[c] = keep + __shfl_xor_sync(0xffffffffu, send, 8);
-    }
-    float y = (b2 ? x[1] : x[0]) + __shfl_xor_sync(0xffffffffu, b2 ? x[0] : x[1], 4);
-    y += __shfl_xor_sync(0xffffffffu, y, 2);
-    y += __shfl_xor_sync(0xffffffffu, y, 1);
-    return y;
+// Packed bf16 operations, each result rounded once to nearest even.
+__device__ __forceinline__ uint32_t mul_bf16x2(uint32_t a, uint32_t b) { uint32_t d; asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b)); return d; }
+__device__ __forceinline__ uint32_t fma_bf16x2(uint32_t a, uint32_t b, uint32_t c) {
+    uint32_t d; asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c)); return d;
 }
-__device__ __forceinline__ int warp_reduce8_column(int lane) { return ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1); }
+__device__ __forceinline__ uint32_t max_bf16x2(uint32_t a, uint32_t b) { uint32_t d; asm("max.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b)); return d; }
 
-// Reductions of the GQA-pooled probabilities of one P tile (128 rows = (head g, query i) x 64 keys, bf16, the
-// swizzled A-operand layout in shared memory).  Warp `ck` (0..7) owns the 8 key columns of 16-byte chunk ck; lane l reads
-// rows l, l + 32, l + 64, l + 96 (one LDS.128 each), pools over the heads (model.py:413-418), and the warp adds the
-// pooled values over the query rows.  QBL = log2(query rows per tile); row = g * QB + i.
-template <int QBL>
-__device__ __forceinline__ void tile_stats(const uint8_t* sP_ptr, float* out_col, float* out_obs, float* out_band, size_t band_stride,
-                                           const PrefillParams& p, int ck, int lane, int i0, int jbase, bool want_obs) {
-    constexpr int QB = 1 << QBL;
-    constexpr int NI = QB >= 32 ? QB / 32 : 1;   // query rows held by one lane
-    constexpr int NK = 4 / NI;                   // heads per query row held by one lane
-    const uint8_t* base = sP_ptr + lane * 128 + ((ck ^ (lane & 7)) << 4);
-    float col[8], obs[8], band[MAX_WINDOWS][8];
-#pragma unroll
-    for (int c = 0; c < 8; ++c) {
-        col[c] = 0.f; obs[c] = 0.f;
-#pragma unroll
-        for (int w = 0; w < MAX_WINDOWS; ++w) band[w][c] = 0.f;
-    }
-    const float fG = (float)p.G, invG = 1.0f / (float)p.G;
-    const bool g_pow2 = (p.G & (p.G - 1)) == 0;
-#pragma unroll
-    for (int ii = 0; ii < NI; ++ii) {
-        f32x2 sum2[4] = {0ull, 0ull, 0ull, 0ull};
-#pragma unroll
-        for (int kk = 0; kk < NK; ++kk) {
-            const int k = ii + NI * kk;                                  // row = lane + 32 k (same swizzle phase)
-            const int g = QB >= 32 ? kk : 2 * kk + (lane >> 4);          // QB = 16: rows l + 32 k hold heads 2k, 2k + 1
-            const uint4 u = *reinterpret_cast<const uint4*>(base + k * 32 * 128);
-            if (g < p.G) {
-                const uint32_t w[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-                for (int c = 0; c < 4; ++c) sum2[c] = add2(sum2[c], pair(bf16x2_lo(w[c]), bf16x2_hi(w[c])));
-            }
-        }
-        float sum[8];
-#pragma unroll
-        for (int c = 0; c < 4; ++c) unpair(sum2[c], sum[2 * c], sum[2 * c + 1]);
-        if (QB < 32) {   // the other half of the heads sits 16 lanes away
-#pragma unroll
-            for (int c = 0; c < 8; ++c) sum[c] += __shfl_xor_sync(0xffffffffu, sum[c], 16);
-        }
-        const int i = QB >= 32 ? lane + 32 * ii : (lane & (QB - 1));
-        const int q_i = i0 + i;
-        const bool counted = (q_i < p.S) && (QB >= 32 || lane < QB);   // QB = 16: lanes 16..31 hold duplicates
-        float pooled[8];
-#pragma unroll
-        for (int c = 0; c < 8; c += 2) {
-            const float a = g_pow2 ? sum[c] * invG : __fdiv_rn(sum[c], fG);
-            const float b = g_pow2 ? sum[c + 1] * invG : __fdiv_rn(sum[c + 1], fG);
-            const uint32_t d = cvt_bf16x2(a, b);
-            pooled[c] = counted ? bf16x2_lo(d) : 0.f;
-            pooled[c + 1] = counted ? bf16x2_hi(d) : 0.f;
-        }
-#pragma unroll
-        for (int c = 0; c < 8; ++c) col[c] += pooled[c];
-        if (want_obs && q_i >= p.obs_start) {
-#pragma unroll
-            for (int c = 0; c < 8; ++c) obs[c] += pooled[c];
-        }
-        if (p.n_windows) {
-#pragma unroll
-            for (int w = 0; w < MAX_WINDOWS; ++w) {
-                if (w < p.n_windows) {
-                    const int lim = q_i - jbase - p.windows[w];   // column c is inside the band iff c > lim
-#pragma unroll
-                    for (int c = 0; c < 8; ++c)
-                        if (c > lim) band[w][c] += pooled[c];
-                }
-            }
-        }
-    }
-    const int oc = ck * 8 + warp_reduce8_column(lane);
-    const bool writer = (lane & 3) == 0;          // eight lanes write the warp's eight columns: one 32-byte sector
-    float r = warp_reduce8(col, lane);
-    if (writer) out_col[oc] = r;
-    if (want_obs) {
-        r = warp_reduce8(obs, lane);
-        if (writer) out_obs[oc] = r;
-    }
-#pragma unroll
-    for (int w = 0; w < MAX_WINDOWS; ++w) {
-        if (w < p.n_windows) {
-            r = warp_reduce8(band[w], lane);
-            if (writer) out_band[w * band_stride + oc] = r;
-        }
-    }
+// Two logits as the reference rounds them: bf16(q.k), then bf16(that times the scale).  1 / sqrt(128) is no bf16 number; x times
+// it, rounded to fp32 and then to bf16, is fma(x, hi, bf16(x lo)) with its two bf16 parts: equal for every finite bf16 x of at
+// least 2^-100 (checked over all of them in tests/test_prefill_rounding.py), and below that both are zero to any exponential.
+// Three instructions for a pair where fp32 takes five.  1 / sqrt(64) is a power of two.
+constexpr uint32_t SCALE128_HI = 0x3db53db5u, SCALE128_LO = 0x371e371eu, SCALE64 = 0x3e003e00u;
+template <int D>
+__device__ __forceinline__ uint32_t round_logits(float x, float y) {
+    const uint32_t d = cvt_bf16x2(x, y);
+    if constexpr (D == 64) return mul_bf16x2(d, SCALE64);
+    else return fma_bf16x2(d, SCALE128_HI, mul_bf16x2(d, SCALE128_LO));
 }
+
+// N pairs of a row's logits: bf16 with the reference's roundings, or fp32.
+template <bool NAIVE, int N = 16>
+struct Logits {
+    uint32_t w[N];
+    template <int D>
+    __device__ __forceinline__ void set(int c, float x, float y, f32x2) { w[c] = round_logits<D>(x, y); }
+    __device__ __forceinline__ f32x2 get(int c) const { return pair(bf16x2_lo(w[c]), bf16x2_hi(w[c])); }
+    __device__ __forceinline__ void hide(int c, bool first, bool second) {
+        if (first) w[c] = (w[c] & 0xffff0000u) | 0xff80u;
+        if (second) w[c] = (w[c] & 0xffffu) | 0xff800000u;
+    }
+    __device__ __forceinline__ float max() const {
+        uint32_t m[4] = {w[0], w[1], w[2], w[3]};
+#pragma unroll
+        for (int c = 4; c < N; ++c) m[c & 3] = max_bf16x2(m[c & 3], w[c]);
+        m[0] = max_bf16x2(max_bf16x2(m[0], m[1]), max_bf16x2(m[2], m[3]));
+        return fmaxf(bf16x2_lo(m[0]), bf16x2_hi(m[0]));
+    }
+};
+template <int N>
+struct Logits<false, N> {
+    f32x2 w[N];
+    template <int D>
+    __device__ __forceinline__ void set(int c, float x, float y, f32x2 scale) { w[c] = mul2(pair(x, y), scale); }
+    __device__ __forceinline__ f32x2 get(int c) const { return w[c]; }
+    __device__ __forceinline__ void hide(int c, bool first, bool second) {
+        float x, y;
+        unpair(w[c], x, y);
+        w[c] = pair(first ? -INFINITY : x, second ? -INFINITY : y);
+    }
+    __device__ __forceinline__ float max() const {
+        float m[2], x, y;
+        unpair(w[0], m[0], m[1]);
+#pragma unroll
+        for (int c = 1; c < N; ++c) {
+            unpair(w[c], x, y);
+            m[0] = fmaxf(m[0], x);
+            m[1] = fmaxf(m[1], y);
+        }
+        return fmaxf(m[0], m[1]);
+    }
+};
 
 // ------------------------------------------------------------------ the kernel
-// grid = n_qtiles * Hkv CTAs (longest query tiles first), 512 threads = two independent KEY-HALF GROUPS of 8 warps.
-// Group g walks the 64-key blocks [128 t + 64 g, +64) of the keys this query block can see, with its own K/V ring,
-// S accumulators, P tile, Y accumulator and barriers, so the two groups drift out of phase and one group's
-// MUFU-bound softmax overlaps the other's rounding / store / reduction phases.  In a group, thread
-// (row = t % 128, ch = t / 128) owns keys [32 ch, 32 ch + 32) of its row of every S block (TMEM lane quarter row / 32).
-// The partial accumulators Y_0 + Y_1 are added in the epilogue (fixed order: bit-reproducible).
-// Bound: latency at four warps per scheduler (issue slots 48 % busy, tensor pipe 23 %, the largest stalls fixed latencies and the
-// group's barrier).  A group has
-// two P blocks so that one barrier per block of sweep 2 is enough: it says that the block is written, and that everyone has
-// read the block before, which the block after it may then overwrite once its MMAs are done.  With one P block there were
-// two barriers per block and the column sums waited in shared memory: 1718 us at 7680 tokens x 32 heads of 128 (8 key/value
-// heads), 1573 with two; 116.2 and 110.7 at 1531 x 28 (4).  The two blocks take 32 KB more: 225 KB of the 227 a CTA may have.
-__device__ __forceinline__ void group_sync(int grp) { asm volatile("bar.sync %0, 256;" :: "r"(grp + 1) : "memory"); }
+struct Small {
+    uint64_t bars[30];
+    uint32_t tmem;
+    int failed;
+    float fin[BM][2];       // minus the offset z(maximum) and one over the sum, of every row
+    float stat[4][BM][3];   // of a row's key quarters: maximum, offset of the sum, sum
+};
+// Tiles of K and V in shared memory (the last one is where Q was), and the pooled probabilities of two tiles, [QB][128 keys] bf16.
+template <int D, int QQ> __host__ __device__ constexpr int stages() { return D == 64 || QQ <= 8 ? 6 : QQ == 16 ? 5 : 4; }
+template <int D, int QQ> constexpr int smem_bytes() {
+    return 1024 + stages<D, QQ>() * (D / 64) * ATOM_BYTES + 2 * 4 * QQ * BN * 2 + (int)sizeof(Small);
+}
 
-template <int D, bool NAIVE>
+// grid = n_qtiles * Hkv CTAs (longest query tiles first).  Rows: TMEM lane quarter j holds QQ = QB / 4 queries, row = QQ g + i, so
+// that all heads of a query lie in one quarter and, read back with tcgen05.ld.16x256b, in one thread (QQ >= 8) or in two that
+// are 16 lanes apart (QQ = 4).  Sixteen warps of softmax in two groups that take every second tile: warp w has lane quarter w % 4,
+// keys 64 (w / 4 % 2) .. + 63 in two steps of 32, and tiles w / 8, + 2, ...  One warp each issues the MMAs and loads K and V, two
+// add up over the queries; nobody meets anybody at a CTA barrier per tile, and while one group waits for the tensor
+// memory or a product the other one has the ALUs.
+//
+// Sweep 1 reads a row per thread.  Its sum is kept relative to a reference that need not be the maximum: the exponentials of a
+// step start at once with the reference there is, and only where the step's own maximum turns out to lie more than 2 above
+// it are they formed again with that maximum as the reference.  Sweep 2 subtracts the maximum itself.
+// Sweep 2 reads four rows x 8 keys per thread: P goes back to tensor memory as the A operand of P V, and a query's heads are
+// added up in registers.  The pooled probabilities go to shared memory, where the two warps of the sums over the queries take them.
+//
+// Bound: issue slots (54 % busy), the exponentials (two per logit at 16 per SM and cycle: 50 %) and the waits between them, at four
+// warps of softmax per scheduler; a 128 x 128 tile takes 1430 cycles in sweep 1 and 2000 in sweep 2, of which the MMAs take 515 and
+// 1030.  Measured at 7680 tokens x 32 heads of 128 (8 key/value heads) / 4096 / 1531 x 28 (4), in us, reduction included:
+// two groups of 256 threads that shared a barrier per 64 keys and issued their own MMAs 1397 / 412 / 105, this 815 / 279 / 85.
+// On the way: MMAs issued by one thread instead of a warp in step 976; mma.sync for the sums over heads and queries 943 (1500
+// cycles a tile: it waits for the tensor pipe behind the tcgen05 MMAs); all warps on the same tile 816; a quarter of the
+// exponentials as polynomials of degree 6 on the FMA pipe 924; the sums over the heads a tile later, among the exponentials, 899.
+template <int D, bool NAIVE, int QQ>
 __global__ void __launch_bounds__(NTHREADS, 1)
 prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
-                    const __grid_constant__ CUtensorMap tm_v, const PrefillParams p) {
-    constexpr int DH = D / 64;                  // 64-column (128-byte) sub-tiles along the head dimension
-    constexpr int Q_BYTES = DH * ATOM_BYTES;    // Q tile: 128 rows
-    constexpr int HALF_ATOM = BNH * 128;        // 64 rows x 128 bytes
-    constexpr int KV_BYTES = DH * HALF_ATOM;    // one K or V block of a group: 64 keys x D
-    constexpr int GROUP_BYTES = 4 * KV_BYTES + 2 * ATOM_BYTES;   // K[2], V[2], P[2] (128 rows x 64 keys)
+                    const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ PrefillParams p) {
+    constexpr int DH = D / 64;                    // 64-column (128-byte) sub-tiles along the head dimension
+    constexpr int TILE_BYTES = DH * ATOM_BYTES;   // 128 rows of Q, K or V
+    constexpr int QB = 4 * QQ;                    // query positions of a CTA
+    constexpr int NS = QQ >= 8 ? QQ / 8 : 1;      // queries of a thread in sweep 2
+    constexpr int STAGES = stages<D, QQ>(), POOL_BYTES = QB * BN * 2;
+    constexpr int TM_Y = 2 * BN, TM_Q = 3 * BN, TM_P = TM_Q + 64;   // tensor memory: logits 2 x 128 | Y, in sweep 1 logits | Q | P
     extern __shared__ uint8_t smem_raw[];
-    __shared__ __align__(8) uint64_t bars[17];  // 0 q; group g at 1 + 8 g: k[2], v[2], s[2], pv[2]
-    __shared__ uint32_t s_tmem_base;
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int grp = tid >> 8, gt = tid & 255, gwarp = gt >> 5;
-    const int row = gt & 127, ch = gt >> 7;
-    // One thread each of three warps of the group issues its Q K^T products, its K loads, and its P V products and V loads:
-    // what one warp issued alone, the other seven waited for at the next barrier (1573 -> 1416 us at 7680 tokens x 32 heads).
-    const bool lead_s = gt == 0, lead_k = gt == 3 * 32, lead_v = gt == 6 * 32;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int h = blockIdx.x % p.Hkv;
     const int qt = p.n_qtiles - 1 - blockIdx.x / p.Hkv;
-    const int i0 = qt * p.QB;
-    const int lim = min(i0 + p.QB, p.S);                        // keys [0, lim) are visible to this query block
-    const int T = max(0, (lim - BNH * grp + BN - 1) / BN);      // 64-key blocks of this group
-    const int T_other = max(0, (lim - BNH * (1 - grp) + BN - 1) / BN);
+    const int i0 = qt * QB;
+    const int lim = min(i0 + QB, p.S);                          // keys [0, lim) are visible to this query block
+    const int T = (lim + BN - 1) / BN;                          // tiles
 
-    const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-    const uint32_t sQ = smem_base;
-    const uint32_t sG = sQ + Q_BYTES + grp * GROUP_BYTES;
-    const uint32_t sK = sG, sV = sG + 2 * KV_BYTES, sP = sG + 4 * KV_BYTES;
-    uint8_t* const sP_ptr = smem_raw + (sP - smem_u32(smem_raw));
-    // row statistics of the four key quarters, between the sweeps, where group 0's P blocks are afterwards
-    float (*s_rowstat)[BM][2] = reinterpret_cast<float (*)[BM][2]>(smem_raw + (sQ + Q_BYTES + 4 * KV_BYTES - smem_u32(smem_raw)));
-    const uint32_t bar0 = smem_u32(bars);
-    const uint32_t BAR_Q = bar0, bG = bar0 + 8u * (1 + 8 * grp);
-    auto BAR_K = [&](int b) { return bG + 8u * b; };
-    auto BAR_V = [&](int b) { return bG + 8u * (2 + b); };
-    auto BAR_S = [&](int b) { return bG + 8u * (4 + b); };
-    auto BAR_PV = [&](int b) { return bG + 8u * (6 + b); };
+    const uint32_t sT = (smem_u32(smem_raw) + 1023u) & ~1023u, sQ = sT + (STAGES - 1) * TILE_BYTES;
+    uint8_t* const q_rows = smem_raw + (sQ - smem_u32(smem_raw));
+    uint8_t* const pools = q_rows + TILE_BYTES;                 // [2][QB][16 chunks of 8 keys], chunks 4 .. of odd rows first
+    Small& sm = *reinterpret_cast<Small*>(pools + 2 * POOL_BYTES);
+    volatile int* const failed = &sm.failed;
+    const uint32_t bar = smem_u32(sm.bars);
+    const uint32_t Q_FULL = bar, Q_READY = bar + 8, Y_DONE = bar + 16;
+    auto FULL = [&](int b) { return bar + 24 + 8u * b; };
+    auto FREE = [&](int b) { return bar + 72 + 8u * b; };
+    auto S_FULL = [&](int b) { return bar + 120 + 8u * b; };
+    auto S_READ = [&](int b) { return bar + 144 + 8u * b; };
+    auto P_FULL = [&](int b) { return bar + 168 + 8u * b; };
+    auto C_FULL = [&](int b) { return bar + 184 + 8u * b; };
+    auto C_READ = [&](int b) { return bar + 200 + 8u * b; };
+    auto PV_DONE = [&](int b) { return bar + 216 + 8u * b; };
+    // Sweep 1 goes round three accumulators (the third where Y comes later), sweep 2 round the first two, after `used` turns each.
+    auto used = [&](int b) { return (T - b + 2) / 3; };
 
     if (tid == 0) {
-        for (int i = 0; i < 17; ++i) mbar_init_u32(bar0 + 8u * i, 1);
+        *failed = 0;
+        mbar_init_u32(Q_FULL, 1);
+        mbar_init_u32(Q_READY, SOFT_WARPS);
+        mbar_init_u32(Y_DONE, 1);
+        for (int b = 0; b < STAGES; ++b) { mbar_init_u32(FULL(b), 1); mbar_init_u32(FREE(b), 1); }
+        for (int b = 0; b < 3; ++b) { mbar_init_u32(S_FULL(b), 1); mbar_init_u32(S_READ(b), SOFT_WARPS / 2); }
+        for (int b = 0; b < 2; ++b) {
+            mbar_init_u32(P_FULL(b), SOFT_WARPS / 2);
+            mbar_init_u32(C_FULL(b), SOFT_WARPS / 2);
+            mbar_init_u32(C_READ(b), 2);
+            mbar_init_u32(PV_DONE(b), 1);
+        }
         mbar_fence_init();
     }
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
-                     :: "r"(smem_u32(&s_tmem_base)), "r"(TMEM_COLS) : "memory");
+                     :: "r"(smem_u32(&sm.tmem)), "r"(TMEM_COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    if (p.G * p.QB < BM) {   // rows the Q box does not cover: zero them once (they only feed unused S rows)
-        uint4* q4 = reinterpret_cast<uint4*>(smem_raw + (sQ - smem_u32(smem_raw)));
-        for (int i = tid; i < Q_BYTES / 16; i += NTHREADS) q4[i] = make_uint4(0, 0, 0, 0);
+    if (p.G * QQ < 32) {   // rows the Q box does not cover: zero them once (they only feed unused S rows)
+        uint4* q4 = reinterpret_cast<uint4*>(q_rows);
+        for (int i = tid; i < TILE_BYTES / 16; i += NTHREADS) q4[i] = make_uint4(0, 0, 0, 0);
         fence_proxy_async();
     }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = s_tmem_base;
-    const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
-    const uint32_t tS = tmem + grp * 128, tY = tmem + 256 + grp * 128;
+    const uint32_t tmem = sm.tmem;
 
-    constexpr uint32_t IDESC_S = make_idesc(BM, BNH, false);
-    constexpr uint32_t IDESC_PV = make_idesc(BM, D, true);
-
-    auto issue_k = [&](int blk, int buf) {
-        mbar_expect_tx_u32(BAR_K(buf), KV_BYTES);
+    if (warp >= SOFT_WARPS) {
+        if (warp == SOFT_WARPS) {
+            constexpr uint32_t IDESC_S = make_idesc(BM, BN, false), IDESC_PV = make_idesc(BM, D, true);
+            const uint64_t k_desc = smem_desc(sT, 16, 1024), v_desc = smem_desc(sT, ATOM_BYTES, 1024);
+            // The tiles come in the order in which they are used: K of sweep 1, then K of tile t + 2 before V of tile t.
+            int st = 0;
+            uint32_t turn = 0;
+            auto next = [&] { if (++st == STAGES) { st = 0; turn ^= 1; } };
+            auto logits = [&](int b) {                   // S[b] = Q K^T: [128 x 128], Q in tensor memory
+                mbar_wait_u32(FULL(st), turn, failed);
+                tc_fence_after();
+                if (elect_one()) {
+                    const uint64_t desc = k_desc + st * (TILE_BYTES >> 4);
 #pragma unroll
-        for (int dh = 0; dh < DH; ++dh)
-            tma_load_3d(sK + buf * KV_BYTES + dh * HALF_ATOM, &tm_k, dh * 64, blk * BN + grp * BNH, h, BAR_K(buf));
-    };
-    auto issue_v = [&](int blk, int buf) {
-        mbar_expect_tx_u32(BAR_V(buf), KV_BYTES);
-#pragma unroll
-        for (int dh = 0; dh < DH; ++dh)
-            tma_load_3d(sV + buf * KV_BYTES + dh * HALF_ATOM, &tm_v, dh * 64, blk * BN + grp * BNH, h, BAR_V(buf));
-    };
-    // S[buf] = Q K_buf^T : [128 x 64], D/16 MMAs of K = 16
-    auto mma_s = [&](int buf) {
-#pragma unroll
-        for (int k = 0; k < D / 16; ++k) {
-            const uint32_t koff = (k & 3) * 32;
-            umma_bf16(tS + buf * BNH, smem_desc(sQ + (k >> 2) * ATOM_BYTES + koff, 16, 1024),
-                      smem_desc(sK + buf * KV_BYTES + (k >> 2) * HALF_ATOM + koff, 16, 1024), IDESC_S, k > 0);
-        }
-        umma_commit(BAR_S(buf));
-    };
-    // Y (+)= P V_buf : 64 keys = 4 MMAs; V is [key][d] in shared memory = MN-major B operand
-    auto mma_pv = [&](int buf, bool first) {
-#pragma unroll
-        for (int k = 0; k < BNH / 16; ++k)
-            umma_bf16(tY, smem_desc(sP + buf * ATOM_BYTES + k * 32, 16, 1024), smem_desc(sV + buf * KV_BYTES + k * 2048, HALF_ATOM, 1024),
-                      IDESC_PV, !(first && k == 0));
-        umma_commit(BAR_PV(buf));
-    };
-
-    const int NT = 2 * T;   // block visits of this group: sweep 1 then sweep 2
-    if (tid == 0) {
-        mbar_expect_tx_u32(BAR_Q, (uint32_t)(DH * p.G * p.QB * 128));
-#pragma unroll
-        for (int dh = 0; dh < DH; ++dh) tma_load_3d(sQ + dh * ATOM_BYTES, &tm_q, dh * 64, i0, h * p.G, BAR_Q);
-    }
-    if (lead_s && T > 0) {
-        issue_k(0, 0);
-        issue_k(1 % T, 1);
-        issue_v(0, 0);
-        if (T > 1) issue_v(1, 1);
-        mbar_wait_u32(BAR_Q, 0);
-        mbar_wait_u32(BAR_K(0), 0);
-        tc_fence_after();
-        mma_s(0);
-    }
-    __syncwarp();
-
-    // this thread's row
-    const int qi = i0 + row % p.QB;
-    float m_run = -INFINITY, s_run = 0.f;
-    float m_fin = 0.f, inv_s = 0.f;
-    const float scale = p.scale;
-
-    // pooled-map reductions: warp = 16-byte chunk of key columns (tile_stats), straight to this query block's partials
-    const bool want_obs = qt >= p.first_obs_tile;
-    float* const out_col = p.part_col + ((size_t)h * p.n_qtiles + qt) * p.S_pad + grp * BNH;
-    float* const out_obs = p.part_obs + ((size_t)h * p.n_obs_tiles + (want_obs ? qt - p.first_obs_tile : 0)) * p.S_pad + grp * BNH;
-    float* const out_band = p.part_band + ((size_t)h * p.n_qtiles + qt) * p.S_pad + grp * BNH;
-    const size_t band_stride = (size_t)p.Hkv * p.n_qtiles * p.S_pad;
-
-    // one block visit up to the logits: l[c] = logit of key (block t, 32 ch + c), -inf past the diagonal
-    auto visit = [&](int n, int t, float (&l)[32]) {
-        const int sb = n & 1;
-        if (lead_s && n + 1 < NT) {   // next block's logits under this block's softmax
-            mbar_wait_u32(BAR_K((n + 1) & 1), ((n + 1) >> 1) & 1);
+                    for (int k = 0; k < D / 16; ++k)
+                        umma_ts(tmem + b * BN, tmem + TM_Q + 8 * k, desc + ((k >> 2) * ATOM_BYTES + (k & 3) * 32) / 16, IDESC_S, k > 0);
+                    umma_commit(S_FULL(b));
+                    umma_commit(FREE(st));
+                }
+                __syncwarp();
+                next();
+            };
+            mbar_wait_u32(Q_READY, 0, failed);
             tc_fence_after();
-            mma_s((n + 1) & 1);
-        }
-        __syncwarp();
-        mbar_wait_u32(BAR_S(sb), (n >> 1) & 1);
-        tc_fence_after();
-        uint32_t v0[32];
-        tmem_ld32(tS + lane_base + sb * BNH + ch * 32, v0);
-        if (lead_k && n + 2 < NT) issue_k((n + 2) % T, sb);   // K[sb] is free: its MMA has completed
-        __syncwarp();
-        const f32x2 scale2 = pair(scale, scale);
-#pragma unroll
-        for (int c = 0; c < 32; c += 2) {
-            float x = __uint_as_float(v0[c]), y = __uint_as_float(v0[c + 1]);
-            if (NAIVE) { x = round_bf16(x); y = round_bf16(y); }
-            unpair(mul2(pair(x, y), scale2), x, y);
-            if (NAIVE && D != 64) { x = round_bf16(x); y = round_bf16(y); }   // D = 64: the scale is 2^-3
-            l[c] = x;
-            l[c + 1] = y;
-        }
-        if (t * BN + grp * BNH + BNH - 1 > i0) {   // the block reaches past the diagonal for some row
-            const int kbase = t * BN + grp * BNH + ch * 32;
-#pragma unroll
-            for (int c = 0; c < 32; ++c)
-                if (kbase + c > qi) l[c] = -INFINITY;
-        }
-    };
-
-    // exp(l - m) = 2^(l log2(e) - z(m)) with z(m) = m log2(e) rounded ONCE: the fma rounds the difference alone, and the rounding
-    // of z is a factor common to all terms that the same m scales.  It cancels because every change of maximum goes from z to z;
-    // a factor formed from m - m' instead left it in the sums (largest weight error at logits near 20 / 100 / 500 / 16384:
-    // 2.2e-6 / 6e-6 / 2.8e-5 / 7.6e-4, from z to z 0.9e-6 throughout, as with the difference formed first).
-    const f32x2 log2e2 = pair(LOG2E, LOG2E);
-    auto in_log2 = [](float m) { return __fmul_rn(m, LOG2E); };
-
-    // ---- sweep 1: softmax statistics
-    for (int n = 0; n < T; ++n) {
-        float l[32];
-        visit(n, n, l);
-        float tm[4] = {l[0], l[1], l[2], l[3]};
-#pragma unroll
-        for (int c = 4; c < 32; ++c) tm[c & 3] = fmaxf(tm[c & 3], l[c]);
-        const float m_new = fmaxf(m_run, fmaxf(fmaxf(tm[0], tm[1]), fmaxf(tm[2], tm[3])));
-        if (m_new > -INFINITY) {
-            const float z_new = in_log2(m_new);
-            const f32x2 off = pair(-z_new, -z_new);
-            f32x2 a[2] = {0ull, 0ull};
-#pragma unroll
-            for (int c = 0; c < 32; c += 2) {
-                float x, y;
-                unpair(fma2(pair(l[c], l[c + 1]), log2e2, off), x, y);
-                a[(c >> 1) & 1] = add2(a[(c >> 1) & 1], pair(ex2(x), ex2(y)));
+            uint32_t read = 1;
+            for (int n = 0, b = 0; n < T && !*failed; ++n) {
+                if (n >= 3) mbar_wait_u32(S_READ(b), read, failed);
+                logits(b);
+                if (++b == 3) { b = 0; read ^= 1; }
             }
-            float a0, a1;
-            unpair(add2(a[0], a[1]), a0, a1);
-            s_run = s_run * ex2(in_log2(m_run) - z_new) + (a0 + a1);
-            m_run = m_new;
+            for (int t = -2; t < T && !*failed; ++t) {
+                if (t + 2 < T) {
+                    const int b = t & 1, turns = used(b) + ((t + 2) >> 1);            // of this accumulator, so far
+                    if (turns > 0) mbar_wait_u32(S_READ(b), (turns - 1) & 1, failed);
+                    logits(b);
+                }
+                if (t < 0) continue;
+                mbar_wait_u32(P_FULL(t & 1), (t >> 1) & 1, failed);
+                mbar_wait_u32(FULL(st), turn, failed);
+                tc_fence_after();
+                const int ksteps = min(BN, lim - t * BN + 15) >> 4;       // keys past the last query's take no part
+                if (elect_one()) {
+                    const uint64_t desc = v_desc + st * (TILE_BYTES >> 4);
+#pragma unroll
+                    for (int k = 0; k < BN / 16; ++k)
+                        if (k < ksteps) umma_ts(tmem + TM_Y, tmem + TM_P + 8 * k, desc + k * 128, IDESC_PV, t > 0 || k > 0);
+                    umma_commit(PV_DONE(t & 1));
+                    umma_commit(FREE(st));
+                }
+                __syncwarp();
+                next();
+            }
+            if (elect_one()) umma_commit(Y_DONE);
+            __syncwarp();
+            mbar_wait_u32(Y_DONE, 0, failed);
+        } else if (warp == SOFT_WARPS + 1) {
+            if (lane == 0) {
+                mbar_expect_tx_u32(Q_FULL, (uint32_t)(4 * DH * p.G * QQ * 128));
+                for (int j = 0; j < 4; ++j)
+#pragma unroll
+                    for (int dh = 0; dh < DH; ++dh) tma_load_3d(sQ + dh * ATOM_BYTES + j * 32 * 128, &tm_q, dh * 64, i0 + j * QQ, h * p.G, Q_FULL);
+                int n = 0;
+                auto load = [&](const CUtensorMap* tm, int tile) {
+                    const int st = n % STAGES;
+                    if (n >= STAGES) mbar_wait_u32(FREE(st), (n / STAGES - 1) & 1, failed);
+                    else if (n == STAGES - 1) mbar_wait_u32(Q_READY, 0, failed);
+                    if (*failed) return;
+                    mbar_expect_tx_u32(FULL(st), TILE_BYTES);
+#pragma unroll
+                    for (int dh = 0; dh < DH; ++dh) tma_load_3d(sT + st * TILE_BYTES + dh * ATOM_BYTES, tm, dh * 64, tile * BN, h, FULL(st));
+                    ++n;
+                };
+                for (int t = 0; t < T; ++t) load(&tm_k, t);
+                for (int t = -2; t < T; ++t) {
+                    if (t + 2 < T) load(&tm_k, t + 2);
+                    if (t >= 0) load(&tm_v, t);
+                }
+                if (*failed) {    // the copies under way end before the CTA does
+                    mbar_wait_out(Q_FULL, 0);
+                    for (int m = max(0, n - STAGES); m < n; ++m) mbar_wait_out(FULL(m % STAGES), (m / STAGES) & 1);
+                }
+            }
+            __syncwarp();
+        } else if (p.stats) {
+            // Sums over the queries, straight to this block's partials.  A warp has 64 keys, a lane 8 of them in every fourth
+            // row: chunk c holds keys 32 (c / 4) + 8 k + 2 (c % 4) + e as pair k.
+            const int c = 8 * (warp - SOFT_WARPS - 2) + (lane & 7), first = lane >> 3, rows = min(QB, p.S - i0);
+            const bool high = lane & 16, odd = lane & 8, obs = qt >= p.first_obs_tile;
+            const int key = 32 * (c >> 2) + 8 * ((high ? 2 : 0) + (odd ? 1 : 0)) + 2 * (c & 3);   // of the pair that this lane stores
+            float* const col = p.part_col + ((size_t)h * p.n_qtiles + qt) * p.S_pad + key;
+            float* const seen = p.part_obs + ((size_t)h * p.n_obs_tiles + (obs ? qt - p.first_obs_tile : 0)) * p.S_pad + key;
+            float* const band = p.part_band + ((size_t)h * p.n_qtiles + qt) * p.S_pad + key;
+            for (int t = 0; t < T; ++t) {
+                const uint8_t* const pool = pools + (t & 1) * POOL_BYTES;
+                mbar_wait_u32(C_FULL(t & 1), (t >> 1) & 1, failed);
+                __syncwarp();
+                auto add = [&](int from, int window, float* out) {       // rows from `from` on, of the last `window` keys each
+                    f32x2 s[4] = {0ull, 0ull, 0ull, 0ull};
+#pragma unroll 4
+                    for (int r = first; r < rows; r += 4) {
+                        uint4 u = *reinterpret_cast<const uint4*>(pool + r * (BN * 2) + ((c ^ ((r & 1) << 2)) << 4));
+                        if (r < from) continue;
+                        if (window > 0) {
+                            const int lo = i0 + r - window - (t * BN + 32 * (c >> 2) + 2 * (c & 3));   // pair k is inside past here
+                            auto inside = [&](uint32_t w, int k) { return (8 * k > lo ? w & 0xffffu : 0u) | (8 * k + 1 > lo ? w & 0xffff0000u : 0u); };
+                            u = make_uint4(inside(u.x, 0), inside(u.y, 1), inside(u.z, 2), inside(u.w, 3));
+                        }
+                        const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) s[k] = add2(s[k], pair(bf16x2_lo(w[k]), bf16x2_hi(w[k])));
+                    }
+                    // over the four rows at a time: lanes 16 and 8 apart swap pairs
+                    f32x2 a[2], b;
+#pragma unroll
+                    for (int k = 0; k < 2; ++k) a[k] = add2(high ? s[k + 2] : s[k], __shfl_xor_sync(0xffffffffu, high ? s[k] : s[k + 2], 16));
+                    b = add2(odd ? a[1] : a[0], __shfl_xor_sync(0xffffffffu, odd ? a[0] : a[1], 8));
+                    float2 f;
+                    unpair(b, f.x, f.y);
+                    if (*failed) f = make_float2(NAN, NAN);
+                    *reinterpret_cast<float2*>(out + t * BN) = f;
+                };
+                add(0, 0, col);
+                if (obs) add(p.obs_start - i0, 0, seen);
+                for (int w = 0; w < p.n_windows; ++w) add(0, p.windows[w], band + (size_t)w * p.Hkv * p.n_qtiles * p.S_pad);
+                __syncwarp();
+                if (lane == 0) mbar_arrive_u32(C_READ(t & 1));
+            }
         }
-        tc_fence_before();
-        group_sync(grp);   // every warp of the group has read S[n & 1] before the MMA two visits ahead overwrites it
-    }
-    // merge the four key quarters of every row (two per group)
-    s_rowstat[grp * 2 + ch][row][0] = m_run;
-    s_rowstat[grp * 2 + ch][row][1] = s_run;
-    __syncthreads();
-    {
-        float mq[4], sq[4];
+    } else {
+        const int quarter = warp & 3, part = warp >> 2;               // row quarter, of Q and Y a quarter of the columns
+        const int half = part & 1, group = part >> 1;                 // half of a tile's keys, of every second tile
+        const uint32_t lanes = (uint32_t)(quarter * 32) << 16;
+        const int row = quarter * 32 + lane, q0 = i0 + quarter * QQ;
+        {   // Q to tensor memory: this row's columns part D / 4 .. (two bf16 a TMEM column)
+            mbar_wait_u32(Q_FULL, 0, failed);
+            __syncwarp();
+            uint32_t w[D / 8];
 #pragma unroll
-        for (int c = 0; c < 4; ++c) { mq[c] = s_rowstat[c][row][0]; sq[c] = s_rowstat[c][row][1]; }
-        m_fin = fmaxf(fmaxf(mq[0], mq[1]), fmaxf(mq[2], mq[3]));   // finite: key 0 is visible to every query
-        float tot = 0.f;
-#pragma unroll
-        for (int c = 0; c < 4; ++c) tot += sq[c] * ex2(in_log2(mq[c]) - in_log2(m_fin));
-        inv_s = 1.0f / tot;
-    }
-    __syncthreads();   // every thread has its statistics: P blocks may take their place
+            for (int c = 0; c < D / 32; ++c) {
+                const int c8 = part * (D / 32) + c;                      // 16-byte chunk of the row
+                const uint4 u = *reinterpret_cast<const uint4*>(q_rows + (c8 >> 3) * ATOM_BYTES + row * 128 + (((c8 & 7) ^ (row & 7)) << 4));
+                w[4 * c] = u.x; w[4 * c + 1] = u.y; w[4 * c + 2] = u.z; w[4 * c + 3] = u.w;
+            }
+            tmem_st_row<D / 8>(tmem + lanes + TM_Q + part * (D / 8), w);
+            tmem_wait_st();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_u32(Q_READY);
+        }
+        const float scale = p.scale;
+        const f32x2 log2e2 = pair(LOG2E, LOG2E), scale2 = pair(scale, scale);
 
-    // ---- sweep 2: probabilities, P V, pooled reductions
-    const f32x2 off2 = pair(-in_log2(m_fin), -in_log2(m_fin)), inv2 = pair(inv_s, inv_s);
-    for (int t = 0; t < T; ++t) {
-        float l[32];
-        visit(T + t, t, l);
-        uint32_t pk[16];
-#pragma unroll
-        for (int c = 0; c < 32; c += 2) {
-            float x, y;
-            unpair(fma2(pair(l[c], l[c + 1]), log2e2, off2), x, y);
-            unpair(mul2(pair(ex2(x), ex2(y)), inv2), x, y);
-            pk[c >> 1] = cvt_bf16x2(x, y);
-        }
-        // P[t & 1] is free: its MMAs of two blocks ago are done, and every warp had read it before the barrier of the last block
-        if (t > 1) mbar_wait_u32(BAR_PV(t & 1), ((t >> 1) - 1) & 1);
-        uint8_t* const P = sP_ptr + (t & 1) * ATOM_BYTES;
+        // exp(l - m) = 2^(l log2(e) - z(m)) with z(m) = m log2(e) rounded ONCE: the fma rounds the difference alone, and the rounding
+        // of z is a factor common to all terms that the same m scales.  It cancels because every change of reference goes from z to z;
+        // a factor formed from m - m' instead left it in the sums (largest weight error at logits near 20 / 100 / 500 / 16384:
+        // 2.2e-6 / 6e-6 / 2.8e-5 / 7.6e-4, from z to z 0.9e-6 throughout, as with the difference formed first).
+        auto in_log2 = [](float m) { return __fmul_rn(m, LOG2E); };
+
+        // ---- sweep 1: softmax statistics of one row per thread.  The logits of tile n + 1 are fetched and rounded among the
+        // exponentials of tile n.
         {
-            uint8_t* prow = P + row * 128;
+            const int qi = q0 + lane % QQ;
+            float m_top = -INFINITY, m_ref = -INFINITY, z_ref = 0.f, s_run = 0.f;
+            uint32_t v[32];
+            Logits<NAIVE> l;
+            // steps: 32 keys at a time, two of a tile
+            auto first_key = [&](int i) { return (group + (i & ~1)) * BN + half * 64 + (i & 1) * 32; };
+            auto fetch = [&](int i) {
+                const int n = group + (i & ~1), b = n % 3;
+                if (!(i & 1)) mbar_wait_u32(S_FULL(b), (n / 3) & 1, failed);
+                __syncwarp();
+                tc_fence_after();
+                tmem_ld_row(tmem + lanes + b * BN + half * 64 + (i & 1) * 32, v);
+            };
+            auto fetched = [&](int i) {
+                tmem_wait_ld(v);
+                tc_fence_before();
+                __syncwarp();
+                if ((i & 1) && lane == 0) mbar_arrive_u32(S_READ((group + (i & ~1)) % 3));
+            };
+            auto cut = [&](int i) {                        // keys past the row's diagonal
+                const int kbase = first_key(i);
+                if (kbase + 31 > q0) {
+                    const int seen = qi - kbase;           // keys 0 .. seen
 #pragma unroll
-            for (int c4 = 0; c4 < 4; ++c4) {
-                const int c8 = ch * 4 + c4;
-                *reinterpret_cast<uint4*>(prow + ((c8 ^ (row & 7)) << 4)) =
-                    make_uint4(pk[4 * c4], pk[4 * c4 + 1], pk[4 * c4 + 2], pk[4 * c4 + 3]);
+                    for (int c = 0; c < 16; ++c) l.hide(c, 2 * c > seen, 2 * c + 1 > seen);
+                }
+            };
+            auto add_up = [&](const Logits<NAIVE>& x, float z, int from, int to, f32x2 (&a)[2]) {
+                const f32x2 off = pair(-z, -z);
+#pragma unroll
+                for (int c = from; c < to; ++c) {
+                    float e, f;
+                    unpair(fma2(x.get(c), log2e2, off), e, f);
+                    a[c & 1] = add2(a[c & 1], pair(ex2(e), ex2(f)));
+                }
+            };
+            auto total = [&](const f32x2 (&a)[2]) {
+                float a0, a1;
+                unpair(add2(a[0], a[1]), a0, a1);
+                return a0 + a1;
+            };
+            auto take = [&](const Logits<NAIVE>& x, float top, float sum) {
+                m_top = fmaxf(m_top, top);
+                if (top > m_ref + 2.f) {       // also for the first finite logit: there is no reference yet
+                    const float z = in_log2(top);
+                    f32x2 a[2] = {0ull, 0ull};
+                    add_up(x, z, 0, 16, a);
+                    s_run = s_run * (m_ref == -INFINITY ? 0.f : ex2(z_ref - z)) + total(a);
+                    m_ref = top;
+                    z_ref = z;
+                } else {
+                    s_run += sum;
+                }
+            };
+            const int steps = T > group ? (T - group + 1) & ~1 : 0;
+            if (steps > 0) {
+                fetch(0);
+                fetched(0);
+#pragma unroll
+                for (int c = 0; c < 16; ++c) l.template set<D>(c, __uint_as_float(v[2 * c]), __uint_as_float(v[2 * c + 1]), scale2);
+                cut(0);
+                for (int i = 1; i < steps; ++i) {
+                    fetch(i);
+                    const Logits<NAIVE> x = l;
+                    const float top = x.max();
+                    f32x2 a[2] = {0ull, 0ull};
+                    add_up(x, z_ref, 0, 8, a);
+                    fetched(i);
+#pragma unroll
+                    for (int c = 0; c < 16; ++c) l.template set<D>(c, __uint_as_float(v[2 * c]), __uint_as_float(v[2 * c + 1]), scale2);
+                    add_up(x, z_ref, 8, 16, a);
+                    take(x, top, total(a));
+                    cut(i);
+                }
+                f32x2 a[2] = {0ull, 0ull};
+                add_up(l, z_ref, 0, 16, a);
+                take(l, l.max(), total(a));
             }
+            sm.stat[part][row][0] = m_top;
+            sm.stat[part][row][1] = m_ref == -INFINITY ? -INFINITY : z_ref;
+            sm.stat[part][row][2] = s_run;
         }
-        fence_proxy_async();
-        tc_fence_before();
-        group_sync(grp);
-        if (lead_v) {
-            tc_fence_after();
-            mbar_wait_u32(BAR_V(t & 1), (t >> 1) & 1);
-            tc_fence_after();
-            mma_pv(t & 1, t == 0);
-            if (t >= 1 && t + 1 < T) {                      // V[(t + 1) & 1] is free once the last block's MMAs are done
-                mbar_wait_u32(BAR_PV((t - 1) & 1), ((t - 1) >> 1) & 1);
-                issue_v(t + 1, (t + 1) & 1);
-            }
+        asm volatile("bar.sync 1, 512;" ::: "memory");
+        if (part == 0) {    // the four parts of every row
+            float m = sm.stat[0][row][0], tot = 0.f;
+#pragma unroll
+            for (int q = 1; q < 4; ++q) m = fmaxf(m, sm.stat[q][row][0]);        // finite: key 0 is visible to every query
+            const float z = in_log2(m);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) tot += sm.stat[q][row][2] * ex2(sm.stat[q][row][1] - z);
+            sm.fin[row][0] = -z;
+            sm.fin[row][1] = 1.0f / tot;
         }
-        __syncwarp();
-        if (p.stats) {
-            const int jbase = t * BN + grp * BNH + gwarp * 8, j = t * BN;
-            switch (p.QB) {
-                case 128: tile_stats<7>(P, out_col + j, out_obs + j, out_band + j, band_stride, p, gwarp, lane, i0, jbase, want_obs); break;
-                case 64:  tile_stats<6>(P, out_col + j, out_obs + j, out_band + j, band_stride, p, gwarp, lane, i0, jbase, want_obs); break;
-                case 32:  tile_stats<5>(P, out_col + j, out_obs + j, out_band + j, band_stride, p, gwarp, lane, i0, jbase, want_obs); break;
-                default:  tile_stats<4>(P, out_col + j, out_obs + j, out_band + j, band_stride, p, gwarp, lane, i0, jbase, want_obs); break;
-            }
-        }
-    }
+        asm volatile("bar.sync 1, 512;" ::: "memory");
 
-    // ---- epilogue: Y_0 + Y_1 (fp32 in TMEM) -> bf16 -> global
-    if (T > 0) mbar_wait_u32(BAR_PV((T - 1) & 1), ((T - 1) >> 1) & 1);
-    tc_fence_after();
-    __syncthreads();   // both groups' accumulators are complete
-    tc_fence_after();
-    {
-        constexpr int CPT = D / 4;   // columns per thread: 32 (D = 128) or 16 (D = 64)
-        const int cq = tid >> 7, orow = tid & 127;
-        const int og = orow / p.QB, oqi = i0 + orow % p.QB;
-        const bool row_ok = (og < p.G) && (oqi < p.S);
-        const bool two = (grp == 0 ? T_other : T) > 0;   // group 1 saw at least one block
-        uint32_t y0[32], y1[32];
-        const uint32_t ycol = (CPT == 32) ? cq * 32 : (cq >> 1) * 32;   // D = 64: load the enclosing 32 columns
-        tmem_ld32(tmem + 256 + lane_base + ycol, y0);
-        if (two) tmem_ld32(tmem + 256 + 128 + lane_base + ycol, y1);
-        __nv_bfloat16* yrow = p.y + (long long)(h * p.G + og) * p.y_stride_h + (long long)oqi * p.y_stride_s + cq * CPT;
-        if (row_ok) {
-            float f[32];
+        // ---- sweep 2: probabilities of rows 8 j + lane / 4 of the quarter, keys 8 k + 2 (lane % 4), + 1 of the warp's 32
+        const int r8 = lane >> 2, c2 = 2 * (lane & 3);
+        f32x2 off[4], inv[4];
 #pragma unroll
-            for (int c = 0; c < 32; ++c) f[c] = __uint_as_float(y0[c]) + (two ? __uint_as_float(y1[c]) : 0.f);
+        for (int j = 0; j < 4; ++j) {
+            const float* const f = sm.fin[quarter * 32 + 8 * j + r8];
+            off[j] = pair(f[0], f[0]);
+            inv[j] = pair(f[1], f[1]);
+        }
+        const float fG = (float)p.G, invG = 1.0f / (float)p.G;
+        const bool g_pow2 = (p.G & (p.G - 1)) == 0, short_heads = p.G * QQ < 32;
+        const f32x2 invG2 = pair(invG, invG);
+        // where this thread's pooled probabilities go: row = query of the block, chunks of the two steps
+        const int pool_row = (quarter * QQ + (QQ == 4 ? r8 & 3 : r8)) * (BN * 2) + half * 128 + ((lane & 3) << 4), pool_swap = (r8 & 1) << 6;
+        uint32_t v[32];                                            // v[16 (j / 2) + 4 k + 2 (j % 2) + e]
+        uint32_t first[4][4], second[4][4];                       // of a tile's two steps
+        auto weigh_all = [&](int kbase, uint32_t (&pk)[4][4]) {
+            auto weigh = [&](auto cut) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const int seen = q0 + (8 * j + r8) % QQ - kbase - c2;   // key 8 k + e is seen up to here
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        const int at_v = 16 * (j >> 1) + 4 * k + 2 * (j & 1);
+                        Logits<NAIVE, 1> l;
+                        l.template set<D>(0, __uint_as_float(v[at_v]), __uint_as_float(v[at_v + 1]), scale2);
+                        if constexpr (decltype(cut)::value) l.hide(0, 8 * k > seen, 8 * k + 1 > seen);
+                        float x, y;
+                        unpair(fma2(l.get(0), log2e2, off[j]), x, y);
+                        unpair(mul2(pair(ex2(x), ex2(y)), inv[j]), x, y);
+                        pk[j][k] = cvt_bf16x2(x, y);
+                    }
+                }
+            };
+            if (kbase + 31 <= q0) {
+                weigh(std::false_type());
+            } else if (kbase < q0 + QQ) {
+                weigh(std::true_type());
+            } else {
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) pk[j][k] = 0u;         // nobody of the quarter sees these keys
+            }
+        };
+        auto pool = [&](int step, uint32_t (&pk)[4][4]) {
+            if (short_heads) {      // rows without a head take no part
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    if (8 * j + r8 >= p.G * QQ)
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) pk[j][k] = 0u;
+            }
+            uint8_t* const at = pools + group * POOL_BYTES + pool_row + ((step << 6) ^ pool_swap);
+#pragma unroll
+            for (int s = 0; s < NS; ++s) {
+                uint32_t w[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    if constexpr (QQ == 32) {
+                        w[k] = pk[s][k];                                    // one head: the probabilities themselves
+                    } else {
+                        f32x2 c = pair(bf16x2_lo(pk[s][k]), bf16x2_hi(pk[s][k]));
+#pragma unroll
+                        for (int j = s + NS; j < 4; j += NS) c = add2(c, pair(bf16x2_lo(pk[j][k]), bf16x2_hi(pk[j][k])));
+                        if constexpr (QQ == 4) c = add2(c, __shfl_xor_sync(0xffffffffu, c, 16));
+                        float x, y;
+                        if (g_pow2) {
+                            unpair(mul2(c, invG2), x, y);
+                        } else {
+                            unpair(c, x, y);
+                            x = __fdiv_rn(x, fG);
+                            y = __fdiv_rn(y, fG);
+                        }
+                        w[k] = cvt_bf16x2(x, y);
+                    }
+                }
+                if (QQ >= 8 || r8 < 4) *reinterpret_cast<uint4*>(at + s * 8 * (BN * 2)) = make_uint4(w[0], w[1], w[2], w[3]);
+            }
+        };
+        for (int t = group; t < T; t += 2) {
+            const int kbase = t * BN + half * 64;
+            const uint32_t at = tmem + lanes + group * BN + half * 64, to = tmem + lanes + TM_P + half * 32;
+            mbar_wait_u32(S_FULL(group), (used(group) + (t >> 1)) & 1, failed);
+            __syncwarp();
+            tc_fence_after();
+            tmem_ld_4rows(at, v);
+            tmem_wait_ld(v);
+            weigh_all(kbase, first);
+            tmem_ld_4rows(at + 32, v);                                 // under the pooling
+            if (p.stats) {
+                if (t >= 2) mbar_wait_u32(C_READ(group), ((t - 2) >> 1) & 1, failed);   // the last contents of this tile's place are summed
+                __syncwarp();
+                pool(0, first);
+            }
+            tmem_wait_ld(v);
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_u32(S_READ(group));
+            weigh_all(kbase + 32, second);
+            if (t > 0) mbar_wait_u32(PV_DONE(group ^ 1), ((t - 1) >> 1) & 1, failed);    // the product of the tile before has been through P
+            __syncwarp();
+            tc_fence_after();
+            tmem_st_4rows(to, first);
+            tmem_st_4rows(to + 16, second);
+            tmem_wait_st();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_u32(P_FULL(group));
+            __syncwarp();
+            if (p.stats) {
+                pool(1, second);
+                __syncwarp();
+                if (lane == 0) mbar_arrive_u32(C_FULL(group));
+            }
+        }
+
+        // ---- epilogue: Y (fp32 in TMEM) -> bf16 -> global; thread = row, columns part D / 4 ..
+        mbar_wait_u32(Y_DONE, 0, failed);
+        __syncwarp();
+        tc_fence_after();
+        constexpr int CPT = D / 4;
+        const int og = lane / QQ, oqi = q0 + lane % QQ;
+        uint32_t y[32];
+        tmem_ld_row(tmem + lanes + TM_Y + (CPT == 32 ? part * 32 : (part >> 1) * 32), y);   // D = 64: the enclosing 32 columns
+        tmem_wait_ld(y);
+        if (og < p.G && oqi < p.S) {
+            __nv_bfloat16* yrow = p.y + (long long)(h * p.G + og) * p.y_stride_h + (long long)oqi * p.y_stride_s + part * CPT;
+            const bool lost = *failed;
 #pragma unroll
             for (int c = 0; c < CPT; c += 8) {
                 float e[8];
 #pragma unroll
-                for (int u = 0; u < 8; ++u) e[u] = (CPT == 32) ? f[c + u] : ((cq & 1) ? f[16 + c + u] : f[c + u]);
+                for (int u = 0; u < 8; ++u) e[u] = lost ? NAN : __uint_as_float((CPT == 16 && (part & 1)) ? y[(16 + c + u) & 31] : y[c + u]);
                 *reinterpret_cast<uint4*>(yrow + c) = make_uint4(pack_bf16(e[0], e[1]), pack_bf16(e[2], e[3]),
                                                                   pack_bf16(e[4], e[5]), pack_bf16(e[6], e[7]));
             }
@@ -586,7 +790,7 @@ __device__ __forceinline__ float sum_tiles(const float* __restrict__ part, size_
 // enough that short prompts reach most of the chip.  Measured at 7680 / 4096 tokens x 8 heads and 1531 x 4 in groups of 7:
 // 16.8 / 8.9 / 5.5 us; CTAs of 256 with the loop as the compiler unrolls it 37.9 / 18.7 / 11.9.
 __global__ void __launch_bounds__(RED_THREADS)
-prefill_reduce_kernel(const PrefillParams p, float* __restrict__ col_sum, float* __restrict__ obs_sum,
+prefill_reduce_kernel(const __grid_constant__ PrefillParams p, float* __restrict__ col_sum, float* __restrict__ obs_sum,
                       float* __restrict__ band_sum) {
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     const int h = blockIdx.y;
@@ -669,19 +873,31 @@ Plan make_plan(int S, int Hkv, int G, int obs_len, int n_windows) {
     return pl;
 }
 
-template <int D, bool NAIVE>
+template <int D, bool NAIVE, int QQ>
 int launch(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const PrefillParams& p, int grid,
            cudaStream_t stream) {
-    const int smem = 1024 + (D / 64) * ATOM_BYTES + 2 * (4 * (D / 64) * BNH * 128 + 2 * ATOM_BYTES);
+    constexpr int smem = smem_bytes<D, QQ>();
+    static_assert(smem <= 232448, "");
     static bool configured = false;
     if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(prefill_attn_kernel<D, NAIVE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        cudaError_t e = cudaFuncSetAttribute(prefill_attn_kernel<D, NAIVE, QQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) return set_cuda_error(e, "cc_prefill_attention: shared memory attribute");
         configured = true;
     }
-    prefill_attn_kernel<D, NAIVE><<<grid, NTHREADS, smem, stream>>>(tq, tk, tv, p);
+    prefill_attn_kernel<D, NAIVE, QQ><<<grid, NTHREADS, smem, stream>>>(tq, tk, tv, p);
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? CC_OK : set_cuda_error(e, "cc_prefill_attention launch");
+}
+
+template <int D, bool NAIVE>
+int launch_group(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const PrefillParams& p, int grid,
+                 cudaStream_t stream) {
+    switch (p.QB) {
+        case 128: return launch<D, NAIVE, 32>(tq, tk, tv, p, grid, stream);
+        case 64:  return launch<D, NAIVE, 16>(tq, tk, tv, p, grid, stream);
+        case 32:  return launch<D, NAIVE, 8>(tq, tk, tv, p, grid, stream);
+        default:  return launch<D, NAIVE, 4>(tq, tk, tv, p, grid, stream);
+    }
 }
 
 }  // namespace
@@ -737,13 +953,13 @@ int prefill_attention_impl(const CcPrefillAttnArgs* a, cudaStream_t stream) {
     }
     CUtensorMap tq, tk, tv;
     int rc;
-    if ((rc = make_map(&tq, a->q, D, S, Hkv * G, a->q_stride_s, a->q_stride_h, pl.QB, G)) != CC_OK) return rc;
-    if ((rc = make_map(&tk, a->k, D, S, Hkv, a->k_stride_s, a->k_stride_h, BNH, 1)) != CC_OK) return rc;
-    if ((rc = make_map(&tv, a->v, D, S, Hkv, a->v_stride_s, a->v_stride_h, BNH, 1)) != CC_OK) return rc;
+    if ((rc = make_map(&tq, a->q, D, S, Hkv * G, a->q_stride_s, a->q_stride_h, pl.QB / 4, G)) != CC_OK) return rc;
+    if ((rc = make_map(&tk, a->k, D, S, Hkv, a->k_stride_s, a->k_stride_h, BN, 1)) != CC_OK) return rc;
+    if ((rc = make_map(&tv, a->v, D, S, Hkv, a->v_stride_s, a->v_stride_h, BN, 1)) != CC_OK) return rc;
     const int grid = pl.n_qtiles * Hkv;
     const bool naive = a->attn_mode == CC_ATTN_NAIVE_BF16;
-    if (D == 128) rc = naive ? launch<128, true>(tq, tk, tv, p, grid, stream) : launch<128, false>(tq, tk, tv, p, grid, stream);
-    else          rc = naive ? launch<64, true>(tq, tk, tv, p, grid, stream) : launch<64, false>(tq, tk, tv, p, grid, stream);
+    if (D == 128) rc = naive ? launch_group<128, true>(tq, tk, tv, p, grid, stream) : launch_group<128, false>(tq, tk, tv, p, grid, stream);
+    else          rc = naive ? launch_group<64, true>(tq, tk, tv, p, grid, stream) : launch_group<64, false>(tq, tk, tv, p, grid, stream);
     if (rc != CC_OK) return rc;
     if (stats) {
         dim3 rgrid((S + RED_THREADS - 1) / RED_THREADS, Hkv);

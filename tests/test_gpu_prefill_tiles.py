@@ -1,0 +1,66 @@
+"""Prompt attention with score reductions (csrc/prefill_attn.cu) at the edges of its tiles, for every group size, against the
+materialised map; tolerances are those of test_gpu_prefill.py, for the same quantities."""
+import pytest
+import torch
+
+from prefill_utils import assert_close_bf16, check_prefill_y
+
+pytestmark = pytest.mark.gpu
+
+
+def _inputs(G, D, S, kv=2):
+    gen = torch.Generator().manual_seed(1000 * G + 10 * S + D)
+    q = torch.randn(1, kv * G, S, D, generator=gen).bfloat16()
+    k = torch.randn(1, kv, S, D, generator=gen).bfloat16()
+    return q, k, torch.randn(1, kv, S, D, generator=gen).bfloat16()
+
+
+def _check(q, k, v, what, strict=0.99):
+    from cold_compress_b200.attention_utils import prefill_attention_stats
+    from oracle.prefill import full_map, reductions
+    S, D = q.shape[2], q.shape[3]
+    windows = (1, max(2, S // 3), S + 5)
+    y, st = prefill_attention_stats(q.cuda(), k.cuda(), v.cuda(), obs_len=16, windows=windows)
+    y_ref, pooled = full_map(q, k, v)
+    ref = reductions(pooled, 16, windows)
+    check_prefill_y(y[0].reshape(-1, D), y_ref[0].reshape(-1, D), what, strict_frac=strict)
+    assert_close_bf16(st.col_sum[0], ref.col_sum[0], f"{what} col_sum", max_ulp=1.0, min_equal=0.85, floor=2.0 ** -14)
+    assert_close_bf16(st.obs_mean[0], ref.obs_mean[0], f"{what} obs_mean", max_ulp=1.0, min_equal=0.85, floor=2.0 ** -14)
+    for w in windows:
+        assert torch.allclose(st.band_sum[w].cpu(), ref.band_sum[w], rtol=1e-2, atol=2e-3), f"{what} band {w}"
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("G", [1, 2, 3, 4, 5, 6, 7, 8])
+@pytest.mark.parametrize("S", [1, 15, 33, 127, 128, 129, 256, 391])
+def test_every_group_at_the_edges_of_tiles(G, D, S):
+    _check(*_inputs(G, D, S), f"G {G} D {D} S {S}")
+
+
+@pytest.mark.parametrize("G,D", [(4, 128), (7, 64)])
+def test_maxima_that_rise_from_tile_to_tile(G, D):
+    """Every tile's maximum lies further above the ones before than a sum's reference may: sums are formed again."""
+    q, k, v = _inputs(G, D, 600)
+    q, k = torch.ones_like(q) + 0.1 * q, (k + torch.arange(600).view(1, 1, -1, 1) / 40).bfloat16()
+    _check(q, k, v, "rising")
+    _check(q, k.flip(2), v, "falling")
+
+
+@pytest.mark.parametrize("G,D,S", [(7, 128, 145), (3, 64, 161), (4, 128, 70)])
+def test_logits_of_minus_infinity(G, D, S):
+    """Keys that no query gives any weight, and rows of the tile without a query or a head, whose logits are NaN there."""
+    q, k, v = _inputs(G, D, S)
+    q[..., 0] = q[..., 0].abs() + 1
+    k[0, :, 5::7, 0] = float("-inf")
+    _check(q, k, v, "minus infinity")
+
+
+def test_without_statistics_in_fp32():
+    from cold_compress_b200.attention_utils import prefill_attention
+    q, k, v = (t.cuda() for t in _inputs(5, 128, 391))
+    y = prefill_attention(q, k, v)
+    w = torch.matmul(q.float(), k.float().repeat_interleave(5, 1).transpose(2, 3)) * 128 ** -0.5
+    w = w.masked_fill(torch.ones(391, 391, dtype=torch.bool, device="cuda").triu(1), float("-inf"))
+    want = torch.softmax(w, -1) @ v.float().repeat_interleave(5, 1)
+    # one rounding of a weight and one of the result: 2^-9 of the largest value each, and half as much again for sums
+    assert (y.float() - want).abs().max() < 3 * 2.0 ** -9 * v.float().abs().max()
