@@ -1442,31 +1442,50 @@ __global__ void cache_append_kernel(const CcSeqAttn a, int t_first) {
     append_row<CT>(a, g, t, p, threadIdx.x, blockDim.x);
 }
 
-// The same for rows of whole 16-byte vectors: thread = vector x of the key row and then of the value row, blockDim.y (token,
-// head) rows per CTA, launched under the attention before it.  (1001 tokens of 4 heads of 128 + 128, with the attention they
-// follow: 77 us with one element per access, 69 with these and the fetch of tiles that straddle runs.)
+// The same for rows of whole 16-byte vectors, launched under the attention before it: thread = vector x of the key row and then of the
+// value row, of APPEND_ROWS (token, head) rows that lie blockDim.y apart and are under way together; positions and marks by a thread
+// per token, so that neighbouring tokens are stored together and a CTA counts its new slots with one addition.
+// Bound: HBM and the launch.  Measured in a chain of launches: 1001 tokens of 4 heads of 128 + 128 bf16 3.6 us, 4096 of 8 5.4; a row per
+// thread, with the row's first thread storing its marks, 10.3 and 22.9 (2.3 and 5.3 without positions and marks).
+constexpr int APPEND_ROWS = 4;
 template <typename CT>
 __global__ void __launch_bounds__(256) cache_append_rows_kernel(const CcSeqAttn a, int t_first) {
     pdl_wait_release();
     constexpr int VEC = 16 / (int)sizeof(CT);
-    const long long row = (long long)blockIdx.x * blockDim.y + threadIdx.y;
-    const int t = t_first + (int)(row / a.G), g = (int)(row % a.G), c = threadIdx.x, kc16 = a.Dk / VEC;
-    if (t >= a.T) return;
-    const int p = a.input_pos[0] + t;
-    if (p >= a.keep_first && p + (a.L - a.keep_first) <= a.input_pos[0] + a.T - 1) return;      // a later row takes this slot
-    const int slot = slot_of(a, p);
+    const int c = threadIdx.x, kc16 = a.Dk / VEC, p0 = a.input_pos[0];
     const bool key = c < kc16;
     const int D = key ? a.Dk : a.Dv, e = (key ? c : c - kc16) * VEC;
-    const CT* src = (key ? (const CT*)a.k_new : (const CT*)a.v_new) + ((size_t)t * a.G + g) * D + e;
-    CT* dst = (key ? (CT*)a.k_cache : (CT*)a.v_cache) + ((size_t)g * a.L + slot) * D + e;
-    *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(src);
-    if (c == 0) {
-        if (a.mask != nullptr) a.mask[(size_t)g * a.L + slot] = 1;
-        if (g == 0) {
-            const int old = a.pos[slot];
-            a.pos[slot] = p;
-            if (old < 0 && a.cache_cts != nullptr) atomicAdd(a.cache_cts, 1);
+    auto kept = [&](int p) { return p < a.keep_first || p + (a.L - a.keep_first) > p0 + a.T - 1; };      // no later row takes its slot
+    const CT* const src = (key ? (const CT*)a.k_new : (const CT*)a.v_new) + e;
+    CT* const dst = (key ? (CT*)a.k_cache : (CT*)a.v_cache) + e;
+    uint4 x[APPEND_ROWS];
+    long long to[APPEND_ROWS];
+#pragma unroll
+    for (int i = 0; i < APPEND_ROWS; ++i) {
+        const unsigned row = (blockIdx.x * APPEND_ROWS + i) * blockDim.y + threadIdx.y, n = row / (unsigned)a.G;
+        const int t = t_first + (int)n, g = (int)(row - n * (unsigned)a.G);
+        to[i] = -1;
+        if (t < a.T && kept(p0 + t)) {
+            to[i] = ((long long)g * a.L + slot_of(a, p0 + t)) * D;
+            x[i] = *reinterpret_cast<const uint4*>(src + ((size_t)t * a.G + g) * D);
         }
+    }
+#pragma unroll
+    for (int i = 0; i < APPEND_ROWS; ++i)
+        if (to[i] >= 0) *reinterpret_cast<uint4*>(dst + to[i]) = x[i];
+    const int threads = blockDim.x * blockDim.y, tid = threadIdx.y * blockDim.x + c;
+    for (long long first = t_first + (long long)blockIdx.x * threads; first < a.T; first += (long long)gridDim.x * threads) {   // the CTA as one
+        const long long t = first + tid;
+        bool fresh = false;
+        if (t < a.T && kept(p0 + (int)t)) {
+            const int p = p0 + (int)t, slot = slot_of(a, p);
+            fresh = a.pos[slot] < 0;
+            a.pos[slot] = p;
+            if (a.mask != nullptr)
+                for (int g = 0; g < a.G; ++g) a.mask[(size_t)g * a.L + slot] = 1;
+        }
+        const int news = __syncthreads_count(fresh);
+        if (tid == 0 && news > 0 && a.cache_cts != nullptr) atomicAdd(a.cache_cts, news);
     }
 }
 
@@ -1871,9 +1890,10 @@ int cc_seq_cache_append(const CcSeqAttn* a, void* stream) {
     const int t_first = (a->keep_first == 0 && a->T > a->L) ? a->T - a->L : 0;   // with kept positions every row's CTA decides
     const int size = a->cache_dtype == CC_DT_BF16 ? 2 : 4, vecs = a->Dk * size % 16 || a->Dv * size % 16 ? 0 : (a->Dk + a->Dv) * size / 16;
     const uintptr_t all = (uintptr_t)a->k_new | (uintptr_t)a->v_new | (uintptr_t)a->k_cache | (uintptr_t)a->v_cache;
-    if ((a->cache_dtype == CC_DT_F32 || a->cache_dtype == CC_DT_BF16) && vecs > 0 && vecs <= 256 && (all & 15) == 0 && a->G > 0) {
+    const long long rows = (long long)(a->T - t_first) * a->G;
+    if ((a->cache_dtype == CC_DT_F32 || a->cache_dtype == CC_DT_BF16) && vecs > 0 && vecs <= 256 && (all & 15) == 0 && a->G > 0 && rows < (1ll << 30)) {
         const dim3 block(vecs, 256 / vecs);
-        const unsigned ctas = (unsigned)(((long long)(a->T - t_first) * a->G + block.y - 1) / block.y);
+        const unsigned per_cta = APPEND_ROWS * block.y, ctas = (unsigned)((rows + per_cta - 1) / per_cta);
         if (size == 2) launch_under(cache_append_rows_kernel<__nv_bfloat16>, dim3(ctas), block, 0, st, *a, t_first);
         else launch_under(cache_append_rows_kernel<float>, dim3(ctas), block, 0, st, *a, t_first);
         return cuda_check("cache_append_rows_kernel");
