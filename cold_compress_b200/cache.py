@@ -274,8 +274,7 @@ class KVCache(nn.Module):
                 seq_ops.seq_attention(*part, seq_ops.ATTN_DECODE_APPEND if h1 == H else seq_ops.ATTN_DECODE,
                                       self._sequence_workspace(16, reach), int(block))
         else:
-            seq_ops.seq_attention(*args, seq_ops.ATTN_CHUNK, None, int(block), *extra)
-            seq_ops.seq_attention(*args, seq_ops.ATTN_APPEND_ONLY, None, int(block), *extra)
+            seq_ops.seq_attention(*args, seq_ops.ATTN_CHUNK_APPEND, None, int(block), *extra)
         return y
 
     def _sequence_workspace(self, n_q_heads, window):

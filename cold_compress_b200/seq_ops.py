@@ -15,7 +15,7 @@ from . import _lib
 
 _library = torch.library.Library("cold_compress_b200", "FRAGMENT")
 
-ATTN_CHUNK, ATTN_DECODE_APPEND, ATTN_APPEND_ONLY, ATTN_DECODE = 0, 1, 2, 3
+ATTN_CHUNK, ATTN_DECODE_APPEND, ATTN_APPEND_ONLY, ATTN_DECODE, ATTN_CHUNK_APPEND = range(5)
 
 _library.define("seq_embed(Tensor tokens, Tensor input_pos, Tensor(a!) prev_token, Tensor embed, Tensor? bigram, "
                 "Tensor inv_freq, Tensor(b!) x, Tensor(c!)? x_act, float scale, int buckets, int mul_prev, int mul_cur) -> ()")
@@ -106,8 +106,11 @@ def _seq_attention(q, k_new, v_new, k_cache, v_cache, pos, mask, cache_cts, inpu
     if workspace is not None:
         a.workspace, a.workspace_bytes = workspace.data_ptr(), workspace.numel() * workspace.element_size()
     lib = _lib.load_seq()
-    if mode == ATTN_CHUNK:
-        _lib.check_seq(lib.cc_seq_attention(C.byref(a), _stream()), "cc_seq_attention")
+    if mode in (ATTN_CHUNK, ATTN_CHUNK_APPEND):
+        stream = _stream()
+        _lib.check_seq(lib.cc_seq_attention(C.byref(a), stream), "cc_seq_attention")
+        if mode == ATTN_CHUNK_APPEND:
+            _lib.check_seq(lib.cc_seq_cache_append(C.byref(a), stream), "cc_seq_cache_append")
     elif mode in (ATTN_DECODE_APPEND, ATTN_DECODE):
         _lib.check_seq(lib.cc_seq_attention_decode(C.byref(a), _stream()), "cc_seq_attention_decode")
     elif mode == ATTN_APPEND_ONLY:
