@@ -11,8 +11,8 @@
 // 32 heads of 64 with keys that are all NaN: 330 us).
 // Rows on other than 16-byte boundaries are staged 4 bytes at a time: the same sums, so the same bits.
 // One multiplication and addition per state element and token more than the plain recurrence, for segments times the parallelism:
-// Back to back in a graph, 4096 tokens of 32 heads of 64 go from 405 us to 152 (57 + 6 + 92 alone), of 4 heads from 387 to 38, of 64
-// heads of 128 from 1663 to 1215.  Now bound by the fp32 pipe (63 % busy in 3., 42 % in 1.; 9 warps of up to 168 registers an SM).
+// Back to back in a graph, 4096 tokens of 32 heads of 64 go from 405 us to 144, of 4 heads from 387 to 38, of 64 heads of 128 from
+// 1663 to 1040.  Now bound by the fp32 pipe (63 % busy in 3., 42 % in 1.; 9 warps of up to 168 registers an SM).
 // Against 64 bits the outputs are as far off as token after token (1.31e-7 and 1.34e-7 of their norm), with other roundings.
 #include <cuda_runtime.h>
 #include <math.h>
@@ -450,15 +450,17 @@ __global__ void __launch_bounds__(Dp) wkv_segment_scan_kernel(const CcSeqWkv a, 
     if (__syncthreads_or(none != none)) wkv_segment_again<Dp>(a, g, sm);
 }
 
-// Segments: as many as give an SM six CTAs (what the scan's registers allow) over heads and column tiles, of at least 32 tokens.
-// With 4 / 5 / 6 / 7 / 8, back to back in a graph: 4096 tokens of 32 heads of 64 166 / 178 / 155 / 166 / 149 us, 2000 of 16 heads 49 / 52
-// / 50 / 51 / 51, 4096 of 64 heads of 128 1157 / 1152 / 1198 / 1033 / 1026 (two waves of shorter segments balance better there; not
-// measured over the range, and more segments are more work for the launch between).  The three launches follow one another in full:
-// started under each other (programmatic launch) 256 tokens of 16 heads take 32 us instead of 20.
-constexpr int MIN_LEN = 32, CTAS = 6;
+// Segments: as many as give an SM six CTAs (what the scan's registers allow) over heads and column tiles, of at least 32 tokens; eight
+// CTAs, so that a second wave of short ones evens out the first, from 2^17 tokens of a tile's columns on.  Six / eight, back to back in a
+// graph, us: 4096 tokens of 32 heads of 64 152 / 144, of 64 294 / 280, of 128 614 / 532, of 64 heads of 128 1214 / 1040, 1024 of 128 heads
+// of 64 169 / 153, 2048 of 64 157 / 154; below that line 3000 of 32 115 / 119, 4096 of 16 83 / 85, of 8 53 / 55, 1024 of 64 84 / 85 and up to
+// 700 tokens no difference (64 heads of 64 at 1500 122 / 118, 9 of 72 at 4096 165 / 158).  Nine and twelve are slower than eight.
+// The three launches follow one another in full: started under each other (programmatic launch) 256 tokens of 16 heads take 32 us
+// instead of 20.
+constexpr int MIN_LEN = 32;
 static Segments plan(int T, int H, int D) {
     const long long per = (long long)H * ((D + TILE - 1) / TILE);
-    long long most = CTAS * 148 / per;
+    long long most = (T * per >= 1 << 17 ? 8 : 6) * 148 / per;
     if (most < 1) most = 1;
     int len = (int)((T + most - 1) / most);
     if (len < MIN_LEN) len = MIN_LEN;
