@@ -23,6 +23,7 @@
 
 #include "../../../include/cc_b200_seq.h"
 #include "launch.cuh"
+#include "tensor_map.cuh"
 
 namespace ccs {
 
@@ -347,32 +348,6 @@ __global__ void __launch_bounds__(THREADS, 1) moe_tc_kernel(const __grid_constan
     }
 }
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
-                                  const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiledFn encode_fn() {
-    static const EncodeTiledFn fn = [] {
-        void* ptr = nullptr;
-        cudaDriverEntryPointQueryResult found;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &found) != cudaSuccess || found != cudaDriverEntryPointSuccess)
-            ptr = nullptr;
-        return (EncodeTiledFn)ptr;
-    }();
-    return fn;
-}
-
-// bf16 [rows, cols], row-major; boxes of 128 rows x 64 columns, columns past the end read as zero
-int make_map(CUtensorMap* tm, const void* p, long long rows, int cols) {
-    EncodeTiledFn fn = encode_fn();
-    if (!fn) return fail(CC_SEQ_ERR_CUDA, "moe_grouped: cuTensorMapEncodeTiled entry point not available");
-    cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows}, strides[1] = {(cuuint64_t)cols * 2};
-    cuuint32_t box[2] = {BK, 128}, one[2] = {1, 1};
-    if (fn(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(p), dims, strides, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE,
-           CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-        return fail(CC_SEQ_ERR_CUDA, "moe_grouped: cuTensorMapEncodeTiled failed");
-    return CC_SEQ_OK;
-}
-
 template <bool UNIT, bool GATED, bool PAIR>
 int launch_tc(const CUtensorMap& tw, const CUtensorMap& ta, const Grouped& p, int grid, cudaStream_t st) {
     auto kern = moe_tc_kernel<UNIT, GATED, PAIR>;
@@ -427,10 +402,10 @@ extern "C" int cc_seq_moe_grouped(const CcSeqMoeGrouped* a, void* stream) {
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     CUtensorMap tgu, td, tx, ta;
+    if (!map_rows(&tgu, a->wgu, wide, a->E) || !map_rows(&td, a->wd, (long long)a->n * a->E, a->F) || !map_rows(&tx, a->xs, a->M, a->E) ||
+        !map_rows(&ta, a->act, a->M, a->F))
+        return fail(CC_SEQ_ERR_CUDA, "moe_grouped: cuTensorMapEncodeTiled failed or is not available");
     int rc;
-    if ((rc = make_map(&tgu, a->wgu, wide, a->E)) || (rc = make_map(&td, a->wd, (long long)a->n * a->E, a->F)) || (rc = make_map(&tx, a->xs, a->M, a->E)) ||
-        (rc = make_map(&ta, a->act, a->M, a->F)))
-        return rc;
     const bool pair = takes_pairs(a->M, a->E, a->n, sms);
     const int tile_rows = pair ? 2 * BM : BM, workers = pair ? sms / 2 : sms;
     const long long row_tiles = (a->M + tile_rows - 1) / tile_rows + (a->n < a->M ? a->n : a->M);      // at most

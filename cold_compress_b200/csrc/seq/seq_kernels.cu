@@ -13,6 +13,7 @@
 
 #include "../../../include/cc_b200_seq.h"
 #include "launch.cuh"
+#include "tensor_map.cuh"
 
 namespace ccs {
 
@@ -1031,9 +1032,9 @@ __global__ void __launch_bounds__(VD_THREADS, RMAX <= 4 ? 2 : 1) attn_decode_row
 // that are zero) are formed again key by key with fp32 multiplications, where such operands give what they give.
 // The keys of a tile are waited for alone, its values land under the scores and the softmax.  The last CTA of a head asks for all
 // partial sums before it knows their weights, and stores the new row under them.
-// Bound: the chain of dependent waits.  Clock stamps after the wait, us: position known 0.5, keys there 4.9 (16.8 MB of rows, asked for
-// up to 4.1, at 0.6 of the HBM rate), scores 6.4, values 8.2, partials out 8.7, counter 9.5, weights of the splits 12.7, end 13.6.
-// 8 layers of 32 / 8 heads of 128, 4096 positions in a graph: 143 us on the kernel above, 109 here.  Against 64 bits (fp32 results,
+// Bound: the chain of dependent waits: position, keys, scores, softmax, values, partials and their counter, combination.  8 layers of 32 / 8
+// heads of 128, 4096 positions in a graph: 143 us on the kernel above, 109 here, 100 since the first tile's rows are asked for in L2 ahead of
+// the wait, tiles come as boxes, and slots' positions are compared after the query has been read.  Against 64 bits (fp32 results,
 // scores of size 4): 2.1e-7 of the norm, 2.4e-7 above.
 constexpr int MD_THREADS = 256, MD_WARPS = MD_THREADS / 32, MD_AHEAD = 17, MD_KEYS = 128;      // MD_KEYS: keys of a tile
 
@@ -1072,6 +1073,11 @@ __device__ __forceinline__ void md_copy_row(void* dst, const void* src, uint32_t
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_at(dst)), "l"(src), "r"(bytes),
                  "r"(smem_at(bar)) : "memory");
 }
+// 128 rows x 64 columns, swizzled, into shared memory
+__device__ __forceinline__ void md_copy_box(void* dst, const CUtensorMap* tm, int column, int row, uint64_t* bar) {
+    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(smem_at(dst)), "l"(tm),
+                 "r"(smem_at(bar)), "r"(column), "r"(row) : "memory");
+}
 // bounded: a copy that does not arrive ends the wait, not the kernel; what it leaves is then no number
 __device__ __forceinline__ bool md_bar_wait(uint64_t* bar, uint32_t parity) {
     for (uint32_t n = 0; n < (1u << 22); ++n) {
@@ -1087,30 +1093,32 @@ struct MdLayout {
     int KU, k_row, v_row;                                   // 16-byte units: padded key row, strides (odd: rows on different banks)
     size_t vs, qs, qb, ps, pb, total;                       // byte offsets
 };
-__host__ __device__ inline MdLayout md_layout(int R, int Dk, int Dv, int buffers) {
+// boxes: tiles as boxes of 64 columns, rows of 128 bytes one after another, 16-byte units swizzled by the row
+__host__ __device__ inline MdLayout md_layout(int R, int Dk, int Dv, int buffers, bool boxes) {
     constexpr int VT = MD_KEYS;
     MdLayout l;
     l.KU = 2 * ((Dk + 15) / 16);
-    l.k_row = l.KU + 1;
-    l.v_row = (Dv / 8) | 1;
+    l.k_row = boxes ? l.KU : l.KU + 1;
+    l.v_row = boxes ? Dv / 8 : (Dv / 8) | 1;
     l.vs = (size_t)buffers * VT * l.k_row * 16;
     l.qs = l.vs + ((size_t)buffers * VT * l.v_row + 1) * 16;        // one more: the second half of an odd last tile is read
     l.qb = l.qs + ((size_t)R * Dk * 4 + 15) / 16 * 16;
     l.ps = l.qb + (size_t)3 * 8 * (l.KU + 1) * 16;
     l.pb = l.ps + (size_t)8 * VT * 4;
-    l.total = l.pb + (size_t)3 * 8 * (VT + 8) * 2;
+    l.total = l.pb + (size_t)3 * 8 * (VT + 8) * 2 + (boxes ? 1024 : 0);      // and the way to a multiple of 1024
     static_assert(MD_KEYS * 3 >= MD_THREADS, "the groups' sums of the combination take the keys' place, three units a row at least");
     return l;
 }
 
-template <typename YT>
-__global__ void __launch_bounds__(MD_THREADS, 2) attn_decode_mma_kernel(const CcSeqAttn a, int buffers, int NS) {
+template <typename YT, bool BOX>
+__global__ void __launch_bounds__(MD_THREADS, 2) attn_decode_mma_kernel(const CcSeqAttn a, int buffers, int NS, const __grid_constant__ CUtensorMap k_map,
+                                                                        const __grid_constant__ CUtensorMap v_map) {
     extern __shared__ float4 smd4[];
     typedef __nv_bfloat16 CT;
     constexpr int VT = MD_KEYS;
-    uint8_t* const sm = reinterpret_cast<uint8_t*>(smd4);
+    uint8_t* const sm = reinterpret_cast<uint8_t*>(smd4) + (BOX ? (1024 - (smem_at(smd4) & 1023)) & 1023 : 0);
     const int R = a.H / a.G, Dk = a.Dk, Dv = a.Dv, kc16 = Dk / 8, vc16 = Dv / 8;
-    const MdLayout lay = md_layout(R, Dk, Dv, buffers);
+    const MdLayout lay = md_layout(R, Dk, Dv, buffers, BOX);
     const int KU = lay.KU, k_row = lay.k_row, v_row = lay.v_row, qb_row = 8 * (KU + 1);      // qb_row in elements
     uint4* const ks = reinterpret_cast<uint4*>(sm);                                 // [buffers][VT][k_row]
     uint4* const vs = reinterpret_cast<uint4*>(sm + lay.vs);                        // [buffers][VT][v_row]
@@ -1118,6 +1126,8 @@ __global__ void __launch_bounds__(MD_THREADS, 2) attn_decode_mma_kernel(const Cc
     CT* const qb = reinterpret_cast<CT*>(sm + lay.qb);                              // [3][8][qb_row] parts of q, zero beyond R and Dk
     float* const Ps = reinterpret_cast<float*>(sm + lay.ps);                        // [8][VT]
     CT* const pb = reinterpret_cast<CT*>(sm + lay.pb);                              // [3][8][VT + 8] parts of the weights, zero beyond R
+    // 16-byte unit c of a row of a tile
+    auto unit = [](uint4* t, int row, int c, int stride) { return BOX ? t + (c >> 3) * 8 * VT + row * 8 + ((c ^ row) & 7) : t + row * stride + c; };
     __shared__ int s_live[2][VT];
     __shared__ float s_M[8], s_L[8], s_corr[8], s_inv[8];
     __shared__ int s_last;
@@ -1129,15 +1139,37 @@ __global__ void __launch_bounds__(MD_THREADS, 2) attn_decode_mma_kernel(const Cc
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     for (int i = tid; i < 3 * 8 * (VT + 8) / 8; i += MD_THREADS) reinterpret_cast<uint4*>(pb)[i] = make_uint4(0, 0, 0, 0);
-    if (KU > kc16)
+    if (!BOX && KU > kc16)
         for (int i = tid; i < buffers * VT; i += MD_THREADS) ks[i * k_row + kc16] = make_uint4(0, 0, 0, 0);
     if (tid < 8) { s_M[tid] = -INFINITY; s_L[tid] = 0.f; s_corr[tid] = 0.f; s_inv[tid] = 0.f; }
+    int j_lo, kx, n, n_tiles, nsplit;                          // keys from position j_lo on behind kx kept ones; runs of n_tiles / nsplit tiles, or of one more
+    auto extent = [&](int p) {
+        j_lo = a.block > 0 ? (p / a.block) * a.block : (a.window > 0 ? max(0, p - a.window + 1) : 0);
+        kx = a.window > 0 ? min(a.keep_first, j_lo) : 0;
+        n = kx + (p - j_lo + 1);
+        n_tiles = (n + VT - 1) / VT;
+        nsplit = min(n_tiles, NS);
+    };
+    if (BOX && tid < 2) asm volatile("prefetch.tensormap [%0];" ::"l"(tid ? &v_map : &k_map) : "memory");
+    // This CTA stands here while the last CTAs of the kernel before it still run: what its first tile's rows will be is asked for in L2 by the
+    // position as it is in memory now.  It may not be this token's yet: the rows of another one are asked for then, within the cache
+    // whatever the number says, and nothing else depends on it (it is read past the L1, which must not keep it).
+    if (tid < 2) {
+        int guess;
+        asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(guess) : "l"(a.input_pos) : "memory");
+        extent(max(0, min(guess, 0x7fffffff - 2 * VT)));
+        const int tile = nsplit > sp ? (int)((long long)sp * n_tiles / nsplit) : 0, u0 = tile * VT, j0 = j_lo + (u0 - kx), ring = a.L - a.keep_first;
+        if (sp < nsplit && u0 >= kx && j0 >= a.keep_first) {
+            const int r0 = (j0 - a.keep_first) % ring, rows = min(min(VT, n - u0), ring - r0), D = tid ? Dv : Dk;
+            const CT* const at = (const CT*)(tid ? a.v_cache : a.k_cache) + ((size_t)g * a.L + a.keep_first + r0) * D;
+            asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(at), "r"((uint32_t)rows * D * 2) : "memory");
+            if (tid == 0)
+                for (int r = 0; r < rows; r += 32) ask_l2(a.pos + a.keep_first + r0 + r);
+        }
+    }
     pdl_wait_release();
     const int p = a.input_pos[0];
-    const int j_lo = a.block > 0 ? (p / a.block) * a.block : (a.window > 0 ? max(0, p - a.window + 1) : 0);
-    const int kx = a.window > 0 ? min(a.keep_first, j_lo) : 0;
-    const int n = kx + (p - j_lo + 1);
-    const int n_tiles = (n + VT - 1) / VT, nsplit = min(n_tiles, NS);      // runs of n_tiles / nsplit tiles, or of one more
+    extent(p);
     if (sp >= nsplit) return;
     const int tile0 = (int)((long long)sp * n_tiles / nsplit), tile_end = (int)((long long)(sp + 1) * n_tiles / nsplit);
     __syncthreads();      // the barriers and the zeros stand
@@ -1148,6 +1180,7 @@ __global__ void __launch_bounds__(MD_THREADS, 2) attn_decode_mma_kernel(const Cc
     const int ht = tid & (MD_THREADS / 2 - 1), D = value ? Dv : Dk, stride = value ? v_row : k_row;
     const CT* const fresh_row = value ? (const CT*)a.v_new + (size_t)g * Dv : (const CT*)a.k_new + (size_t)g * Dk;
     const CT* const cached = (value ? (const CT*)a.v_cache : (const CT*)a.k_cache) + (size_t)g * a.L * D;
+    int held = 0;
     auto fetch = [&](int tile) {
         const int b = buffers > 1 ? (tile - tile0) & 1 : 0, u0 = tile * VT, rows = min(VT, n - u0);
         uint64_t* const bar = &bars[b][value];
@@ -1157,30 +1190,78 @@ __global__ void __launch_bounds__(MD_THREADS, 2) attn_decode_mma_kernel(const Cc
             const int j = position(row);
             return j == p ? fresh_row : cached + (size_t)slot_of(a, j) * D;
         };
-        if (ht < rows) {
+        if constexpr (BOX) {
+            // One run of slots, but for the token itself, which is put over what was fetched in its place: boxes.  Otherwise a row
+            // per thread (at the end of a ring, or beside kept positions).
+            const int ring = a.L - a.keep_first, j0 = position(0), r0 = j0 >= a.keep_first ? (j0 - a.keep_first) % ring : ring;
+            const int old = rows - (u0 + rows == n ? 1 : 0);           // rows that the cache holds
+            if (u0 >= kx && r0 + old <= ring) {
+                if (ht == 0 && old > 0) {
+                    md_bar_expect(bar, (uint32_t)VT * D * 2);
+                    for (int c = 0; c < D; c += 64) md_copy_box(dst + c * (VT / 8), value ? &v_map : &k_map, c, g * a.L + a.keep_first + r0, bar);
+                } else {
+                    md_bar_arrive(bar);
+                }
+            } else {
+                if (ht < rows) {
+                    const uint4* const src = reinterpret_cast<const uint4*>(source(ht));
+#pragma unroll 8
+                    for (int c = 0; c < D / 8; ++c) *unit(dst, ht, c, stride) = src[c];
+                }
+                md_bar_arrive(bar);
+            }
+        } else if (ht < rows) {
             md_bar_expect(bar, (uint32_t)D * 2);
             md_copy_row(dst + ht * stride, source(ht), (uint32_t)D * 2, bar);
         } else {
             md_bar_arrive(bar);
         }
-        if (value) {      // no position: whatever lay there must not meet a weight of zero
+        if (value && !BOX) {      // no position: whatever lay there must not meet a weight of zero
             if (ht >= rows)
                 for (int c = 0; c < vc16; ++c) dst[ht * stride + c] = make_uint4(0, 0, 0, 0);
-        } else {
-            const int j = position(ht);
-            s_live[(tile - tile0) & 1][ht] = ht < rows && (j == p || a.pos[slot_of(a, j)] == j);
         }
+        // whether the key's slot holds its position: asked for here, looked at by mark()
+        const int j = position(ht);
+        held = ht < rows ? j : j - 1;
+        if (!value && ht < rows && j != p) held = a.pos[slot_of(a, j)];
+    };
+    auto mark = [&](int tile) {
+        const int u = tile * VT + ht, j = u < kx ? u : j_lo + (u - kx);
+        if (!value) s_live[(tile - tile0) & 1][ht] = held == j;
     };
     fetch(tile0);
-    for (int i = tid; i < 8 * KU * 8; i += MD_THREADS) {
+    // boxes: the token's own row goes over what was fetched for it, and values without a position that meet a weight of zero become zero
+    uint4 own = make_uint4(0, 0, 0, 0);
+    if (BOX && ht < D / 8 && tile_end == n_tiles) own = reinterpret_cast<const uint4*>(fresh_row)[ht];
+    auto finish = [&](int tile, uint4* t) {                  // the half of the CTA whose rows they are, before a barrier of the CTA
+        const int rows = n - tile * VT;
+        if (ht < D / 8) *unit(t, rows - 1, ht, stride) = own;
+        if (value)
+            for (int r = rows + ht / 8; r < ((rows + 15) & ~15); r += MD_THREADS / 16)      // of the 16 that a step of the product takes
+                for (int c = ht & 7; c < D / 8; c += 8) *unit(t, r, c, stride) = make_uint4(0, 0, 0, 0);
+    };
+    const bool q16 = ((uintptr_t)a.q & 15) == 0;
+    for (int i = 4 * tid; i < 8 * KU * 8; i += 4 * MD_THREADS) {      // four columns of a query row
         const int r = i / (KU * 8), d = i - r * (KU * 8);
-        float x = 0.f;
-        if (r < R && d < Dk) qs[r * Dk + d] = x = a.q[((size_t)g * R + r) * Dk + d];
-        CT part[3];
-        three_parts(x, part);
+        float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (r < R && d < Dk) {                                            // Dk is a multiple of 8
+            const float* const at = a.q + ((size_t)g * R + r) * Dk + d;
+            x = q16 ? *reinterpret_cast<const float4*>(at) : make_float4(at[0], at[1], at[2], at[3]);
+            *reinterpret_cast<float4*>(qs + r * Dk + d) = x;
+        }
+        __align__(8) CT part[3][4];
+        CT three[3];
+        const float e[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
-        for (int q = 0; q < 3; ++q) qb[(q * 8 + r) * qb_row + d] = part[q];
+        for (int c = 0; c < 4; ++c) {
+            three_parts(e[c], three);
+#pragma unroll
+            for (int q = 0; q < 3; ++q) part[q][c] = three[q];
+        }
+#pragma unroll
+        for (int q = 0; q < 3; ++q) *reinterpret_cast<uint2*>(qb + (q * 8 + r) * qb_row + d) = *reinterpret_cast<const uint2*>(part[q]);
     }
+    mark(tile0);
     const int row_r = lane >> 2, col2 = (lane & 3) * 2;      // of an accumulator
     float acc[2][2][2];                                      // [pair of column tiles][tile][column]: head row_r
 #pragma unroll
@@ -1192,10 +1273,14 @@ __global__ void __launch_bounds__(MD_THREADS, 2) attn_decode_mma_kernel(const Cc
         const int b = buffers > 1 ? (tile - tile0) & 1 : 0, u0 = tile * VT;
         const int* live = s_live[(tile - tile0) & 1];
         const uint32_t turn = (buffers > 1 ? (tile - tile0) >> 1 : tile - tile0) & 1;
-        if (buffers > 1 && tile + 1 < tile_end) fetch(tile + 1);
+        if (buffers > 1 && tile + 1 < tile_end) {
+            fetch(tile + 1);
+            mark(tile + 1);
+        }
         bool landed = md_bar_wait(&bars[b][0], turn);
+        uint4* const kt = ks + b * VT * k_row;
+        if (BOX && !value && tile == n_tiles - 1) finish(tile, kt);
         __syncthreads();
-        const uint4* const kt = ks + b * VT * k_row;
         for (int mt = warp; mt < VT / 16; mt += MD_WARPS) {
             float d[2][4], small[2][4];      // sums of even and odd steps; of the two smaller parts
 #pragma unroll
@@ -1203,7 +1288,7 @@ __global__ void __launch_bounds__(MD_THREADS, 2) attn_decode_mma_kernel(const Cc
 #pragma unroll 4
             for (int k = 0; k < KU / 2; ++k) {
                 uint32_t ka[4];
-                ldsm4(ka, kt + (16 * mt + (lane & 15)) * k_row + 2 * k + (lane >> 4));
+                ldsm4(ka, unit(kt, 16 * mt + (lane & 15), 2 * k + (lane >> 4), k_row));
                 float step[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
                 for (int q = 2; q >= 0; --q) {
@@ -1223,9 +1308,8 @@ __global__ void __launch_bounds__(MD_THREADS, 2) attn_decode_mma_kernel(const Cc
                 if (r >= R) continue;
                 float s = (d[0][e] + d[1][e]) + (small[0][e] + small[1][e]);
                 if (!finite(s) && live[k]) {
-                    const CT* kr = reinterpret_cast<const CT*>(kt + k * k_row);
                     s = 0.f;
-                    for (int c = 0; c < Dk; ++c) s = fmaf(qs[r * Dk + c], __bfloat162float(kr[c]), s);
+                    for (int c = 0; c < Dk; ++c) s = fmaf(qs[r * Dk + c], __bfloat162float(reinterpret_cast<const CT*>(unit(kt, k, c >> 3, k_row))[c & 7]), s);
                 }
                 Ps[r * VT + k] = live[k] ? shape_score(a, s * a.scale, g * R + r, p - j) : -INFINITY;
             }
@@ -1256,20 +1340,22 @@ __global__ void __launch_bounds__(MD_THREADS, 2) attn_decode_mma_kernel(const Cc
             }
         }
         landed = md_bar_wait(&bars[b][1], turn) && landed;
+        uint4* const vt = vs + b * VT * v_row;
+        if (BOX && value && tile == n_tiles - 1) finish(tile, vt);
         __syncthreads();
-        const uint4* const vt = vs + b * VT * v_row;
         const float corr = s_corr[row_r];
+        const int steps = min(VT, n - u0 + 15) >> 4;             // further rows have no position
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
             const int np = warp + MD_WARPS * i;
             if (16 * np >= Dv) break;
             float d[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}}, odd[2][2] = {{0.f, 0.f}, {0.f, 0.f}}, small[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
 #pragma unroll 4
-            for (int k = 0; k < VT / 16; ++k) {
+            for (int k = 0; k < steps; ++k) {
                 uint32_t pa[4], pc[2], vb[4];
                 ldsm4(pa, pb + (((lane >> 3) & 1) * 8 + (lane & 7)) * (VT + 8) + 16 * k + (lane >> 4) * 8);
                 ldsm2(pc, pb + (16 + (lane & 7)) * (VT + 8) + 16 * k + ((lane >> 3) & 1) * 8);
-                ldsm4_t(vb, vt + (16 * k + (lane & 15)) * v_row + 2 * np + (lane >> 4));
+                ldsm4_t(vb, unit(vt, 16 * k + (lane & 15), 2 * np + (lane >> 4), v_row));
 #pragma unroll
                 for (int t = 0; t < 2; ++t) {
                     float step[4] = {0.f, 0.f, 0.f, 0.f};
@@ -1292,7 +1378,7 @@ __global__ void __launch_bounds__(MD_THREADS, 2) attn_decode_mma_kernel(const Cc
                     if (!finite(sum) && row_r < R && c < Dv) {
                         sum = 0.f;
                         for (int k = 0; k < VT; ++k)
-                            if (live[k]) sum = fmaf(Ps[row_r * VT + k], __bfloat162float(reinterpret_cast<const CT*>(vt + k * v_row)[c]), sum);
+                            if (live[k]) sum = fmaf(Ps[row_r * VT + k], __bfloat162float(reinterpret_cast<const CT*>(unit(vt, k, c >> 3, v_row))[c & 7]), sum);
                     }
                     if (!landed) sum = NAN;
                     acc[i][t][e] = tile > tile0 ? fmaf(acc[i][t][e], corr, sum) : sum;
@@ -1300,7 +1386,10 @@ __global__ void __launch_bounds__(MD_THREADS, 2) attn_decode_mma_kernel(const Cc
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // reads before the copies that follow
         __syncthreads();      // the tile is consumed: its buffers may be filled again
-        if (buffers == 1 && tile + 1 < tile_end) fetch(tile + 1);
+        if (buffers == 1 && tile + 1 < tile_end) {
+            fetch(tile + 1);
+            mark(tile + 1);
+        }
     }
     int* counters = (int*)a.workspace;
     float* part_m = (float*)(counters + ((a.G + 3) & ~3));
@@ -1767,7 +1856,14 @@ static bool decode_mma_serves(const CcSeqAttn* a) {
 template <typename YT>
 static int launch_decode_mma(const CcSeqAttn* a, cudaStream_t st) {
     const int reach = attn_reach(*a), R = a->H / a->G;
-    auto bytes = [&](int buffers) { return md_layout(R, a->Dk, a->Dv, buffers).total; };
+    // Tiles as boxes of one TMA copy per 64 columns where rows are whole boxes wide, by a copy per row otherwise.  8 layers with L2 flushed
+    // before, start / rows / boxes in us (the first without what is asked for ahead of the wait): 32 / 8 heads of 128, 300 positions
+    // 90 / 88 / 82, 4096 119 / 104 / 104, 12000 229 / 221 / 203; 16 / 4 at 1000 92 / 90 / 84, in a window of 1000 92 / 90 / 82.
+    const long long rows = (long long)a->G * a->L;
+    CUtensorMap k_map = {}, v_map = {};
+    const bool boxes = a->Dk % 64 == 0 && a->Dv % 64 == 0 && rows >= MD_KEYS && rows < (1ll << 31) - MD_KEYS && map_rows(&k_map, a->k_cache, rows, a->Dk) &&
+                       map_rows(&v_map, a->v_cache, rows, a->Dv);
+    auto bytes = [&](int buffers) { return md_layout(R, a->Dk, a->Dv, buffers, boxes).total; };
     const size_t half = 111 * 1024, all = 223 * 1024;
     // Two CTAs per SM where a tile fits half of the shared memory, one otherwise (rows of 256 + 256 fit it whole).  8 / 2 heads of
     // 256, 300 / 2000 / 4096 / 8000 positions, us a layer: two CTAs with tiles of 64 keys 12.0 / 16.3 / 27.2 / 29.3, one of 128
@@ -1776,10 +1872,10 @@ static int launch_decode_mma(const CcSeqAttn* a, cudaStream_t st) {
     const long long tiles = vd_tiles(a->L, reach, MD_KEYS);
     const int NS = vd_splits(tiles, a->G, per_sm), buffers = tiles > NS && bytes(2) <= (per_sm == 2 ? half : all) ? 2 : 1;
     const size_t smem = bytes(buffers);
-    auto kern = attn_decode_mma_kernel<YT>;
+    auto kern = boxes ? attn_decode_mma_kernel<YT, true> : attn_decode_mma_kernel<YT, false>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return fail(CC_SEQ_ERR_CUDA, cudaGetErrorString(e));
-    launch_under(kern, dim3(NS, a->G), dim3(MD_THREADS), smem, st, *a, buffers, NS);
+    launch_under(kern, dim3(NS, a->G), dim3(MD_THREADS), smem, st, *a, buffers, NS, k_map, v_map);
     return cuda_check("attn_decode_mma_kernel");
 }
 
