@@ -53,7 +53,7 @@ class CcTpArgs(C.Structure):
 class CcPrefillAttnArgs(C.Structure):
     _fields_ = [f for t in "qkvy" for f in ((t, C.c_void_p), (f"{t}_stride_s", C.c_int64), (f"{t}_stride_h", C.c_int64))] + [
         (n, C.c_int32) for n in ("seq_len", "n_kv_heads", "q_per_kv", "head_dim", "attn_mode", "obs_len", "n_windows")] + [
-        ("windows", C.c_int32 * 4), ("reserved0", C.c_int32)] + [
+        ("windows", C.c_int32 * 4), ("stats_bf16", C.c_int32)] + [
         (n, C.c_void_p) for n in ("col_sum", "obs_sum", "band_sum", "workspace")] + [("workspace_bytes", C.c_uint64)]
 
 

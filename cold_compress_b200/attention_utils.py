@@ -71,7 +71,7 @@ def prefill_attention_stats(q, k, v, obs_len: int = 16, windows=()):
     q [1, Hq, S, D], k/v [1, Hkv, S, D] (bf16, post-RoPE; any row/head strides).  Returns
     (y [1, Hq, S, D], PrefillAttnStats).  ONE tcgen05 kernel (csrc/prefill_attn.cu) + a fixed-order reduction
     of its per-tile partial sums; the reference's rounding points (naive path) are applied in the kernel,
-    the final bf16 roundings of the reductions (prompt_compression.py:175, 192) here."""
+    the final bf16 roundings of the reductions (prompt_compression.py:175, 192) in the reduction."""
     if not q.is_cuda:
         raise _lib.CcError("prefill_attention_stats is CUDA-only (cc_prefill_attention); there is no CPU path")
     _, Hq, S, D = q.shape
@@ -81,12 +81,11 @@ def prefill_attention_stats(q, k, v, obs_len: int = 16, windows=()):
     windows = [int(w) for w in windows]
     dev = q.device
     y = torch.empty(S, Hq, D, dtype=q.dtype, device=dev)
-    col = torch.empty(Hkv, S, dtype=torch.float32, device=dev)
-    obs = torch.empty(Hkv, S, dtype=torch.float32, device=dev)
+    col = torch.empty(1, Hkv, S, dtype=q.dtype, device=dev)
+    obs = torch.empty(1, Hkv, S, dtype=q.dtype, device=dev)
     band = torch.empty(len(windows), Hkv, S, dtype=torch.float32, device=dev) if windows else None
     ws = _scratch(dev, ops.prefill_attention_workspace(S, Hkv, G, obs_len, len(windows)))
     ops.prefill_attention(q[0], k[0], v[0], y.permute(1, 0, 2), _lib.ATTN_NAIVE_BF16, obs_len, windows, col, obs, band, ws)
-    stats = PrefillAttnStats(col_sum=col.to(q.dtype).unsqueeze(0),
-                             obs_mean=(obs / obs_len).to(q.dtype).unsqueeze(0), obs_len=obs_len,
+    stats = PrefillAttnStats(col_sum=col, obs_mean=obs, obs_len=obs_len,
                              band_sum={w: band[i] for i, w in enumerate(windows)} if windows else None)
     return y.permute(1, 0, 2).unsqueeze(0), stats

@@ -785,22 +785,29 @@ __device__ __forceinline__ float sum_tiles(const float* __restrict__ part, size_
     return acc;
 }
 
-// Fixed-order sum of the per-tile partials: one thread per (head, column).  Bound: latency, a column's sum is a chain of
+// Fixed-order sum of the per-tile partials, rounded for its consumers on the way out (three launches of tensor operations behind it: 8 of
+// the 81 us that 1531 tokens took): one thread per (head, column).  Bound: latency, a column's sum is a chain of
 // as many loads as there are query tiles behind it; so RED_AHEAD of them are under way at once and the CTAs are small
 // enough that short prompts reach most of the chip.  Measured at 7680 / 4096 tokens x 8 heads and 1531 x 4 in groups of 7:
 // 16.8 / 8.9 / 5.5 us; CTAs of 256 with the loop as the compiler unrolls it 37.9 / 18.7 / 11.9.
+// BF16: as the consumers take them, the column sums and the mean of the observed rows in bf16; fp32 sums otherwise.
+template <bool BF16>
 __global__ void __launch_bounds__(RED_THREADS)
-prefill_reduce_kernel(const __grid_constant__ PrefillParams p, float* __restrict__ col_sum, float* __restrict__ obs_sum,
-                      float* __restrict__ band_sum) {
+prefill_reduce_kernel(const __grid_constant__ PrefillParams p, void* __restrict__ col_sum, void* __restrict__ obs_sum,
+                      float* __restrict__ band_sum, float per_obs_row) {
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     const int h = blockIdx.y;
     if (j >= p.S) return;
-    const size_t slab = (size_t)p.S_pad;
+    const size_t slab = (size_t)p.S_pad, at = (size_t)h * p.S + j;
     const int qt0 = j / p.QB;
-    col_sum[(size_t)h * p.S + j] = sum_tiles(p.part_col + (size_t)h * p.n_qtiles * slab + j, slab, qt0, p.n_qtiles);
+    const float col = sum_tiles(p.part_col + (size_t)h * p.n_qtiles * slab + j, slab, qt0, p.n_qtiles);
+    if (BF16) ((__nv_bfloat16*)col_sum)[at] = __float2bfloat16_rn(col);
+    else ((float*)col_sum)[at] = col;
     if (obs_sum) {
         const int first = max(qt0, p.first_obs_tile) - p.first_obs_tile;
-        obs_sum[(size_t)h * p.S + j] = sum_tiles(p.part_obs + (size_t)h * p.n_obs_tiles * slab + j, slab, first, p.n_obs_tiles);
+        const float obs = sum_tiles(p.part_obs + (size_t)h * p.n_obs_tiles * slab + j, slab, first, p.n_obs_tiles);
+        if (BF16) ((__nv_bfloat16*)obs_sum)[at] = __float2bfloat16_rn(__fmul_rn(obs, per_obs_row));
+        else ((float*)obs_sum)[at] = obs;
     }
     for (int w = 0; w < p.n_windows; ++w) {
         const int qt1 = min(p.n_qtiles - 1, (j + p.windows[w] - 1) / p.QB);   // later query tiles are outside the band
@@ -963,7 +970,9 @@ int prefill_attention_impl(const CcPrefillAttnArgs* a, cudaStream_t stream) {
     if (rc != CC_OK) return rc;
     if (stats) {
         dim3 rgrid((S + RED_THREADS - 1) / RED_THREADS, Hkv);
-        prefill_reduce_kernel<<<rgrid, RED_THREADS, 0, stream>>>(p, a->col_sum, obs_len > 0 ? a->obs_sum : nullptr, a->band_sum);
+        auto reduce = a->stats_bf16 ? prefill_reduce_kernel<true> : prefill_reduce_kernel<false>;
+        reduce<<<rgrid, RED_THREADS, 0, stream>>>(p, a->col_sum, obs_len > 0 ? a->obs_sum : nullptr, a->band_sum,
+                                                  obs_len > 0 ? 1.0f / (float)obs_len : 0.f);
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return set_cuda_error(e, "cc_prefill_attention reduce launch");
     }

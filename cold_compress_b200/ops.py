@@ -143,6 +143,10 @@ def _prefill_attention(q, k, v, y, attn_mode, obs_len, windows, col_sum, obs_sum
     for i, w in enumerate(windows):
         a.windows[i] = int(w)
     a.col_sum, a.obs_sum, a.band_sum = _optr(col_sum), _optr(obs_sum), _optr(band_sum)
+    if col_sum is not None:
+        if col_sum.dtype not in (torch.float32, torch.bfloat16) or (obs_sum is not None and obs_sum.dtype != col_sum.dtype):
+            raise _lib.CcError("prefill_attention: col_sum and obs_sum are both fp32 (sums) or both bf16 (sums, mean over the observed rows)")
+        a.stats_bf16 = int(col_sum.dtype == torch.bfloat16)
     a.workspace = _optr(workspace)
     a.workspace_bytes = 0 if workspace is None else workspace.numel() * workspace.element_size()
     _lib.check(_lib.load().cc_prefill_attention(C.byref(a), _stream()), "cc_prefill_attention")

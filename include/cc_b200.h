@@ -241,9 +241,9 @@ typedef struct CcPrefillAttnArgs {
     int32_t obs_len;         /* SnapKV observation window (prompt_compression.py:157) */
     int32_t n_windows;       /* 0..4                                        */
     int32_t windows[4];      /* window sizes in tokens                      */
-    int32_t reserved0;
-    float*  col_sum;
-    float*  obs_sum;
+    int32_t stats_bf16;      /* 0: col_sum, obs_sum fp32.  1: bf16, col_sum rounded and obs_sum the mean over the observed rows */
+    void*   col_sum;
+    void*   obs_sum;
     float*  band_sum;
     void*   workspace;
     uint64_t workspace_bytes;
