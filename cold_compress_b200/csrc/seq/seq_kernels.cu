@@ -1033,9 +1033,8 @@ __global__ void __launch_bounds__(VD_THREADS, RMAX <= 4 ? 2 : 1) attn_decode_row
 // The keys of a tile are waited for alone, its values land under the scores and the softmax.  The last CTA of a head asks for all
 // partial sums before it knows their weights, and stores the new row under them.
 // Bound: the chain of dependent waits: position, keys, scores, softmax, values, partials and their counter, combination.  8 layers of 32 / 8
-// heads of 128, 4096 positions in a graph: 143 us on the kernel above, 109 here, 100 since the first tile's rows are asked for in L2 ahead of
-// the wait, tiles come as boxes, and slots' positions are compared after the query has been read.  Against 64 bits (fp32 results,
-// scores of size 4): 2.1e-7 of the norm, 2.4e-7 above.
+// heads of 128, 4096 positions in a graph: 143 us on the kernel above, 109 here, 107 since tiles come as boxes and slots' positions are
+// compared after the query has been read.  Against 64 bits (fp32 results, scores of size 4): 2.1e-7 of the norm, 2.4e-7 above.
 constexpr int MD_THREADS = 256, MD_WARPS = MD_THREADS / 32, MD_AHEAD = 17, MD_KEYS = 128;      // MD_KEYS: keys of a tile
 
 __device__ __forceinline__ uint32_t smem_at(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -1142,34 +1141,13 @@ __global__ void __launch_bounds__(MD_THREADS, 2) attn_decode_mma_kernel(const Cc
     if (!BOX && KU > kc16)
         for (int i = tid; i < buffers * VT; i += MD_THREADS) ks[i * k_row + kc16] = make_uint4(0, 0, 0, 0);
     if (tid < 8) { s_M[tid] = -INFINITY; s_L[tid] = 0.f; s_corr[tid] = 0.f; s_inv[tid] = 0.f; }
-    int j_lo, kx, n, n_tiles, nsplit;                          // keys from position j_lo on behind kx kept ones; runs of n_tiles / nsplit tiles, or of one more
-    auto extent = [&](int p) {
-        j_lo = a.block > 0 ? (p / a.block) * a.block : (a.window > 0 ? max(0, p - a.window + 1) : 0);
-        kx = a.window > 0 ? min(a.keep_first, j_lo) : 0;
-        n = kx + (p - j_lo + 1);
-        n_tiles = (n + VT - 1) / VT;
-        nsplit = min(n_tiles, NS);
-    };
     if (BOX && tid < 2) asm volatile("prefetch.tensormap [%0];" ::"l"(tid ? &v_map : &k_map) : "memory");
-    // This CTA stands here while the last CTAs of the kernel before it still run: what its first tile's rows will be is asked for in L2 by the
-    // position as it is in memory now.  It may not be this token's yet: the rows of another one are asked for then, within the cache
-    // whatever the number says, and nothing else depends on it (it is read past the L1, which must not keep it).
-    if (tid < 2) {
-        int guess;
-        asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(guess) : "l"(a.input_pos) : "memory");
-        extent(max(0, min(guess, 0x7fffffff - 2 * VT)));
-        const int tile = nsplit > sp ? (int)((long long)sp * n_tiles / nsplit) : 0, u0 = tile * VT, j0 = j_lo + (u0 - kx), ring = a.L - a.keep_first;
-        if (sp < nsplit && u0 >= kx && j0 >= a.keep_first) {
-            const int r0 = (j0 - a.keep_first) % ring, rows = min(min(VT, n - u0), ring - r0), D = tid ? Dv : Dk;
-            const CT* const at = (const CT*)(tid ? a.v_cache : a.k_cache) + ((size_t)g * a.L + a.keep_first + r0) * D;
-            asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(at), "r"((uint32_t)rows * D * 2) : "memory");
-            if (tid == 0)
-                for (int r = 0; r < rows; r += 32) ask_l2(a.pos + a.keep_first + r0 + r);
-        }
-    }
     pdl_wait_release();
     const int p = a.input_pos[0];
-    extent(p);
+    const int j_lo = a.block > 0 ? (p / a.block) * a.block : (a.window > 0 ? max(0, p - a.window + 1) : 0);
+    const int kx = a.window > 0 ? min(a.keep_first, j_lo) : 0;
+    const int n = kx + (p - j_lo + 1);
+    const int n_tiles = (n + VT - 1) / VT, nsplit = min(n_tiles, NS);      // runs of n_tiles / nsplit tiles, or of one more
     if (sp >= nsplit) return;
     const int tile0 = (int)((long long)sp * n_tiles / nsplit), tile_end = (int)((long long)(sp + 1) * n_tiles / nsplit);
     __syncthreads();      // the barriers and the zeros stand
@@ -1857,8 +1835,9 @@ template <typename YT>
 static int launch_decode_mma(const CcSeqAttn* a, cudaStream_t st) {
     const int reach = attn_reach(*a), R = a->H / a->G;
     // Tiles as boxes of one TMA copy per 64 columns where rows are whole boxes wide, by a copy per row otherwise.  8 layers with L2 flushed
-    // before, start / rows / boxes in us (the first without what is asked for ahead of the wait): 32 / 8 heads of 128, 300 positions
-    // 90 / 88 / 82, 4096 119 / 104 / 104, 12000 229 / 221 / 203; 16 / 4 at 1000 92 / 90 / 84, in a window of 1000 92 / 90 / 82.
+    // before, us by rows / by boxes: 32 / 8 heads of 128, 300 positions 90 / 80, 4096 119 / 117, 12000 229 / 215; 16 / 4 at 1000 92 / 84, in a
+    // window of 1000 92 / 84.  (The rows asked for in L2 ahead of the wait, by the position that memory held then, gave 104 at 4096 and 203
+    // at 12000; but no value is taken from memory there.)
     const long long rows = (long long)a->G * a->L;
     CUtensorMap k_map = {}, v_map = {};
     const bool boxes = a->Dk % 64 == 0 && a->Dv % 64 == 0 && rows >= MD_KEYS && rows < (1ll << 31) - MD_KEYS && map_rows(&k_map, a->k_cache, rows, a->Dk) &&
