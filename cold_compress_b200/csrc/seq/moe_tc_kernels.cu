@@ -5,16 +5,16 @@
 // come to the host; at 2048 tokens and 16 experts of 1536 that was 32 products of ~450 rows with the GPU idle before and
 // between them, and the gate and up rows made a round trip through memory in fp32.
 //
-// A persistent CTA per SM walks 128 x 256 tiles, or a pair of CTAs 256 x 256 ones, expert by expert, the row tiles of one weight tile next
-// to one another so that the weights are read from HBM once.  Both operands come by TMA: the token rows are gathered by a copy kernel first
-// (fetched row by row with cp.async inside the product they held the tensor pipe at 23 %: 237 us where the TMA form took
+// A persistent CTA per SM walks 128 x 256 tiles, expert by expert, the row tiles of one weight tile next to one another so
+// that the weights are read from HBM once.  Both operands come by TMA: the token rows are gathered by a copy kernel first
+// (fetched row by row with cp.async inside the product they held the tensor pipe at 23 %: 237 us where the TMA form takes
 // 96 and the copy 10; 2048 tokens, 4 of 16 experts of 1536, width 2048).  A gated tile holds 128 gate columns beside the 128 up columns they
 // belong to, so the unit is applied on the way out of tensor memory, four warps emptying one accumulator while the next tile
 // fills the other; fp32 results go by way of shared memory, so that rows are stored as whole lines (the unit's bf16 results that way:
-// 10 us slower at 400 to 512 tokens).
-// Bound: what an SM takes from L2 and, from 4096 tokens on, power.  A 128 x 256 x 64 stage is 48 KB for 512 cycles of MMAs; of a pair each CTA
-// brings its own rows and half of the weights, 32 KB for the same MMAs.  Both products of that case with gathering and grouping: 171 us,
-// results as whole lines 166, pairs 156.
+// 10 us slower at 400 to 512 tokens).  Bound: the 64 bytes per clock that an SM takes from L2; a 128 x 256 x 64 stage is 48 KB (768 cycles) for
+// 512 cycles of MMAs.  The whole mixture with a shared expert of 2048 in a graph, over seconds: results 16 bytes of a row at a time and
+// MMAs issued by one thread 247 us, this 240; 4096 tokens 430 / 416; experts of 1000 216 / 207; 1024 tokens 152 / 146.  Pairs of CTAs
+// (cta_group::2) on 256 x 256 tiles, which read half of the weights each: 254, 422, 215 and 158.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -34,12 +34,8 @@ namespace {
 
 typedef __nv_bfloat16 bf16;
 
-constexpr int BM = 128, BN = 256, BK = 64;      // BM: rows of a CTA; BK: one 128-byte swizzled row of a tile
-constexpr int A_BYTES = BM * 128, OUT_BYTES = 4 * 32 * 128;
-// A CTA alone holds 128 rows and all 256 weight rows of its tile; of a pair each CTA holds its 128 of 256 rows and half of the weights.
-template <bool PAIR> struct Stage {
-    static constexpr int B_ROWS = PAIR ? BN / 2 : BN, BYTES = A_BYTES + B_ROWS * 128, N = PAIR ? 6 : 4, TILE_ROWS = PAIR ? 2 * BM : BM;
-};
+constexpr int BM = 128, BN = 256, BK = 64;      // BK: one 128-byte swizzled row of a tile
+constexpr int STAGES = 4, A_BYTES = BM * 128, B_BYTES = BN * 128, STAGE_BYTES = A_BYTES + B_BYTES, OUT_BYTES = 4 * 32 * 128;
 constexpr int W_OUT = 4, W_MMA = 4, W_TMA = 5, THREADS = 192;   // warps 0-3 empty tensor memory
 constexpr uint32_t WAIT_LIMIT = 1u << 22;
 
@@ -76,44 +72,17 @@ __device__ __forceinline__ bool elect_one() {
     asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(one));
     return one != 0;
 }
-template <bool PAIR>
+constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
 __device__ __forceinline__ void mma_ss(uint32_t d, uint64_t a, uint64_t b, uint32_t acc) {
-    constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(Stage<PAIR>::TILE_ROWS >> 4) << 24);
-    if constexpr (PAIR)
-        asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n}\n"
-                     ::"r"(d), "l"(a), "l"(b), "r"(IDESC), "r"(acc) : "memory");
-    else
-        asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
-                     ::"r"(d), "l"(a), "l"(b), "r"(IDESC), "r"(acc) : "memory");
+    asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
+                 ::"r"(d), "l"(a), "l"(b), "r"(IDESC), "r"(acc) : "memory");
 }
-// arrives on the barrier at this place, of a pair in both CTAs
-template <bool PAIR>
 __device__ __forceinline__ void mma_commit(uint32_t bar) {
-    if constexpr (PAIR)
-        asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"((uint16_t)3) : "memory");
-    else
-        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
-// into this CTA's memory; the barrier may be the other CTA's of a pair
-template <bool PAIR>
 __device__ __forceinline__ void tma_load(uint32_t dst, const CUtensorMap* tm, int x, int y, uint32_t bar) {
-    if constexpr (PAIR)
-        asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-                     ::"r"(dst), "l"(tm), "r"(bar), "r"(x), "r"(y) : "memory");
-    else
-        asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-                     ::"r"(dst), "l"(tm), "r"(bar), "r"(x), "r"(y) : "memory");
-}
-__device__ __forceinline__ uint32_t in_cta(uint32_t addr, uint32_t rank) {
-    uint32_t r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
-    return r;
-}
-__device__ __forceinline__ void mbar_arrive_in(uint32_t bar) {
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+                 ::"r"(dst), "l"(tm), "r"(bar), "r"(x), "r"(y) : "memory");
 }
 __device__ __forceinline__ void tmem_ld32(uint32_t t, float* v) {
     asm volatile(
@@ -146,13 +115,13 @@ struct Grouped {
     int kind;
 };
 
-// The tiles in order: expert, column tile, row tile.  A role walks the ids of its CTA or pair: first, + step, ...
+// The tiles in order: expert, column tile, row tile.  A role walks the ids blockIdx.x, + gridDim.x, ...
 struct Walk {
     int e, first_row, first_id, rows, row_tiles, col_tiles;
     const int32_t* counts;
-    int n, tile_rows;
-    __device__ __forceinline__ void start(const int32_t* c, int n_experts, int ct, int tr) {
-        counts = c; n = n_experts; col_tiles = ct; tile_rows = tr;
+    int n;
+    __device__ __forceinline__ void start(const int32_t* c, int n_experts, int ct) {
+        counts = c; n = n_experts; col_tiles = ct;
         e = -1; first_row = 0; first_id = 0; rows = 0; row_tiles = 0;
     }
     // moves on to the expert of tile `id`; false when there is none
@@ -161,7 +130,7 @@ struct Walk {
             if (e >= 0) { first_id += row_tiles * col_tiles; first_row += rows; }
             if (++e >= n) return false;
             rows = counts[e];
-            row_tiles = (rows + tile_rows - 1) / tile_rows;
+            row_tiles = (rows + BM - 1) / BM;
         }
         return true;
     }
@@ -170,7 +139,7 @@ struct Walk {
 };
 
 struct Small {
-    uint64_t bars[2 * 6 + 4];          // full, empty, accumulator full[2], empty[2]
+    uint64_t bars[2 * STAGES + 4];     // full, empty, accumulator full[2], empty[2]
     uint32_t tmem;
     int failed;
 };
@@ -187,16 +156,13 @@ __global__ void __launch_bounds__(256) moe_rows_kernel(const uint4* __restrict__
 }
 
 // GATED: 128 gate and 128 up columns per tile, out = unit(gate) up.  UNIT: the first product (bf16 out through the unit),
-// otherwise the second (fp32 out).  PAIR: two CTAs (a cluster) on a tile of 256 rows, the first of which issues the MMAs of both.
-template <bool UNIT, bool GATED, bool PAIR>
+// otherwise the second (fp32 out).
+template <bool UNIT, bool GATED>
 __global__ void __launch_bounds__(THREADS, 1) moe_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_a, const Grouped p) {
-    typedef Stage<PAIR> S;
-    constexpr int STAGES = S::N;
     extern __shared__ __align__(1024) uint8_t smem_raw[];      // the stages, results on their way out, then Small: no static shared memory in front of them
-    uint8_t* const outs = smem_raw + STAGES * S::BYTES;
+    uint8_t* const outs = smem_raw + STAGES * STAGE_BYTES;
     Small& sm = *reinterpret_cast<Small*>(outs + OUT_BYTES);
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
-    const int rank = PAIR ? blockIdx.x & 1 : 0, first_tile = PAIR ? blockIdx.x >> 1 : blockIdx.x, step = PAIR ? gridDim.x >> 1 : gridDim.x;
     const uint32_t base = smem_u32(smem_raw), bar = smem_u32(sm.bars);
     const uint32_t FULL = bar, EMPTY = bar + 8 * STAGES, ACC_FULL = bar + 16 * STAGES, ACC_EMPTY = ACC_FULL + 16;
     volatile int* const failed = &sm.failed;
@@ -208,22 +174,16 @@ __global__ void __launch_bounds__(THREADS, 1) moe_tc_kernel(const __grid_constan
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(ACC_FULL + 8 * b, 1);
-            mbar_init(ACC_EMPTY + 8 * b, PAIR ? 2 * W_OUT : W_OUT);
+            mbar_init(ACC_EMPTY + 8 * b, W_OUT);
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) {
-        if constexpr (PAIR) {
-            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sm.tmem)), "r"(512) : "memory");
-            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
-        } else {
-            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sm.tmem)), "r"(512) : "memory");
-            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-        }
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sm.tmem)), "r"(512) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     fence_before();
     __syncthreads();
-    if constexpr (PAIR) cluster_sync();                        // the barriers of both stand
     fence_after();
     const uint32_t tmem = sm.tmem;
     pdl_wait_release();
@@ -231,61 +191,58 @@ __global__ void __launch_bounds__(THREADS, 1) moe_tc_kernel(const __grid_constan
     const int cols = GATED ? BN / 2 : BN;          // output columns of a tile
     const int k_iters = (p.K + BK - 1) / BK;
     Walk w;
-    w.start(p.counts, p.n, (p.N + cols - 1) / cols, S::TILE_ROWS);
+    w.start(p.counts, p.n, (p.N + cols - 1) / cols);
 
     if (warp == W_TMA) {
         if (lane == 0) {
-            const uint32_t full = PAIR ? in_cta(FULL, 0) : FULL;      // a pair's copies count in the first CTA
             int it = 0;
-            for (int id = first_tile; w.seek(id) && !*failed; id += step) {
-                const int c0 = w.col_tile(id) * cols, r0 = w.first_row + w.row_tile(id) * S::TILE_ROWS + rank * BM;
+            for (int id = blockIdx.x; w.seek(id) && !*failed; id += gridDim.x) {
+                const int c0 = w.col_tile(id) * cols, r0 = w.first_row + w.row_tile(id) * BM;
                 const int b0 = w.e * p.w_rows + c0, b1 = GATED ? b0 + p.N : b0 + BN / 2;
                 for (int k = 0; k < k_iters; ++k, ++it) {
                     const int s = it % STAGES;
                     if (it >= STAGES) mbar_wait(EMPTY + 8 * s, (it / STAGES - 1) & 1, failed);
                     if (*failed) break;
-                    const uint32_t sA = base + s * S::BYTES, sB = sA + A_BYTES;
-                    if (rank == 0) mbar_expect(FULL + 8 * s, PAIR ? 2 * S::BYTES : S::BYTES);
-                    tma_load<PAIR>(sB, &tm_w, k * BK, PAIR && rank ? b1 : b0, full + 8 * s);
-                    if constexpr (!PAIR) tma_load<PAIR>(sB + S::B_ROWS / 2 * 128, &tm_w, k * BK, b1, full + 8 * s);
-                    tma_load<PAIR>(sA, &tm_a, k * BK, r0, full + 8 * s);
+                    const uint32_t sA = base + s * STAGE_BYTES, sB = sA + A_BYTES;
+                    mbar_expect(FULL + 8 * s, STAGE_BYTES);
+                    tma_load(sB, &tm_w, k * BK, b0, FULL + 8 * s);
+                    tma_load(sB + B_BYTES / 2, &tm_w, k * BK, b1, FULL + 8 * s);
+                    tma_load(sA, &tm_a, k * BK, r0, FULL + 8 * s);
                 }
             }
-            if (*failed && rank == 0)      // the copies under way end before the CTAs do
+            if (*failed)      // the copies under way end before the CTA does
                 for (int m = it < STAGES ? 0 : it - STAGES; m < it; ++m)
                     for (uint32_t n = 0; n < WAIT_LIMIT && !mbar_try(FULL + 8 * (m % STAGES), (m / STAGES) & 1); ++n) {}
         }
         __syncwarp();
     } else if (warp == W_MMA) {
-        if (rank == 0) {
-            int s = 0, n_tile = 0;
-            uint32_t turn = 0;
-            const uint64_t a_desc = smem_desc(base), b_desc = smem_desc(base + A_BYTES);
-            for (int id = first_tile; w.seek(id) && !*failed; id += step, ++n_tile) {
-                const int b = n_tile & 1;
-                if (n_tile >= 2) mbar_wait(ACC_EMPTY + 8 * b, (n_tile / 2 - 1) & 1, failed);
-                for (int k = 0; k < k_iters; ++k) {
-                    mbar_wait(FULL + 8 * s, turn, failed);
-                    __syncwarp();
-                    fence_after();
-                    if (elect_one()) {
-                        const uint64_t at = s * (S::BYTES >> 4);
+        int s = 0, n_tile = 0;
+        uint32_t turn = 0;
+        const uint64_t a_desc = smem_desc(base), b_desc = smem_desc(base + A_BYTES);
+        for (int id = blockIdx.x; w.seek(id) && !*failed; id += gridDim.x, ++n_tile) {
+            const int b = n_tile & 1;
+            if (n_tile >= 2) mbar_wait(ACC_EMPTY + 8 * b, (n_tile / 2 - 1) & 1, failed);
+            for (int k = 0; k < k_iters; ++k) {
+                mbar_wait(FULL + 8 * s, turn, failed);
+                __syncwarp();
+                fence_after();
+                if (elect_one()) {
+                    const uint64_t at = s * (STAGE_BYTES >> 4);
 #pragma unroll
-                        for (int kk = 0; kk < BK / 16; ++kk) mma_ss<PAIR>(tmem + b * BN, a_desc + at + 2 * kk, b_desc + at + 2 * kk, k > 0 || kk > 0);
-                        mma_commit<PAIR>(EMPTY + 8 * s);
-                        if (k == k_iters - 1) mma_commit<PAIR>(ACC_FULL + 8 * b);
-                    }
-                    __syncwarp();
-                    if (++s == STAGES) { s = 0; turn ^= 1; }
+                    for (int kk = 0; kk < BK / 16; ++kk) mma_ss(tmem + b * BN, a_desc + at + 2 * kk, b_desc + at + 2 * kk, k > 0 || kk > 0);
+                    mma_commit(EMPTY + 8 * s);
+                    if (k == k_iters - 1) mma_commit(ACC_FULL + 8 * b);
                 }
+                __syncwarp();
+                if (++s == STAGES) { s = 0; turn ^= 1; }
             }
         }
     } else {
         int n_tile = 0;
-        const uint32_t lanes = (uint32_t)(warp * 32) << 16, free_bar = PAIR ? in_cta(ACC_EMPTY, 0) : ACC_EMPTY;
+        const uint32_t lanes = (uint32_t)(warp * 32) << 16;
         uint8_t* const mine = outs + warp * 32 * 128;           // 32 rows of 128 bytes, 16-byte chunks swizzled by the row
-        for (int id = first_tile; w.seek(id); id += step, ++n_tile) {
-            const int b = n_tile & 1, c0 = w.col_tile(id) * cols, row0 = w.row_tile(id) * S::TILE_ROWS + rank * BM + warp * 32;
+        for (int id = blockIdx.x; w.seek(id); id += gridDim.x, ++n_tile) {
+            const int b = n_tile & 1, c0 = w.col_tile(id) * cols, row0 = w.row_tile(id) * BM + warp * 32;
             mbar_wait(ACC_FULL + 8 * b, (n_tile / 2) & 1, failed);
             __syncwarp();
             fence_after();
@@ -333,56 +290,23 @@ __global__ void __launch_bounds__(THREADS, 1) moe_tc_kernel(const __grid_constan
             }
             fence_before();
             __syncwarp();
-            if (lane == 0) {
-                if constexpr (PAIR) mbar_arrive_in(free_bar + 8 * b);
-                else mbar_arrive(free_bar + 8 * b);
-            }
+            if (lane == 0) mbar_arrive(ACC_EMPTY + 8 * b);
         }
     }
     fence_before();
     __syncthreads();
-    if constexpr (PAIR) cluster_sync();                        // nobody reads or arrives here any more
-    if (warp == 0) {
-        if constexpr (PAIR) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
-        else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
-    }
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
 }
 
-template <bool UNIT, bool GATED, bool PAIR>
+template <bool UNIT, bool GATED>
 int launch_tc(const CUtensorMap& tw, const CUtensorMap& ta, const Grouped& p, int grid, cudaStream_t st) {
-    auto kern = moe_tc_kernel<UNIT, GATED, PAIR>;
-    const int smem = Stage<PAIR>::N * Stage<PAIR>::BYTES + OUT_BYTES + (int)sizeof(Small);
+    auto kern = moe_tc_kernel<UNIT, GATED>;
+    const int smem = STAGES * STAGE_BYTES + OUT_BYTES + (int)sizeof(Small);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return fail(CC_SEQ_ERR_CUDA, cudaGetErrorString(e));
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(THREADS);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[2];
-    int n = 0;
-    if (pdl_enabled()) {
-        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[n++].val.programmaticStreamSerializationAllowed = 1;
-    }
-    if (PAIR) {
-        attr[n].id = cudaLaunchAttributeClusterDimension;
-        attr[n].val.clusterDim.x = 2;
-        attr[n].val.clusterDim.y = attr[n].val.clusterDim.z = 1;
-        ++n;
-    }
-    cfg.attrs = attr;
-    cfg.numAttrs = n;
-    cudaLaunchKernelEx(&cfg, kern, tw, ta, p);
+    launch_under(kern, dim3(grid), dim3(THREADS), smem, st, tw, ta, p);
     return cuda_check("moe_tc_kernel");
 }
-
-// Pairs read half of the weights per CTA but need 256 rows of an expert to fill a tile, and their two CTAs wait for one another on every
-// accumulator.  Both products with gathering and grouping, 4 of 16 experts, CTAs alone / pairs in us: width 2048, experts of 1536, 700 tokens (175
-// rows an expert) 101 / 94, 1024 105 / 98, 2048 166 / 156, 4096 273 / 267; of 1000 86 / 79, 88 / 82, 140 / 126, 225 / 205; of 512 59 / 58 to
-// 142 / 139; below that, 560 tokens of 768 63 / 70, 8 of 1536 77 / 79.  Width 1024 59 / 58 to 162 / 156 (of 1000), but 70 / 72 to 196 / 204
-// (of 1536) and 39 / 42 to 106 / 108 (of 512); width 512 47 / 49 to 124 / 128.
-bool takes_pairs(int M, int E, int n, int sms) { return sms % 2 == 0 && E >= 2048 && M / n >= BM + BM / 4; }
 
 }  // namespace
 }  // namespace ccs
@@ -406,22 +330,17 @@ extern "C" int cc_seq_moe_grouped(const CcSeqMoeGrouped* a, void* stream) {
         !map_rows(&ta, a->act, a->M, a->F))
         return fail(CC_SEQ_ERR_CUDA, "moe_grouped: cuTensorMapEncodeTiled failed or is not available");
     int rc;
-    const bool pair = takes_pairs(a->M, a->E, a->n, sms);
-    const int tile_rows = pair ? 2 * BM : BM, workers = pair ? sms / 2 : sms;
-    const long long row_tiles = (a->M + tile_rows - 1) / tile_rows + (a->n < a->M ? a->n : a->M);      // at most
+    const long long row_tiles = (a->M + BM - 1) / BM + (a->n < a->M ? a->n : a->M);      // at most
     auto grid = [&](int N, int cols) {
         const long long t = row_tiles * ((N + cols - 1) / cols);
-        return (int)(t < workers ? t : workers) * (pair ? 2 : 1);
+        return (int)(t < sms ? t : sms);
     };
     const long long copies = ((long long)a->M * (a->E / 8) + 255) / 256;
     moe_rows_kernel<<<(unsigned)(copies < 16 * sms ? copies : 16 * sms), 256, 0, st>>>((const uint4*)a->h, a->perm, a->counts, a->n, (uint4*)a->xs, a->E / 8);
     if ((rc = cuda_check("moe_rows_kernel"))) return rc;
     const Grouped up = {a->counts, a->act, a->n, a->E, a->F, (a->gated ? 2 : 1) * a->F, a->kind};
+    rc = a->gated ? launch_tc<true, true>(tgu, tx, up, grid(a->F, BN / 2), st) : launch_tc<true, false>(tgu, tx, up, grid(a->F, BN), st);
+    if (rc) return rc;
     const Grouped down = {a->counts, a->y, a->n, a->F, a->E, a->E, CC_ACT_NONE};
-    if (pair) {
-        rc = a->gated ? launch_tc<true, true, true>(tgu, tx, up, grid(a->F, BN / 2), st) : launch_tc<true, false, true>(tgu, tx, up, grid(a->F, BN), st);
-        return rc ? rc : launch_tc<false, false, true>(td, ta, down, grid(a->E, BN), st);
-    }
-    rc = a->gated ? launch_tc<true, true, false>(tgu, tx, up, grid(a->F, BN / 2), st) : launch_tc<true, false, false>(tgu, tx, up, grid(a->F, BN), st);
-    return rc ? rc : launch_tc<false, false, false>(td, ta, down, grid(a->E, BN), st);
+    return launch_tc<false, false>(td, ta, down, grid(a->E, BN), st);
 }
