@@ -298,11 +298,13 @@ template <int D, int QQ> constexpr int smem_bytes() {
 //
 // Bound: issue slots (54 % busy), the exponentials (two per logit at 16 per SM and cycle: 50 %) and the waits between them, at four
 // warps of softmax per scheduler; a 128 x 128 tile takes 1430 cycles in sweep 1 and 2000 in sweep 2, of which the MMAs take 515 and
-// 1030.  Measured at 7680 tokens x 32 heads of 128 (8 key/value heads) / 4096 / 1531 x 28 (4), in us, reduction included:
-// two groups of 256 threads that shared a barrier per 64 keys and issued their own MMAs 1397 / 412 / 105, this 815 / 279 / 85.
+// 1030.  Measured at 7680 tokens x 32 heads of 128 (8 key/value heads) / 4096 / 1531 x 28 (4), in us, reduction included, in bursts: two
+// groups of 256 threads that shared a barrier per 64 keys and issued their own MMAs 1397 / 412 / 105, this 814 / 268 / 75 (904 and 70
+// over seconds with L2 flushed between calls, where power takes part).
 // On the way: MMAs issued by one thread instead of a warp in step 976; mma.sync for the sums over heads and queries 943 (1500
 // cycles a tile: it waits for the tensor pipe behind the tcgen05 MMAs); all warps on the same tile 816; a quarter of the
-// exponentials as polynomials of degree 6 on the FMA pipe 924; the sums over the heads a tile later, among the exponentials, 899.
+// exponentials as polynomials of degree 6 on the FMA pipe 924; the sums over the heads a tile later, among the exponentials, 899; the next
+// tile's logits fetched under the pooling 840; Q in shared memory and two P 839.
 template <int D, bool NAIVE, int QQ>
 __global__ void __launch_bounds__(NTHREADS, 1)
 prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
