@@ -468,13 +468,13 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
                 const uint8_t* const pool = pools + (t & 1) * POOL_BYTES;
                 mbar_wait_u32(C_FULL(t & 1), (t >> 1) & 1, failed);
                 __syncwarp();
-                auto add = [&](int from, int window, float* out) {       // rows from `from` on, of the last `window` keys each
+                auto add = [&](auto banded, int from, int window, float* out) {       // rows from `from` on, banded: of the last `window` keys each
                     f32x2 s[4] = {0ull, 0ull, 0ull, 0ull};
 #pragma unroll 4
                     for (int r = first; r < rows; r += 4) {
                         uint4 u = *reinterpret_cast<const uint4*>(pool + r * (BN * 2) + ((c ^ ((r & 1) << 2)) << 4));
                         if (r < from) continue;
-                        if (window > 0) {
+                        if constexpr (decltype(banded)::value) {
                             const int lo = i0 + r - window - (t * BN + 32 * (c >> 2) + 2 * (c & 3));   // pair k is inside past here
                             auto inside = [&](uint32_t w, int k) { return (8 * k > lo ? w & 0xffffu : 0u) | (8 * k + 1 > lo ? w & 0xffff0000u : 0u); };
                             u = make_uint4(inside(u.x, 0), inside(u.y, 1), inside(u.z, 2), inside(u.w, 3));
@@ -493,9 +493,9 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
                     if (*failed) f = make_float2(NAN, NAN);
                     *reinterpret_cast<float2*>(out + t * BN) = f;
                 };
-                add(0, 0, col);
-                if (obs) add(p.obs_start - i0, 0, seen);
-                for (int w = 0; w < p.n_windows; ++w) add(0, p.windows[w], band + (size_t)w * p.Hkv * p.n_qtiles * p.S_pad);
+                add(std::false_type(), 0, 0, col);
+                if (obs) add(std::false_type(), p.obs_start - i0, 0, seen);
+                for (int w = 0; w < p.n_windows; ++w) add(std::true_type(), 0, p.windows[w], band + (size_t)w * p.Hkv * p.n_qtiles * p.S_pad);
                 __syncwarp();
                 if (lane == 0) mbar_arrive_u32(C_READ(t & 1));
             }
@@ -947,7 +947,8 @@ int prefill_attention_impl(const CcPrefillAttnArgs* a, cudaStream_t stream) {
     p.obs_start = obs_len > 0 ? S - obs_len : S;
     p.first_obs_tile = pl.first_obs_tile; p.n_obs_tiles = pl.n_obs_tiles;
     p.n_windows = stats ? a->n_windows : 0;
-    for (int w = 0; w < MAX_WINDOWS; ++w) p.windows[w] = w < p.n_windows ? a->windows[w] : 0;
+    for (int w = 0; w < MAX_WINDOWS; ++w)      // no rows at all from 0 down, every row from S on
+        p.windows[w] = w < p.n_windows ? (a->windows[w] < 0 ? 0 : a->windows[w] > S ? S : a->windows[w]) : 0;
     p.scale = (float)(1.0 / sqrt((double)D));
     p.stats = stats ? 1 : 0;
     p.part_col = p.part_obs = p.part_band = nullptr;

@@ -64,3 +64,15 @@ def test_without_statistics_in_fp32():
     want = torch.softmax(w, -1) @ v.float().repeat_interleave(5, 1)
     # one rounding of a weight and one of the result: 2^-9 of the largest value each, and half as much again for sums
     assert (y.float() - want).abs().max() < 3 * 2.0 ** -9 * v.float().abs().max()
+
+
+@pytest.mark.parametrize("G,D,S", [(4, 128, 40), (1, 64, 300), (8, 128, 129)])
+def test_windows_of_no_token_and_of_every_token(G, D, S):
+    """A row i counts for key j while i - j < w: none does for w <= 0, all do for any w of at least S."""
+    from cold_compress_b200.attention_utils import prefill_attention_stats
+    q, k, v = (t.cuda() for t in _inputs(G, D, S))
+    top = 2 ** 31 - 1
+    _, st = prefill_attention_stats(q, k, v, obs_len=16, windows=(0, -3, -top - 1, top))
+    for w in (0, -3, -top - 1):
+        assert not st.band_sum[w].any(), f"band {w}"
+    assert torch.equal(st.band_sum[top].to(torch.bfloat16), st.col_sum[0])
