@@ -91,6 +91,7 @@ __device__ __forceinline__ void mbar_wait_u32(uint32_t bar, uint32_t parity, vol
     for (uint32_t n = 0; !mbar_try_u32(bar, parity); ++n)
         if (n >= WAIT_LIMIT || *failed) { *failed = 1; return; }
 }
+// What was started is waited for also after another wait has run out: its shared and its tensor memory go to another CTA.
 __device__ __forceinline__ void mbar_wait_out(uint32_t bar, uint32_t parity) {
     for (uint32_t n = 0; n < WAIT_LIMIT && !mbar_try_u32(bar, parity); ++n) {}
 }
@@ -426,7 +427,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
             }
             if (elect_one()) umma_commit(Y_DONE);
             __syncwarp();
-            mbar_wait_u32(Y_DONE, 0, failed);
+            mbar_wait_out(Y_DONE, 0);
         } else if (warp == SOFT_WARPS + 1) {
             if (lane == 0) {
                 mbar_expect_tx_u32(Q_FULL, (uint32_t)(4 * DH * p.G * QQ * 128));
@@ -449,10 +450,8 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
                     if (t + 2 < T) load(&tm_k, t + 2);
                     if (t >= 0) load(&tm_v, t);
                 }
-                if (*failed) {    // the copies under way end before the CTA does
-                    mbar_wait_out(Q_FULL, 0);
-                    for (int m = max(0, n - STAGES); m < n; ++m) mbar_wait_out(FULL(m % STAGES), (m / STAGES) & 1);
-                }
+                mbar_wait_out(Q_FULL, 0);
+                for (int m = max(0, n - STAGES); m < n; ++m) mbar_wait_out(FULL(m % STAGES), (m / STAGES) & 1);
             }
             __syncwarp();
         } else if (p.stats) {

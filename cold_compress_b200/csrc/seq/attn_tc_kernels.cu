@@ -67,6 +67,10 @@ __device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity, volatil
     for (uint32_t n = 0; !mbar_try(bar, parity); ++n)
         if (n >= WAIT_LIMIT || *failed) { *failed = 1; return; }
 }
+// What was started is waited for also after another wait has run out: its shared and its tensor memory go to another CTA.
+__device__ __forceinline__ void mbar_wait_out(uint32_t bar, uint32_t parity) {
+    for (uint32_t n = 0; n < WAIT_LIMIT && !mbar_try(bar, parity); ++n) {}
+}
 __device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_async() { asm volatile("fence.proxy.async;" ::: "memory"); }
@@ -278,7 +282,7 @@ __device__ __forceinline__ void copy_tile(uint32_t dst, const CcSeqAttn& a, cons
 }
 
 struct Small {
-    uint64_t bars[12];          // k full[2], v full[2], scores[2], weights[2], product[2], result read, queries
+    uint64_t bars[13];          // k full[2], v full[2], scores[2], weights[2], product[2], result read, queries, everything done
     uint32_t tmem;
     int failed;
     float max[4][BM];           // row maxima over a quarter of a tile's keys; the sums' meeting place at the end
@@ -377,7 +381,7 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const CcSeqAttn a) 
     Small& sm = *reinterpret_cast<Small*>(smem_raw + 5 * q_part + 2 * v_tile);
     volatile int* const failed = &sm.failed;
     const uint32_t bar = smem_u32(sm.bars);
-    const uint32_t K_FULL = bar, V_FULL = bar + 16, S_DONE = bar + 32, P_DONE = bar + 48, PV_DONE = bar + 64, O_READ = bar + 80, Q_FULL = bar + 88;
+    const uint32_t K_FULL = bar, V_FULL = bar + 16, S_DONE = bar + 32, P_DONE = bar + 48, PV_DONE = bar + 64, O_READ = bar + 80, Q_FULL = bar + 88, DONE = bar + 96;
 
     if (tid < BM / 32) sm.redo[tid] = 0;
     if (tid == 0) {
@@ -391,6 +395,7 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const CcSeqAttn a) 
         }
         mbar_init(O_READ, SOFT_THREADS / 32);
         mbar_init(Q_FULL, SOFT_THREADS);
+        mbar_init(DONE, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) {
@@ -449,6 +454,8 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const CcSeqAttn a) 
                         }
                     mma_commit(PV_DONE + 8 * b);
                 }
+                mma_commit(DONE);
+                mbar_wait_out(DONE, 0);
             }
             __syncwarp();
         } else if (warp == SOFT_THREADS / 32 + 1) {

@@ -62,6 +62,10 @@ __device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity, volatil
     for (uint32_t n = 0; !mbar_try(bar, parity); ++n)
         if (n >= WAIT_LIMIT || *failed) { *failed = 1; return; }
 }
+// What was started is waited for also after another wait has run out: its shared and its tensor memory go to another CTA.
+__device__ __forceinline__ void mbar_wait_out(uint32_t bar, uint32_t parity) {
+    for (uint32_t n = 0; n < WAIT_LIMIT && !mbar_try(bar, parity); ++n) {}
+}
 __device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ uint64_t smem_desc(uint32_t addr) {   // 128-byte swizzle, rows of 128 bytes, descriptor version 1
@@ -139,7 +143,7 @@ struct Walk {
 };
 
 struct Small {
-    uint64_t bars[2 * STAGES + 4];     // full, empty, accumulator full[2], empty[2]
+    uint64_t bars[2 * STAGES + 5];     // full, empty, accumulator full[2], empty[2], everything done
     uint32_t tmem;
     int failed;
 };
@@ -164,7 +168,7 @@ __global__ void __launch_bounds__(THREADS, 1) moe_tc_kernel(const __grid_constan
     Small& sm = *reinterpret_cast<Small*>(outs + OUT_BYTES);
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const uint32_t base = smem_u32(smem_raw), bar = smem_u32(sm.bars);
-    const uint32_t FULL = bar, EMPTY = bar + 8 * STAGES, ACC_FULL = bar + 16 * STAGES, ACC_EMPTY = ACC_FULL + 16;
+    const uint32_t FULL = bar, EMPTY = bar + 8 * STAGES, ACC_FULL = bar + 16 * STAGES, ACC_EMPTY = ACC_FULL + 16, DONE = ACC_EMPTY + 16;
     volatile int* const failed = &sm.failed;
     if (tid == 0) {
         *failed = 0;
@@ -176,6 +180,7 @@ __global__ void __launch_bounds__(THREADS, 1) moe_tc_kernel(const __grid_constan
             mbar_init(ACC_FULL + 8 * b, 1);
             mbar_init(ACC_EMPTY + 8 * b, W_OUT);
         }
+        mbar_init(DONE, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) {
@@ -210,9 +215,7 @@ __global__ void __launch_bounds__(THREADS, 1) moe_tc_kernel(const __grid_constan
                     tma_load(sA, &tm_a, k * BK, r0, FULL + 8 * s);
                 }
             }
-            if (*failed)      // the copies under way end before the CTA does
-                for (int m = it < STAGES ? 0 : it - STAGES; m < it; ++m)
-                    for (uint32_t n = 0; n < WAIT_LIMIT && !mbar_try(FULL + 8 * (m % STAGES), (m / STAGES) & 1); ++n) {}
+            for (int m = it < STAGES ? 0 : it - STAGES; m < it; ++m) mbar_wait_out(FULL + 8 * (m % STAGES), (m / STAGES) & 1);
         }
         __syncwarp();
     } else if (warp == W_MMA) {
@@ -237,6 +240,9 @@ __global__ void __launch_bounds__(THREADS, 1) moe_tc_kernel(const __grid_constan
                 if (++s == STAGES) { s = 0; turn ^= 1; }
             }
         }
+        if (elect_one()) mma_commit(DONE);
+        __syncwarp();
+        mbar_wait_out(DONE, 0);
     } else {
         int n_tile = 0;
         const uint32_t lanes = (uint32_t)(warp * 32) << 16;

@@ -1,0 +1,35 @@
+"""CPU: waits that run out, read as text.  A wait has a limit, and after it a kernel runs to its end.  Its shared and tensor memory then go to
+another CTA, so that what it started has to be over: the last products by a commit of their own, the last copies by their barriers,
+each waited for whether or not another wait has run out."""
+import re
+from pathlib import Path
+
+import pytest
+
+CSRC = Path(__file__).resolve().parent.parent / "cold_compress_b200" / "csrc"
+WITH_TENSOR_MEMORY = [f for f in sorted(CSRC.rglob("*.cu")) if "tcgen05.alloc" in f.read_text()]
+
+
+def _bare(path):
+    return re.sub(r"//[^\n]*", "", path.read_text())
+
+
+def test_the_kernels_are_found():
+    assert {f.name for f in WITH_TENSOR_MEMORY} == {"prefill_attn.cu", "attn_tc_kernels.cu", "moe_tc_kernels.cu"}
+
+
+@pytest.mark.parametrize("path", WITH_TENSOR_MEMORY, ids=lambda f: f.stem)
+def test_products_are_over_before_tensor_memory_is_given_back(path):
+    text = _bare(path)
+    assert re.search(r"mbar_wait_out\(uint32_t bar, uint32_t parity\) \{\s*for \(uint32_t n = 0; n < WAIT_LIMIT && !mbar_try\w*\(bar, parity\); \+\+n\) \{\}\s*\}", text)
+    last = text[text.rindex("mma_commit("):]
+    assert re.match(r"mma_commit\((\w+)\);\s*(__syncwarp\(\);\s*)?mbar_wait_out\(\1, 0\);", last)      # nothing on the way asks for `failed`
+    assert "tcgen05.mma" not in last and not re.search(r"\bu?mma_[st]s\(", last) and "tcgen05.dealloc" in last
+
+
+@pytest.mark.parametrize("path", [f for f in WITH_TENSOR_MEMORY if "tma_load" in f.read_text()], ids=lambda f: f.stem)
+def test_copies_are_over_before_the_end(path):
+    text = _bare(path)
+    after = text[[m.end() for m in re.finditer(r"tma_load\w*\(", text)][-1]:]
+    drain = re.search(r"\n([^\n]*)for \(int m = [^;]*; m < (\w+); \+\+m\) mbar_wait_out\(FULL[^;]*, \(m / STAGES\) & 1\);", after)
+    assert drain and not drain.group(1).strip() and not re.search(r"if \(\*failed\)([^;]*|\s*\{[^}]*)$", after[:drain.start()])
