@@ -381,6 +381,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
             int st = 0;
             uint32_t turn = 0;
             auto next = [&] { if (++st == STAGES) { st = 0; turn ^= 1; } };
+            auto lost = [&] { return __any_sync(0xffffffffu, *failed) != 0; };      // the same for all lanes, which elect_one wants together
             auto logits = [&](int b) {                   // S[b] = Q K^T: [128 x 128], Q in tensor memory
                 mbar_wait_u32(FULL(st), turn, failed);
                 tc_fence_after();
@@ -398,12 +399,12 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
             mbar_wait_u32(Q_READY, 0, failed);
             tc_fence_after();
             uint32_t read = 1;
-            for (int n = 0, b = 0; n < T && !*failed; ++n) {
+            for (int n = 0, b = 0; n < T && !lost(); ++n) {
                 if (n >= 3) mbar_wait_u32(S_READ(b), read, failed);
                 logits(b);
                 if (++b == 3) { b = 0; read ^= 1; }
             }
-            for (int t = -2; t < T && !*failed; ++t) {
+            for (int t = -2; t < T && !lost(); ++t) {
                 if (t + 2 < T) {
                     const int b = t & 1, turns = used(b) + ((t + 2) >> 1);            // of this accumulator, so far
                     if (turns > 0) mbar_wait_u32(S_READ(b), (turns - 1) & 1, failed);

@@ -222,7 +222,8 @@ __global__ void __launch_bounds__(THREADS, 1) moe_tc_kernel(const __grid_constan
         int s = 0, n_tile = 0;
         uint32_t turn = 0;
         const uint64_t a_desc = smem_desc(base), b_desc = smem_desc(base + A_BYTES);
-        for (int id = blockIdx.x; w.seek(id) && !*failed; id += gridDim.x, ++n_tile) {
+        // the flag is the same for all lanes, which elect_one wants together
+        for (int id = blockIdx.x; w.seek(id) && !__any_sync(0xffffffffu, *failed); id += gridDim.x, ++n_tile) {
             const int b = n_tile & 1;
             if (n_tile >= 2) mbar_wait(ACC_EMPTY + 8 * b, (n_tile / 2 - 1) & 1, failed);
             for (int k = 0; k < k_iters; ++k) {

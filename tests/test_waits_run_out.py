@@ -33,3 +33,15 @@ def test_copies_are_over_before_the_end(path):
     after = text[[m.end() for m in re.finditer(r"tma_load\w*\(", text)][-1]:]
     drain = re.search(r"\n([^\n]*)for \(int m = [^;]*; m < (\w+); \+\+m\) mbar_wait_out\(FULL[^;]*, \(m / STAGES\) & 1\);", after)
     assert drain and not drain.group(1).strip() and not re.search(r"if \(\*failed\)([^;]*|\s*\{[^}]*)$", after[:drain.start()])
+
+
+@pytest.mark.parametrize("path", [f for f in WITH_TENSOR_MEMORY if "elect_one()" in f.read_text()], ids=lambda f: f.stem)
+def test_lanes_that_elect_one_leave_a_loop_together(path):
+    """Loops around elect.sync, which wants all lanes of the warp, ask for `failed` as a warp."""
+    text = _bare(path)
+    role = text[text.rindex("warp == ", 0, text.index("umma_commit(S_FULL" if "umma_commit(S_FULL" in text else "mma_commit(EMPTY")):text.rindex("elect_one()")]
+    heads = re.findall(r"for \(([^;]*;[^;]*;[^{]*)\{", role)
+    asking = [h for h in heads if "failed" in h or "lost()" in h]
+    assert asking and all("lost()" in h or "__any_sync(0xffffffffu, *failed)" in h for h in asking)
+    assert "lost()" not in role or re.search(r"auto lost = \[&\] \{ return __any_sync\(0xffffffffu, \*failed\) != 0; \};", role)
+    assert not re.search(r"if \(\*failed\)", role)
