@@ -1077,7 +1077,7 @@ __device__ __forceinline__ void md_copy_box(void* dst, const CUtensorMap* tm, in
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(smem_at(dst)), "l"(tm),
                  "r"(smem_at(bar)), "r"(column), "r"(row) : "memory");
 }
-// bounded: a copy that does not arrive ends the wait, not the kernel; what it leaves is then no number
+// bounded: a copy that does not arrive ends the wait, not the kernel, whose results are then no numbers
 __device__ __forceinline__ bool md_bar_wait(uint64_t* bar, uint32_t parity) {
     for (uint32_t n = 0; n < (1u << 22); ++n) {
         uint32_t done;
@@ -1130,10 +1130,12 @@ __global__ void __launch_bounds__(MD_THREADS, 2) attn_decode_mma_kernel(const Cc
     __shared__ int s_live[2][VT];
     __shared__ float s_M[8], s_L[8], s_corr[8], s_inv[8];
     __shared__ int s_last;
+    __shared__ volatile int s_lost;
     __shared__ __align__(8) uint64_t bars[2][2];      // [buffer][keys, values]
 
     const int sp = blockIdx.x, g = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if (tid == 0) {
+        s_lost = 0;
         for (int i = 0; i < 4; ++i) md_bar_init(&bars[i >> 1][i & 1], MD_THREADS / 2);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -1320,7 +1322,9 @@ __global__ void __launch_bounds__(MD_THREADS, 2) attn_decode_mma_kernel(const Cc
         landed = md_bar_wait(&bars[b][1], turn) && landed;
         uint4* const vt = vs + b * VT * v_row;
         if (BOX && value && tile == n_tiles - 1) finish(tile, vt);
+        if (!landed) s_lost = 1;
         __syncthreads();
+        const bool lost = s_lost;                                // read by all between two barriers without a wait in between
         const float corr = s_corr[row_r];
         const int steps = min(VT, n - u0 + 15) >> 4;             // further rows have no position
 #pragma unroll
@@ -1358,13 +1362,24 @@ __global__ void __launch_bounds__(MD_THREADS, 2) attn_decode_mma_kernel(const Cc
                         for (int k = 0; k < VT; ++k)
                             if (live[k]) sum = fmaf(Ps[row_r * VT + k], __bfloat162float(reinterpret_cast<const CT*>(unit(vt, k, c >> 3, v_row))[c & 7]), sum);
                     }
-                    if (!landed) sum = NAN;
                     acc[i][t][e] = tile > tile0 ? fmaf(acc[i][t][e], corr, sum) : sum;
                 }
         }
+        if (lost) {           // a copy did not arrive: those under way end before the CTA goes on
+            for (int i = 0; i < 2; ++i) {
+                md_bar_wait(&bars[b][i], turn);
+                if (buffers > 1 && tile + 1 < tile_end) md_bar_wait(&bars[b ^ 1][i], ((tile + 1 - tile0) >> 1) & 1);
+            }
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+#pragma unroll
+                for (int t = 0; t < 2; ++t) acc[i][t][0] = acc[i][t][1] = NAN;
+            break;
+        }
+        if (tile + 1 == tile_end) break;
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // reads before the copies that follow
         __syncthreads();      // the tile is consumed: its buffers may be filled again
-        if (buffers == 1 && tile + 1 < tile_end) {
+        if (buffers == 1) {
             fetch(tile + 1);
             mark(tile + 1);
         }

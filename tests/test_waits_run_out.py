@@ -45,3 +45,19 @@ def test_lanes_that_elect_one_leave_a_loop_together(path):
     assert asking and all("lost()" in h or "__any_sync(0xffffffffu, *failed)" in h for h in asking)
     assert "lost()" not in role or re.search(r"auto lost = \[&\] \{ return __any_sync\(0xffffffffu, \*failed\) != 0; \};", role)
     assert not re.search(r"if \(\*failed\)", role)
+
+
+def test_one_token_attention_fetches_nothing_more_and_waits_for_what_is_under_way():
+    """attn_decode_mma_kernel has a flag of its own: it is raised before a barrier and looked at between that one and the next."""
+    text = _bare(CSRC / "seq" / "seq_kernels.cu")
+    body = text[text.index("attn_decode_mma_kernel(const CcSeqAttn a"):]
+    loop = body[body.index("for (int tile = tile0; tile < tile_end; ++tile) {"):body.index("int* counters")]
+    assert loop.count("md_bar_wait(&bars[b][0], turn)") == loop.count("md_bar_wait(&bars[b][1], turn)") == 1
+    marked = loop.index("if (!landed) s_lost = 1;")
+    met, known, done = (loop.index(x, marked) for x in ("__syncthreads();", "const bool lost = s_lost;", "if (lost) {"))
+    assert loop.rindex("md_bar_wait(&bars[b][1], turn)", 0, marked) and met < known < done < loop.index("__syncthreads();", known)      # the same for all threads
+    assert "md_bar_wait(" not in loop[marked:done]
+    end = loop[done:]
+    lost, rest = end[:end.index("break;")], end[end.index("break;"):]
+    assert "md_bar_wait(&bars[b][i], turn);" in lost and "md_bar_wait(&bars[b ^ 1][i], ((tile + 1 - tile0) >> 1) & 1);" in lost and "NAN" in lost
+    assert "fetch(" not in lost and loop.count("fetch(tile + 1)") == 2 and rest.count("fetch(tile + 1)") == 1      # the other one is of two buffers, before the waits
