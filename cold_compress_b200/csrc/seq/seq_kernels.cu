@@ -1171,8 +1171,11 @@ __global__ void __launch_bounds__(MD_THREADS, 2) attn_decode_mma_kernel(const Cc
             return j == p ? fresh_row : cached + (size_t)slot_of(a, j) * D;
         };
         if constexpr (BOX) {
-            // One run of slots, but for the token itself, which is put over what was fetched in its place: boxes.  Otherwise a row
-            // per thread (at the end of a ring, or beside kept positions).
+            // One run of slots, but for the token itself, which is put over what was fetched in its place: boxes.  Otherwise (at the end
+            // of a ring, or beside kept positions) rows by asynchronous copies of 16 bytes, neighbouring lanes in neighbouring bytes, that
+            // arrive at the same barrier.  One such tile a head sets the time of all: 8 layers in a graph, us a layer by a row per thread through
+            // registers / by these, 32 / 8 heads of 128, windows of 1000 behind 1128 positions 11.8 / 9.5, of 1000 and 4 kept 11.8 / 9.5, of 4096 and 128
+            // kept 16.0 / 13.1, 8 / 2 heads of 256 15.6 / 11.2 (a bulk copy per row, all tiles so: 10.5, 10.5, 13.5, 12.0).
             const int ring = a.L - a.keep_first, j0 = position(0), r0 = j0 >= a.keep_first ? (j0 - a.keep_first) % ring : ring;
             const int old = rows - (u0 + rows == n ? 1 : 0);           // rows that the cache holds
             if (u0 >= kx && r0 + old <= ring) {
@@ -1183,12 +1186,20 @@ __global__ void __launch_bounds__(MD_THREADS, 2) attn_decode_mma_kernel(const Cc
                     md_bar_arrive(bar);
                 }
             } else {
-                if (ht < rows) {
-                    const uint4* const src = reinterpret_cast<const uint4*>(source(ht));
-#pragma unroll 8
-                    for (int c = 0; c < D / 8; ++c) *unit(dst, ht, c, stride) = src[c];
+                // a warp's 32 rows, 16 bytes a lane of rows one after another, all under way together
+                const unsigned long long mine = ht < rows ? (unsigned long long)source(ht) : 0ull;
+                const int units = D / 8, down = 32 / units, right = 32 - down * units;      // units: 8, 16, 24 or 32
+                int r = lane / units, c = lane - r * units;
+#pragma unroll 4
+                for (int i = 0; i < units; ++i) {
+                    const unsigned long long from = __shfl_sync(0xffffffffu, mine, r);
+                    if (from != 0ull)
+                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_at(unit(dst, (ht & ~31) + r, c, stride))), "l"(from + 16 * c) : "memory");
+                    r += down;
+                    c += right;
+                    if (c >= units) { c -= units; ++r; }
                 }
-                md_bar_arrive(bar);
+                asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_at(bar)) : "memory");
             }
         } else if (ht < rows) {
             md_bar_expect(bar, (uint32_t)D * 2);

@@ -50,3 +50,9 @@ def test_query_rows_on_a_boundary_of_a_float():
         cache.sequence_step(q[shift:shift + H * D].view(1, H, D), k1, v1, ip, y, sink_mode=_lib.SINK_NONE, scale=D ** -0.5)
         got.append(y)
     assert all(torch.equal(y, got[0]) for y in got)
+
+
+@pytest.mark.parametrize("past,window,keep", [(1128, 1000, 0), (3000, 1000, 7), (300, 128, 4), (131, 100, 30)])
+def test_widest_rows_of_rings_and_kept_positions(past, window, keep):
+    """Rows of a tile that is no single run, copied 16 bytes a lane: 32 of them a row."""
+    _check(*_run(16, 2, 256, 256, past, window, keep, 0), 256, past)
