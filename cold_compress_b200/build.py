@@ -36,7 +36,7 @@ def seq_sources():
 def seq_needs_build() -> bool:
     if not SEQ_SO.exists():
         return True
-    newest = max(p.stat().st_mtime for p in [*(CSRC / "seq").glob("*"), SEQ_HEADER])
+    newest = max(p.stat().st_mtime for p in [*(CSRC / "seq").glob("*"), *CSRC.glob("*.cuh"), SEQ_HEADER])
     return SEQ_SO.stat().st_mtime < newest
 
 

@@ -445,18 +445,19 @@ static int launch_split(K1 k1, K2 k2, K4 k4, K8 k8, const P& p, int n_pairs, int
     // (sharing the input staging between the CTAs of a cluster over DSMEM was measured 5-8 us per launch SLOWER:
     // gang scheduling + two cluster barriers)
     auto go = [&](auto kernel) -> int {
-        static thread_local const void* raised[16] = {};
-        if (smem > 48 * 1024) {  // raise the per-function cap once, to the device limit
+        static thread_local struct { const void* kernel; int dev; } raised[64] = {};
+        if (smem > 48 * 1024) {  // raise the cap once per function and device, to the device limit
             bool done = false;
-            for (int i = 0; i < 16; ++i) done |= raised[i] == (const void*)kernel;
+            int dev = 0;
+            cudaGetDevice(&dev);
+            for (int i = 0; i < 64; ++i) done |= raised[i].kernel == (const void*)kernel && raised[i].dev == dev;
             if (!done) {
-                int dev = 0, optin = 0;
-                cudaGetDevice(&dev);
+                int optin = 0;
                 cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
                 cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
                 if (e != cudaSuccess) return set_cuda_error(e, what);
-                for (int i = 0; i < 16; ++i)
-                    if (!raised[i]) { raised[i] = (const void*)kernel; break; }
+                for (int i = 0; i < 64; ++i)
+                    if (!raised[i].kernel) { raised[i].kernel = (const void*)kernel; raised[i].dev = dev; break; }
             }
         }
         cudaLaunchConfig_t cfg = {};

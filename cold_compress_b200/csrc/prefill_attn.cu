@@ -33,6 +33,7 @@
 
 #include "common.cuh"
 #include "internal.h"
+#include "smem_limit.cuh"
 
 namespace cc {
 namespace {
@@ -887,14 +888,11 @@ int launch(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, 
            cudaStream_t stream) {
     constexpr int smem = smem_bytes<D, QQ>();
     static_assert(smem <= 232448, "");
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(prefill_attn_kernel<D, NAIVE, QQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (e != cudaSuccess) return set_cuda_error(e, "cc_prefill_attention: shared memory attribute");
-        configured = true;
-    }
+    static SmemLimit limit;
+    cudaError_t e = limit.allow(prefill_attn_kernel<D, NAIVE, QQ>, smem);
+    if (e != cudaSuccess) return set_cuda_error(e, "cc_prefill_attention: shared memory attribute");
     prefill_attn_kernel<D, NAIVE, QQ><<<grid, NTHREADS, smem, stream>>>(tq, tk, tv, p);
-    cudaError_t e = cudaGetLastError();
+    e = cudaGetLastError();
     return e == cudaSuccess ? CC_OK : set_cuda_error(e, "cc_prefill_attention launch");
 }
 

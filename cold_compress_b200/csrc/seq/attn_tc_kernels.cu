@@ -649,7 +649,8 @@ template <typename YT, int NO, bool SHAPED>
 int launch_tc(const CcSeqAttn* a, cudaStream_t st) {
     const size_t smem = sizeof(Small) + (size_t)TILE_BYTES * (5 * ((a->Dk + 63) / 64) + 2 * ((a->Dv + 63) / 64));
     auto kern = attn_tc_kernel<YT, NO, SHAPED>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    static SmemLimit limit;
+    const cudaError_t e = limit.allow(kern, smem);
     if (e != cudaSuccess) return fail(CC_SEQ_ERR_CUDA, cudaGetErrorString(e));
     const long long tiles = ((long long)a->T * (a->H / a->G) + BM - 1) / BM;
     launch_under(kern, dim3((unsigned)(tiles * a->G)), dim3(THREADS), smem, st, *a);

@@ -596,12 +596,8 @@ template <int CH>
 static int launch_scan(const CcSeqMlstm* a, cudaStream_t st) {
     const int P = (a->D + CH - 1) / CH, TB = a->T < SCAN_TB ? a->T : SCAN_TB;
     const size_t smem = sizeof(float) * (size_t)TB * (2 * P * CH + SCAN_J + P * SCAN_J);
-    static size_t configured = 40 * 1024;      // beside the static arrays
-    if (smem > configured) {
-        configured = smem;
-        if (cudaFuncSetAttribute(mlstm_scan_kernel<CH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-            return cuda_check("mlstm: shared memory");
-    }
+    static SmemLimit limit;
+    if (limit.allow(mlstm_scan_kernel<CH>, smem) != cudaSuccess) return cuda_check("mlstm: shared memory");
     ccs::launch_under(mlstm_scan_kernel<CH>, dim3(a->H, (a->V + SCAN_J - 1) / SCAN_J), dim3((P + 1) * 32), smem, st, *a);
     return cuda_check("mlstm_scan_kernel");
 }

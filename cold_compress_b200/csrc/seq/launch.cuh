@@ -11,6 +11,8 @@
 #include <cuda_runtime.h>
 #include <stdlib.h>
 
+#include "../smem_limit.cuh"
+
 namespace ccs {
 
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

@@ -1003,12 +1003,8 @@ static int launch_latent_decode(const CcSeqLatentDecode* a, cudaStream_t st) {
     const int Dkp = ld_stride(a->Dk);
     const size_t smem = sizeof(float) * ((size_t)(LD_HG + LD_TK) * Dkp + LD_HG * LD_TK) + sizeof(int) * LD_TK;
     auto kern = latent_decode_kernel<CT, NC>;
-    static size_t configured = 48 * 1024;
-    if (smem > configured) {
-        configured = smem;
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-            return cuda_check("latent_decode: shared memory");
-    }
+    static SmemLimit limit;
+    if (limit.allow(kern, smem) != cudaSuccess) return cuda_check("latent_decode: shared memory");
     const int kpr = ld_keys_per_run(a->L);
     dim3 grid((a->L + kpr - 1) / kpr, (a->H + LD_HG - 1) / LD_HG);
     ccs::launch_under(kern, grid, dim3(LD_THREADS), smem, st, *a);
@@ -1329,12 +1325,8 @@ template <int TB, int CH, int J>
 static int launch_wkv(const CcSeqWkv* a, cudaStream_t st) {
     const int P = (a->D + CH - 1) / CH;
     const size_t smem = sizeof(float) * (2 * (size_t)TB * (3 * P * CH + J) + (size_t)TB * P * J);
-    static size_t configured = 48 * 1024;
-    if (smem > configured) {
-        configured = smem;
-        if (cudaFuncSetAttribute(wkv_kernel<TB, CH, J>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-            return cuda_check("wkv: shared memory");
-    }
+    static SmemLimit limit;
+    if (limit.allow(wkv_kernel<TB, CH, J>, smem) != cudaSuccess) return cuda_check("wkv: shared memory");
     dim3 grid(a->H, (a->D + J - 1) / J);
     wkv_kernel<TB, CH, J><<<grid, P * J, smem, st>>>(*a);
     return cuda_check("wkv_kernel");
@@ -1397,12 +1389,8 @@ int cc_seq_gated_group_norm(const CcSeqGatedNorm* g, void* stream) {
 #define CALL(ST)                                                                                                     \
     {                                                                                                                \
         auto kern = gated_group_norm_kernel<ST>;                                                                     \
-        static size_t configured = 48 * 1024;                                                                        \
-        if (smem > configured) {                                                                                     \
-            configured = smem;                                                                                       \
-            if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)   \
-                return cuda_check("gated_group_norm: shared memory");                                                \
-        }                                                                                                            \
+        static SmemLimit limit;                                                                                      \
+        if (limit.allow(kern, smem) != cudaSuccess) return cuda_check("gated_group_norm: shared memory");            \
         kern<<<dim3(g->T, g->groups), 256, smem, st>>>(*g);                                                          \
     }
     CCM_ST(g->act_dtype, CALL);
@@ -1640,12 +1628,8 @@ int cc_seq_gemv_multi(const CcSeqGemvMulti* g, void* stream) {
 #define CALL3(ST, PRE, KS, PAIR)                                                                                   \
     {                                                                                                              \
         auto kern = gemv_multi_kernel<ST, PRE, KS, PAIR>;                                                          \
-        static size_t configured = 48 * 1024;                                                                      \
-        if (smem > configured) {                                                                                   \
-            configured = smem;                                                                                     \
-            if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) \
-                return cuda_check("gemv_multi: shared memory");                                                    \
-        }                                                                                                          \
+        static SmemLimit limit;                                                                                    \
+        if (limit.allow(kern, smem) != cudaSuccess) return cuda_check("gemv_multi: shared memory");                \
         ccs::launch_under(kern, dim3(blocks), dim3(256), smem, st, *g, split.rows_per_cta);                        \
     }
 #define CALL2(ST, PRE, KS)                                                                                         \

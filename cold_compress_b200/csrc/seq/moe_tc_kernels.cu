@@ -309,7 +309,8 @@ template <bool UNIT, bool GATED>
 int launch_tc(const CUtensorMap& tw, const CUtensorMap& ta, const Grouped& p, int grid, cudaStream_t st) {
     auto kern = moe_tc_kernel<UNIT, GATED>;
     const int smem = STAGES * STAGE_BYTES + OUT_BYTES + (int)sizeof(Small);
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    static SmemLimit limit;
+    const cudaError_t e = limit.allow(kern, smem);
     if (e != cudaSuccess) return fail(CC_SEQ_ERR_CUDA, cudaGetErrorString(e));
     launch_under(kern, dim3(grid), dim3(THREADS), smem, st, tw, ta, p);
     return cuda_check("moe_tc_kernel");

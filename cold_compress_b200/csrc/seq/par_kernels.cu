@@ -10,6 +10,7 @@
 #include <stdint.h>
 
 #include "../../../include/cc_b200_seq.h"
+#include "../smem_limit.cuh"
 
 namespace ccs {
 int fail(int code, const char* msg);
@@ -322,14 +323,9 @@ int cc_seq_par_norm(const CcSeqParNorm* g, void* stream) {
     const int threads = g->T <= 4 ? 1024 : 256;      // few rows: every pass is a chain of dependent loads
     const size_t smem = sizeof(float) * (size_t)g->E * (fused ? 1 + 2 * g->n_out : 1);
     if (smem > 200 * 1024) return fail(CC_SEQ_ERR_UNSUPPORTED_SHAPE, "par_norm: row too wide");
-    if (smem > 48 * 1024) {
-        static size_t configured = 48 * 1024;
-        if (smem > configured) {
-            configured = smem;
-            cudaFuncSetAttribute(par_norm_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            cudaFuncSetAttribute(par_norm_kernel<bf16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        }
-    }
+    static SmemLimit limits[2];
+    if (limits[0].allow(par_norm_kernel<float>, smem) != cudaSuccess || limits[1].allow(par_norm_kernel<bf16>, smem) != cudaSuccess)
+        return cuda_check("par_norm: shared memory");
     if (g->n_out == 0 && !g->rinv) return fail(CC_SEQ_ERR_INVALID_ARG, "par_norm: nothing to write");
 #define CALL(ST) par_norm_kernel<ST><<<g->T, threads, smem, st>>>(*g, fused)
     CCP_ST(g->act_dtype, CALL);

@@ -8,6 +8,7 @@
 #include <stdint.h>
 
 #include "../../../include/cc_b200_seq.h"
+#include "../smem_limit.cuh"
 
 namespace ccs {
 int fail(int code, const char* msg);
@@ -221,20 +222,12 @@ __global__ void __launch_bounds__(1024) post_norm_route_kernel(const CcSeqPostNo
     for (int k = lane; k < top; k += 32) wts[t * top + k] /= sum;
 }
 
-template <typename K>
-static int more_smem(K kern, size_t smem, size_t& configured) {
-    if (smem <= configured) return CC_SEQ_OK;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return cuda_check("post_norm: shared memory");
-    configured = smem;
-    return CC_SEQ_OK;
-}
-
 template <typename AT, int VEC>
 static int launch_post_norm(const CcSeqPostNorm* a, cudaStream_t st) {
     const size_t smem = sizeof(float) * (size_t)((a->E + 3) & ~3);
-    static size_t configured = 48 * 1024;
+    static SmemLimit limit;
     auto kern = post_norm_kernel<AT, VEC>;
-    if (int rc = more_smem(kern, smem, configured)) return rc;
+    if (limit.allow(kern, smem) != cudaSuccess) return cuda_check("post_norm: shared memory");
     const int want = ((a->E + VEC - 1) / VEC + 31) / 32 * 32, most = a->T < 64 ? 1024 : 256;
     kern<<<a->T, want < most ? want : most, smem, st>>>(*a);
     return cuda_check("post_norm_kernel");
@@ -243,9 +236,9 @@ static int launch_post_norm(const CcSeqPostNorm* a, cudaStream_t st) {
 template <typename AT, int VEC>
 static int launch_post_norm_route(const CcSeqPostNorm* a, const void* Wr, const float* bias, int n, int top, int32_t* ids, float* wts, cudaStream_t st) {
     const size_t smem = sizeof(float) * (size_t)(((a->E + 3) & ~3) + n);
-    static size_t configured = 48 * 1024;
+    static SmemLimit limit;
     auto kern = post_norm_route_kernel<AT, VEC>;
-    if (int rc = more_smem(kern, smem, configured)) return rc;
+    if (limit.allow(kern, smem) != cudaSuccess) return cuda_check("post_norm: shared memory");
     int threads = ((a->E + VEC - 1) / VEC + 31) / 32 * 32;
     threads = threads > n * 32 ? threads : n * 32;      // at least a warp per expert
     kern<<<a->T, threads < 1024 ? threads : 1024, smem, st>>>(*a, (const AT*)Wr, bias, n, top, ids, wts);

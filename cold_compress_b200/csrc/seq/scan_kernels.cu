@@ -613,22 +613,12 @@ __global__ void softcap_kernel(float* __restrict__ x, int64_t n, float cap) {
 }
 
 // ------------------------------------------------------------------------------------------------ host side
-template <typename K>
-static int set_smem(K kern, size_t smem, size_t& configured) {
-    if (smem > configured) {
-        configured = smem;
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-            return cuda_check("shared memory size");
-    }
-    return CC_SEQ_OK;
-}
-
 template <int CH, int TB>
 static int launch_ssd(const CcSeqSsdScan* a, cudaStream_t st) {
     const int P = (a->N + CH - 1) / CH;
     const size_t smem = sizeof(float) * (2 * (size_t)TB * (2 * P * CH + SCAN_J + 2) + (size_t)TB * P * SCAN_J);
-    static size_t configured = 48 * 1024;
-    if (int rc = set_smem(ssd_scan_kernel<CH, TB>, smem, configured)) return rc;
+    static SmemLimit limit;
+    if (limit.allow(ssd_scan_kernel<CH, TB>, smem) != cudaSuccess) return cuda_check("shared memory size");
     dim3 grid(a->H, (a->V + SCAN_J - 1) / SCAN_J);
     ssd_scan_kernel<CH, TB><<<grid, P * 32, smem, st>>>(*a);
     return cuda_check("ssd_scan_kernel");
@@ -637,9 +627,9 @@ static int launch_ssd(const CcSeqSsdScan* a, cudaStream_t st) {
 template <int CH, int NC, int TB, int J, bool HD>
 static int launch_delta_j(const CcSeqDeltaScan* a, cudaStream_t st) {
     const size_t smem = sizeof(float) * 2 * (size_t)delta_buf_floats(DL_PARTS * (CH + 4), J, TB, HD);
-    static size_t configured = 48 * 1024;
+    static SmemLimit limit;
     auto kern = delta_scan_kernel<CH, NC, TB, J, HD>;
-    if (int rc = set_smem(kern, smem, configured)) return rc;
+    if (limit.allow(kern, smem) != cudaSuccess) return cuda_check("shared memory size");
     dim3 grid(a->H, (a->V + J - 1) / J);
     kern<<<grid, J / (4 * NC) * 32, smem, st>>>(*a);
     return cuda_check("delta_scan_kernel");
@@ -684,8 +674,9 @@ int cc_seq_sum_norm(const CcSeqSumNorm* a, void* stream) {
     const int threads = a->T < 64 ? (a->E >= 1024 ? 1024 : ((a->E + 31) / 32) * 32) : 256;
 #define CALL(AT)                                                                 \
     {                                                                            \
-        static size_t configured = 48 * 1024;                                    \
-        if (int rc = set_smem(sum_norm_kernel<AT>, smem, configured)) return rc; \
+        static SmemLimit limit;                                                  \
+        if (limit.allow(sum_norm_kernel<AT>, smem) != cudaSuccess)               \
+            return cuda_check("shared memory size");                             \
         sum_norm_kernel<AT><<<a->T, threads, smem, st>>>(*a);                    \
     }
     CCN_ST(a->out_act ? a->act_dtype : CC_DT_F32, CALL);

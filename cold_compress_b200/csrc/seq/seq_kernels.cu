@@ -1731,12 +1731,9 @@ template <typename WT, typename XT, typename OT>
 static int launch_gemv(const CcSeqGemv* g, cudaStream_t st) {
     const size_t smem = sizeof(float) * (size_t)((g->K + 3) & ~3);
     auto kern = gemv_kernel<WT, XT, OT>;
-    static size_t configured = 48 * 1024;
-    if (smem > configured) {
-        configured = smem;
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return fail(CC_SEQ_ERR_CUDA, cudaGetErrorString(e));
-    }
+    static SmemLimit limit;
+    const cudaError_t e = limit.allow(kern, smem);
+    if (e != cudaSuccess) return fail(CC_SEQ_ERR_CUDA, cudaGetErrorString(e));
     kern<<<(g->N + GEMV_ROWS - 1) / GEMV_ROWS, GEMV_THREADS, smem, st>>>(*g);
     return cuda_check("gemv_kernel");
 }
@@ -1767,12 +1764,9 @@ static int launch_chunk(const CcSeqAttn* a, cudaStream_t st) {
     const int Dkp = vec_stride(a->Dk);
     const size_t smem = sizeof(float) * ((size_t)(BQ + BK) * Dkp + (size_t)BK * 64 * DV4 + (size_t)BQ * (BK + 4)) + sizeof(int) * 2 * BK;
     auto kern = attn_chunk_kernel<CT, YT, DV4>;
-    static size_t configured = 48 * 1024;
-    if (smem > configured) {
-        configured = smem;
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return fail(CC_SEQ_ERR_CUDA, cudaGetErrorString(e));
-    }
+    static SmemLimit limit;
+    const cudaError_t e = limit.allow(kern, smem);
+    if (e != cudaSuccess) return fail(CC_SEQ_ERR_CUDA, cudaGetErrorString(e));
     dim3 grid((a->T + BQ - 1) / BQ, a->H);
     kern<<<grid, ATT_THREADS, smem, st>>>(*a);
     return cuda_check("attn_chunk_kernel");
@@ -1794,12 +1788,9 @@ static int launch_decode_r(const CcSeqAttn* a, cudaStream_t st) {
     const size_t red = (RMAX * vecw <= 64 && a->Dv % vecw == 0 && a->Dv / vecw <= DEC_THREADS) ? (size_t)(DEC_THREADS / (a->Dv / vecw)) * R * a->Dv : 0;
     const size_t smem = sizeof(float) * ((size_t)R * ((a->Dk + 7) & ~7) + (size_t)R * KS + red) + sizeof(int) * KS;
     auto kern = attn_decode_kernel<CT, YT, RMAX>;
-    static size_t configured = 48 * 1024;
-    if (smem > configured) {
-        configured = smem;
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return fail(CC_SEQ_ERR_CUDA, cudaGetErrorString(e));
-    }
+    static SmemLimit limit;
+    const cudaError_t e = limit.allow(kern, smem);
+    if (e != cudaSuccess) return fail(CC_SEQ_ERR_CUDA, cudaGetErrorString(e));
     dim3 grid(decode_max_splits(a->L, attn_reach(*a)), a->G);
     kern<<<grid, DEC_THREADS, smem, st>>>(*a);
     return cuda_check("attn_decode_kernel");
@@ -1834,7 +1825,8 @@ static int launch_decode_rows(const CcSeqAttn* a, cudaStream_t st) {
     if constexpr (sizeof(CT) == 4) {
         if (VT == 64) kern = attn_decode_rows_kernel<CT, YT, RMAX, 64>;
     }
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    static SmemLimit limits[2];
+    const cudaError_t e = limits[VT == 64].allow(kern, smem);
     if (e != cudaSuccess) return fail(CC_SEQ_ERR_CUDA, cudaGetErrorString(e));
     launch_under(kern, dim3(NS, a->G), dim3(VD_THREADS), smem, st, *a, buffers, NS);
     return cuda_check("attn_decode_rows_kernel");
@@ -1878,7 +1870,8 @@ static int launch_decode_mma(const CcSeqAttn* a, cudaStream_t st) {
     const int NS = vd_splits(tiles, a->G, per_sm), buffers = tiles > NS && bytes(2) <= (per_sm == 2 ? half : all) ? 2 : 1;
     const size_t smem = bytes(buffers);
     auto kern = boxes ? attn_decode_mma_kernel<YT, true> : attn_decode_mma_kernel<YT, false>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    static SmemLimit limits[2];
+    const cudaError_t e = limits[boxes].allow(kern, smem);
     if (e != cudaSuccess) return fail(CC_SEQ_ERR_CUDA, cudaGetErrorString(e));
     launch_under(kern, dim3(NS, a->G), dim3(MD_THREADS), smem, st, *a, buffers, NS, k_map, v_map);
     return cuda_check("attn_decode_mma_kernel");

@@ -19,6 +19,7 @@
 #include <stdint.h>
 
 #include "../../../include/cc_b200_seq.h"
+#include "../smem_limit.cuh"
 
 namespace ccs {
 int fail(int code, const char* msg);
@@ -484,10 +485,8 @@ static uint64_t workspace_floats(const Segments& g, int T, int H, int D) {
 template <int Dp, bool VEC>
 static int launch_scan(const CcSeqWkv* a, const Segments& g, cudaStream_t st) {
     const size_t smem = 2 * sizeof(float) * (3 * TB * Dp + TB * TILE);
-    if (smem > 48 * 1024) {
-        const cudaError_t e = cudaFuncSetAttribute(wkv_segment_scan_kernel<Dp, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return cuda_check("wkv_segments: shared memory");
-    }
+    static SmemLimit limit;
+    if (limit.allow(wkv_segment_scan_kernel<Dp, VEC>, smem) != cudaSuccess) return cuda_check("wkv_segments: shared memory");
     wkv_segment_scan_kernel<Dp, VEC><<<dim3(g.n, a->H, (a->D + TILE - 1) / TILE), Dp, smem, st>>>(*a, g);
     return cuda_check("wkv_segment_scan_kernel");
 }
