@@ -64,3 +64,12 @@ def test_launchers_ask_for_it_so():
         assert f.name in own or "cudaFuncAttributeMaxDynamicSharedMemorySize" not in text, f.name
         assert not re.search(r"static (bool|size_t) configured", text), f.name
     assert "raised[i].dev == dev" in (CSRC / "gemv.cu").read_text()
+
+
+def test_what_is_looked_up_once_is_there_for_every_thread():
+    """A flag that says 'looked up' before the result is stored let a second thread go on without it."""
+    for f in (CSRC / "prefill_attn.cu", CSRC / "seq" / "tensor_map.cuh"):
+        text = f.read_text()
+        body = text[text.index("EncodeTiledFn encode_fn() {"):]
+        body = body[:body.index("\n}\n")]
+        assert re.findall(r"\bstatic\b.*", body) and all(x.startswith("static const EncodeTiledFn fn = [] {") for x in re.findall(r"\bstatic\b.*", body)), f.name
