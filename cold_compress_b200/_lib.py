@@ -14,7 +14,7 @@ import os
 
 SO_PATH = Path(os.environ.get("CC_B200_LIB", PKG / "libcc_b200.so"))  # override: another build of the library
 
-ABI_VERSION = 1
+ABI_VERSION = 2
 CC_OK = 0
 POLICY_EXTERNAL, POLICY_RECENT_GLOBAL, POLICY_L2, POLICY_HEAVY_HITTER, POLICY_HYBRID = range(5)
 ATTN_MATH_FP32, ATTN_NAIVE_BF16 = 0, 1

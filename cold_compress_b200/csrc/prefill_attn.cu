@@ -922,6 +922,7 @@ int prefill_attention_impl(const CcPrefillAttnArgs* a, cudaStream_t stream) {
         return set_error(CC_ERR_INVALID_ARG, "cc_prefill_attention: at most 4 band windows");
     if (a->attn_mode != CC_ATTN_NAIVE_BF16 && a->attn_mode != CC_ATTN_MATH_FP32)
         return set_error(CC_ERR_INVALID_ARG, "cc_prefill_attention: bad attn_mode");
+    if (a->stats_bf16 != 0 && a->stats_bf16 != 1) return set_error(CC_ERR_INVALID_ARG, "cc_prefill_attention: stats_bf16 is 0 or 1");
     const long long strides[] = {a->q_stride_s, a->q_stride_h, a->k_stride_s, a->k_stride_h, a->v_stride_s,
                                  a->v_stride_h, a->y_stride_s, a->y_stride_h};
     for (long long s : strides)

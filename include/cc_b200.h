@@ -24,7 +24,7 @@
 extern "C" {
 #endif
 
-#define CC_ABI_VERSION 1
+#define CC_ABI_VERSION 2
 
 /* ---- error codes ------------------------------------------------------- */
 #define CC_OK                     0
@@ -222,10 +222,12 @@ int cc_requantize_cache(void* k_cache, void* v_cache, int32_t n_kv_heads, int32_
  *   the sliding-window masses of KVCacheHybrid.build_masks                 cache.py:1066-1173
  * q [Hkv*G, S, D], k / v [Hkv, S, D], y [Hkv*G, S, D]: bf16, D contiguous, row / head strides in ELEMENTS
  * (multiples of 8), so the [S, H, D] layout the projections produce is taken as is.
- * Outputs (fp32, the caller applies the reference's final bf16 roundings):
+ * Outputs:
  *   col_sum [Hkv, S]            sum over query rows i of pooled[h, i, j]        (NULL: attention only)
  *   obs_sum [Hkv, S]            the same over the last obs_len query rows       (NULL or obs_len 0: skipped)
- *   band_sum [n_windows, Hkv, S] sum over rows i with i - j < windows[w]        (n_windows 0: skipped)
+ *   band_sum [n_windows, Hkv, S] sum over rows i with i - j < windows[w], fp32; none for windows[w] <= 0   (n_windows 0: skipped)
+ * stats_bf16 0: col_sum and obs_sum are fp32 sums, and the reference's final bf16 roundings are the caller's.  1: both are bf16 with those
+ * roundings, col_sum that of the sum and obs_sum that of the mean over the observed rows (min(obs_len, S)).  Any other value is an error.
  * where pooled[h, i, j] = bf16(mean over the G query heads of bf16 softmax probabilities).
  * attn_mode CC_ATTN_NAIVE_BF16 keeps the reference's naive-path roundings (bf16 after q.k, after *scale,
  * after softmax); CC_ATTN_MATH_FP32 keeps fp32 logits (F.scaled_dot_product_attention semantics).
@@ -241,7 +243,7 @@ typedef struct CcPrefillAttnArgs {
     int32_t obs_len;         /* SnapKV observation window (prompt_compression.py:157) */
     int32_t n_windows;       /* 0..4                                        */
     int32_t windows[4];      /* window sizes in tokens                      */
-    int32_t stats_bf16;      /* 0: col_sum, obs_sum fp32.  1: bf16, col_sum rounded and obs_sum the mean over the observed rows */
+    int32_t stats_bf16;      /* 0 or 1, see above; since ABI version 2          */
     void*   col_sum;
     void*   obs_sum;
     float*  band_sum;

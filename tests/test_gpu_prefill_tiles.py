@@ -76,3 +76,19 @@ def test_windows_of_no_token_and_of_every_token(G, D, S):
     for w in (0, -3, -top - 1):
         assert not st.band_sum[w].any(), f"band {w}"
     assert torch.equal(st.band_sum[top].to(torch.bfloat16), st.col_sum[0])
+
+
+@pytest.mark.parametrize("S,obs_len", [(7, 16), (15, 16), (40, 1), (40, 3), (391, 7), (391, 16), (391, 100)])
+def test_sums_in_bf16_are_the_rounded_sums(S, obs_len):
+    """Bit for bit what tensor operations make of the fp32 sums, for means over any number of rows."""
+    from cold_compress_b200 import _lib, ops
+    q, k, v = (t[0].cuda() for t in _inputs(4, 64, S))
+    n = min(obs_len, S)
+    ws = torch.empty(ops.prefill_attention_workspace(S, 2, 4, n, 0), dtype=torch.uint8, device="cuda")
+    got = []
+    for dtype in (torch.float32, torch.bfloat16):
+        col, obs = (torch.full((2, S), 7.0, dtype=dtype, device="cuda") for _ in range(2))
+        ops.prefill_attention(q, k, v, torch.empty_like(q), _lib.ATTN_NAIVE_BF16, n, [], col, obs, None, ws)
+        got.append((col, obs))
+    (col, obs), (col16, obs16) = got
+    assert torch.equal(col16, col.bfloat16()) and torch.equal(obs16, (obs / n).bfloat16())
