@@ -42,18 +42,6 @@ def scaled_dot_product_attention(query, key, value, attn_mask=None, dropout_p=0.
     return p @ value, p
 
 
-_workspace: dict = {}
-
-
-def _scratch(device, nbytes: int) -> torch.Tensor:
-    """Per-device scratch for the partial column sums (grown on demand, reused across layers)."""
-    buf = _workspace.get(device)
-    if buf is None or buf.numel() < nbytes:
-        buf = torch.empty(nbytes, dtype=torch.uint8, device=device)
-        _workspace[device] = buf
-    return buf
-
-
 @torch.no_grad()
 def prefill_attention(q, k, v, attn_mode: int = _lib.ATTN_MATH_FP32):
     """Causal GQA attention over a prompt on the tensor cores, no statistics (caches that keep no scores).
@@ -84,7 +72,8 @@ def prefill_attention_stats(q, k, v, obs_len: int = 16, windows=()):
     col = torch.empty(1, Hkv, S, dtype=q.dtype, device=dev)
     obs = torch.empty(1, Hkv, S, dtype=q.dtype, device=dev)
     band = torch.empty(len(windows), Hkv, S, dtype=torch.float32, device=dev) if windows else None
-    ws = _scratch(dev, ops.prefill_attention_workspace(S, Hkv, G, obs_len, len(windows)))
+    # of this call alone: calls on other streams or from other threads have sums of their own under way
+    ws = torch.empty(ops.prefill_attention_workspace(S, Hkv, G, obs_len, len(windows)), dtype=torch.uint8, device=dev)
     ops.prefill_attention(q[0], k[0], v[0], y.permute(1, 0, 2), _lib.ATTN_NAIVE_BF16, obs_len, windows, col, obs, band, ws)
     stats = PrefillAttnStats(col_sum=col, obs_mean=obs, obs_len=obs_len,
                              band_sum={w: band[i] for i, w in enumerate(windows)} if windows else None)
