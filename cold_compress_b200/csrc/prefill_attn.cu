@@ -20,6 +20,8 @@
 // GQA mean; MATH: fp32 logits, one rounding of P for the tensor core).
 // K and V are staged by TMA (cp.async.bulk.tensor, 128-byte swizzle) through a ring of tiles; the logits of the next tiles are formed
 // under the current tile's softmax.
+// A row with a logit that is NaN or +inf is NaN in y, and in the pooled map as far as its block of queries reaches (the reference's map
+// carries it on to every later key; those tiles are not visited).  What a query does not see takes no part in its row.
 // Per-tile partial column sums go to a scratch buffer and are added in a fixed order by a second small
 // kernel: results are bit-reproducible run to run (no floating-point atomics).
 #include <cuda.h>
@@ -632,12 +634,15 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         // ---- sweep 2: probabilities of rows 8 j + lane / 4 of the quarter, keys 8 k + 2 (lane % 4), + 1 of the warp's 32
         const int r8 = lane >> 2, c2 = 2 * (lane & 3);
         f32x2 off[4], inv[4];
+        bool no_number = false;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const float* const f = sm.fin[quarter * 32 + 8 * j + r8];
             off[j] = pair(f[0], f[0]);
             inv[j] = pair(f[1], f[1]);
+            no_number |= f[1] != f[1];
         }
+        no_number = __any_sync(0xffffffffu, no_number);            // a row that is NaN is so for the keys that it does not see, too
         const float fG = (float)p.G, invG = 1.0f / (float)p.G;
         const bool g_pow2 = (p.G & (p.G - 1)) == 0, short_heads = p.G * QQ < 32;
         const f32x2 invG2 = pair(invG, invG);
@@ -665,7 +670,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
             };
             if (kbase + 31 <= q0) {
                 weigh(std::false_type());
-            } else if (kbase < q0 + QQ) {
+            } else if (kbase < q0 + QQ || no_number) {
                 weigh(std::true_type());
             } else {
 #pragma unroll

@@ -92,3 +92,30 @@ def test_sums_in_bf16_are_the_rounded_sums(S, obs_len):
         got.append((col, obs))
     (col, obs), (col16, obs16) = got
     assert torch.equal(col16, col.bfloat16()) and torch.equal(obs16, (obs / n).bfloat16())
+
+
+@pytest.mark.parametrize("G,QB,D", [(1, 128, 64), (2, 64, 128), (4, 32, 128), (7, 16, 64)])
+@pytest.mark.parametrize("value", [float("nan"), float("inf")])
+@pytest.mark.parametrize("row", [0, 37, 130])
+def test_rows_that_are_no_numbers(G, QB, D, value, row):
+    """A query whose logits are NaN or +inf: its row of y, and the sums over every key before the end of its block of queries."""
+    from cold_compress_b200.attention_utils import prefill_attention_stats
+    from oracle.prefill import full_map, reductions
+    S, windows = 200, (150, 300)
+    q, k, v = _inputs(G, D, S)
+    k[..., 0] = k[..., 0].abs() + 1                  # +inf times these: no key's logit is -inf
+    q[0, 0, row, 0] = value
+    y, st = prefill_attention_stats(q.cuda(), k.cuda(), v.cuda(), obs_len=100, windows=windows)
+    _, pooled = full_map(q, k, v)
+    assert y[0, 0, row].isnan().all() and int(y.isnan().sum()) == D      # (the restatement's product on the CPU takes it on to a neighbour)
+    end = min(S, (row // QB + 1) * QB)
+    assert pooled[0, 0, row].isnan().all() and int(pooled.isnan().sum()) == S
+    pooled[0, 0, row, end:] = 0                      # not visited
+    ref = reductions(pooled, 100, windows)
+    for got, want, what in ((st.col_sum[0].cpu(), ref.col_sum[0], "col_sum"), (st.obs_mean[0].cpu(), ref.obs_mean[0], "obs_mean")):
+        assert torch.equal(got.isnan(), want.isnan()), what
+        assert_close_bf16(got.nan_to_num(), want.nan_to_num(), what, max_ulp=1.0, min_equal=0.85, floor=2.0 ** -14)
+    for w in windows:
+        inside = (row - torch.arange(S)) < w         # the kernel leaves out what lies outside, the restatement multiplies it by zero
+        assert torch.equal(st.band_sum[w][0].cpu().isnan(), (torch.arange(S) < end) & inside)
+        assert not st.band_sum[w][1:].isnan().any()
