@@ -459,8 +459,9 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
             }
             __syncwarp();
         } else if (p.stats) {
-            // Sums over the queries, straight to this block's partials.  A warp has 64 keys, a lane 8 of them in every fourth
-            // row: chunk c holds keys 32 (c / 4) + 8 k + 2 (c % 4) + e as pair k.
+            // Sums over the queries, straight to this block's partials; sums of their own for a band only in tiles that its edge crosses
+            // (2047 tokens, two windows, us with sums of their own in every tile / so: 8 heads of 128 without groups 103 / 68, 32 / 8 107 / 90).
+            // A warp has 64 keys, a lane 8 of them in every fourth row: chunk c holds keys 32 (c / 4) + 8 k + 2 (c % 4) + e as pair k.
             const int c = 8 * (warp - SOFT_WARPS - 2) + (lane & 7), first = lane >> 3, rows = min(QB, p.S - i0);
             const bool high = lane & 16, odd = lane & 8, obs = qt >= p.first_obs_tile;
             const int key = 32 * (c >> 2) + 8 * ((high ? 2 : 0) + (odd ? 1 : 0)) + 2 * (c & 3);   // of the pair that this lane stores
@@ -495,10 +496,17 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
                     unpair(b, f.x, f.y);
                     if (*failed) f = make_float2(NAN, NAN);
                     *reinterpret_cast<float2*>(out + t * BN) = f;
+                    return f;
                 };
-                add(std::false_type(), 0, 0, col);
+                const float2 all = add(std::false_type(), 0, 0, col);
                 if (obs) add(std::false_type(), p.obs_start - i0, 0, seen);
-                for (int w = 0; w < p.n_windows; ++w) add(std::true_type(), 0, p.windows[w], band + (size_t)w * p.Hkv * p.n_qtiles * p.S_pad);
+                for (int w = 0; w < p.n_windows; ++w) {
+                    const int window = p.windows[w], from = i0 - t * BN;                 // of the first row, from the tile's first key
+                    float* const out = band + (size_t)w * p.Hkv * p.n_qtiles * p.S_pad;
+                    if (from - (BN - 1) >= window) continue;                             // no row has a key of the tile inside: never read
+                    if (from + rows - 1 < window) *reinterpret_cast<float2*>(out + t * BN) = all;   // every row has every key inside
+                    else add(std::true_type(), 0, window, out);
+                }
                 __syncwarp();
                 if (lane == 0) mbar_arrive_u32(C_READ(t & 1));
             }

@@ -119,3 +119,17 @@ def test_rows_that_are_no_numbers(G, QB, D, value, row):
         inside = (row - torch.arange(S)) < w         # the kernel leaves out what lies outside, the restatement multiplies it by zero
         assert torch.equal(st.band_sum[w][0].cpu().isnan(), (torch.arange(S) < end) & inside)
         assert not st.band_sum[w][1:].isnan().any()
+
+
+@pytest.mark.parametrize("G,D", [(1, 64), (3, 128), (8, 64)])
+@pytest.mark.parametrize("S", [391, 512])
+def test_bands_whose_edges_lie_anywhere_in_a_tile(G, D, S):
+    """Tiles of keys inside a window, outside of it and crossed by its edge, around the sizes of tiles and of blocks of queries."""
+    from cold_compress_b200.attention_utils import prefill_attention_stats
+    from oracle.prefill import full_map, reductions
+    q, k, v = _inputs(G, D, S)
+    ref = reductions(full_map(q, k, v)[1], 16, every := (1, 2, 16, 31, 32, 33, 63, 64, 96, 127, 128, 129, 160, 255, 256, 257, 300, S - 1, S, S + 1))
+    for i in range(0, len(every), 4):
+        _, st = prefill_attention_stats(q.cuda(), k.cuda(), v.cuda(), obs_len=16, windows=every[i:i + 4])
+        for w in every[i:i + 4]:
+            assert torch.allclose(st.band_sum[w].cpu(), ref.band_sum[w], rtol=1e-2, atol=2e-3), f"band {w}"
