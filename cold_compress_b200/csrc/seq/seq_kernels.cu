@@ -1536,12 +1536,11 @@ __global__ void cache_append_kernel(const CcSeqAttn a, int t_first) {
 }
 
 // The same for rows of whole 16-byte vectors, launched under the attention before it: thread = vector x of the key row and then of the
-// value row, of APPEND_ROWS (token, head) rows that lie blockDim.y apart and are under way together; positions and marks by a thread
-// per token, so that neighbouring tokens are stored together and a CTA counts its new slots with one addition.
-// Bound: HBM and the launch.  Measured in a chain of launches: 1001 tokens of 4 heads of 128 + 128 bf16 3.6 us, 4096 of 8 5.4; a row per
-// thread, with the row's first thread storing its marks, 10.3 and 22.9 (2.3 and 5.3 without positions and marks).
-constexpr int APPEND_ROWS = 4;
-template <typename CT>
+// value row, of ROWS (token, head) rows that lie blockDim.y apart and are under way together; positions and marks by a thread
+// per mark, neighbouring tokens in neighbouring threads, new slots counted by the warp.
+// Bound: HBM and the launch.  Measured in a chain of launches, with a row per thread whose first thread stores its marks / so, us: 2 tokens of 8
+// heads of 128 + 128 bf16 1.65 / 1.65, 64 4.9 / 1.65, 1001 12.7 / 3.3, 4096 of one head 16 / 3.1, of 8 19.5 / 5.75.
+template <typename CT, int ROWS>
 __global__ void __launch_bounds__(256) cache_append_rows_kernel(const CcSeqAttn a, int t_first) {
     pdl_wait_release();
     constexpr int VEC = 16 / (int)sizeof(CT);
@@ -1551,11 +1550,11 @@ __global__ void __launch_bounds__(256) cache_append_rows_kernel(const CcSeqAttn 
     auto kept = [&](int p) { return p < a.keep_first || p + (a.L - a.keep_first) > p0 + a.T - 1; };      // no later row takes its slot
     const CT* const src = (key ? (const CT*)a.k_new : (const CT*)a.v_new) + e;
     CT* const dst = (key ? (CT*)a.k_cache : (CT*)a.v_cache) + e;
-    uint4 x[APPEND_ROWS];
-    long long to[APPEND_ROWS];
+    uint4 x[ROWS];
+    long long to[ROWS];
 #pragma unroll
-    for (int i = 0; i < APPEND_ROWS; ++i) {
-        const unsigned row = (blockIdx.x * APPEND_ROWS + i) * blockDim.y + threadIdx.y, n = row / (unsigned)a.G;
+    for (int i = 0; i < ROWS; ++i) {
+        const unsigned row = (blockIdx.x * ROWS + i) * blockDim.y + threadIdx.y, n = row / (unsigned)a.G;
         const int t = t_first + (int)n, g = (int)(row - n * (unsigned)a.G);
         to[i] = -1;
         if (t < a.T && kept(p0 + t)) {
@@ -1564,21 +1563,23 @@ __global__ void __launch_bounds__(256) cache_append_rows_kernel(const CcSeqAttn 
         }
     }
 #pragma unroll
-    for (int i = 0; i < APPEND_ROWS; ++i)
+    for (int i = 0; i < ROWS; ++i)
         if (to[i] >= 0) *reinterpret_cast<uint4*>(dst + to[i]) = x[i];
-    const int threads = blockDim.x * blockDim.y, tid = threadIdx.y * blockDim.x + c;
-    for (long long first = t_first + (long long)blockIdx.x * threads; first < a.T; first += (long long)gridDim.x * threads) {   // the CTA as one
-        const long long t = first + tid;
+    const unsigned threads = blockDim.x * blockDim.y, tid = threadIdx.y * blockDim.x + c, tokens = a.T - t_first, marks = tokens * (unsigned)a.G;
+    for (unsigned long long first = (unsigned long long)blockIdx.x * threads; first < marks; first += (unsigned long long)gridDim.x * threads) {
+        const unsigned i = (unsigned)first + tid, g = i / tokens;
+        const int t = t_first + (int)(i - g * tokens), p = p0 + t;
         bool fresh = false;
-        if (t < a.T && kept(p0 + (int)t)) {
-            const int p = p0 + (int)t, slot = slot_of(a, p);
-            fresh = a.pos[slot] < 0;
-            a.pos[slot] = p;
-            if (a.mask != nullptr)
-                for (int g = 0; g < a.G; ++g) a.mask[(size_t)g * a.L + slot] = 1;
+        if (i < marks && kept(p)) {
+            const int slot = slot_of(a, p);
+            if (a.mask != nullptr) a.mask[(size_t)g * a.L + slot] = 1;
+            if (g == 0) {
+                fresh = a.pos[slot] < 0;
+                a.pos[slot] = p;
+            }
         }
-        const int news = __syncthreads_count(fresh);
-        if (tid == 0 && news > 0 && a.cache_cts != nullptr) atomicAdd(a.cache_cts, news);
+        const unsigned here = __activemask(), some = __ballot_sync(here, fresh);
+        if (some != 0 && (tid & 31) == __ffs(here) - 1 && a.cache_cts != nullptr) atomicAdd(a.cache_cts, __popc(some));
     }
 }
 
@@ -1987,9 +1988,14 @@ int cc_seq_cache_append(const CcSeqAttn* a, void* stream) {
     const long long rows = (long long)(a->T - t_first) * a->G;
     if ((a->cache_dtype == CC_DT_F32 || a->cache_dtype == CC_DT_BF16) && vecs > 0 && vecs <= 256 && (all & 15) == 0 && a->G > 0 && rows < (1ll << 30)) {
         const dim3 block(vecs, 256 / vecs);
-        const unsigned per_cta = APPEND_ROWS * block.y, ctas = (unsigned)((rows + per_cta - 1) / per_cta);
-        if (size == 2) launch_under(cache_append_rows_kernel<__nv_bfloat16>, dim3(ctas), block, 0, st, *a, t_first);
-        else launch_under(cache_append_rows_kernel<float>, dim3(ctas), block, 0, st, *a, t_first);
+        auto launch = [&](auto kern, unsigned rows_each) {
+            launch_under(kern, dim3((unsigned)((rows + rows_each * block.y - 1) / (rows_each * block.y))), block, 0, st, *a, t_first);
+        };
+        // A row per thread until that takes 24 CTAs an SM, four from there on.  One / four, us: 8 heads of 128 at 1001 tokens (6.8 CTAs an SM) 3.3
+        // / 4.1, at 3000 (20) 4.85 / 5.65, at 4096 (28) 5.95 / 5.75; 64 heads of 64 at 256 (7) 3.2 / 3.6, at 1001 (27) 5.95 / 5.75, at 4096 25.8 / 22.
+        const bool one = rows <= (long long)block.y * 148 * 24;
+        if (size == 2) one ? launch(cache_append_rows_kernel<__nv_bfloat16, 1>, 1) : launch(cache_append_rows_kernel<__nv_bfloat16, 4>, 4);
+        else one ? launch(cache_append_rows_kernel<float, 1>, 1) : launch(cache_append_rows_kernel<float, 4>, 4);
         return cuda_check("cache_append_rows_kernel");
     }
     dim3 grid(a->T - t_first, a->G);

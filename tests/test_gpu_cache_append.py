@@ -32,3 +32,9 @@ def test_append_stores_what_the_rule_says(T, G, Dk, Dv, L, keep, p0, dtype):
                           ring if keep else 0, 0, 1.0, seq_ops.ATTN_APPEND_ONLY, None, 0, keep)
     for a, b, what in zip(got, (kc, vc, pos, mask, cts), ("keys", "values", "positions", "marks", "count")):
         assert torch.equal(a.cpu(), b), what
+
+
+@pytest.mark.parametrize("T,G,Dk,Dv,L,keep,p0", [(4201, 17, 64, 64, 4400, 0, 11), (4201, 17, 64, 64, 3000, 5, 2), (2, 64, 64, 64, 70, 4, 3), (1, 300, 8, 16, 9, 0, 0)])
+def test_many_rows_and_few_tokens_of_many_heads(T, G, Dk, Dv, L, keep, p0):
+    """Above the line from which a thread stores four rows, and marks that are many more than tokens."""
+    test_append_stores_what_the_rule_says(T, G, Dk, Dv, L, keep, p0, torch.bfloat16)
