@@ -451,17 +451,20 @@ __global__ void __launch_bounds__(Dp) wkv_segment_scan_kernel(const CcSeqWkv a, 
     if (__syncthreads_or(none != none)) wkv_segment_again<Dp>(a, g, sm);
 }
 
-// Segments: as many as give an SM six CTAs (what the scan's registers allow) over heads and column tiles, of at least 32 tokens; eight
-// CTAs, so that a second wave of short ones evens out the first, from 2^17 tokens of a tile's columns on.  Six / eight, back to back in a
-// graph, us: 4096 tokens of 32 heads of 64 152 / 144, of 64 294 / 280, of 128 614 / 532, of 64 heads of 128 1214 / 1040, 1024 of 128 heads
-// of 64 169 / 153, 2048 of 64 157 / 154; below that line 3000 of 32 115 / 119, 4096 of 16 83 / 85, of 8 53 / 55, 1024 of 64 84 / 85 and up to
-// 700 tokens no difference (64 heads of 64 at 1500 122 / 118, 9 of 72 at 4096 165 / 158).  Nine and twelve are slower than eight.
+// Segments: as many as give an SM six CTAs (what the scan's registers allow) over heads and column tiles, of at least 32 tokens.  Eight, so that
+// a second wave evens out the first, while segments keep 100 tokens: each has a start of its own (a state to load, a batch to wait for),
+// which shorter ones repeat more often than an even end is worth.  Time with six over time with eight, back to back in a graph, by the length
+// that eight leave: up to 90 tokens 0.92 to 1.13, and as often below one as above (3000 tokens of 32 heads of 64 0.97, 512 of 40 of 100 0.92); at 92 to
+// 99 0.98 to 1.06; at 100 1.00 to 1.12; at 110 (4096 of 32 of 64) 1.06, at 120 1.005 to 1.14, at 220 1.01 to 1.15 (9 to 128 heads of 16 to 128).
+// Where six give a single segment or two and eight one more, 1.15 to 1.8 (256 to 1024 tokens of 460 to 592 heads of 64, 222 to 296 of 100 to
+// 128).  Nine and twelve are slower than eight, and seven than six for most numbers of heads.
 // The three launches follow one another in full: started under each other (programmatic launch) 256 tokens of 16 heads take 32 us
 // instead of 20.
-constexpr int MIN_LEN = 32;
+constexpr int MIN_LEN = 32, LONG_LEN = 100;
 static Segments plan(int T, int H, int D) {
     const long long per = (long long)H * ((D + TILE - 1) / TILE);
-    long long most = (T * per >= 1 << 17 ? 8 : 6) * 148 / per;
+    long long most = 8 * 148 / per;
+    if (T < LONG_LEN * most) most = 6 * 148 / per;
     if (most < 1) most = 1;
     int len = (int)((T + most - 1) / most);
     if (len < MIN_LEN) len = MIN_LEN;

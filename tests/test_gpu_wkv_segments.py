@@ -42,6 +42,12 @@ def test_segments_against_the_recurrence(T, H, D, w0, monkeypatch):
     assert all(a <= 1.25 * b + 2.0 ** -26 for a, b in zip(cut, plain))      # and no further off than token after token
 
 
+@pytest.mark.parametrize("T, H, D", [(1100, 128, 64), (901, 128, 60), (420, 128, 128), (259, 500, 64), (384, 230, 100)])
+def test_eight_segments_an_sm_against_the_recurrence(T, H, D, monkeypatch):
+    """Long enough for the second cut, among them heads that six segments an SM would leave uncut."""
+    test_segments_against_the_recurrence(T, H, D, -2.0, monkeypatch)
+
+
 def test_what_is_not_served_goes_token_after_token():
     from cold_compress_b200 import _lib, seq_ops
     lib = _lib.load_seq()

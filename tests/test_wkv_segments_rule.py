@@ -18,3 +18,23 @@ def test_shapes_that_are_slower_in_segments_go_token_after_token(T, H, D):
 def test_shapes_that_are_faster_in_segments_go_in_segments(T, H, D):
     from cold_compress_b200 import _lib
     assert _lib.load_seq().cc_seq_wkv_segments_workspace(T, H, D) > 0
+
+
+def _segments(T, H, D):
+    """How many, from the floats that each takes in the workspace."""
+    from cold_compress_b200 import _lib
+    floats = _lib.load_seq().cc_seq_wkv_segments_workspace(T, H, D) // 4 - (T * H * D + 3) // 4 * 4
+    assert floats % (H * D * (D + 1)) == 0
+    return floats // (H * D * (D + 1))
+
+
+@pytest.mark.parametrize("T,H,D,n", [(3699, 32, 64, 27), (3700, 32, 64, 37), (4096, 32, 64, 37), (899, 128, 64, 6), (900, 128, 64, 9), (7299, 16, 64, 55), (7400, 16, 64, 74),
+                                     (399, 128, 128, 3), (400, 128, 128, 4), (1399, 40, 100, 11), (1400, 40, 100, 14), (256, 460, 64, 2), (256, 592, 64, 2), (256, 290, 128, 2)])
+def test_eight_segments_an_sm_while_they_keep_a_hundred_tokens_and_six_otherwise(T, H, D, n):
+    assert _segments(T, H, D) == n
+
+
+@pytest.mark.parametrize("T,H,D", [(4096, 593, 64), (4096, 297, 128), (256, 290, 100), (300, 290, 104)])
+def test_more_heads_than_leave_two_segments_go_token_after_token(T, H, D):
+    from cold_compress_b200 import _lib
+    assert _lib.load_seq().cc_seq_wkv_segments_workspace(T, H, D) == 0
