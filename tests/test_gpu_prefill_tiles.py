@@ -15,7 +15,7 @@ def _inputs(G, D, S, kv=2):
     return q, k, torch.randn(1, kv, S, D, generator=gen).bfloat16()
 
 
-def _check(q, k, v, what, strict=0.99):
+def _check(q, k, v, what):
     from cold_compress_b200.attention_utils import prefill_attention_stats
     from oracle.prefill import full_map, reductions
     S, D = q.shape[2], q.shape[3]
@@ -23,9 +23,9 @@ def _check(q, k, v, what, strict=0.99):
     y, st = prefill_attention_stats(q.cuda(), k.cuda(), v.cuda(), obs_len=16, windows=windows)
     y_ref, pooled = full_map(q, k, v)
     ref = reductions(pooled, 16, windows)
-    check_prefill_y(y[0].reshape(-1, D), y_ref[0].reshape(-1, D), what, strict_frac=strict)
-    assert_close_bf16(st.col_sum[0], ref.col_sum[0], f"{what} col_sum", max_ulp=1.0, min_equal=0.85, floor=2.0 ** -14)
-    assert_close_bf16(st.obs_mean[0], ref.obs_mean[0], f"{what} obs_mean", max_ulp=1.0, min_equal=0.85, floor=2.0 ** -14)
+    check_prefill_y(y[0].reshape(-1, D), y_ref[0].reshape(-1, D), what)
+    assert_close_bf16(st.col_sum[0], ref.col_sum[0], f"{what} col_sum", max_ulp=1.0, min_equal=0.90, floor=2.0 ** -14)
+    assert_close_bf16(st.obs_mean[0], ref.obs_mean[0], f"{what} obs_mean", max_ulp=1.0, min_equal=0.90, floor=2.0 ** -14)
     for w in windows:
         assert torch.allclose(st.band_sum[w].cpu(), ref.band_sum[w], rtol=1e-2, atol=2e-3), f"{what} band {w}"
 
@@ -114,7 +114,7 @@ def test_rows_that_are_no_numbers(G, QB, D, value, row):
     ref = reductions(pooled, 100, windows)
     for got, want, what in ((st.col_sum[0].cpu(), ref.col_sum[0], "col_sum"), (st.obs_mean[0].cpu(), ref.obs_mean[0], "obs_mean")):
         assert torch.equal(got.isnan(), want.isnan()), what
-        assert_close_bf16(got.nan_to_num(), want.nan_to_num(), what, max_ulp=1.0, min_equal=0.85, floor=2.0 ** -14)
+        assert_close_bf16(got.nan_to_num(), want.nan_to_num(), what, max_ulp=1.0, min_equal=0.90, floor=2.0 ** -14)
     for w in windows:
         inside = (row - torch.arange(S)) < w         # the kernel leaves out what lies outside, the restatement multiplies it by zero
         assert torch.equal(st.band_sum[w][0].cpu().isnan(), (torch.arange(S) < end) & inside)
