@@ -10,7 +10,7 @@
 // Bound: tensor pipe and the shared memory it reads: 2 x 24 MMAs of 128 x 128 x 16 per 128 x 128 scores at head size 128,
 // 107 cycles each with both operands in shared memory (scores) and 74 with the weights in tensor memory (values) by stamps of the
 // SM's clock, where the pipe itself needs 64 (ncu: tensor pipe 49 % active, issue slots 38 %); together 4350 of the
-// 5000 cycles that a tile takes; the other pipes need ~10 instructions per score beside them.  Layout that
+// 4400 to 5000 cycles that a tile takes (long prompts / short ones); the other pipes need ~10 instructions per score beside them.  Layout that
 // follows: the query parts stay in shared memory (96 KB) and the weight parts go to tensor memory, over the scores they came
 // from, as the A operand.  Sixteen warps of softmax, four threads per row.
 //

@@ -12,9 +12,10 @@
 // belong to, so the unit is applied on the way out of tensor memory, four warps emptying one accumulator while the next tile
 // fills the other; fp32 results go by way of shared memory, so that rows are stored as whole lines (the unit's bf16 results that way:
 // 10 us slower at 400 to 512 tokens).  Bound: the 64 bytes per clock that an SM takes from L2; a 128 x 256 x 64 stage is 48 KB (768 cycles) for
-// 512 cycles of MMAs.  The whole mixture with a shared expert of 2048 in a graph, over seconds: results 16 bytes of a row at a time and
-// MMAs issued by one thread 247 us, this 240; 4096 tokens 430 / 416; experts of 1000 216 / 207; 1024 tokens 152 / 146.  Pairs of CTAs
-// (cta_group::2) on 256 x 256 tiles, which read half of the weights each: 254, 422, 215 and 158.
+// 512 cycles of MMAs.  The whole mixture with a shared expert of 2048 in a graph, four turns of each side that agree within 1 %: results 16
+// bytes of a row at a time and MMAs issued by one thread 251 us, this 241; 4096 tokens 434 / 408; experts of 1000 221 / 208.6; 1024 tokens
+// 151 / 147.7, 300 108.4 / 105.2, 64 97.0 / 94.5.  Pairs of CTAs (cta_group::2) on 256 x 256 tiles, which read half of the weights each, beside
+// 240, 416, 207 and 146 of this form: 254 at 2048 tokens, 422 at 4096, 215 with experts of 1000 and 158 at 1024.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>

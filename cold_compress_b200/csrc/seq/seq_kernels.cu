@@ -1033,7 +1033,7 @@ __global__ void __launch_bounds__(VD_THREADS, RMAX <= 4 ? 2 : 1) attn_decode_row
 // The keys of a tile are waited for alone, its values land under the scores and the softmax.  The last CTA of a head asks for all
 // partial sums before it knows their weights, and stores the new row under them.
 // Bound: the chain of dependent waits: position, keys, scores, softmax, values, partials and their counter, combination.  8 layers of 32 / 8
-// heads of 128, 4096 positions in a graph: 143 us on the kernel above, 109 here, 107 since tiles come as boxes and slots' positions are
+// heads of 128, 4096 positions in a graph: 143 us on the kernel above, 109 here, 106 since tiles come as boxes and slots' positions are
 // compared after the query has been read.  Against 64 bits (fp32 results, scores of size 4): 2.1e-7 of the norm, 2.4e-7 above.
 constexpr int MD_THREADS = 256, MD_WARPS = MD_THREADS / 32, MD_AHEAD = 17, MD_KEYS = 128;      // MD_KEYS: keys of a tile
 

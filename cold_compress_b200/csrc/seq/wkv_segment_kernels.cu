@@ -12,7 +12,7 @@
 // Rows on other than 16-byte boundaries are staged 4 bytes at a time: the same sums, so the same bits.
 // One multiplication and addition per state element and token more than the plain recurrence, for segments times the parallelism:
 // Back to back in a graph, 4096 tokens of 32 heads of 64 go from 405 us to 144, of 4 heads from 387 to 38, of 64 heads of 128 from
-// 1663 to 1040.  Now bound by the fp32 pipe (63 % busy in 3., 42 % in 1.; 9 warps of up to 168 registers an SM).
+// 1663 to 1040.  Now bound by the fp32 pipe (69 % busy in 3., 50 % in 1.; 9 warps of up to 168 registers an SM).
 // Against 64 bits the outputs are as far off as token after token (1.31e-7 and 1.34e-7 of their norm), with other roundings.
 #include <cuda_runtime.h>
 #include <math.h>
